@@ -47,8 +47,11 @@ struct bfs_graph {
 	RunCtx rc{};
 	uint32_t batch = 1;
 	int grid = 0;
-	int grid_max = 0;  // CTAs of the cooperative grid at full occupancy (grid: as the options ask)
 	size_t smem = 0;
+	// by bottom-up variant: CTAs of the cooperative grid at full occupancy and
+	// their shared memory (grid, smem: as the options ask)
+	int grid_max[2] = {0, 0};
+	size_t smem_of[2] = {0, 0};
 	std::vector<DevBuf> bufs;
 	size_t device_bytes = 0;
 	int32_t *level_buf = nullptr;    // internal outputs for bfs_run
@@ -369,6 +372,14 @@ int upload_big_in(bfs_graph *g, const std::vector<uint32_t> &in_off) {
 	return dev_upload(g, &g->ms_chunk_beg, chunk_beg);
 }
 
+// The traversal's launch shape for the graph's options: the occupancy bound
+// found at set-up, or fewer CTAs per SM.
+void apply_grid(bfs_graph *g) {
+	const int most = g->grid_max[g->opt.bottom_up];
+	g->grid = g->opt.ctas_per_sm ? std::min(most, (int) g->opt.ctas_per_sm * g->num_sms) : most;
+	g->smem = g->smem_of[g->opt.bottom_up];
+}
+
 // Run context, events and the persistent grid.
 int alloc_run(bfs_graph *g) {
 	DevGraph &d = g->dg;
@@ -398,9 +409,10 @@ int alloc_run(bfs_graph *g) {
 			cudaEventCreate(&g->evm) != cudaSuccess)
 		return BFS_ECUDA;
 	g->batch = std::max<uint32_t>(1, std::min<uint32_t>(kMaxSliceBatch, kSliceBudgetWords / std::max<uint32_t>(1, d.slice_words)));
-	st = persistent_grid(d, g->batch, g->num_sms, &g->grid, &g->smem);
-	g->grid_max = g->grid;
-	return st;
+	for (uint32_t bu : {BFS_BU_PULL, BFS_BU_STREAM})
+		if ((st = persistent_grid(d, g->batch, bu, g->device, g->num_sms, &g->grid_max[bu], &g->smem_of[bu]))) return st;
+	apply_grid(g);
+	return BFS_OK;
 }
 
 // Builds the device copy of a validated host graph.
@@ -1855,9 +1867,7 @@ int bfs_set_options(bfs_graph *g, const bfs_options *opt) {
 		return BFS_EARG;
 	std::lock_guard<std::mutex> lk(g->mu);
 	g->opt = *opt;
-	// the cooperative grid: the occupancy bound found at set-up, or fewer CTAs per SM
-	if (!g->host_only && g->grid_max)
-		g->grid = opt->ctas_per_sm ? std::min(g->grid_max, (int) opt->ctas_per_sm * g->num_sms) : g->grid_max;
+	if (!g->host_only) apply_grid(g);
 	return BFS_OK;
 }
 

@@ -40,6 +40,9 @@ struct DevGraph {
 struct StepCounters {
 	unsigned int tail[3];       // queue bucket tails (top-down appends, to_sparse)
 	unsigned int work;          // dynamic work counter (column groups)
+	unsigned int levels;        // steps the round took (0: one, by the whole grid)
+	unsigned int pad;
+	unsigned long long solo_deg;  // out-edges of the frontiers inside a round of several steps
 };
 
 // Per-run statistics gathered on the device.

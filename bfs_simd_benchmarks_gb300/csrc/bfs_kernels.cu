@@ -182,13 +182,12 @@ __device__ __forceinline__ uint32_t block_incl_scan(uint32_t x) {
 // The frontier's queue sizes nS, nM, nL (small, medium, large out-degree)
 // come from the caller, which loads them together with the step totals.
 __device__ __forceinline__ void phase_expand(const DevGraph &g, const RunCtx &r, const StepParams &p, uint32_t step,
-		uint32_t nS, uint32_t nM, uint32_t nL, uint32_t *smem, ThreadAcc &acc) {
+		int32_t nl, uint32_t nS, uint32_t nM, uint32_t nL, uint32_t *smem, ThreadAcc &acc) {
 	const uint32_t cur = step & 1, nxt = (step + 1) & 1;
 	StepCounters *out = r.ctr + step % 3;
 	uint32_t *nbm = r.bm[step % 3];
 	const uint32_t *qS = r.q[cur][0], *qM = r.q[cur][1], *qL = r.q[cur][2];
 	uint32_t *const qn[3] = {r.q[nxt][0], r.q[nxt][1], r.q[nxt][2]};
-	const int32_t nl = (int32_t) step + 1;
 	const unsigned lane = lane_id(), wid = warp_id();
 	// warps numbered across CTAs first, so that a small amount of work is
 	// spread over all SMs rather than the first CTAs' warps
@@ -643,14 +642,13 @@ __device__ __forceinline__ uint32_t dense_window(const DevGraph &g, const uint8_
 }
 
 // Generic bottom-up step: slices staged with plain loads (any tile width).
-__device__ __forceinline__ void phase_dense_generic(const DevGraph &g, const RunCtx &r, uint32_t step, uint32_t batch,
-		uint32_t *smem, ThreadAcc &acc) {
+__device__ __forceinline__ void phase_dense_generic(const DevGraph &g, const RunCtx &r, uint32_t step, int32_t nl,
+		uint32_t batch, uint32_t *smem, ThreadAcc &acc) {
 	const uint32_t *cur = r.bm[(step + 2) % 3];
 	uint32_t *nxt = r.bm[step % 3];
 	const uint8_t *sf_cur = r.sf[(step + 2) % 3];
 	uint8_t *sf_nxt = r.sf[step % 3];
 	StepCounters *out = r.ctr + step % 3;
-	const int32_t nl = (int32_t) step + 1;
 	const unsigned tid = threadIdx.x;
 	uint32_t *vis_s = smem;
 	uint32_t *nxt_s = vis_s + g.max_group_words + 1;
@@ -775,13 +773,13 @@ __device__ void dense_tma_init() {
 // barrier, test its edges and release the stage on its "empty" barrier, so
 // no CTA-wide barrier separates batches.  Needs S*W to be a multiple of 128
 // so that every slice starts on a 16-byte boundary.
-__device__ __forceinline__ void phase_dense_tma(const DevGraph &g, const RunCtx &r, uint32_t step, uint32_t *smem, ThreadAcc &acc) {
+__device__ __forceinline__ void phase_dense_tma(const DevGraph &g, const RunCtx &r, uint32_t step, int32_t nl, uint32_t *smem,
+		ThreadAcc &acc) {
 	const uint32_t *cur = r.bm[(step + 2) % 3];
 	uint32_t *nxt = r.bm[step % 3];
 	const uint8_t *sf_cur = r.sf[(step + 2) % 3];
 	uint8_t *sf_nxt = r.sf[step % 3];
 	StepCounters *out = r.ctr + step % 3;
-	const int32_t nl = (int32_t) step + 1;
 	const unsigned tid = threadIdx.x, wid = warp_id(), lane = lane_id();
 	const uint32_t stage_words = kTmaEdgeWords + g.tma_batch * g.slice_words;
 	uint32_t *stages = smem;
@@ -912,12 +910,11 @@ __device__ __forceinline__ bool frontier_bit(const uint32_t *cur, uint32_t u) {
 	return (ld_cg(cur + (u >> 5)) >> (u & 31)) & 1u;
 }
 
-__device__ __forceinline__ void phase_pull(const DevGraph &g, const RunCtx &r, uint32_t step, uint32_t *smem,
+__device__ __forceinline__ void phase_pull(const DevGraph &g, const RunCtx &r, uint32_t step, int32_t nl, uint32_t *smem,
 		ThreadAcc &acc) {
 	const uint32_t *cur = r.bm[(step + 2) % 3];
 	uint32_t *nxt = r.bm[step % 3];
 	StepCounters *out = r.ctr + step % 3;
-	const int32_t nl = (int32_t) step + 1;
 	const unsigned wid = warp_id(), lane = lane_id();
 	const uint32_t mgw = g.max_group_words + 1;
 	uint32_t *vis_s = smem;
@@ -1035,10 +1032,10 @@ __device__ __forceinline__ void phase_pull(const DevGraph &g, const RunCtx &r, u
 }
 
 __device__ __forceinline__ void phase_dense(const DevGraph &g, const RunCtx &r, const StepParams &p, uint32_t step,
-		uint32_t batch, uint32_t *smem, ThreadAcc &acc) {
-	if (p.bottom_up == 0) phase_pull(g, r, step, smem, acc);
-	else if (g.tma) phase_dense_tma(g, r, step, smem, acc);
-	else phase_dense_generic(g, r, step, batch, smem, acc);
+		int32_t nl, uint32_t batch, uint32_t *smem, ThreadAcc &acc) {
+	if (p.bottom_up == 0) phase_pull(g, r, step, nl, smem, acc);
+	else if (g.tma) phase_dense_tma(g, r, step, nl, smem, acc);
+	else phase_dense_generic(g, r, step, nl, batch, smem, acc);
 }
 
 // ---------------------------------------------------------------------------
@@ -1054,6 +1051,8 @@ __device__ __forceinline__ void clear_slot(const DevGraph &g, const RunCtx &r, u
 		StepCounters *c = r.ctr + slot;
 		c->tail[0] = c->tail[1] = c->tail[2] = 0;
 		c->work = 0;
+		c->levels = 0;
+		c->solo_deg = 0;
 	}
 }
 
@@ -1081,15 +1080,19 @@ __device__ __forceinline__ void flush_step(ThreadAcc &acc, const RunCtx &r, uint
 }
 
 // Sums the partials of `slot` over the grid (all threads call), and loads
-// the slot's three queue tails in the same round trip.
+// the slot's three queue tails -- and what one CTA by itself (phase_solo) did
+// to get there -- in the same round trip.
 __device__ __forceinline__ void step_totals(const RunCtx &r, uint32_t slot, uint32_t *count,
-		unsigned long long *degsum, uint32_t (&tails)[3]) {
+		unsigned long long *degsum, uint32_t (&tails)[3], uint32_t *levels, unsigned long long *solo_deg) {
 	// every thread loads at most a few partials (one L2 round trip), then a
 	// block reduction; three threads load the tails (every thread loading
 	// them put hundreds of thousands of requests on one hot line)
 	__shared__ unsigned long long red[2][kWarps];
-	__shared__ uint32_t s_tails[3];
+	__shared__ uint32_t s_tails[3], s_levels;
+	__shared__ unsigned long long s_solo_deg;
 	if (threadIdx.x < 3) s_tails[threadIdx.x] = __ldcg(&r.ctr[slot].tail[threadIdx.x]);
+	else if (threadIdx.x == 32) s_levels = __ldcg(&r.ctr[slot].levels);
+	else if (threadIdx.x == 64) s_solo_deg = __ldcg(&r.ctr[slot].solo_deg);
 	unsigned long long c = 0, d = 0;
 	const unsigned long long *pc = part_at(r, slot, 0), *pd = part_at(r, slot, 1);
 	for (uint32_t i = threadIdx.x; i < gridDim.x; i += blockDim.x) {
@@ -1108,6 +1111,8 @@ __device__ __forceinline__ void step_totals(const RunCtx &r, uint32_t slot, uint
 	tails[0] = s_tails[0];
 	tails[1] = s_tails[1];
 	tails[2] = s_tails[2];
+	*levels = s_levels;
+	*solo_deg = s_solo_deg;
 	__syncthreads();
 }
 
@@ -1213,6 +1218,210 @@ __global__ void k_seed(DevGraph g, RunCtx r, StepParams p) {
 	if (blockIdx.x == 0 && threadIdx.x == 0) seed_source(g, r, p);
 }
 
+// ---------------------------------------------------------------------------
+// Small frontiers: top-down steps by one CTA
+// ---------------------------------------------------------------------------
+// The direction of the step that expands this frontier (apps/bfs_simd/bfs.cpp:
+// 829-834, or Beamer's rule); `seen` includes the frontier's own out-edges.
+__device__ __forceinline__ bool goes_dense(const DevGraph &g, const StepParams &p, uint32_t fsize,
+		unsigned long long dsum, unsigned long long seen, bool last_dense) {
+	if (p.switch_rule == 0) {
+		const unsigned long long thr = last_dense ? p.to_sparse_threshold : p.to_dense_threshold;
+		return (unsigned long long) fsize + dsum > thr;
+	}
+	const unsigned long long unseen = g.m > seen ? g.m - seen : 0ull;
+	return last_dense ? (unsigned long long) fsize * p.beta >= g.n : dsum * p.alpha > unseen;
+}
+
+// A step of the whole grid costs about 6 us however little it does: the grid
+// barrier, the totals and a chain of round trips.  While the frontier has at
+// most kSoloCap vertices and out-edges, CTA 0 therefore takes the steps by
+// itself -- one __syncthreads each, the frontier in shared memory -- and the
+// other CTAs wait at the round's grid barrier.  A level of up to 512 edges is
+// two round trips (edge; claim and row offsets) and one block barrier: 1.05 us
+// against 6.9 us of the grid (1.9 us with the claim as a compare-and-swap on
+// the level in L2, as graphs too large for the visited bits in shared memory
+// take it).  A 301 x 287 street grid of 395 levels: 2.78 -> 0.79 ms; at 2048
+// edges a level takes about as long as half a grid step, and the five words
+// per edge of two lists still fit the shared memory that the grid's own
+// top-down step uses.
+constexpr uint32_t kSoloCap = 2048;
+// Steps in one round: bounds the other CTAs' wait.
+constexpr uint32_t kSoloLevels = 128;
+constexpr uint32_t kSoloWords = 5 * kSoloCap;  // dynamic shared memory of its lists ...
+constexpr uint32_t kSoloVisWords = 8192;       // ... and of the visited bits of graphs of at most 2^18 vertices
+static_assert(kSoloCap <= 0x10000, "owners are 16-bit");
+
+// One of the two frontier lists: vertex u[x] owns the out-edge slots off ..
+// off + deg - 1 of its list, fb[x] = (first edge) - off, owner[slot] = x.
+struct SoloList {
+	uint32_t *u, *fb;
+	uint16_t *owner;
+};
+__device__ __forceinline__ SoloList solo_list(uint32_t *smem, uint32_t which) {
+	uint32_t *b = smem + (size_t) which * (kSoloWords / 2);
+	return {b, b + kSoloCap, (uint16_t *) (b + 2 * kSoloCap)};
+}
+
+// Appends the lanes' vertices v[q] (ok[q]; out-edges beg[q], deg[q]) to `l`;
+// cnt[0], cnt[1]: its vertices and out-edges.  All 32 lanes call it.  Slots
+// past kSoloCap are not filled: a list with that many edges is never expanded
+// here.
+template <int Q>
+__device__ __forceinline__ void solo_append(const SoloList &l, uint32_t *cnt, const bool (&ok)[Q], const uint32_t (&v)[Q],
+		const uint32_t (&beg)[Q], const uint32_t (&deg)[Q]) {
+	const unsigned lane = lane_id();
+	uint32_t c = 0, d = 0;
+#pragma unroll
+	for (int q = 0; q < Q; ++q) {
+		c += ok[q];
+		d += ok[q] ? deg[q] : 0u;
+	}
+	if (!__ballot_sync(kFull, c)) return;
+	const uint32_t ci = warp_incl_scan(c), di = warp_incl_scan(d);
+	const uint32_t ct = __shfl_sync(kFull, ci, 31);
+	uint32_t b = 0;
+	if (lane >= 30) b = atomicAdd(cnt + (lane - 30), lane == 30 ? ct : di);
+	uint32_t pos = __shfl_sync(kFull, b, 30) + ci - c, off = __shfl_sync(kFull, b, 31) + di - d;
+#pragma unroll
+	for (int q = 0; q < Q; ++q) {
+		const uint32_t dq = ok[q] ? deg[q] : 0u;
+		if (ok[q]) {
+			l.u[pos] = v[q];
+			l.fb[pos] = beg[q] - off;
+		}
+		const bool wide = dq > 8;
+		if (!wide)
+			for (uint32_t i = off; i < min(off + dq, kSoloCap); ++i) l.owner[i] = (uint16_t) pos;
+		for (uint32_t m = __ballot_sync(kFull, wide); m; m &= m - 1) {
+			const int j = __ffs(m) - 1;
+			const uint32_t jo = __shfl_sync(kFull, off, j), jd = __shfl_sync(kFull, dq, j), jp = __shfl_sync(kFull, pos, j);
+			const uint32_t je = jo >= kSoloCap ? jo : jo + min(jd, kSoloCap - jo);
+			for (uint32_t i = jo + lane; i < je; i += 32) l.owner[i] = (uint16_t) jp;
+		}
+		pos += ok[q];
+		off += dq;
+	}
+}
+
+// Expands the list `cur` (ne out-edges) into `nxt`, Q edges per lane in
+// flight.  The claim and the out-edge range of its vertex, whether it wins or
+// not, go out together: two round trips per edge.
+template <int Q>
+__device__ __forceinline__ void solo_expand(const DevGraph &g, const RunCtx &r, const SoloList &cur, const SoloList &nxt,
+		uint32_t *cn, uint32_t ne, int32_t nl, uint32_t *vis_s) {
+	const unsigned lane = lane_id();
+	for (uint32_t f0 = threadIdx.x - lane; f0 < ne; f0 += Q * kThreads) {
+		bool ok[Q];
+		uint32_t u[Q], v[Q], beg[Q], end[Q];
+		int32_t old[Q];
+#pragma unroll
+		for (int q = 0; q < Q; ++q) {
+			const uint32_t f = f0 + q * kThreads + lane;
+			ok[q] = f < ne;
+			const uint32_t j = ok[q] ? cur.owner[f] : 0u;
+			u[q] = ok[q] ? cur.u[j] : 0u;
+			v[q] = ok[q] ? __ldg(g.col + (cur.fb[j] + f)) : 0u;
+		}
+#pragma unroll
+		for (int q = 0; q < Q; ++q) {
+			beg[q] = ok[q] ? __ldg(g.row_off + v[q]) : 0u;
+			end[q] = ok[q] ? __ldg(g.row_off + v[q] + 1) : 0u;
+			const uint32_t bit = 1u << (v[q] & 31);
+			if (!ok[q]) old[q] = 0;
+			else if (vis_s) old[q] = (atomicOr(vis_s + (v[q] >> 5), bit) & bit) ? 0 : -1;
+			else old[q] = atomicCAS((int *) r.level + v[q], -1, nl);
+		}
+#pragma unroll
+		for (int q = 0; q < Q; ++q) {
+			ok[q] = ok[q] && old[q] == -1;
+			end[q] -= beg[q];
+			if (ok[q]) {
+				if (vis_s) r.level[v[q]] = nl;
+				atomicOr(r.vis + (v[q] >> 5), 1u << (v[q] & 31));
+				if (r.parent) r.parent[v[q]] = u[q];
+			}
+		}
+		solo_append<Q>(nxt, cn, ok, v, beg, end);
+	}
+}
+
+// Called by every thread of CTA 0: expands the frontier of `step` (queue
+// sizes tails[]) and the ones after it until one is too large, goes
+// bottom-up, is empty, or kSoloLevels steps are done; that one becomes the
+// round's output like any step's.
+__device__ __forceinline__ void phase_solo(const DevGraph &g, const RunCtx &r, const StepParams &p, uint32_t rnd,
+		uint32_t step, const uint32_t (&tails)[3], unsigned long long seen, uint32_t *smem, ThreadAcc &acc,
+		unsigned long long &st_reached, unsigned long long &st_edges) {
+	__shared__ uint32_t cnt[3][2];
+	__shared__ uint32_t s_tail[3];
+	const uint32_t tid = threadIdx.x, in = rnd & 1, out = (rnd + 1) & 1;
+	if (tid < 6) cnt[tid / 2][tid % 2] = 0;
+	if (tid < 3) s_tail[tid] = 0;
+	uint32_t *vis_s = g.nwords <= kSoloVisWords ? smem + kSoloWords : nullptr;
+	if (vis_s)
+		for (uint32_t i = tid; i < g.nwords; i += kThreads) vis_s[i] = ld_cg(r.vis + i);
+	__syncthreads();
+	const uint32_t n0 = tails[0], n1 = n0 + tails[1], n2 = n1 + tails[2];
+	for (uint32_t x0 = 0; x0 < n2; x0 += kThreads) {
+		const uint32_t x = x0 + tid;
+		const bool ok[1] = {x < n2};
+		uint32_t v[1] = {0}, beg[1] = {0}, deg[1] = {0};
+		if (ok[0]) {
+			v[0] = ld_cg(x < n0 ? r.q[in][0] + x : x < n1 ? r.q[in][1] + (x - n0) : r.q[in][2] + (x - n1));
+			beg[0] = __ldg(g.row_off + v[0]);
+			deg[0] = __ldg(g.row_off + v[0] + 1) - beg[0];
+		}
+		solo_append<1>(solo_list(smem, 0), cnt[0], ok, v, beg, deg);
+	}
+	__syncthreads();
+	uint32_t nv = cnt[0][0], ne = cnt[0][1], done = 0;
+	unsigned long long skipped = 0;
+	for (;;) {
+		const SoloList cur = solo_list(smem, done & 1), nxt = solo_list(smem, (done & 1) ^ 1);
+		uint32_t *cn = cnt[(done + 1) % 3];
+		if (tid == 0) {
+			cnt[(done + 2) % 3][0] = cnt[(done + 2) % 3][1] = 0;
+			acc.td_edges += ne;
+			acc.td_vertices += nv;
+		}
+		const int32_t nl = (int32_t) (step + done) + 1;
+		if (ne <= kThreads) solo_expand<1>(g, r, cur, nxt, cn, ne, nl, vis_s);
+		else solo_expand<kTdPerLane>(g, r, cur, nxt, cn, ne, nl, vis_s);
+		__syncthreads();
+		++done;
+		nv = cn[0];
+		ne = cn[1];
+		if (nv == 0 || ne > kSoloCap || done == kSoloLevels ||
+				goes_dense(g, p, nv, ne, seen + skipped + ne, false))
+			break;
+		skipped += ne;
+		if (tid == 0) {
+			st_reached += nv;
+			st_edges += ne;
+			if (step + done < 257) r.stats->t_step[step + done] = global_timer_ns();
+		}
+	}
+	// the frontier left over: the next round's queues and bitmap
+	const SoloList last = solo_list(smem, done & 1);
+	uint32_t *nbm = r.bm[rnd % 3];
+	for (uint32_t x = tid; x < nv; x += kThreads) {
+		const uint32_t v = last.u[x];
+		const uint32_t deg = __ldg(g.row_off + v + 1) - __ldg(g.row_off + v), bk = bucket_of(deg, p);
+		atomicOr(nbm + (v >> 5), 1u << (v & 31));
+		r.q[out][bk][atomicAdd(&s_tail[bk], 1u)] = v;
+		acc.count++;
+		acc.degsum += deg;
+	}
+	__syncthreads();
+	StepCounters *c = r.ctr + rnd % 3;
+	if (tid < 3) c->tail[tid] = s_tail[tid];
+	if (tid == 0) {
+		c->levels = done;
+		c->solo_deg = skipped;
+	}
+}
+
 // All steps of one traversal in one cooperative launch, the clearing of the
 // run state and the seeding of the source included (one grid barrier after
 // them).  The run statistics that only CTA 0 keeps are held in its
@@ -1238,59 +1447,56 @@ __global__ void __launch_bounds__(kThreads, 2) k_bfs_persistent(DevGraph g, RunC
 	CTA_STAMP(15, 1);
 	ok = grid_sync(r.bar, epoch, r.err, p.wait_limit_ns, p.hold_barrier);
 	CTA_STAMP(15, 2);
-	for (; ok; ++step) {
-		uint32_t fsize, tails[3];
-		unsigned long long dsum;
+	// A round is one step of the whole grid, or several of CTA 0 alone
+	// (phase_solo); queues, bitmaps and counters rotate by round.
+	for (uint32_t rnd = 0; ok; ++rnd) {
+		uint32_t fsize, tails[3], levels;
+		unsigned long long dsum, solo_deg;
 		CTA_STAMP(step, 0);
-		step_totals(r, (step + 2) % 3, &fsize, &dsum, tails);
+		step_totals(r, (rnd + 2) % 3, &fsize, &dsum, tails, &levels, &solo_deg);
 		CTA_STAMP(step, 1);
+		if (rnd > 0) step += levels ? levels : 1u;
 		if (leader) {
 			st_reached += fsize;
 			st_edges += dsum;
 			if (step < 257) r.stats->t_step[step] = global_timer_ns();
 		}
 		if (fsize == 0) break;
-		seen += dsum;
-		bool dense = false;
-		if (step > 0) {
-			if (p.switch_rule == 0) {
-				unsigned long long thr = last_dense ? p.to_sparse_threshold : p.to_dense_threshold;
-				dense = (unsigned long long) fsize + dsum > thr;
-			} else {
-				const unsigned long long unseen = g.m > seen ? g.m - seen : 0ull;
-				dense = last_dense ? (unsigned long long) fsize * p.beta >= g.n : dsum * p.alpha > unseen;
-			}
-		}
-		clear_slot(g, r, (step + 1) % 3);
+		seen += solo_deg + dsum;
+		const bool dense = step > 0 && goes_dense(g, p, fsize, dsum, seen, last_dense);
+		clear_slot(g, r, (rnd + 1) % 3);
 		CTA_STAMP(step, 2);
+		bool solo = false;
 		if (dense) {
 			// the top-down step that produced this frontier also set its
 			// bitmap; only the streaming variant needs the stripe flags built
 			if (!last_dense && p.bottom_up != 0) {
-				phase_to_dense(g, r, step, true);
+				phase_to_dense(g, r, rnd, true);
 				if (!(ok = grid_sync(r.bar, epoch, r.err, p.wait_limit_ns, p.hold_barrier))) break;
 				if (leader && step < 256) r.stats->t_conv[step] = global_timer_ns();
 			}
 			CTA_STAMP(step, 3);
-			phase_dense(g, r, p, step, batch, smem, acc);
+			phase_dense(g, r, p, rnd, (int32_t) step + 1, batch, smem, acc);
 		} else {
 			if (last_dense) {
-				phase_to_sparse(g, r, p, step);
+				phase_to_sparse(g, r, p, rnd);
 				if (!(ok = grid_sync(r.bar, epoch, r.err, p.wait_limit_ns, p.hold_barrier))) break;
 				if (leader && step < 256) r.stats->t_conv[step] = global_timer_ns();
-				if (threadIdx.x < 3) s_conv_tails[threadIdx.x] = __ldcg(&r.ctr[(step + 2) % 3].tail[threadIdx.x]);
+				if (threadIdx.x < 3) s_conv_tails[threadIdx.x] = __ldcg(&r.ctr[(rnd + 2) % 3].tail[threadIdx.x]);
 				__syncthreads();
 				tails[0] = s_conv_tails[0];
 				tails[1] = s_conv_tails[1];
 				tails[2] = s_conv_tails[2];
 			}
 			CTA_STAMP(step, 3);
-			phase_expand(g, r, p, step, tails[0], tails[1], tails[2], smem, acc);
+			solo = fsize <= kSoloCap && dsum <= kSoloCap;
+			if (!solo) phase_expand(g, r, p, rnd, (int32_t) step + 1, tails[0], tails[1], tails[2], smem, acc);
+			else if (blockIdx.x == 0) phase_solo(g, r, p, rnd, step, tails, seen, smem, acc, st_reached, st_edges);
 		}
 		CTA_STAMP(step, 4);
-		flush_step(acc, r, step % 3);
+		flush_step(acc, r, rnd % 3);
 		CTA_STAMP(step, 5);
-		if (threadIdx.x == 0 && step < 256) {
+		if (threadIdx.x == 0 && step < 256 && !solo) {
 			const unsigned long long t = global_timer_ns();
 			atomicMax(&r.stats->t_work_max[step], t);
 			atomicMax(&r.stats->t_work_min_inv[step], ~t);
@@ -1337,7 +1543,7 @@ __global__ void __launch_bounds__(kThreads) k_step_expand(DevGraph g, RunCtx r, 
 	extern __shared__ __align__(128) uint32_t smem[];
 	ThreadAcc acc{0, 0, 0, 0, 0, 0, 0, 0};
 	const StepCounters *in = r.ctr + (step + 2) % 3;
-	phase_expand(g, r, p, step, ld_volatile(&in->tail[0]), ld_volatile(&in->tail[1]), ld_volatile(&in->tail[2]),
+	phase_expand(g, r, p, step, (int32_t) step + 1, ld_volatile(&in->tail[0]), ld_volatile(&in->tail[1]), ld_volatile(&in->tail[2]),
 			smem, acc);
 	flush_step(acc, r, step % 3);
 	flush_stats(acc, r.stats);
@@ -1347,7 +1553,7 @@ __global__ void __launch_bounds__(kThreads, 2) k_step_dense(DevGraph g, RunCtx r
 	extern __shared__ __align__(128) uint32_t smem[];
 	ThreadAcc acc{0, 0, 0, 0, 0, 0, 0, 0};
 	dense_tma_init();
-	phase_dense(g, r, p, step, batch, smem, acc);
+	phase_dense(g, r, p, step, (int32_t) step + 1, batch, smem, acc);
 	flush_step(acc, r, step % 3);
 	flush_stats(acc, r.stats);
 }
@@ -1355,25 +1561,38 @@ __global__ void __launch_bounds__(kThreads, 2) k_step_dense(DevGraph g, RunCtx r
 // ---------------------------------------------------------------------------
 // Host-side launchers
 // ---------------------------------------------------------------------------
-size_t dense_smem_bytes(const DevGraph &g, uint32_t batch) {
+// Dynamic shared memory of the traversal kernels for a bottom-up variant: the
+// pull needs less than half of what the streamed variant stages, so that two
+// CTAs fit an SM whatever the graph's column groups are (Twitter shape: one
+// CTA per SM with the streamed variant's 112 KB; the first pull step took
+// 3.33 ms, with two 1.86 ms).
+size_t traversal_smem_bytes(const DevGraph &g, uint32_t batch, uint32_t bottom_up) {
 	size_t words = (size_t) 2 * (g.max_group_words + 1) + 3 * kThreads;
 	if (g.tma) words += (size_t) kTmaStages * (kTmaEdgeWords + (size_t) g.tma_batch * g.slice_words);
 	else words += (size_t) batch * g.slice_words;
 	const size_t pull = (size_t) 3 * (g.max_group_words + 1) + g.pull_long_cap;
 	const size_t expand = (size_t) kWarps * 3 * kWqCap + 3 * (size_t) kFlatChunk;
-	size_t need = words > pull ? words : pull;
+	size_t need = bottom_up == BFS_BU_PULL || pull > words ? pull : words;
 	need = need > expand ? need : expand;
+	const size_t solo = kSoloWords + (g.nwords <= kSoloVisWords ? g.nwords : 0u);
+	need = need > solo ? need : solo;
 	return sizeof(uint32_t) * need;
 }
 
-int persistent_grid(const DevGraph &g, uint32_t batch, int num_sms, int *grid, size_t *smem) {
-	*smem = dense_smem_bytes(g, batch);
-	if (cudaFuncSetAttribute(k_bfs_persistent, cudaFuncAttributeMaxDynamicSharedMemorySize, (int) *smem) != cudaSuccess)
-		return BFS_ECUDA;
-	if (cudaFuncSetAttribute(k_step_dense, cudaFuncAttributeMaxDynamicSharedMemorySize, (int) *smem) != cudaSuccess)
-		return BFS_ECUDA;
-	if (cudaFuncSetAttribute(k_step_expand, cudaFuncAttributeMaxDynamicSharedMemorySize, (int) *smem) != cudaSuccess)
-		return BFS_ECUDA;
+// The grid and the shared memory of a traversal with the given bottom-up
+// variant.  The kernels' shared-memory limit is the device's, the same for
+// every graph: a limit of this graph's own need would be that of all graphs.
+int persistent_grid(const DevGraph &g, uint32_t batch, uint32_t bottom_up, int device, int num_sms, int *grid, size_t *smem) {
+	*smem = traversal_smem_bytes(g, batch, bottom_up);
+	int optin = 0;
+	if (cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, device) != cudaSuccess) return BFS_ECUDA;
+	for (const void *fn : {(const void *) k_bfs_persistent, (const void *) k_step_dense, (const void *) k_step_expand}) {
+		cudaFuncAttributes at{};
+		if (cudaFuncGetAttributes(&at, fn) != cudaSuccess) return BFS_ECUDA;
+		const int most = optin - (int) at.sharedSizeBytes;
+		if (*smem > (size_t) most) return BFS_ECUDA;
+		if (cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, most) != cudaSuccess) return BFS_ECUDA;
+	}
 	int per_sm = 0;
 	if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_bfs_persistent, kThreads, *smem) != cudaSuccess)
 		return BFS_ECUDA;

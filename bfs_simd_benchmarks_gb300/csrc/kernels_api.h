@@ -22,8 +22,9 @@ constexpr uint32_t kTmaSliceWords = 4096;
 
 enum StepKind { kStepSeed = 0, kStepClear, kStepToDense, kStepToSparse, kStepExpand, kStepDense };
 
-size_t dense_smem_bytes(const DevGraph &g, uint32_t batch);
-int persistent_grid(const DevGraph &g, uint32_t batch, int num_sms, int *grid, size_t *smem);
+// The cooperative grid at full occupancy and the dynamic shared memory of a
+// traversal whose bottom-up steps are `bottom_up` (BFS_BU_*).
+int persistent_grid(const DevGraph &g, uint32_t batch, uint32_t bottom_up, int device, int num_sms, int *grid, size_t *smem);
 // Clears the run state for the stepwise mode (the persistent kernel clears
 // and seeds by itself).
 int launch_init(const DevGraph &g, const RunCtx &r, cudaStream_t st, int num_sms);

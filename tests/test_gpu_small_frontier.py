@@ -1,0 +1,111 @@
+"""Single-source traversals whose frontiers are small enough for one CTA to take
+several steps by itself: the edges of that rule (2048 vertices and out-edges,
+128 steps, 2^18 vertices) and what it hands back to the whole grid, against the
+oracle (levels and direction trace bit-exact, parents a valid tree)."""
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+
+def _star(leaves, fan):
+    """0 -> leaves 1..d; leaf i -> fan[i % len(fan)] of its own grandchildren and one shared vertex."""
+    src, dst, n = [0] * leaves, list(range(1, leaves + 1)), leaves + 2
+    shared = leaves + 1
+    for i in range(leaves):
+        for _ in range(fan[i % len(fan)]):
+            src.append(i + 1)
+            dst.append(n)
+            n += 1
+        src.append(i + 1)
+        dst.append(shared)
+    return n, src, dst
+
+
+def _chain(levels, width, n=0):
+    """`levels` layers of `width` vertices, each layer's vertices to all of the next; isolated vertices up to n."""
+    src, dst = [], []
+    for l in range(levels):
+        for i in range(width):
+            for j in range(width):
+                src.append(l * width + i)
+                dst.append((l + 1) * width + j)
+    return max(n, (levels + 1) * width), src, dst
+
+
+def _ladder_into_hub(hub):
+    """A chain of 5, a hub of `hub` out-edges, and a second chain behind its last leaf."""
+    n, src, dst = 5, [0, 1, 2, 3], [1, 2, 3, 4]
+    first = n
+    src += [4] * hub
+    dst += range(first, first + hub)
+    n += hub
+    for i in range(6):
+        src.append(n - 1)
+        dst.append(n)
+        n += 1
+    return n, src, dst
+
+
+CASES = {
+    "star_2047": _star(2047, [0]),
+    "star_2048": _star(2048, [0]),
+    "star_2049": _star(2049, [0]),
+    "star_grows": _star(300, [1, 9, 0, 40]),
+    "star_edges_past_cap": _star(200, [10]),
+    "chain_127": _chain(127, 1),
+    "chain_128": _chain(128, 1),
+    "chain_129": _chain(129, 1),
+    "chain_300x3": _chain(300, 3),
+    "layers_45": _chain(6, 45),
+    "layers_46": _chain(6, 46),
+    "chain_2p18": _chain(140, 2, 1 << 18),
+    "chain_2p18_plus": _chain(140, 2, (1 << 18) + 1),
+    "hub_2048": _ladder_into_hub(2048),
+    "hub_5000": _ladder_into_hub(5000),
+}
+
+
+@pytest.mark.parametrize("rule", [0, 1])
+@pytest.mark.parametrize("degree_order", [False, True])
+@pytest.mark.parametrize("name", list(CASES))
+def test_small_frontiers(native, oracle, name, degree_order, rule):
+    import bfs_simd_benchmarks_gb300 as B
+    n, src, dst = CASES[name]
+    src, dst = np.asarray(src + src[:3], np.uint32), np.asarray(dst + dst[:3], np.uint32)  # with duplicate edges
+    arr = oracle.arrays_from_edges(n, src, dst, 64, 4)
+    deg = arr["degrees"].astype(np.uint64)
+    with B.Graph.from_edges(n, src, dst, 64, 4, degree_order=degree_order) as g:
+        g.set_options(switch_rule=rule)
+        for s in (0, 1):
+            ref = oracle.bfs_levels(arr, s)
+            lev, par, st = g.run(s)
+            np.testing.assert_array_equal(lev, ref)
+            assert oracle.check_parents(arr, s, lev, par) == 0
+            assert st["status"] == 0
+            assert st["num_steps"] == ref.max() + 1
+            assert st["reached"] == int((ref >= 0).sum())
+            assert st["edges_traversed"] == int(deg[ref >= 0].sum())
+            if rule == 0:
+                _, _, trace, _ = oracle.bfs_hybrid(arr, s)
+                k = min(len(trace), st["num_steps"], 256)
+                assert list(st["trace"][:k]) == list(trace[:k])
+
+
+def test_a_smaller_graph_leaves_a_larger_one_callable(native, oracle):
+    """Each graph's traversals ask for their own amount of shared memory, whatever was built since."""
+    import bfs_simd_benchmarks_gb300 as B
+    n = 1 << 15
+    src, dst = B.gen_rmat(n, 4 * n, seed=77, permute=True)
+    arr = oracle.arrays_from_edges(n, src, dst, 1024, 16)
+    s = int(B.pick_sources(arr["degrees"], 1, seed=3)[0])
+    ref = oracle.bfs_levels(arr, s)
+    with B.Graph.from_edges(n, src, dst, 1024, 16) as g:
+        with B.Graph.from_edges(3, [0, 1], [1, 2], 64, 4) as small:
+            for bottom_up in ("pull", "stream"):
+                for mode in ("persistent", "stepwise"):
+                    g.set_options(bottom_up=bottom_up, mode=mode)
+                    lev, _, st = g.run(s)
+                    assert st["status"] == 0
+                    np.testing.assert_array_equal(lev, ref)
+            np.testing.assert_array_equal(small.run(0)[0], [0, 1, 2])
