@@ -112,11 +112,13 @@ struct bfs_graph {
 	// batched betweenness state, allocated by the first batched bfs_bc_* call
 	struct BcBatch {
 		uint32_t *sigma = nullptr, *partial = nullptr, *d_sources = nullptr;
+		unsigned *chunks_done = nullptr;
 		float *dsum = nullptr;
 		float *delta = nullptr;      // [64][n] staging of host outputs (allocated when first asked for)
 		uint32_t *paths = nullptr;
 		uint32_t *blist = nullptr, *ilist = nullptr, *olist = nullptr;  // per-level work lists
 		uint32_t list_planes = 0;    // levels they have room for
+		uint32_t state_words = 0;    // words of 64 sources the state and the lists hold
 		std::vector<DevBuf> lbufs;
 		BbControl *ctl = nullptr;
 		BbControl *h_ctl = nullptr;  // pinned
@@ -129,9 +131,9 @@ struct bfs_graph {
 		size_t bytes = 0;
 		std::vector<DevBuf> bufs;
 	} bb;
-	// out-edge chunks of vertices with many out-edges (batched betweenness)
-	const uint32_t *bb_ochunk_v = nullptr, *bb_ochunk_beg = nullptr;
-	uint32_t bb_noch = 0;
+	// edge chunks of vertices with many in- or out-edges (batched betweenness)
+	const uint32_t *bb_ichunk_v = nullptr, *bb_ichunk_beg = nullptr, *bb_ochunk_v = nullptr, *bb_ochunk_beg = nullptr;
+	uint32_t bb_nich = 0, bb_noch = 0;
 	bool bb_chunks_ready = false;
 	bool bc_last_batched = false;    // bfs_bc_last_stats describes a batched run
 	std::mutex mu;
@@ -1230,32 +1232,76 @@ template <class T> int bb_alloc(bfs_graph *g, T **out, size_t count) {
 
 static_assert(BFS_BC_BATCH_MAX_SOURCES == kBbMaxWords * kBbMaxSources, "a batch is at most kBbMaxWords launches");
 
-// Out-edge chunks (once per graph), the per-(vertex, source) state, and
-// (host_out) the [64][n] staging of host outputs.
-int bb_prepare(bfs_graph *g, bool host_deps, bool host_paths) {
+// Words of 64 sources that one launch takes.  On small graphs a level of one
+// word has fewer list items than the grid has warps; all of a call's words
+// together fill it and pass its barriers once.  R-MAT scale 16, 201 sources,
+// with the chunks and parts below: 5.9 -> 1.9 ms.  Above kBbFuseMaxVertices a
+// word fills the grid by itself, and the state of four words (2 KB per vertex)
+// would only cost memory.
+constexpr uint32_t kBbFuseMaxVertices = 1u << 19;
+uint32_t bb_launch_words(const bfs_graph *g, uint32_t num_sources) {
+	const uint32_t K = std::min(kBbMaxWords, (num_sources + kBbMaxSources - 1) / kBbMaxSources);
+	return g->n <= kBbFuseMaxVertices ? K : 1u;
+}
+
+// Edges per chunk of the sweeps: a vertex's (or a block's) edges are a serial
+// chain on one warp, which on a small graph outlasts everything else of a
+// level; on a large one longer chunks save partial rows.  Measured per call,
+// with 64 / 128 / 256 edges: R-MAT scale 16, 64 sources 739 / 779 / 885 us;
+// scale 18, 256 sources 4.64 / 4.51 / 4.42 ms; scale 19, 64 sources 2.85 / 2.70 /
+// 2.88 ms; Pokec shape, 64 sources 8.25 / 7.8 / 7.33 ms.
+uint32_t bb_chunk_edges(const bfs_graph *g) { return g->m <= 1u << 21 ? 64u : g->m <= 1u << 24 ? 128u : kMsChunk; }
+// Blocks of 32 vertices (over a launch's words) from which a list item is a
+// whole block; below, quarters of blocks give the grid's warps more items
+// (scale 18, 64 sources: 1.86 -> 1.74 ms with quarters; scale 19: 2.70 -> 2.73).
+constexpr size_t kBbWholeBlocks = 1u << 14;
+
+// Edge chunks (once per graph) of the vertices with more than `chunk` edges in
+// the rows `d_off`, uploaded.
+int bb_upload_chunks(bfs_graph *g, const uint32_t *d_off, uint32_t chunk, const uint32_t **chunk_v,
+		const uint32_t **chunk_beg, uint32_t *count) {
+	std::vector<uint32_t> off((size_t) g->n + 1);
+	if (cudaMemcpy(off.data(), d_off, sizeof(uint32_t) * off.size(), cudaMemcpyDeviceToHost) != cudaSuccess)
+		return BFS_ECUDA;
+	std::vector<uint32_t> cv, cb;
+	for (uint32_t v = 0; v < g->n; ++v) {
+		if (off[v + 1] - off[v] <= chunk) continue;
+		for (uint32_t e = off[v]; e < off[v + 1]; e += chunk) {
+			cv.push_back(v);
+			cb.push_back(e);
+		}
+	}
+	*count = (uint32_t) cv.size();
+	const int rc = dev_upload(g, chunk_v, cv);
+	return rc ? rc : dev_upload(g, chunk_beg, cb);
+}
+
+// Edge chunks (once per graph), the per-(vertex, source) state, and
+// (host_out) the [256][n] staging of host outputs.
+int bb_prepare(bfs_graph *g, uint32_t num_sources, bool host_deps, bool host_paths) {
 	int rc;
 	if (!g->bb_chunks_ready) {
-		std::vector<uint32_t> off((size_t) g->n + 1);
-		if (cudaMemcpy(off.data(), g->dg.row_off, sizeof(uint32_t) * off.size(), cudaMemcpyDeviceToHost) != cudaSuccess)
-			return BFS_ECUDA;
-		std::vector<uint32_t> cv, cb;
-		for (uint32_t v = 0; v < g->n; ++v) {
-			if (off[v + 1] - off[v] <= kBbBig) continue;
-			for (uint32_t e = off[v]; e < off[v + 1]; e += kBbChunk) {
-				cv.push_back(v);
-				cb.push_back(e);
-			}
+		const uint32_t chunk = bb_chunk_edges(g);
+		if ((rc = bb_upload_chunks(g, g->dg.row_off, chunk, &g->bb_ochunk_v, &g->bb_ochunk_beg, &g->bb_noch))) return rc;
+		if (chunk == kMsChunk) {  // the batched pull's
+			g->bb_ichunk_v = g->ms_chunk_v;
+			g->bb_ichunk_beg = g->ms_chunk_beg;
+			g->bb_nich = g->ms_nchunks;
+		} else if ((rc = bb_upload_chunks(g, g->dg.in_off, chunk, &g->bb_ichunk_v, &g->bb_ichunk_beg, &g->bb_nich))) {
+			return rc;
 		}
-		g->bb_noch = (uint32_t) cv.size();
-		if ((rc = dev_upload(g, &g->bb_ochunk_v, cv)) || (rc = dev_upload(g, &g->bb_ochunk_beg, cb))) return rc;
 		g->bb_chunks_ready = true;
 	}
 	auto &b = g->bb;
+	const uint32_t words = bb_launch_words(g, num_sources);
+	if (b.ctl && b.state_words < words) release_bb(g);  // its cudaFree waits for earlier calls
 	if (!b.ctl) {
-		const size_t rows = (size_t) g->n * kBbMaxSources;
-		const size_t part = (size_t) std::max(g->ms_nchunks, g->bb_noch) * kBbMaxSources;
+		const size_t rows = (size_t) words * g->n * kBbMaxSources;
+		const size_t part = (size_t) words * std::max(g->bb_nich, g->bb_noch);
+		b.state_words = words;
 		if ((rc = bb_alloc(g, &b.sigma, rows)) || (rc = bb_alloc(g, &b.dsum, rows)) ||
-				(rc = bb_alloc(g, &b.partial, part)) || (rc = bb_alloc(g, &b.ctl, kBbMaxWords)) ||
+				(rc = bb_alloc(g, &b.partial, part * kBbMaxSources)) || (rc = bb_alloc(g, &b.chunks_done, part)) ||
+				(rc = bb_alloc(g, &b.ctl, kBbMaxWords)) ||
 				(rc = bb_alloc(g, &b.d_sources, kBbMaxWords * kBbMaxSources))) {
 			release_bb(g);
 			return rc;
@@ -1292,8 +1338,8 @@ int bb_enqueue(bfs_graph *g, const uint32_t *sources, uint32_t ns, float *delta,
 		for (auto &x : b.lbufs) cudaFree(x.p);
 		b.lbufs.clear();
 		b.list_planes = 0;
-		const size_t nblk = (g->n + 31) / 32;
-		const size_t sizes[3] = {planes * nblk, (size_t) planes * g->ms_nchunks, (size_t) planes * g->bb_noch};
+		const size_t nblk = (g->n + 31) / 32, levels = (size_t) planes * b.state_words;
+		const size_t sizes[3] = {levels * nblk, levels * g->bb_nich, levels * g->bb_noch};
 		uint32_t **dst[3] = {&b.blist, &b.ilist, &b.olist};
 		for (int i = 0; i < 3; ++i) {
 			void *p = nullptr;
@@ -1324,15 +1370,17 @@ int bb_enqueue(bfs_graph *g, const uint32_t *sources, uint32_t ns, float *delta,
 	x.hist = a.hist;
 	x.vis = a.vis;
 	x.ms = a.ctl;
-	x.ichunk_v = g->ms_chunk_v;
-	x.ichunk_beg = g->ms_chunk_beg;
-	x.nich = g->ms_nchunks;
+	x.ichunk_v = g->bb_ichunk_v;
+	x.ichunk_beg = g->bb_ichunk_beg;
+	x.nich = g->bb_nich;
+	x.chunk = bb_chunk_edges(g);
 	x.ochunk_v = g->bb_ochunk_v;
 	x.ochunk_beg = g->bb_ochunk_beg;
 	x.noch = g->bb_noch;
 	x.sigma = b.sigma;
 	x.dsum = b.dsum;
 	x.partial = b.partial;
+	x.chunks_done = b.chunks_done;
 	x.blist = b.blist;
 	x.ilist = b.ilist;
 	x.olist = b.olist;
@@ -1340,11 +1388,15 @@ int bb_enqueue(bfs_graph *g, const uint32_t *sources, uint32_t ns, float *delta,
 	x.wait_limit_ns = wait_limit_ns(g->opt);
 	x.hold_barrier = g->opt.test_hold_barrier;
 	x.ctas_per_sm = g->opt.ctas_per_sm;
-	// one launch (and output pass) per word of 64 sources, in source order, so
-	// that acc receives the sources in order
-	for (uint32_t w = 0; w < K; ++w) {
+	// the words of 64 sources, in launches (and output passes) of up to
+	// bb_launch_words, in source order, so that acc receives the sources in order
+	const uint32_t fused = bb_launch_words(g, ns);
+	for (uint32_t w = 0; w < K; w += fused) {
 		x.word = w;
-		x.ns = std::min<uint32_t>(kBbMaxSources, ns - w * kBbMaxSources);
+		x.words = std::min(fused, K - w);
+		x.ns = std::min<uint32_t>(x.words * kBbMaxSources, ns - w * kBbMaxSources);
+		// parts of a block: enough list items for the grid's warps
+		x.split = (size_t) ((g->n + 31) / 32) * x.words >= kBbWholeBlocks ? 1 : 4;
 		x.ctl = b.ctl + w;
 		const size_t row0 = (size_t) w * kBbMaxSources * g->n;
 		BbOut o{b.d_sources + w * kBbMaxSources, delta ? delta + row0 : nullptr, paths ? paths + row0 : nullptr, acc};
@@ -2048,7 +2100,7 @@ int bfs_bc_run_batch(bfs_graph *g, const uint32_t *sources, uint32_t num_sources
 	for (uint32_t i = 0; i < num_sources; ++i)
 		if (sources[i] >= g->n) return BFS_EARG;
 	if (cudaSetDevice(g->device) != cudaSuccess) return BFS_ECUDA;
-	int rc = bb_prepare(g, dependencies != nullptr, num_paths != nullptr);
+	int rc = bb_prepare(g, num_sources, dependencies != nullptr, num_paths != nullptr);
 	if (rc) return rc;
 	auto &b = g->bb;
 	if ((rc = bb_enqueue(g, sources, num_sources, dependencies ? b.delta : nullptr, num_paths ? b.paths : nullptr,
@@ -2082,7 +2134,7 @@ int bfs_bc_run_batch_device(bfs_graph *g, const uint32_t *sources, uint32_t num_
 	for (uint32_t i = 0; i < num_sources; ++i)
 		if (sources[i] >= g->n) return BFS_EARG;
 	if (cudaSetDevice(g->device) != cudaSuccess) return BFS_ECUDA;
-	int rc = bb_prepare(g, false, false);
+	int rc = bb_prepare(g, num_sources, false, false);
 	if (rc) return rc;
 	return bb_enqueue(g, sources, num_sources, dependencies, num_paths, nullptr, (cudaStream_t) stream);
 }
@@ -2098,7 +2150,7 @@ int bfs_bc_accumulate(bfs_graph *g, const uint32_t *sources, uint32_t num_source
 	int rc = bc_prepare(g);
 	if (rc) return rc;
 	auto &b = g->bc;
-	if (g->opt.bc_batch && (rc = bb_prepare(g, false, false))) return rc;
+	if (g->opt.bc_batch && (rc = bb_prepare(g, num_sources, false, false))) return rc;
 	if (cudaMemsetAsync(b.acc, 0, sizeof(float) * g->n, 0) != cudaSuccess) return BFS_ECUDA;
 	cudaEvent_t start = nullptr, end = nullptr;
 	if (cudaEventCreate(&start) != cudaSuccess || cudaEventCreate(&end) != cudaSuccess ||

@@ -1,5 +1,5 @@
-// bc_batch.cu -- betweenness dependencies of 64 sources (one word of a batched
-// traversal) in one pass.
+// bc_batch.cu -- betweenness dependencies of many sources (64 per word of a
+// batched traversal, one to four words per launch) in one pass.
 //
 // No counterpart in the reference, whose BC() (apps/betweennessCentrality_simd/
 // bc.cpp:1717-2097) handles one source per call; for every source the results
@@ -11,7 +11,7 @@
 //
 // The batched traversal (msbfs.cu) leaves, for every level L, the plane
 // hist[L][v]: the sources that reached v first at level L (a launch takes one
-// 64-bit word of it).  u -> v is a shortest-path edge of source s exactly when
+// or more of its 64-bit words, which share nothing but the levels' barriers).  u -> v is a shortest-path edge of source s exactly when
 // bit s is set in both hist[L-1][u] and hist[L][v], so one AND of two words
 // gives all the sources an edge serves.  The state is per (vertex, source):
 // sigma[v][64] and dsum[v][64], a 256-byte row each.
@@ -22,8 +22,8 @@
 //   reverse, L = depth-1 .. 0:
 //     dsum[v][s] = (sum of dsum[w][s] over out-edges v -> w, s in hist[L][v] & hist[L+1][w])
 //                  + 1 / sigma[v][s].
-// The launch first lists, per level, the blocks of 32 consecutive vertices
-// and the edge chunks that have a vertex at that level; a level then hands
+// The launch first lists, per level and word, the blocks of 32 consecutive
+// vertices and the edge chunks that have a vertex at that level; a level then hands
 // its list items to warps one at a time through a counter.  A warp takes a
 // block and walks the concatenated edge lists of its vertices at that level,
 // 32 edges per step (each edge's vertex found by a binary search over the
@@ -33,10 +33,10 @@
 // neighbour's row, read where any of the 4 is served); a vertex's sum is its
 // half-0 sum plus its half-1 sum.  The finish of chunked vertices keeps lane l
 // on sources l and l + 32.
-// Vertices with more than kBbBig edges in the sweep's direction are cut into
-// kBbChunk-edge chunks, one list item each; the partial rows are added in
-// chunk order after a grid barrier.  Every sum has a fixed order, so repeated
-// runs give identical bits.
+// Vertices with more than BbArgs::chunk edges in the sweep's direction are cut
+// into chunks of that many, one list item each; the warp that completes a
+// vertex's last chunk adds the partial rows in chunk order.  Every sum has a
+// fixed order, so repeated runs give identical bits.
 // The output pass (its own launch) turns the [v][64] rows into [source][v]
 // rows through a shared-memory transpose, 0 for unreached pairs, and/or adds
 // each vertex's dependencies into an accumulator in source order.
@@ -61,18 +61,18 @@ __device__ __forceinline__ uint64_t bb_shfl64(uint64_t x, int src) {
 	return (uint64_t) __shfl_sync(kFull, (unsigned long long) x, src);
 }
 __device__ __forceinline__ uint64_t bb_ldg64(const uint64_t *p) { return __ldg((const unsigned long long *) p); }
-// Plane L of the launch's word, and vertex v's entry in it (planes hold K words per vertex).
-__device__ __forceinline__ const uint64_t *bb_plane(const BbArgs &a, uint32_t L) {
-	return a.hist + (size_t) L * a.n * a.K + a.word;
+// Plane L of the launch's word w, and vertex v's entry in it (planes hold K words per vertex).
+__device__ __forceinline__ const uint64_t *bb_plane(const BbArgs &a, uint32_t L, uint32_t w) {
+	return a.hist + (size_t) L * a.n * a.K + a.word + w;
 }
 __device__ __forceinline__ uint64_t bb_word(const uint64_t *plane, const BbArgs &a, uint32_t v) {
 	return bb_ldg64(plane + (size_t) v * a.K);
 }
 
-// A warp's counts over a sweep: edges read (lane 0), edges that serve a
+// A warp's counts over a level: edges read (lane 0), edges that serve a
 // source (lane 0), and (edge, source) pairs summed (every lane its own edges).
 struct BbCount {
-	unsigned long long edges, matched, served;
+	uint32_t edges, matched, served;
 };
 
 // The two sweeps: forward reads in-edges and path counts, reverse reads
@@ -248,26 +248,27 @@ __device__ __forceinline__ void bb_add_pair(const BbArgs &a, uint32_t vb, uint64
 		for (int i = 0; i < 4; ++i) op.acc[i] += x[i];
 }
 
-// Block b of 32 consecutive vertices in one level of a sweep: those with at
-// most kBbBig edges in the sweep's direction.  `has_nb`: the neighbour level
-// exists (the reverse sweep's deepest level has none; its vertices get
-// 1/sigma alone).
+// Vertices lo .. hi - 1 of block b (32 consecutive vertices) in one level of a
+// sweep: those with at most a.big edges in the sweep's direction.  `has_nb`:
+// the neighbour level exists (the reverse sweep's deepest level has none; its
+// vertices get 1/sigma alone).
 template <bool kFwd>
-__device__ void bb_block(const BbArgs &a, uint32_t L, bool has_nb, uint32_t b, BbCount &cnt) {
+__device__ void bb_block(const BbArgs &a, uint32_t L, uint32_t w, bool has_nb, uint32_t b, uint32_t lo, uint32_t hi,
+		BbCount &cnt) {
 	using D = BbDir<kFwd>;
 	using T = typename D::T;
 	const unsigned lane = lane_id();
-	const uint64_t *own = bb_plane(a, L);
-	const uint64_t *nb = bb_plane(a, kFwd ? L - 1 : L + 1);
+	const uint64_t *own = bb_plane(a, L, w);
+	const uint64_t *nb = bb_plane(a, kFwd ? L - 1 : L + 1, w);
 	const uint32_t *off = D::off(a), *adj = D::adj(a);
-	const uint32_t vb = b * 32, v = vb + lane;
-	const uint64_t hv = v < a.n ? bb_word(own, a, v) : 0ull;
+	const uint32_t rw = w * a.n, vb = b * 32 + rw, v = b * 32 + lane;  // rw: row of the word's vertex 0
+	const uint64_t hv = v < a.n && lane >= lo && lane < hi ? bb_word(own, a, v) : 0ull;
 	uint32_t beg = 0, end = 0;
 	if (hv) {
 		beg = __ldg(off + v);
 		end = __ldg(off + v + 1);
 	}
-	const bool part = hv != 0ull && end - beg <= kBbBig;
+	const bool part = hv != 0ull && end - beg <= a.chunk;
 	const uint32_t pm = __ballot_sync(kFull, part);
 	if (!pm) return;
 	const uint32_t d = part && has_nb ? end - beg : 0u;
@@ -294,6 +295,7 @@ __device__ void bb_block(const BbArgs &a, uint32_t L, bool has_nb, uint32_t b, B
 		if (e < total) {
 			u = __ldg(adj + obeg + (e - oex));
 			m = ohv & bb_word(nb, a, u);
+			u += rw;
 		}
 		uint32_t bal = __ballot_sync(kFull, m != 0ull);
 		if (lane == 0) {
@@ -358,17 +360,51 @@ __device__ void bb_block(const BbArgs &a, uint32_t L, bool has_nb, uint32_t b, B
 	}
 }
 
-// Chunk c (kBbChunk edges of a vertex with more than kBbBig edges) in one
-// level of a sweep: the sums of its edges into partial[c].
+// After the chunk sums of vertex v (first chunk c0, k of them): adds its
+// chunks' partial rows in chunk order and writes its sums.
 template <bool kFwd>
-__device__ void bb_chunk(const BbArgs &a, uint32_t L, bool has_nb, uint32_t c, uint32_t v, uint64_t hv,
-		BbCount &cnt) {
+__device__ __forceinline__ void bb_finish(const BbArgs &a, uint32_t w, uint32_t v, uint64_t hv, uint32_t c0, uint32_t k) {
 	using D = BbDir<kFwd>;
 	using T = typename D::T;
 	const unsigned lane = lane_id();
-	const uint64_t *nb = bb_plane(a, kFwd ? L - 1 : L + 1);
+	const bool w0 = (hv >> lane) & 1ull, w1 = (hv >> (lane + 32)) & 1ull;
+	const uint32_t vr = v + w * a.n;
+	const BbPre pre = bb_pre<kFwd>(a, vr, hv);
+	const size_t r0 = (size_t) w * D::nchunks(a) + c0;
+	T acc0 = T(0), acc1 = T(0);
+	for (uint32_t i = 0; i < k; i += kBbUnroll) {
+		T x0[kBbUnroll], x1[kBbUnroll];
+#pragma unroll
+		for (int j = 0; j < kBbUnroll; ++j) {
+			const bool in = i + j < k;
+			const size_t row = (r0 + i + j) * 64;
+			x0[j] = in && w0 ? D::from_bits(ld_cg(a.partial + row + lane)) : T(0);
+			x1[j] = in && w1 ? D::from_bits(ld_cg(a.partial + row + lane + 32)) : T(0);
+		}
+#pragma unroll
+		for (int j = 0; j < kBbUnroll; ++j) {
+			acc0 += x0[j];
+			acc1 += x1[j];
+		}
+	}
+	bb_flush<kFwd>(a, vr, hv, acc0, acc1, pre);
+}
+
+// Chunk c (a.chunk edges of a vertex with more of them) in one level of a
+// sweep: the sums of its edges into its row of partial[].  The warp that
+// completes the last of a vertex's chunks finishes the vertex (no barrier
+// between the chunks and their finish), and leaves the count at 0.
+template <bool kFwd>
+__device__ void bb_chunk(const BbArgs &a, uint32_t L, uint32_t w, bool has_nb, uint32_t c, BbCount &cnt) {
+	using D = BbDir<kFwd>;
+	using T = typename D::T;
+	const unsigned lane = lane_id();
+	const uint64_t *nb = bb_plane(a, kFwd ? L - 1 : L + 1, w);
 	const uint32_t *off = D::off(a), *adj = D::adj(a), *cb = D::chunk_beg(a);
-	const uint32_t beg = __ldg(cb + c), end = min(beg + kBbChunk, __ldg(off + v + 1));
+	const uint32_t v = __ldg(D::chunk_v(a) + c), rw = w * a.n;
+	const uint64_t hv = bb_word(bb_plane(a, L, w), a, v);
+	const uint32_t beg = __ldg(cb + c), vbeg = __ldg(off + v), vend = __ldg(off + v + 1);
+	const uint32_t end = min(beg + a.chunk, vend);
 	T acc[4] = {T(0), T(0), T(0), T(0)};
 	for (uint32_t e0 = beg; has_nb && e0 < end; e0 += 32) {
 		const uint32_t e = e0 + lane;
@@ -377,6 +413,7 @@ __device__ void bb_chunk(const BbArgs &a, uint32_t L, bool has_nb, uint32_t c, u
 		if (e < end) {
 			u = __ldg(adj + e);
 			m = hv & bb_word(nb, a, u);
+			u += rw;
 		}
 		uint32_t bal = __ballot_sync(kFull, m != 0ull);
 		if (lane == 0) {
@@ -406,68 +443,39 @@ __device__ void bb_chunk(const BbArgs &a, uint32_t L, bool has_nb, uint32_t c, u
 #pragma unroll
 	for (int i = 0; i < 4; ++i) acc[i] += __shfl_xor_sync(kFull, acc[i], 16);
 	const uint32_t bits = (uint32_t) (hv >> bb_quad()) & 0xFu;
+	const size_t crow = (size_t) w * D::nchunks(a) + c;
 	if (lane < 16u && bits) {
-		const size_t row = (size_t) c * 64 + bb_quad();
 #pragma unroll
 		for (int i = 0; i < 4; ++i)
-			if ((bits >> i) & 1u) a.partial[row + i] = D::to_bits(acc[i]);
+			if ((bits >> i) & 1u) a.partial[crow * 64 + bb_quad() + i] = D::to_bits(acc[i]);
 	}
+	const uint32_t k = (vend - vbeg + a.chunk - 1) / a.chunk, c0 = c - (beg - vbeg) / a.chunk;
+	unsigned *done = a.chunks_done + (size_t) w * D::nchunks(a) + c0;
+	__syncwarp();
+	uint32_t before = 0;
+	// releases the warp's row to, and acquires the other warps' rows from, the others that count here
+	if (lane == 0)
+		asm volatile("atom.acq_rel.gpu.global.add.u32 %0, [%1], 1;" : "=r"(before) : "l"(done) : "memory");
+	before = __shfl_sync(kFull, before, 0);
+	if (before != k - 1) return;
+	__syncwarp();
+	bb_finish<kFwd>(a, w, v, hv, c0, k);
+	if (lane == 0) *done = 0u;
 }
 
-// After the chunk sums of a level: each chunked vertex of that level adds its
-// chunks' partial rows in chunk order (by the warp that meets its first chunk
-// in the level's list).
-template <bool kFwd>
-__device__ void bb_finish(const BbArgs &a, uint32_t L) {
-	using D = BbDir<kFwd>;
-	using T = typename D::T;
-	const uint32_t ncl = ld_volatile(kFwd ? &a.ctl->ni_at[L] : &a.ctl->no_at[L]);
-	const uint32_t *clist = (kFwd ? a.ilist : a.olist) + (size_t) L * D::nchunks(a);
-	const unsigned lane = lane_id();
-	const uint64_t *own = bb_plane(a, L);
-	const uint32_t *off = D::off(a), *cv = D::chunk_v(a), *cb = D::chunk_beg(a);
-	const uint32_t gwarp = blockIdx.x * kBbWarps + warp_id(), nwarps = gridDim.x * kBbWarps;
-	for (uint32_t i = gwarp; i < ncl; i += nwarps) {
-		const uint32_t c = __ldcg(clist + i);
-		const uint32_t v = __ldg(cv + c);
-		const uint32_t b0 = __ldg(off + v);
-		if (__ldg(cb + c) != b0) continue;
-		const uint64_t hv = bb_word(own, a, v);
-		const uint32_t k = (__ldg(off + v + 1) - b0 + kBbChunk - 1) / kBbChunk;
-		const bool w0 = (hv >> lane) & 1ull, w1 = (hv >> (lane + 32)) & 1ull;
-		T acc0 = T(0), acc1 = T(0);
-		for (uint32_t i2 = 0; i2 < k; i2 += kBbUnroll) {
-			T x0[kBbUnroll], x1[kBbUnroll];
-#pragma unroll
-			for (int j = 0; j < kBbUnroll; ++j) {
-				const bool in = i2 + j < k;
-				const size_t row = (size_t) (c + i2 + j) * 64;
-				x0[j] = in && w0 ? D::from_bits(ld_cg(a.partial + row + lane)) : T(0);
-				x1[j] = in && w1 ? D::from_bits(ld_cg(a.partial + row + lane + 32)) : T(0);
-			}
-#pragma unroll
-			for (int j = 0; j < kBbUnroll; ++j) {
-				acc0 += x0[j];
-				acc1 += x1[j];
-			}
-		}
-		bb_flush<kFwd>(a, v, hv, acc0, acc1, bb_pre<kFwd>(a, v, hv));
-	}
-}
-
-// Lists, per level, of the blocks of 32 vertices and of the edge chunks
-// that have a vertex at that level, so that a level's work is only its own
-// (the planes are final once the traversal has ended).  A warp takes 32
-// consecutive blocks (lane j: block j) or 32 chunks; one atomic per warp and
-// level places them.
+// Lists, per level and word, of the blocks of 32 vertices and of the edge
+// chunks that have a vertex at that level, so that a level's work is only its
+// own (the planes are final once the traversal has ended).  A warp takes 32
+// consecutive blocks (lane j: block j) or 32 chunks of one word; one atomic
+// per warp and level places them.
 __device__ void bb_lists(const BbArgs &a, uint32_t depth) {
-	BbControl *ctl = a.ctl;
 	const unsigned lane = lane_id();
 	const uint32_t gwarp = blockIdx.x * kBbWarps + warp_id(), nwarps = gridDim.x * kBbWarps;
-	const uint32_t nblk = (a.n + 31) / 32;
-	for (uint32_t wb = gwarp; wb * 32 < nblk; wb += nwarps) {
+	const uint32_t nblk = (a.n + 31) / 32, nwb = (nblk + 31) / 32;
+	for (uint32_t t = gwarp; t < nwb * a.words; t += nwarps) {
+		const uint32_t w = t / nwb, wb = t % nwb;
 		for (uint32_t L = 0; L < depth; ++L) {
-			const uint64_t *pl = bb_plane(a, L);
+			const uint64_t *pl = bb_plane(a, L, w);
 			uint32_t act = 0;
 #pragma unroll 8
 			for (uint32_t j = 0; j < 32; ++j) {
@@ -477,68 +485,84 @@ __device__ void bb_lists(const BbArgs &a, uint32_t depth) {
 			}
 			if (!act) continue;
 			uint32_t base = 0;
-			if (lane == 0) base = atomicAdd(&ctl->nb_at[L], (unsigned) __popc(act));
+			if (lane == 0) base = atomicAdd(&a.ctl[w].nb_at[L], (unsigned) __popc(act));
 			base = __shfl_sync(kFull, base, 0);
-			if ((act >> lane) & 1u) a.blist[(size_t) L * nblk + base + __popc(act & lanemask_lt())] = wb * 32 + lane;
+			if ((act >> lane) & 1u)
+				a.blist[((size_t) w * a.planes + L) * nblk + base + __popc(act & lanemask_lt())] = wb * 32 + lane;
 		}
 	}
 	for (int dir = 0; dir < 2; ++dir) {
-		const uint32_t nch = dir ? a.noch : a.nich;
+		const uint32_t nch = dir ? a.noch : a.nich, ncg = (nch + 31) / 32;
 		const uint32_t *cv = dir ? a.ochunk_v : a.ichunk_v;
 		uint32_t *list = dir ? a.olist : a.ilist;
-		unsigned *cnt = dir ? ctl->no_at : ctl->ni_at;
-		for (uint32_t c0 = gwarp * 32; c0 < nch; c0 += nwarps * 32) {
-			const uint32_t c = c0 + lane;
+		for (uint32_t t = gwarp; t < ncg * a.words; t += nwarps) {
+			const uint32_t w = t / ncg, c = (t % ncg) * 32 + lane;
 			const uint32_t v = c < nch ? __ldg(cv + c) : 0u;
+			if (c < nch) a.chunks_done[(size_t) w * nch + c] = 0u;
 			for (uint32_t L = 0; L < depth; ++L) {
-				const bool at = c < nch && bb_word(bb_plane(a, L), a, v) != 0ull;
+				const bool at = c < nch && bb_word(bb_plane(a, L, w), a, v) != 0ull;
 				const uint32_t m = __ballot_sync(kFull, at);
 				if (!m) continue;
+				unsigned *cnt = (dir ? a.ctl[w].no_at : a.ctl[w].ni_at) + L;
 				uint32_t base = 0;
-				if (lane == 0) base = atomicAdd(cnt + L, (unsigned) __popc(m));
+				if (lane == 0) base = atomicAdd(cnt, (unsigned) __popc(m));
 				base = __shfl_sync(kFull, base, 0);
-				if (at) list[(size_t) L * nch + base + __popc(m & lanemask_lt())] = c;
+				if (at) list[((size_t) w * a.planes + L) * nch + base + __popc(m & lanemask_lt())] = c;
 			}
 		}
 	}
 }
 
-// One level of a sweep: the level's chunks, then its blocks of 32 vertices,
-// from the level's lists, handed out one at a time through a counter (the
-// cost of a block varies with the edges of its vertices that serve a source;
-// a fixed deal left warps waiting at the level's barrier).  The next item is
-// claimed while the current one runs.
+// One level of a sweep: the level's chunks, then its blocks of 32 vertices (or
+// their parts), of every word of the launch, from the level's lists, handed
+// out one at a time through a counter (the cost of a block varies with the
+// edges of its vertices that serve a source; a fixed deal left warps waiting
+// at the level's barrier).  The next item is claimed while the current one runs.
 template <bool kFwd>
-__device__ void bb_level(const BbArgs &a, uint32_t L, bool has_nb, unsigned *counter, BbCount &cnt) {
+__device__ void bb_level(const BbArgs &a, uint32_t L, bool has_nb, unsigned *counter,
+		unsigned long long *counts) {
 	using D = BbDir<kFwd>;
+	__shared__ uint32_t s_nc[kBbMaxWords], s_nb[kBbMaxWords];
 	const uint32_t nblk = (a.n + 31) / 32;
-	const uint32_t ncl = ld_volatile(kFwd ? &a.ctl->ni_at[L] : &a.ctl->no_at[L]);
-	const uint32_t nbl = ld_volatile(&a.ctl->nb_at[L]);
+	__syncthreads();
+	if (threadIdx.x < a.words) {
+		const BbControl *ctl = a.ctl + threadIdx.x;
+		s_nc[threadIdx.x] = ld_volatile(kFwd ? &ctl->ni_at[L] : &ctl->no_at[L]);
+		s_nb[threadIdx.x] = ld_volatile(&ctl->nb_at[L]) * a.split;
+	}
+	__syncthreads();
 	const uint32_t *clist = (kFwd ? a.ilist : a.olist) + (size_t) L * D::nchunks(a);
 	const uint32_t *blist = a.blist + (size_t) L * nblk;
-	const uint32_t items = ncl + nbl;
+	uint32_t ncl = 0, items = 0;
+	for (uint32_t w = 0; w < a.words; ++w) {
+		ncl += s_nc[w];
+		items += s_nc[w] + s_nb[w];
+	}
 	const unsigned lane = lane_id();
+	BbCount cnt{0, 0, 0};
 	uint32_t item = lane == 0 ? atomicAdd(counter, 1u) : 0u;
 	item = __shfl_sync(kFull, item, 0);
-	while (item < items) {
+	// two loops, so that neither keeps the other's loop invariants in registers
+	while (item < ncl) {
 		const uint32_t next = lane == 0 ? atomicAdd(counter, 1u) : 0u;
-		if (item < ncl) {
-			const uint32_t c = __ldcg(clist + item);
-			const uint32_t v = __ldg(D::chunk_v(a) + c);
-			bb_chunk<kFwd>(a, L, has_nb, c, v, bb_word(bb_plane(a, L), a, v), cnt);
-		} else {
-			bb_block<kFwd>(a, L, has_nb, __ldcg(blist + (item - ncl)), cnt);
-		}
+		uint32_t w = 0;
+		for (; item >= s_nc[w]; ++w) item -= s_nc[w];
+		bb_chunk<kFwd>(a, L, w, has_nb, __ldcg(clist + (size_t) w * a.planes * D::nchunks(a) + item), cnt);
 		item = __shfl_sync(kFull, next, 0);
 	}
-}
-
-__device__ __forceinline__ void bb_add_counts(unsigned long long *dst, const BbCount &c) {
-	const unsigned long long served = warp_sum(c.served);
-	if (lane_id() == 0) {
-		if (c.edges) atomicAdd(dst, c.edges);
-		if (c.matched) atomicAdd(dst + 1, c.matched);
-		if (served) atomicAdd(dst + 2, served);
+	while (item < items) {
+		const uint32_t next = lane == 0 ? atomicAdd(counter, 1u) : 0u;
+		uint32_t w = 0;
+		for (item -= ncl; item >= s_nb[w]; ++w) item -= s_nb[w];
+		const uint32_t per = 32 / a.split, lo = (item % a.split) * per;
+		bb_block<kFwd>(a, L, w, has_nb, __ldcg(blist + (size_t) w * a.planes * nblk + item / a.split), lo, lo + per, cnt);
+		item = __shfl_sync(kFull, next, 0);
+	}
+	const unsigned long long served = warp_sum((unsigned long long) cnt.served);
+	if (lane == 0 && cnt.edges) {
+		atomicAdd(counts, (unsigned long long) cnt.edges);
+		atomicAdd(counts + 1, (unsigned long long) cnt.matched);
+		atomicAdd(counts + 2, served);
 	}
 }
 
@@ -561,105 +585,110 @@ __global__ void __launch_bounds__(kBbThreads, 2) k_bc_batch(BbArgs a) {
 	if (leader) ctl->depth = depth;
 	unsigned epoch = 0;
 	const uint32_t t0 = blockIdx.x * blockDim.x + threadIdx.x, stride = gridDim.x * blockDim.x;
-	for (uint32_t v = t0; v < a.n; v += stride) {
-		uint64_t h = bb_word(bb_plane(a, 0), a, v);
+	for (uint32_t r = t0; r < a.n * a.words; r += stride) {
+		uint64_t h = bb_word(bb_plane(a, 0, r / a.n), a, r % a.n);
 		while (h) {
-			a.sigma[(size_t) v * 64 + (__ffsll((long long) h) - 1)] = 1u;
+			a.sigma[(size_t) r * 64 + (__ffsll((long long) h) - 1)] = 1u;
 			h &= h - 1ull;
 		}
 	}
 	bb_lists(a, depth);
 	bool ok = grid_sync(ctl->bar, epoch, &ctl->err, a.wait_limit_ns, a.hold_barrier);
 	if (leader) ctl->t_fwd[0] = global_timer_ns();
-	BbCount cf{0, 0, 0}, cr{0, 0, 0};
+	__shared__ unsigned long long s_counts[2][3];  // this CTA's, per sweep
+	if (threadIdx.x < 6) s_counts[threadIdx.x / 3][threadIdx.x % 3] = 0;
 	for (uint32_t L = 1; ok && L < depth; ++L) {
-		bb_level<true>(a, L, true, &ctl->work[0][L], cf);
-		if (ld_volatile(&ctl->ni_at[L])) {
-			if (!(ok = grid_sync(ctl->bar, epoch, &ctl->err, a.wait_limit_ns, a.hold_barrier))) break;
-			bb_finish<true>(a, L);
-		}
+		bb_level<true>(a, L, true, &ctl->work[0][L], s_counts[0]);
 		ok = grid_sync(ctl->bar, epoch, &ctl->err, a.wait_limit_ns, a.hold_barrier);
 		if (leader && L < kBbTraceLevels) ctl->t_fwd[L] = global_timer_ns();
 	}
 	if (leader) ctl->t[1] = global_timer_ns();
 	for (int L = (int) depth - 1; ok && L >= 0; --L) {
 		const bool has_nb = (uint32_t) L + 1 < depth;
-		bb_level<false>(a, (uint32_t) L, has_nb, &ctl->work[1][L], cr);
-		if (ld_volatile(&ctl->no_at[L])) {
-			if (!(ok = grid_sync(ctl->bar, epoch, &ctl->err, a.wait_limit_ns, a.hold_barrier))) break;
-			bb_finish<false>(a, (uint32_t) L);
-		}
+		bb_level<false>(a, (uint32_t) L, has_nb, &ctl->work[1][L], s_counts[1]);
 		if (L > 0) ok = grid_sync(ctl->bar, epoch, &ctl->err, a.wait_limit_ns, a.hold_barrier);
 		if (leader && (uint32_t) L < kBbTraceLevels) ctl->t_rev[L] = global_timer_ns();
 	}
 	if (leader) ctl->t[2] = global_timer_ns();
-	bb_add_counts(ctl->fwd, cf);
-	bb_add_counts(ctl->rev, cr);
+	__syncthreads();
+	if (threadIdx.x < 6) atomicAdd((threadIdx.x < 3 ? ctl->fwd : ctl->rev) + threadIdx.x % 3, s_counts[threadIdx.x / 3][threadIdx.x % 3]);
 }
 
 // Output pass: [v][64] rows -> dependencies and path counts [source][v]
 // (0 for unreached pairs) and/or acc[v] += dependencies of the sources != v,
-// in source order; counts the vertices each source reached.
+// in source order (a tile's words one after the other); counts the vertices
+// each source reached.
 __global__ void __launch_bounds__(kBbOutThreads) k_bc_batch_out(BbArgs a, BbOut o) {
 	if (*(const volatile int *) &a.ctl->err) return;
 	__shared__ float sd[kBbOutV][kBbMaxSources + 1];
 	__shared__ uint32_t sp[kBbOutV][kBbMaxSources + 1];
 	__shared__ uint64_t svis[kBbOutV];
-	__shared__ uint32_t ssrc[kBbMaxSources];
-	const uint32_t t = threadIdx.x, ns = a.ns;
-	if (t < kBbMaxSources) ssrc[t] = t < ns ? o.sources[t] : 0xFFFFFFFFu;
-	const uint64_t smask = ns >= 64 ? ~0ull : (1ull << ns) - 1ull;
-	uint32_t reached = 0;  // threads 64..127: vertices reached from source t - 64
+	__shared__ uint32_t ssrc[kBbMaxWords * kBbMaxSources];
+	__shared__ uint32_t sreached[kBbMaxWords * kBbMaxSources];
+	const uint32_t t = threadIdx.x;
+	static_assert(kBbOutThreads >= kBbMaxWords * kBbMaxSources, "a thread per source");
+	if (t < kBbMaxWords * kBbMaxSources) {
+		ssrc[t] = t < a.ns ? o.sources[t] : 0xFFFFFFFFu;
+		sreached[t] = 0;
+	}
 	for (uint32_t v0 = blockIdx.x * kBbOutV; v0 < a.n; v0 += gridDim.x * kBbOutV) {
 		const uint32_t nv = min(kBbOutV, a.n - v0);
-		__syncthreads();
-		if (t < nv) svis[t] = bb_ldg64(a.vis + (size_t) (v0 + t) * a.K + a.word) & smask;
-		__syncthreads();
-		// 16-byte loads: 4 sources of a row per thread (streamed, not kept in L2)
-		for (uint32_t i = t; i < nv * 16; i += blockDim.x) {
-			const uint32_t j = i / 16, s0 = 4 * (i % 16);
-			const uint32_t r = (uint32_t) (svis[j] >> s0) & 0xFu;
-			uint4 sg4 = make_uint4(0u, 0u, 0u, 0u), dv4 = make_uint4(0u, 0u, 0u, 0u);
-			if (r) {
-				const size_t x = (size_t) (v0 + j) * 64 + s0;
-				sg4 = __ldcs(reinterpret_cast<const uint4 *>(a.sigma + x));
-				dv4 = __ldcs(reinterpret_cast<const uint4 *>(a.dsum + x));
-			}
-			const uint32_t sg[4] = {sg4.x, sg4.y, sg4.z, sg4.w}, dv[4] = {dv4.x, dv4.y, dv4.z, dv4.w};
+		for (uint32_t w = 0; w < a.words; ++w) {
+			const uint32_t s_base = w * kBbMaxSources, ns = min(kBbMaxSources, a.ns - s_base);
+			const uint64_t smask = ns >= 64 ? ~0ull : (1ull << ns) - 1ull;
+			__syncthreads();
+			if (t < nv) svis[t] = bb_ldg64(a.vis + (size_t) (v0 + t) * a.K + a.word + w) & smask;
+			__syncthreads();
+			// 16-byte loads: 4 sources of a row per thread (streamed, not kept in L2)
+			for (uint32_t i = t; i < nv * 16; i += blockDim.x) {
+				const uint32_t j = i / 16, s0 = 4 * (i % 16);
+				const uint32_t r = (uint32_t) (svis[j] >> s0) & 0xFu;
+				uint4 sg4 = make_uint4(0u, 0u, 0u, 0u), dv4 = make_uint4(0u, 0u, 0u, 0u);
+				if (r) {
+					const size_t x = ((size_t) w * a.n + v0 + j) * 64 + s0;
+					sg4 = __ldcs(reinterpret_cast<const uint4 *>(a.sigma + x));
+					dv4 = __ldcs(reinterpret_cast<const uint4 *>(a.dsum + x));
+				}
+				const uint32_t sg[4] = {sg4.x, sg4.y, sg4.z, sg4.w}, dv[4] = {dv4.x, dv4.y, dv4.z, dv4.w};
 #pragma unroll
-			for (int k = 0; k < 4; ++k) {
-				const uint32_t g = ((r >> k) & 1u) ? sg[k] : 0u;
-				const float inv = g ? 1.0f / (float) (int) g : 0.0f;
-				sd[j][s0 + k] = inv != 0.0f ? (__uint_as_float(dv[k]) - inv) / inv : 0.0f;
-				sp[j][s0 + k] = g;
+				for (int k = 0; k < 4; ++k) {
+					const uint32_t g = ((r >> k) & 1u) ? sg[k] : 0u;
+					const float inv = g ? 1.0f / (float) (int) g : 0.0f;
+					sd[j][s0 + k] = inv != 0.0f ? (__uint_as_float(dv[k]) - inv) / inv : 0.0f;
+					sp[j][s0 + k] = g;
+				}
+			}
+			__syncthreads();
+			if (o.delta || o.paths)
+				for (uint32_t i = t; i < ns * kBbOutV; i += blockDim.x) {
+					const uint32_t s = i / kBbOutV, j = i % kBbOutV;
+					if (j >= nv) continue;
+					const size_t x = (size_t) (s_base + s) * a.n + v0 + j;
+					if (o.delta) __stcs(o.delta + x, sd[j][s]);
+					if (o.paths) __stcs(o.paths + x, sp[j][s]);
+				}
+			if (o.acc && t < nv) {
+				const uint32_t v = v0 + t;
+				float x = o.acc[v];
+				for (uint32_t s = 0; s < ns; ++s)
+					if (ssrc[s_base + s] != v) x += sd[t][s];
+				o.acc[v] = x;
+			}
+			if (t >= 64 && t < 64 + ns) {
+				uint32_t reached = 0;
+				for (uint32_t j = 0; j < nv; ++j) reached += (uint32_t) ((svis[j] >> (t - 64)) & 1ull);
+				sreached[s_base + t - 64] += reached;
 			}
 		}
-		__syncthreads();
-		if (o.delta || o.paths)
-			for (uint32_t i = t; i < ns * kBbOutV; i += blockDim.x) {
-				const uint32_t s = i / kBbOutV, j = i % kBbOutV;
-				if (j >= nv) continue;
-				const size_t x = (size_t) s * a.n + v0 + j;
-				if (o.delta) __stcs(o.delta + x, sd[j][s]);
-				if (o.paths) __stcs(o.paths + x, sp[j][s]);
-			}
-		if (o.acc && t < nv) {
-			const uint32_t v = v0 + t;
-			float x = o.acc[v];
-			for (uint32_t s = 0; s < ns; ++s)
-				if (ssrc[s] != v) x += sd[t][s];
-			o.acc[v] = x;
-		}
-		if (t >= 64 && t < 64 + ns)
-			for (uint32_t j = 0; j < nv; ++j) reached += (uint32_t) ((svis[j] >> (t - 64)) & 1ull);
 	}
-	if (t >= 64 && t < 64 + ns && reached) atomicAdd(&a.ctl->reached[t - 64], reached);
+	__syncthreads();
+	if (t < a.ns && sreached[t]) atomicAdd(&a.ctl[t / kBbMaxSources].reached[t % kBbMaxSources], sreached[t]);
 }
 
 } // namespace
 
 int bb_launch(const BbArgs &a, const BbOut &o, int num_sms, cudaStream_t st, int *grid, cudaEvent_t between) {
-	if (a.ns == 0 || a.ns > kBbMaxSources) return BFS_EARG;
+	if (a.words == 0 || a.words > kBbMaxWords || a.ns == 0 || a.ns > a.words * kBbMaxSources) return BFS_EARG;
 	int per_sm = 0;
 	if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_bc_batch, kBbThreads, 0) != cudaSuccess || per_sm < 1)
 		return BFS_ECUDA;
@@ -667,7 +696,7 @@ int bb_launch(const BbArgs &a, const BbOut &o, int num_sms, cudaStream_t st, int
 	if (a.ctas_per_sm) per_sm = std::min(per_sm, (int) a.ctas_per_sm);
 	const int g = num_sms * per_sm;
 	if (grid) *grid = g;
-	if (cudaMemsetAsync(a.ctl, 0, sizeof(BbControl), st) != cudaSuccess) return BFS_ECUDA;
+	if (cudaMemsetAsync(a.ctl, 0, a.words * sizeof(BbControl), st) != cudaSuccess) return BFS_ECUDA;
 	BbArgs aa = a;
 	void *args[] = {&aa};
 	if (cudaLaunchCooperativeKernel((const void *) k_bc_batch, dim3(g), dim3(kBbThreads), args, 0, st) != cudaSuccess)

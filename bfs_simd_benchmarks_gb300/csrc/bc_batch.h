@@ -1,5 +1,5 @@
 // bc_batch.h -- betweenness dependencies of many sources at once (64 per
-// launch, up to 4 launches per call), on the bit-sliced batched traversal
+// word, up to 4 words per call, together or one launch each), on the bit-sliced batched traversal
 // (internal).
 #pragma once
 
@@ -10,10 +10,8 @@
 
 namespace bfsg {
 
-constexpr uint32_t kBbMaxSources = 64;       // sources per launch: one 64-bit word of the traversal
-constexpr uint32_t kBbMaxWords = 4;          // words per call (BFS_BC_BATCH_MAX_SOURCES = 256 sources)
-constexpr uint32_t kBbBig = kMsPullBig;      // degree above which a vertex's edges are summed in chunks ...
-constexpr uint32_t kBbChunk = kMsChunk;      // ... of this many edges (the batched pull's in-edge chunks)
+constexpr uint32_t kBbMaxSources = 64;       // sources per 64-bit word of the traversal
+constexpr uint32_t kBbMaxWords = 4;          // words per call and per launch (BFS_BC_BATCH_MAX_SOURCES = 256 sources)
 constexpr uint32_t kBbTraceLevels = 64;      // per-level timers kept for the first levels
 
 struct BbControl {
@@ -35,26 +33,29 @@ struct BbControl {
 };
 
 struct BbArgs {
-	uint32_t n, ns;                    // ns: sources of this launch's word (1..64)
-	uint32_t K, word;                  // the traversal's words per vertex; the word this launch takes
+	uint32_t n, ns;                    // ns: sources of this launch's words (64 each, the last one 1..64)
+	uint32_t K, word, words;           // the traversal's words per vertex; the first one this launch takes, how many
+	uint32_t chunk;                    // a vertex with more edges than this is summed in chunks of as many
+	uint32_t split;                    // list items per block of 32 vertices (1, 2, 4 ...)
 	const uint32_t *row_off, *col;     // CSR
 	const uint32_t *in_off, *in_src;   // in-edge lists
 	const uint64_t *hist;              // [planes][n][K]: sources that reached v first at level L
 	const uint64_t *vis;               // [n][K] sources that reached v
 	const MsControl *ms;               // the traversal's control block (depth, completion, status)
-	const uint32_t *ichunk_v, *ichunk_beg;  // in-edge chunks of vertices with in-degree > kBbBig
+	const uint32_t *ichunk_v, *ichunk_beg;  // in-edge chunks of vertices with in-degree > chunk
 	uint32_t nich;
-	const uint32_t *ochunk_v, *ochunk_beg;  // out-edge chunks of vertices with out-degree > kBbBig
+	const uint32_t *ochunk_v, *ochunk_beg;  // out-edge chunks of vertices with out-degree > chunk
 	uint32_t noch;
-	uint32_t *sigma;                   // [n][64] path counts (mod 2^32)
-	float *dsum;                       // [n][64] 1/sigma + the dependency sums of the next level
-	uint32_t *partial;                 // [max(nich, noch)][64] chunk sums (value bits)
-	// per level L < planes, built at the start of the launch (any order):
-	uint32_t *blist;                   // [planes][ceil(n / 32)] blocks of 32 vertices with a vertex at level L
-	uint32_t *ilist;                   // [planes][nich] in-edge chunks of vertices at level L
-	uint32_t *olist;                   // [planes][noch] out-edge chunks of vertices at level L
+	uint32_t *sigma;                   // [words][n][64] path counts (mod 2^32)
+	float *dsum;                       // [words][n][64] 1/sigma + the dependency sums of the next level
+	uint32_t *partial;                 // [words][max(nich, noch)][64] chunk sums (value bits)
+	unsigned *chunks_done;             // [words][max(nich, noch)] at a vertex's first chunk: its chunks summed so far
+	// per word and level L < planes, built at the start of the launch (any order):
+	uint32_t *blist;                   // [words][planes][ceil(n / 32)] blocks of 32 vertices with a vertex at level L
+	uint32_t *ilist;                   // [words][planes][nich] in-edge chunks of vertices at level L
+	uint32_t *olist;                   // [words][planes][noch] out-edge chunks of vertices at level L
 	uint32_t planes;                   // levels the lists have room for
-	BbControl *ctl;
+	BbControl *ctl;                    // [words]; barrier, status, timers and work counters in the first
 	unsigned long long wait_limit_ns;  // bound of every grid-barrier wait
 	uint32_t hold_barrier;             // tests: CTA 0 skips its arrival at this barrier (0 = off)
 	uint32_t ctas_per_sm;              // 0 = as many as fit (at most 2)
@@ -68,8 +69,9 @@ struct BbOut {
 };
 
 // Enqueues, after the batched traversal that filled a.hist / a.vis / a.ms,
-// the cooperative path-count and dependency launch for the sources of word
-// a.word and the output pass; the control block is cleared first.  `between` (may be null) is recorded
+// the cooperative path-count and dependency launch for the sources of words
+// a.word .. a.word + a.words - 1 and the output pass; the control blocks are
+// cleared first.  `between` (may be null) is recorded
 // between the two launches; *grid gets the CTA count.
 int bb_launch(const BbArgs &a, const BbOut &o, int num_sms, cudaStream_t st, int *grid, cudaEvent_t between);
 

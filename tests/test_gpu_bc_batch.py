@@ -219,3 +219,53 @@ def test_bc_batch_arguments(native):
             g.set_options(no_such=1)
         with pytest.raises(N.BfsError):
             g.set_options(bc_batch=2)
+
+
+@pytest.mark.parametrize("degree", [63, 64, 65, 128, 129])
+def test_bc_batch_degrees_at_the_chunk_length(native, oracle, degree):
+    """Two layers of `degree` vertices, all to all, behind a source and in front of a
+    sink, twice with a 40-vertex block between: in- and out-degrees at the edges of
+    a chunk of the sweeps (64 edges on a graph this small), state grown from one
+    word of sources to four and used with fewer again."""
+    import bfs_simd_benchmarks_gb300 as B
+    d = degree
+    a, b = np.arange(1, d + 1), np.arange(d + 1, 2 * d + 1)
+    sink = 2 * d + 1
+    far = sink + 1 + np.arange(40)
+    src = np.concatenate([np.zeros(d), np.repeat(a, d), b, np.full(40, sink), far, far[:7]])
+    dst = np.concatenate([a, np.tile(b, d), np.full(d, sink), far, np.full(40, 0), far[1:8]])
+    n = int(far[-1]) + 1
+    arr = oracle.csr_arrays(n, src.astype(np.uint32), dst.astype(np.uint32))
+    with B.Graph.from_edges(n, src, dst, 64, 4) as g:
+        rng = np.random.default_rng(degree)
+        for k in (1, 65, 200, 5):
+            sources = rng.integers(0, n, size=k).astype(np.uint32)
+            sources[0] = 0
+            dep, sig, st = g.bc_batch(sources)
+            assert st["status"] == 0 and st["batched_sources"] == k
+            _check_rows(oracle, arr, sources, dep, sig, st)
+            total, _ = g.betweenness(sources)
+            want = np.zeros(n)
+            scale = np.zeros(n)
+            for s in sources:
+                _, odep, _, oscale = oracle.bc_single(arr, int(s))
+                odep, oscale = np.array(odep, np.float64), np.array(oscale, np.float64)
+                odep[s] = oscale[s] = 0
+                want += odep
+                scale += np.abs(oscale) + 1
+            assert bc_close(total, want, scale).all()
+
+
+@pytest.mark.parametrize("m", [1 << 21, (1 << 21) + 1, 1 << 24, (1 << 24) + 1])
+def test_bc_batch_chunk_length_by_edges(native, oracle, m):
+    """The graphs on both sides of the edge counts where the sweeps' chunks grow."""
+    import bfs_simd_benchmarks_gb300 as B
+    n = 1 << 16
+    s, d = B.gen_rmat_device(n, m, seed=5, dedup=False)
+    src, dst = s.cpu().numpy().astype(np.uint32), d.cpu().numpy().astype(np.uint32)
+    arr = oracle.csr_arrays(n, src, dst)
+    with B.Graph.from_edges(n, src, dst, 256, 4, device_build=True) as g:
+        sources = B.pick_sources(g.degrees(), 3, seed=11).astype(np.uint32)
+        dep, sig, st = g.bc_batch(sources)
+        assert st["status"] == 0 and st["batched_sources"] == 3
+        _check_rows(oracle, arr, sources, dep, sig, st)
