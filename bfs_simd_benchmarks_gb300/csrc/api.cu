@@ -867,7 +867,7 @@ int batch_prepare(bfs_graph *g, uint32_t K, uint32_t *planes_out) {
 	if (b.have_run && cudaEventSynchronize(b.e1) != cudaSuccess) return BFS_ECUDA;
 	release_batch(g);
 	const size_t fixed = (size_t) g->n * K * 8 + (size_t) g->n * (2 + 4 + 8) + sizeof(MsControl) +
-			4 * BFS_BATCH_MAX_SOURCES;
+			4 * BFS_BATCH_MAX_SOURCES + 4 * (size_t) g->ms_nchunks + (size_t) g->ms_nbig_in * (4 + 8 * (size_t) K);
 	size_t free_b = 0, total_b = 0;
 	if (cudaMemGetInfo(&free_b, &total_b) != cudaSuccess) return BFS_ECUDA;
 	const size_t usable = free_b > (size_t) 1 << 30 ? free_b - ((size_t) 1 << 30) : 0;  // leave 1 GiB
@@ -881,9 +881,13 @@ int batch_prepare(bfs_graph *g, uint32_t K, uint32_t *planes_out) {
 	if ((st = batch_alloc(g, &a.vis, (size_t) g->n * K))) return st;
 	if ((st = batch_alloc(g, &a.hist, (size_t) planes * g->n * K))) return st;
 	if ((st = batch_alloc(g, &a.pmask, (size_t) planes * g->n))) return st;
-	if ((st = batch_alloc(g, &a.touched, g->n))) return st;
+	if ((st = batch_alloc(g, &a.touched, (g->n + 3) & ~size_t(3)))) return st;  // claimed in 32-bit words
 	if ((st = batch_alloc(g, &a.done, g->n))) return st;
 	if ((st = batch_alloc(g, &a.seed_flag, g->n))) return st;
+	if ((st = batch_alloc(g, &a.chunk_slot, g->ms_nchunks)) || (st = batch_alloc(g, &a.big_cnt, g->ms_nbig_in)) ||
+			(st = batch_alloc(g, &a.big_acc, (size_t) g->ms_nbig_in * K)) ||
+			(st = ms_chunk_slots(g->ms_chunk_v, g->ms_nchunks, g->ms_in_big, g->ms_nbig_in, a.chunk_slot)))
+		return st;
 	if ((st = batch_alloc(g, &a.queue[0], g->n))) return st;
 	if ((st = batch_alloc(g, &a.queue[1], g->n))) return st;
 	if ((st = batch_alloc(g, &a.ctl, 1))) return st;

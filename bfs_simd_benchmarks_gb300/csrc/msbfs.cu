@@ -17,11 +17,16 @@
 //     frontier vertex, loads its K words once and ORs the non-zero ones into
 //     every out-neighbour's next words (64-bit atomics); a high-degree vertex
 //     has its edges spread over every warp of the grid; or
-//   - pull (bottom-up) once it holds many: a warp owns a destination, gathers
-//     the non-zero words of its frontier in-neighbours that the destination
-//     still lacks and stops as soon as every source has reached it
-//     (per-destination early exit); destinations with many in-edges are cut
-//     into chunks that warps all over the grid gather and OR together.
+//   - pull (bottom-up) once it holds many: destinations gather the words of
+//     their frontier in-neighbours and stop as soon as every source that has a
+//     frontier has reached them (per-destination early exit).  Up to
+//     kMsRowWords words per vertex a lane (or 8 lanes) takes a destination and
+//     reads whole rows; with more, a warp takes one and reads the non-zero
+//     words it still lacks.  Destinations with many in-edges are cut into
+//     chunks that warps all over the grid gather and OR together; the last one
+//     finishes the destination, so that a pull level has one grid barrier.
+//     (R-MAT scale 22, 4096 sources: the level with the most gathers 7.8 ->
+//     6.1 ms; Pokec shape, 64 sources: 0.54 -> 0.26 ms.)
 // Clearing, seeding, all levels and the edge count run in one cooperative
 // launch, levels separated by a bounded-spin grid barrier; the output pass,
 // its own launch, turns planes into uint8 levels [source][vertex] (255 =
@@ -43,15 +48,15 @@ constexpr int kMsWarps = kMsThreads / 32;
 constexpr uint32_t kMsWq = 64;          // per-warp staged queue appends (pull)
 constexpr uint32_t kMsBig = 1024;       // push: higher-degree vertices are spread over the grid
 constexpr int kMsGather = 4;            // pull: frontier rows gathered per round
-constexpr uint32_t kLaneMaxWords = 2;   // pull: up to this many words per vertex ...
-constexpr uint32_t kLaneMaxDeg = 32;    // ... destinations of at most this in-degree go one per lane
+constexpr uint32_t kLaneMaxDeg = 32;    // pull, few words: destinations of at most this in-degree go one per lane
 constexpr uint32_t kGroupMaxWords = 8;  // pull: up to this many words, in-neighbour rows in lane groups
-constexpr uint32_t kEmitW = 4;          // output tile: kV vertices x 4 words (256 sources), kV = threads / 4
+constexpr uint32_t kEmitW = 4;          // output tile: kV vertices x kW words (4: 256 sources), kV = threads / kW
 // shared bytes of an output tile of kV vertices: rows of one source quad (kV + 4
 // words, 16-byte aligned; `bufs` copies) and the nibble table
-__host__ __device__ constexpr uint32_t emit_bytes(uint32_t kV, uint32_t bufs = 1) {
-	return (bufs * kEmitW * 16 * (kV + 4) + 16) * 4;
+__host__ __device__ constexpr uint32_t emit_bytes(uint32_t kV, uint32_t bufs = 1, uint32_t kW = kEmitW) {
+	return (bufs * kW * 16 * (kV + 4) + 16) * 4;
 }
+constexpr uint32_t kMsRowWords = 4;     // pull: up to this many words per vertex, rows are read whole
 constexpr uint32_t kEmitV = kMsThreads / kEmitW;  // the traversal kernel's tiles (its early output passes)
 constexpr uint32_t kEmitBytes = emit_bytes(kEmitV);
 // The output pass launch: tiles of 64 vertices (256 threads, 4 CTAs per SM)
@@ -303,16 +308,6 @@ __device__ __forceinline__ bool ms_gather(const MsArgs &a, const uint64_t *cur, 
 	return done;
 }
 
-// A bijection of [0, 2^bits): xor-shift, multiply by an odd constant, xor-shift.
-__device__ __forceinline__ uint32_t block_perm(uint32_t x, uint32_t bits) {
-	const uint32_t mask = bits >= 32 ? 0xFFFFFFFFu : (1u << bits) - 1u;
-	const uint32_t h = (bits + 1) / 2;
-	x ^= x >> h;
-	x = (x * 0x9E3779B1u) & mask;
-	x ^= x >> h;
-	return x;
-}
-
 __device__ __forceinline__ uint64_t warp_or64(uint64_t x) {
 #pragma unroll
 	for (int d = 16; d > 0; d >>= 1) x |= shfl_xor64(x, d);
@@ -364,270 +359,385 @@ __device__ __forceinline__ void ms_gather_grouped(const MsArgs &a, const uint64_
 	gathered += loads;
 }
 
-// ms_gather for K <= 2 words per vertex: lanes take in-edges (32 per step)
-// instead of words, read the neighbour's needed non-zero words and OR them
-// across the warp.  Inputs and outputs are word 0 / word 1 in every lane.
-__device__ __forceinline__ void ms_gather_edges(const MsArgs &a, const uint64_t *cur, const uint64_t *actc,
-		uint32_t beg, uint32_t end, uint64_t f0, uint64_t f1, uint64_t vis0, uint64_t vis1, uint64_t &acc0,
-		uint64_t &acc1, unsigned long long &gathered) {
-	const uint32_t K = a.K;
-	const unsigned lane = lane_id();
-	for (uint32_t e0 = beg; e0 < end; e0 += 32) {
-		const bool n0 = ((vis0 | acc0) & f0) != f0, n1 = ((vis1 | acc1) & f1) != f1;
-		if (!n0 && !n1) break;  // uniform: every lane holds the same words
-		const uint32_t e = e0 + lane;
-		const uint32_t u = e < end ? __ldg(a.in_src + e) : 0u;
-		const uint64_t m = e < end ? ld_cg64(actc + u) : 0ull;
-		const bool l0 = n0 && (m & 1ull), l1 = n1 && (m & 2ull);
-		const uint64_t g0 = l0 ? ld_cg64(cur + (size_t) u * K) : 0ull;
-		const uint64_t g1 = l1 ? ld_cg64(cur + (size_t) u * K + 1) : 0ull;
-		gathered += (unsigned long long) l0 + l1;
-		acc0 |= warp_or64(g0);
-		acc1 |= warp_or64(g1);
+// What a pull level works on.
+struct MsPull {
+	const uint64_t *cur, *actc;  // the frontier's plane and word masks
+	uint64_t *nxt, *actn;        // the next level's
+	const unsigned long long *act;  // sources with a frontier at this level (null: every source)
+	MsCounters *cn;
+	uint32_t *qn;                // the next level's queue
+	// a destination without a new word: its row of nxt is not written.  Every
+	// reader of the planes goes by the masks (more than kMsRowWords words per
+	// vertex, and no later pass over the planes that reads them whole).
+	bool masked;
+};
+
+// ---- pull with at most kMsRowWords words per vertex -----------------------
+// A row is one sector at most, so a neighbour's row is read straight away
+// (zero where it is not in the frontier) instead of its mask first and its
+// words then: one round trip less per step.
+
+template <int KK> __device__ __forceinline__ void row_ld(const uint64_t *p, uint64_t (&x)[KK]) {
+	if constexpr (KK % 2 == 0) {
+#pragma unroll
+		for (int k = 0; k < KK; k += 2) {
+			const ulonglong2 t = __ldcg(reinterpret_cast<const ulonglong2 *>(p + k));
+			x[k] = t.x;
+			x[k + 1] = t.y;
+		}
+	} else {
+#pragma unroll
+		for (int k = 0; k < KK; ++k) x[k] = ld_cg64(p + k);
 	}
 }
+// ORs the frontier rows of U in-neighbours, in_src[e + stride * t] below end, into acc.
+template <int KK, int U>
+__device__ __forceinline__ uint32_t rows_or(const MsArgs &a, const uint64_t *cur, uint32_t e, uint32_t stride, uint32_t end,
+		uint64_t (&acc)[KK]) {
+	uint32_t u[U], read = 0;
+#pragma unroll
+	for (int t = 0; t < U; ++t) u[t] = e + stride * t < end ? __ldg(a.in_src + e + stride * t) : 0xFFFFFFFFu;
+	uint64_t x[U][KK];
+#pragma unroll
+	for (int t = 0; t < U; ++t) {
+#pragma unroll
+		for (int k = 0; k < KK; ++k) x[t][k] = 0ull;
+		if (u[t] != 0xFFFFFFFFu) {
+			row_ld<KK>(cur + (size_t) u[t] * KK, x[t]);
+			read += KK;
+		}
+	}
+#pragma unroll
+	for (int t = 0; t < U; ++t)
+#pragma unroll
+		for (int k = 0; k < KK; ++k) acc[k] |= x[t][k];
+	return read;
+}
+template <int KK>
+__device__ __forceinline__ bool row_complete(const uint64_t (&x)[KK], const uint64_t (&y)[KK], const uint64_t (&f)[KK]) {
+	bool r = true;
+#pragma unroll
+	for (int k = 0; k < KK; ++k) r &= ((x[k] | y[k]) & f[k]) == f[k];
+	return r;
+}
 
-// Pull of one destination by one lane (K <= kLaneMaxWords words per vertex,
-// at most kLaneMaxDeg in-edges): the lane walks the in-edges four at a time,
-// reads a neighbour's word only where its mask is set and the destination
-// still lacks sources, and stops when every source has arrived.  Lanes with
-// `mine` false only take part in the warp-wide appends.
-__device__ __forceinline__ void ms_pull_lane(const MsArgs &a, const uint64_t *cur, const uint64_t *actc,
-		uint64_t *nxt, uint64_t *actn, uint32_t v, uint32_t beg, uint32_t end, bool mine, unsigned long long &actdeg,
-		unsigned long long &gathered, MsCounters *cn, uint32_t *qn, uint64_t act0, uint64_t act1, uint64_t &new0,
-		uint64_t &new1) {
-	const uint32_t K = a.K;
-	const uint64_t last = a.last_bits == 64 ? ~0ull : ((1ull << a.last_bits) - 1);
-	const uint64_t f0 = (K == 1 ? last : ~0ull) & act0, f1 = (K == 2 ? last : 0ull) & act1;
-	uint64_t vis0 = 0, vis1 = 0, acc0 = 0, acc1 = 0;
-	bool any = false;
-	uint32_t d = 0;
-	if (mine) {
-		const size_t row = (size_t) v * K;
-		vis0 = ld_cg64(a.vis + row);
-		vis1 = K == 2 ? ld_cg64(a.vis + row + 1) : 0ull;
-		for (uint32_t e = beg; e < end; e += 4) {
-			if (((vis0 | acc0) & f0) == f0 && ((vis1 | acc1) & f1) == f1) break;
-			uint32_t u[4];
-			uint64_t m[4];
+// The 32 destinations from vb (those of at most kMsPullBig in-edges): lanes
+// walk the lists of up to kLaneMaxDeg in-edges, each its own, kRows rows per
+// round trip; then groups of 8 lanes take the longer lists, four destinations
+// at a time, 32 edges of each per round; a list's walk stops when every source
+// that has a frontier has arrived.  All lanes then write their own destination.
+template <int KK>
+__device__ __forceinline__ void ms_pull_rows(const MsArgs &a, const MsPull &p, uint32_t vb, const uint64_t (&f)[KK],
+		uint64_t (&newacc)[KK], unsigned long long &actdeg, unsigned long long &gathered) {
+	constexpr int kRows = KK == 1 ? 8 : 4;
+	const unsigned lane = lane_id();
+	const uint32_t v = vb + lane;
+	const bool valid = v < a.n;
+	const uint32_t beg = valid ? __ldg(a.in_off + v) : 0u, end = valid ? __ldg(a.in_off + v + 1) : 0u;
+	const bool small = valid && end - beg <= kMsPullBig;
+	const bool needy = small && end > beg && !ld_cg_u8(a.done + v);
+	uint64_t vis[KK], acc[KK];
 #pragma unroll
-			for (int t = 0; t < 4; ++t) u[t] = e + t < end ? __ldg(a.in_src + e + t) : 0xFFFFFFFFu;
+	for (int k = 0; k < KK; ++k) vis[k] = acc[k] = 0ull;
+	if (needy) row_ld<KK>(a.vis + (size_t) v * KK, vis);
+	const bool open = needy && !row_complete(vis, acc, f);
+	uint32_t read = 0;
+	if (open && end - beg <= kLaneMaxDeg)
+		for (uint32_t e = beg; e < end && !row_complete(vis, acc, f); e += kRows)
+			read += rows_or<KK, kRows>(a, p.cur, e, 1, end, acc);
+	__syncwarp();
+	for (uint32_t wm = __ballot_sync(kFull, open && end - beg > kLaneMaxDeg); wm;) {
+		int j = -1;
+		uint32_t m = wm;
 #pragma unroll
-			for (int t = 0; t < 4; ++t) m[t] = u[t] != 0xFFFFFFFFu ? ld_cg64(actc + u[t]) : 0ull;
-			const bool n0 = ((vis0 | acc0) & f0) != f0, n1 = ((vis1 | acc1) & f1) != f1;
-			uint64_t g0[4], g1[4];
+		for (uint32_t g = 0; g < 4; ++g) {
+			if (m && lane / 8 == g) j = __ffs(m) - 1;
+			m &= m - 1u;
+		}
+		const uint32_t taken = wm & ~m;
+		wm = m;
+		const int src = j < 0 ? 0 : j;
+		uint64_t gv[KK], ga[KK];
 #pragma unroll
-			for (int t = 0; t < 4; ++t) {
-				const bool l0 = n0 && (m[t] & 1ull), l1 = n1 && (m[t] & 2ull);
-				g0[t] = l0 ? ld_cg64(cur + (size_t) u[t] * K) : 0ull;
-				g1[t] = l1 ? ld_cg64(cur + (size_t) u[t] * K + 1) : 0ull;
-				gathered += (unsigned long long) l0 + l1;
+		for (int k = 0; k < KK; ++k) {
+			gv[k] = shfl64(vis[k], src);
+			ga[k] = 0ull;
+		}
+		uint32_t e = __shfl_sync(kFull, beg, src);
+		const uint32_t ge = __shfl_sync(kFull, end, src);
+		for (bool go = j >= 0; __any_sync(kFull, go);) {
+			if (go) read += rows_or<KK, 4>(a, p.cur, e + (lane & 7u), 8, ge, ga);
+			e += 32;
+#pragma unroll
+			for (int k = 0; k < KK; ++k)
+#pragma unroll
+				for (int d = 4; d > 0; d >>= 1) ga[k] |= shfl_xor64(ga[k], d);
+			go = go && e < ge && !row_complete(gv, ga, f);
+		}
+		// each destination's words from its group to its lane
+		const int from = 8 * (__popc(taken & lanemask_lt()) & 3);
+#pragma unroll
+		for (int k = 0; k < KK; ++k) {
+			const uint64_t x = shfl64(ga[k], from);
+			if ((taken >> lane) & 1u) acc[k] = x;
+		}
+	}
+	gathered += read;
+	uint64_t mask = 0;
+	if (small) {
+		uint64_t w[KK];
+#pragma unroll
+		for (int k = 0; k < KK; ++k) {
+			w[k] = acc[k] & ~vis[k] & f[k];
+			newacc[k] |= w[k];
+			if (w[k]) {
+				mask |= 1ull << k;
+				a.vis[(size_t) v * KK + k] = vis[k] | w[k];
 			}
-#pragma unroll
-			for (int t = 0; t < 4; ++t) { acc0 |= g0[t]; acc1 |= g1[t]; }
+			p.nxt[(size_t) v * KK + k] = w[k];
 		}
-		const uint64_t w0 = acc0 & ~vis0 & f0, w1 = acc1 & ~vis1 & f1;
-		new0 |= w0;
-		new1 |= w1;
-		nxt[row] = w0;
-		if (w0) a.vis[row] = vis0 | w0;
-		if (K == 2) {
-			nxt[row + 1] = w1;
-			if (w1) a.vis[row + 1] = vis1 | w1;
-		}
-		actn[v] = (w0 ? 1ull : 0ull) | (w1 ? 2ull : 0ull);
-		if (((vis0 | w0) & f0) == f0 && ((vis1 | w1) & f1) == f1) a.done[v] = 1;
-		any = (w0 | w1) != 0ull;
-		if (any) {
-			d = deg_of(a, v);
-			actdeg += d;
-		}
+		p.actn[v] = mask;
+		if (needy && row_complete(vis, w, f)) a.done[v] = 1;
 	}
-	ms_append(a, cn, qn, v, any && d <= kMsBig, any && d > kMsBig);
+	const uint32_t d = mask ? deg_of(a, v) : 0u;
+	actdeg += d;
+	ms_append(a, p.cn, p.qn, v, mask && d <= kMsBig, mask && d > kMsBig);
 }
 
-// Pull, destinations with at most kMsPullBig in-edges.  A warp screens 32
-// consecutive destinations at once (their in-edge ranges and "every source
-// has arrived" flags, lane-parallel), clears the rows of those with nothing
-// to do as one contiguous block, then works through the others one at a
-// time: lane l owns words l and l + 32.  The rows of many-in-edge
-// destinations are cleared here and filled by ms_pull_chunks.
-__device__ void ms_pull(const MsArgs &a, uint32_t lvl, const uint64_t *cur, const uint64_t *actc, uint64_t *nxt,
-		uint64_t *actn, unsigned long long &actdeg, unsigned long long &gathered, uint32_t *wq_base,
-		const unsigned long long *act, unsigned long long *s_act) {
-	const uint32_t K = a.K;
-	uint32_t *qn = a.queue[(lvl + 1) & 1];
-	MsCounters *cn = &a.ctl->ctr[(lvl + 1) % 3];
+// A chunk's frontier words for KK words per vertex: OR over its in-edges, in
+// every lane's acc.
+template <int KK>
+__device__ __forceinline__ uint64_t ms_chunk_rows(const MsArgs &a, const uint64_t *cur, uint32_t beg, uint32_t end,
+		unsigned long long &gathered) {
+	constexpr int kRows = KK == 1 ? 8 : 4;
 	const unsigned lane = lane_id();
-	const uint32_t gwarp = blockIdx.x * kMsWarps + warp_id();
-	const uint32_t nwarps = gridDim.x * kMsWarps;
+	uint64_t acc[KK];
+#pragma unroll
+	for (int k = 0; k < KK; ++k) acc[k] = 0ull;
+	uint32_t read = 0;
+	for (uint32_t e = beg + lane; e < end; e += 32 * kRows) read += rows_or<KK, kRows>(a, cur, e, 32, end, acc);
+	__syncwarp();
+	gathered += read;
+	uint64_t mine = 0;
+#pragma unroll
+	for (int k = 0; k < KK; ++k) {
+		const uint64_t x = warp_or64(acc[k]);
+		if (lane == (unsigned) k) mine = x;
+	}
+	return mine;
+}
+
+// ---- pull with more words per vertex --------------------------------------
+// A warp screens 32 consecutive destinations at once (their in-edge ranges and
+// "every source has arrived" flags, lane-parallel), then works through those
+// with something to do one at a time: lane l owns words l and l + 32.
+__device__ __forceinline__ void ms_pull_words(const MsArgs &a, const MsPull &p, uint32_t vb, const FullMask &fm,
+		uint64_t &new0, uint64_t &new1, unsigned long long &actdeg, unsigned long long &gathered, uint32_t *wbuf,
+		uint32_t &wn) {
+	const uint32_t K = a.K;
+	const unsigned lane = lane_id();
 	const bool w0 = lane < K, w1 = lane + 32 < K;
-	const FullMask fm(a, lane, act);
-	const uint64_t lact0 = act ? ld_cg64((const uint64_t *) act) : ~0ull;
-	const uint64_t lact1 = act && K > 1 ? ld_cg64((const uint64_t *) act + 1) : ~0ull;
-	uint64_t new_lane0 = 0, new_lane1 = 0;  // new words lane / lane + 32 (warp-per-destination paths)
-	uint64_t new_w0 = 0, new_w1 = 0;        // new words 0 / 1 (lane-per-destination path)
-	uint32_t *wbuf = wq_base + warp_id() * kMsWq;
-	uint32_t wn = 0;
-	// blocks of 32 destinations in a hashed order: in-degree follows the id
-	// bits of R-MAT-like graphs, so a plain stride gives some warps the heavy
-	// blocks every time
-	const uint32_t nblk = (a.n + 31) / 32;
-	const uint32_t pbits = 32 - __clz(max(nblk - 1, 1u));
-	for (uint32_t i = gwarp; i < (1u << pbits); i += nwarps) {
-		const uint32_t bi = block_perm(i, pbits);
-		if (bi >= nblk) continue;
-		const uint32_t vb = bi * 32;
-		const uint32_t vl = vb + lane;
-		const bool valid = vl < a.n;
-		const uint32_t lbeg = valid ? __ldg(a.in_off + vl) : 0u, lend = valid ? __ldg(a.in_off + vl + 1) : 0u;
-		const bool big = lend - lbeg > kMsPullBig;
-		const bool needy = valid && !big && lend > lbeg && !ld_cg_u8(a.done + vl);
-		const uint32_t needm = __ballot_sync(kFull, needy);
-		if (valid && !needy && !big) actn[vl] = 0;
-		// rows of the block with nothing to do (and of big destinations) are zero
+	const uint32_t vl = vb + lane;
+	const bool valid = vl < a.n;
+	const uint32_t lbeg = valid ? __ldg(a.in_off + vl) : 0u, lend = valid ? __ldg(a.in_off + vl + 1) : 0u;
+	const bool big = lend - lbeg > kMsPullBig;
+	const bool needy = valid && !big && lend > lbeg && !ld_cg_u8(a.done + vl);
+	const uint32_t needm = __ballot_sync(kFull, needy);
+	if (valid && !needy && !big) p.actn[vl] = 0;
+	if (!p.masked) {
+		// rows of the block with nothing to do are zero
+		const uint32_t bigm = __ballot_sync(kFull, big);
 		const uint32_t nb = min(32u, a.n - vb);
-		uint64_t *blk = nxt + (size_t) vb * K;
+		uint64_t *blk = p.nxt + (size_t) vb * K;
 		for (uint32_t x = lane; x < nb * K; x += 32)
-			if (!((needm >> (x / K)) & 1u)) blk[x] = 0ull;
-		// few words per vertex: every lane takes its own low in-degree destination
-		uint32_t warpm = needm;
-		if (K <= kLaneMaxWords) {
-			const bool mine = needy && lend - lbeg <= kLaneMaxDeg;
-			warpm &= ~__ballot_sync(kFull, mine);
-			ms_pull_lane(a, cur, actc, nxt, actn, vl, lbeg, lend, mine, actdeg, gathered, cn, qn, lact0, lact1, new_w0,
-					new_w1);
-		}
-		for (uint32_t m = warpm; m; m &= m - 1) {
-			const int jj = __ffs(m) - 1;
-			const uint32_t v = vb + jj;
-			const uint32_t beg = __shfl_sync(kFull, lbeg, jj), end = __shfl_sync(kFull, lend, jj);
-			const size_t row = (size_t) v * K;
-			const uint64_t vis0 = w0 ? ld_cg64(a.vis + row + lane) : 0ull;
-			const uint64_t vis1 = w1 ? ld_cg64(a.vis + row + lane + 32) : 0ull;
-			uint64_t acc0 = 0, acc1 = 0;
-			if (K <= kLaneMaxWords) {
-				// lanes hold words lane; the edge-parallel gather wants both words everywhere
-				uint64_t a0 = 0, a1 = 0;
-				ms_gather_edges(a, cur, actc, beg, end, shfl64(fm.f0, 0), shfl64(fm.f0, 1), shfl64(vis0, 0),
-						shfl64(vis0, 1), a0, a1, gathered);
-				acc0 = lane == 0 ? a0 : (lane == 1 ? a1 : 0ull);
-			} else if (K <= kGroupMaxWords) {
-				const uint32_t kp = K <= 4 ? 4 : 8;
-				const uint32_t kw = lane & (kp - 1);
-				uint64_t ag = 0;
-				ms_gather_grouped(a, cur, actc, beg, end, kp, shfl64(fm.f0, kw), shfl64(vis0, kw), ag, gathered);
-				acc0 = lane < kp ? ag : 0ull;
-			} else if (!fm.complete(vis0, vis1)) {
-				ms_gather(a, cur, actc, beg, end, fm, vis0, vis1, acc0, acc1, gathered);
-			}
-			const uint64_t n0 = acc0 & ~vis0 & fm.f0, n1 = acc1 & ~vis1 & fm.f1;
-			new_lane0 |= n0;
-			new_lane1 |= n1;
-			if (w0) { nxt[row + lane] = n0; if (n0) a.vis[row + lane] = vis0 | n0; }
-			if (w1) { nxt[row + lane + 32] = n1; if (n1) a.vis[row + lane + 32] = vis1 | n1; }
-			const uint64_t mask = row_mask(n0, n1);
-			const bool full = fm.complete(vis0 | n0, vis1 | n1);
-			if (lane == 0) {
-				actn[v] = mask;
-				if (full) a.done[v] = 1;
-			}
-			if (mask) {
-				const uint32_t d = deg_of(a, v);
-				if (lane == 0) actdeg += d;
-				if (d > kMsBig) {
-					if (lane == 0) qn[a.n - 1 - atomicAdd(&cn->nbig, 1u)] = v;
-				} else {
-					if (lane == 0) wbuf[wn] = v;
-					if (++wn == kMsWq) ms_wq_flush(cn, qn, wbuf, wn);
-				}
-			}
-		}
+			if (!(((needm | bigm) >> (x / K)) & 1u)) blk[x] = 0ull;
 	}
-	ms_wq_flush(cn, qn, wbuf, wn);
-	if (w0 && new_lane0) atomicOr(s_act + lane, (unsigned long long) new_lane0);
-	if (w1 && new_lane1) atomicOr(s_act + lane + 32, (unsigned long long) new_lane1);
-	if (new_w0) atomicOr(s_act, (unsigned long long) new_w0);
-	if (new_w1) atomicOr(s_act + 1, (unsigned long long) new_w1);
-}
-
-// Pull, destinations with many in-edges: warps take chunks of kMsChunk
-// in-edges over the whole grid and OR what they gather into the row.
-__device__ void ms_pull_chunks(const MsArgs &a, const uint64_t *cur, const uint64_t *actc, uint64_t *nxt,
-		unsigned long long &gathered, const unsigned long long *act) {
-	const uint32_t K = a.K;
-	const unsigned lane = lane_id();
-	const uint32_t gwarp = blockIdx.x * kMsWarps + warp_id();
-	const uint32_t nwarps = gridDim.x * kMsWarps;
-	const bool w0 = lane < K, w1 = lane + 32 < K;
-	const FullMask fm(a, lane, act);
-	for (uint32_t c = gwarp; c < a.nchunks; c += nwarps) {
-		const uint32_t v = __ldg(a.chunk_v + c), beg = __ldg(a.chunk_beg + c);
-		const uint32_t end = min(beg + kMsChunk, __ldg(a.in_off + v + 1));
+	for (uint32_t m = needm; m; m &= m - 1) {
+		const int jj = __ffs(m) - 1;
+		const uint32_t v = vb + jj;
+		const uint32_t beg = __shfl_sync(kFull, lbeg, jj), end = __shfl_sync(kFull, lend, jj);
 		const size_t row = (size_t) v * K;
 		const uint64_t vis0 = w0 ? ld_cg64(a.vis + row + lane) : 0ull;
 		const uint64_t vis1 = w1 ? ld_cg64(a.vis + row + lane + 32) : 0ull;
-		if (fm.complete(vis0, vis1)) continue;
 		uint64_t acc0 = 0, acc1 = 0;
-		if (K <= kLaneMaxWords) {
-			uint64_t a0 = 0, a1 = 0;
-			ms_gather_edges(a, cur, actc, beg, end, shfl64(fm.f0, 0), shfl64(fm.f0, 1), shfl64(vis0, 0), shfl64(vis0, 1),
-					a0, a1, gathered);
-			acc0 = lane == 0 ? a0 : (lane == 1 ? a1 : 0ull);
-		} else if (K <= kGroupMaxWords) {
-			const uint32_t kp = K <= 4 ? 4 : 8;
-			const uint32_t kw = lane & (kp - 1);
+		if (K <= kGroupMaxWords) {
+			const uint32_t kw = lane & 7u;
 			uint64_t ag = 0;
-			ms_gather_grouped(a, cur, actc, beg, end, kp, shfl64(fm.f0, kw), shfl64(vis0, kw), ag, gathered);
-			acc0 = lane < kp ? ag : 0ull;
-		} else {
-			ms_gather(a, cur, actc, beg, end, fm, vis0, vis1, acc0, acc1, gathered);
+			ms_gather_grouped(a, p.cur, p.actc, beg, end, 8, shfl64(fm.f0, kw), shfl64(vis0, kw), ag, gathered);
+			acc0 = lane < 8 ? ag : 0ull;
+		} else if (!fm.complete(vis0, vis1)) {
+			ms_gather(a, p.cur, p.actc, beg, end, fm, vis0, vis1, acc0, acc1, gathered);
 		}
 		const uint64_t n0 = acc0 & ~vis0 & fm.f0, n1 = acc1 & ~vis1 & fm.f1;
-		if (n0) atomicOr((unsigned long long *) (nxt + row + lane), (unsigned long long) n0);
-		if (n1) atomicOr((unsigned long long *) (nxt + row + lane + 32), (unsigned long long) n1);
-	}
-}
-
-// After ms_pull_chunks: the many-in-edge destinations' rows hold their new
-// bits; update vis, the frontier mask and the queue.
-__device__ void ms_pull_chunks_finish(const MsArgs &a, uint32_t lvl, uint64_t *nxt, uint64_t *actn,
-		unsigned long long &actdeg, unsigned long long *s_act) {
-	const uint32_t K = a.K;
-	uint32_t *qn = a.queue[(lvl + 1) & 1];
-	MsCounters *cn = &a.ctl->ctr[(lvl + 1) % 3];
-	const unsigned lane = lane_id();
-	const uint32_t gwarp = blockIdx.x * kMsWarps + warp_id();
-	const uint32_t nwarps = gridDim.x * kMsWarps;
-	const bool w0 = lane < K, w1 = lane + 32 < K;
-	uint64_t new0 = 0, new1 = 0;
-	for (uint32_t j = gwarp; j < a.nbig_in; j += nwarps) {
-		const uint32_t v = __ldg(a.in_big + j);
-		const size_t row = (size_t) v * K;
-		uint64_t n0 = 0, n1 = 0;
-		if (w0) {
-			n0 = ld_cg64(nxt + row + lane);
-			if (n0) a.vis[row + lane] = ld_cg64(a.vis + row + lane) | n0;
-		}
-		if (w1) {
-			n1 = ld_cg64(nxt + row + lane + 32);
-			if (n1) a.vis[row + lane + 32] = ld_cg64(a.vis + row + lane + 32) | n1;
-		}
 		new0 |= n0;
 		new1 |= n1;
 		const uint64_t mask = row_mask(n0, n1);
+		if (mask || !p.masked) {
+			if (w0) p.nxt[row + lane] = n0;
+			if (w1) p.nxt[row + lane + 32] = n1;
+		}
+		if (n0) a.vis[row + lane] = vis0 | n0;
+		if (n1) a.vis[row + lane + 32] = vis1 | n1;
+		const bool full = fm.complete(vis0 | n0, vis1 | n1);
 		if (lane == 0) {
-			actn[v] = mask;
-			if (mask) {
-				const uint32_t d = deg_of(a, v);
-				actdeg += d;
-				if (d > kMsBig) qn[a.n - 1 - atomicAdd(&cn->nbig, 1u)] = v;
-				else qn[atomicAdd(&cn->nact, 1u)] = v;
+			p.actn[v] = mask;
+			if (full) a.done[v] = 1;
+		}
+		if (mask) {
+			const uint32_t d = deg_of(a, v);
+			if (lane == 0) actdeg += d;
+			if (d > kMsBig) {
+				if (lane == 0) p.qn[a.n - 1 - atomicAdd(&p.cn->nbig, 1u)] = v;
+			} else {
+				if (lane == 0) wbuf[wn] = v;
+				if (++wn == kMsWq) ms_wq_flush(p.cn, p.qn, wbuf, wn);
 			}
 		}
 	}
-	if (w0 && new0) atomicOr(s_act + lane, (unsigned long long) new0);
-	if (w1 && new1) atomicOr(s_act + lane + 32, (unsigned long long) new1);
+}
+
+// Chunk c of kMsChunk in-edges of a destination with more than kMsPullBig: the
+// words it gathers are OR-ed into the destination's row of big_acc; the warp
+// that completes the destination's last chunk writes its row, mask and queue
+// entry and leaves its row of big_acc and its count at 0.
+__device__ __forceinline__ void ms_pull_chunk(const MsArgs &a, const MsPull &p, uint32_t c, const FullMask &fm,
+		uint64_t &new0, uint64_t &new1, unsigned long long &actdeg, unsigned long long &gathered) {
+	const uint32_t K = a.K;
+	const unsigned lane = lane_id();
+	const bool w0 = lane < K, w1 = lane + 32 < K;
+	const uint32_t v = __ldg(a.chunk_v + c), beg = __ldg(a.chunk_beg + c), slot = __ldg(a.chunk_slot + c);
+	const uint32_t vbeg = __ldg(a.in_off + v), vend = __ldg(a.in_off + v + 1);
+	const uint32_t end = min(beg + kMsChunk, vend);
+	const size_t row = (size_t) v * K;
+	const uint64_t vis0 = w0 ? ld_cg64(a.vis + row + lane) : 0ull;
+	const uint64_t vis1 = w1 ? ld_cg64(a.vis + row + lane + 32) : 0ull;
+	uint64_t *bacc = a.big_acc + (size_t) slot * K;
+	if (!fm.complete(vis0, vis1)) {
+		uint64_t acc0 = 0, acc1 = 0;
+		switch (K) {
+		case 1: acc0 = ms_chunk_rows<1>(a, p.cur, beg, end, gathered); break;
+		case 2: acc0 = ms_chunk_rows<2>(a, p.cur, beg, end, gathered); break;
+		case 3: acc0 = ms_chunk_rows<3>(a, p.cur, beg, end, gathered); break;
+		case 4: acc0 = ms_chunk_rows<4>(a, p.cur, beg, end, gathered); break;
+		default:
+			if (K <= kGroupMaxWords) {
+				const uint32_t kw = lane & 7u;
+				uint64_t ag = 0;
+				ms_gather_grouped(a, p.cur, p.actc, beg, end, 8, shfl64(fm.f0, kw), shfl64(vis0, kw), ag, gathered);
+				acc0 = lane < 8 ? ag : 0ull;
+			} else {
+				ms_gather(a, p.cur, p.actc, beg, end, fm, vis0, vis1, acc0, acc1, gathered);
+			}
+		}
+		const uint64_t n0 = acc0 & ~vis0 & fm.f0, n1 = acc1 & ~vis1 & fm.f1;
+		if (n0) atomicOr((unsigned long long *) (bacc + lane), (unsigned long long) n0);
+		if (n1) atomicOr((unsigned long long *) (bacc + lane + 32), (unsigned long long) n1);
+	}
+	__syncwarp();
+	uint32_t before = 0;
+	// releases this warp's words to, and acquires the other warps' from, those that count here
+	if (lane == 0)
+		asm volatile("atom.acq_rel.gpu.global.add.u32 %0, [%1], 1;" : "=r"(before) : "l"(a.big_cnt + slot) : "memory");
+	before = __shfl_sync(kFull, before, 0);
+	if (before != (vend - vbeg + kMsChunk - 1) / kMsChunk - 1) return;
+	__syncwarp();
+	const uint64_t n0 = w0 ? ld_cg64(bacc + lane) : 0ull, n1 = w1 ? ld_cg64(bacc + lane + 32) : 0ull;
+	if (n0) bacc[lane] = 0ull;
+	if (n1) bacc[lane + 32] = 0ull;
+	new0 |= n0;
+	new1 |= n1;
+	const uint64_t mask = row_mask(n0, n1);
+	if (mask || !p.masked) {
+		if (w0) p.nxt[row + lane] = n0;
+		if (w1) p.nxt[row + lane + 32] = n1;
+	}
+	if (n0) a.vis[row + lane] = vis0 | n0;
+	if (n1) a.vis[row + lane + 32] = vis1 | n1;
+	if (lane == 0) {
+		a.big_cnt[slot] = 0u;
+		p.actn[v] = mask;
+		if (mask) {
+			const uint32_t d = deg_of(a, v);
+			actdeg += d;
+			if (d > kMsBig) p.qn[a.n - 1 - atomicAdd(&p.cn->nbig, 1u)] = v;
+			else p.qn[atomicAdd(&p.cn->nact, 1u)] = v;
+		}
+	}
+}
+
+// The chunks from `item` on; returns the first item after them that this warp got.
+__device__ __noinline__ uint32_t ms_pull_chunks(const MsArgs &a, const MsPull &p, uint32_t item, unsigned *counter,
+		const FullMask &fm, unsigned long long &actdeg, unsigned long long &gathered, unsigned long long *s_act) {
+	const unsigned lane = lane_id();
+	uint64_t new0 = 0, new1 = 0;
+	while (item < a.nchunks) {
+		const uint32_t next = lane == 0 ? atomicAdd(counter, 1u) : 0u;
+		ms_pull_chunk(a, p, item, fm, new0, new1, actdeg, gathered);
+		item = __shfl_sync(kFull, next, 0);
+	}
+	if (new0) atomicOr(s_act + lane, (unsigned long long) new0);
+	if (new1) atomicOr(s_act + lane + 32, (unsigned long long) new1);
+	return item;
+}
+
+// The blocks of 32 destinations from `item` on, for KK words per vertex (0:
+// more than kMsRowWords).
+template <int KK>
+__device__ __noinline__ void ms_pull_blocks(const MsArgs &a, const MsPull &p, uint32_t item, unsigned *counter,
+		const FullMask &fm, unsigned long long &actdeg, unsigned long long &gathered, uint32_t *wbuf,
+		unsigned long long *s_act) {
+	const unsigned lane = lane_id();
+	const uint32_t nblk = (a.n + 31) / 32;
+	constexpr int kN = KK ? KK : 2;
+	uint64_t f[kN], acc[kN];
+#pragma unroll
+	for (int k = 0; k < kN; ++k) {
+		f[k] = KK ? shfl64(fm.f0, k) : 0ull;
+		acc[k] = 0ull;
+	}
+	uint32_t wn = 0;
+	while (item < a.nchunks + nblk) {
+		const uint32_t next = lane == 0 ? atomicAdd(counter, 1u) : 0u;
+		const uint32_t vb = (item - a.nchunks) * 32;
+		if constexpr (KK != 0) ms_pull_rows<KK>(a, p, vb, f, acc, actdeg, gathered);
+		else ms_pull_words(a, p, vb, fm, acc[0], acc[1], actdeg, gathered, wbuf, wn);
+		item = __shfl_sync(kFull, next, 0);
+	}
+	if constexpr (KK != 0) {
+#pragma unroll
+		for (int k = 0; k < KK; ++k) {
+			const uint64_t x = warp_or64(acc[k]);
+			if (lane == 0 && x) atomicOr(s_act + k, (unsigned long long) x);
+		}
+	} else {
+		ms_wq_flush(p.cn, p.qn, wbuf, wn);
+		if (acc[0]) atomicOr(s_act + lane, (unsigned long long) acc[0]);
+		if (acc[1]) atomicOr(s_act + lane + 32, (unsigned long long) acc[1]);
+	}
+}
+
+// A pull level: the chunks of the many-in-edge destinations, then the blocks of
+// 32 destinations, handed to the warps one at a time through a counter (the
+// next one claimed while one runs), so that no barrier is needed between them.
+__device__ __forceinline__ void ms_pull(const MsArgs &a, const MsPull &p, unsigned *counter, unsigned long long &actdeg_out,
+		unsigned long long &gathered_out, uint32_t *wq_base, unsigned long long *s_act) {
+	const unsigned lane = lane_id();
+	const FullMask fm(a, lane, p.act);
+	unsigned long long actdeg = 0, gathered = 0;
+	uint32_t item = lane == 0 ? atomicAdd(counter, 1u) : 0u;
+	item = __shfl_sync(kFull, item, 0);
+	if (item < a.nchunks) item = ms_pull_chunks(a, p, item, counter, fm, actdeg, gathered, s_act);
+	uint32_t *wbuf = wq_base + warp_id() * kMsWq;
+	switch (a.K) {
+	case 1: ms_pull_blocks<1>(a, p, item, counter, fm, actdeg, gathered, wbuf, s_act); break;
+	case 2: ms_pull_blocks<2>(a, p, item, counter, fm, actdeg, gathered, wbuf, s_act); break;
+	case 3: ms_pull_blocks<3>(a, p, item, counter, fm, actdeg, gathered, wbuf, s_act); break;
+	case 4: ms_pull_blocks<4>(a, p, item, counter, fm, actdeg, gathered, wbuf, s_act); break;
+	default: ms_pull_blocks<0>(a, p, item, counter, fm, actdeg, gathered, wbuf, s_act); break;
+	}
+	static_assert(kMsRowWords == 4, "a case for each");
+	actdeg_out += actdeg;
+	gathered_out += gathered;
 }
 
 // Planes [first, last] (levels base + p) -> uint8 levels [source][vertex].
@@ -702,10 +812,10 @@ __device__ __forceinline__ uint64_t emit_ld(const uint64_t *p) {
 // kCached also selects two row buffers used in turn, so that a tile needs one
 // barrier (between its two phases): a buffer is written again two tiles
 // later, after the barrier that every thread reaches once done reading it.
-template <bool kCached, uint32_t kV>
+template <bool kCached, uint32_t kV, uint32_t kW>
 __device__ __noinline__ void ms_emit(const MsArgs &a, uint8_t *levels, uint32_t ns, uint32_t base, uint32_t first, uint32_t last,
 		bool merge, uint8_t *lev) {
-	constexpr uint32_t kEmitV = kV, kEmitRow = kV + 4;
+	constexpr uint32_t kEmitV = kV, kEmitW = kW, kEmitRow = kV + 4;
 	constexpr uint32_t kBufs = kCached ? 2 : 1, kBufWords = kEmitW * 16 * kEmitRow;
 	constexpr uint32_t kRows = kEmitW * 64;
 	const uint32_t K = a.K, n = a.n;
@@ -797,7 +907,7 @@ __device__ __noinline__ void ms_emit(const MsArgs &a, uint8_t *levels, uint32_t 
 	}
 }
 
-__global__ void __launch_bounds__(kMsThreads, 2) k_ms_bfs(MsArgs a, const uint32_t *sources, uint32_t ns,
+__global__ void __launch_bounds__(kMsThreads, 2) k_ms_bfs(const __grid_constant__ MsArgs a, const uint32_t *sources, uint32_t ns,
 		uint8_t *levels) {
 	__shared__ unsigned long long red[kMsWarps];
 	__shared__ uint32_t wq[kMsWarps * kMsWq];
@@ -811,6 +921,8 @@ __global__ void __launch_bounds__(kMsThreads, 2) k_ms_bfs(MsArgs a, const uint32
 	if (leader) ctl->stats.t_start = global_timer_ns();
 	// clear (the control block was zeroed by the host)
 	for (size_t i = t0; i < nK; i += stride) { a.vis[i] = 0; a.hist[i] = 0; }
+	for (size_t i = t0; i < (size_t) a.nbig_in * a.K; i += stride) a.big_acc[i] = 0;
+	for (uint32_t i = t0; i < a.nbig_in; i += stride) a.big_cnt[i] = 0;
 	for (uint32_t i = t0; i < a.n; i += stride) {
 		a.pmask[i] = 0;
 		a.done[i] = 0;
@@ -860,7 +972,7 @@ __global__ void __launch_bounds__(kMsThreads, 2) k_ms_bfs(MsArgs a, const uint32
 				break;
 			}
 			// planes full: write them out, keep the frontier's plane as plane 0
-			ms_emit<false, kEmitV>(a, levels, ns, base, base == 0 ? 0 : 1, lvl - base, base != 0, lev);
+			ms_emit<false, kEmitV, kEmitW>(a, levels, ns, base, base == 0 ? 0 : 1, lvl - base, base != 0, lev);
 			if (!(ok = grid_sync(ctl->bar, epoch, &ctl->err, a.wait_limit_ns, a.hold_barrier))) break;
 			const uint64_t *src = a.hist + (size_t) (lvl - base) * nK;
 			for (size_t i = t0; i < nK; i += stride) a.hist[i] = ld_cg64(src + i);
@@ -904,15 +1016,9 @@ __global__ void __launch_bounds__(kMsThreads, 2) k_ms_bfs(MsArgs a, const uint32
 			if (leader && tph) tph[1] = global_timer_ns();
 			ms_push_finish(a, lvl, nxt, actn, actdeg, s_act);
 		} else {
-			ms_pull(a, lvl, cur, actc, nxt, actn, actdeg, gathered, wq, act, s_act);
-			if (a.nbig_in) {
-				if (!(ok = grid_sync(ctl->bar, epoch, &ctl->err, a.wait_limit_ns, a.hold_barrier))) break;
-				if (leader && tph) tph[0] = global_timer_ns();
-				ms_pull_chunks(a, cur, actc, nxt, gathered, act);
-				if (!(ok = grid_sync(ctl->bar, epoch, &ctl->err, a.wait_limit_ns, a.hold_barrier))) break;
-				if (leader && tph) tph[1] = global_timer_ns();
-				ms_pull_chunks_finish(a, lvl, nxt, actn, actdeg, s_act);
-			}
+			const MsPull p{cur, actc, nxt, actn, act, &ctl->ctr[(lvl + 1) % 3], a.queue[(lvl + 1) & 1],
+					levels != nullptr && a.K > kMsRowWords};
+			ms_pull(a, p, &ctl->work[lvl], actdeg, gathered, wq, s_act);
 		}
 		// the next frontier's out-degree: per-CTA sum, one atomic per CTA
 		const unsigned long long d = warp_sum(actdeg);
@@ -966,17 +1072,40 @@ __global__ void __launch_bounds__(kMsThreads, 2) k_ms_bfs(MsArgs a, const uint32
 // the cooperative kernel, so more plane loads in flight).  Plane depth - base
 // is the empty frontier; after an early output pass, plane 0 was written too.
 // A tile's plane loads and its barriers form a chain of round trips; narrow
-// tiles on small CTAs keep more chains going per SM.
-template <int kThreads>
+// tiles on small CTAs keep more chains going per SM.  A tile is kW words wide,
+// a thread per (vertex, word): with one or two words per vertex, tiles of four
+// would leave most threads idle.
+template <int kThreads, uint32_t kW>
 __global__ void __launch_bounds__(kThreads, kThreads == 256 ? 4 : 2) k_ms_emit(MsArgs a, uint32_t ns, uint8_t *levels) {
-	constexpr uint32_t kV = kThreads / kEmitW;
-	__shared__ __align__(16) uint8_t lev[emit_bytes(kV, 2)];
+	constexpr uint32_t kV = kThreads / kW;
+	__shared__ __align__(16) uint8_t lev[emit_bytes(kV, 2, kW)];
 	const MsStats &st = a.ctl->stats;
 	if (!st.complete) return;
 	const uint32_t base = st.base, depth = st.depth;
 	const uint32_t first = base == 0 ? 0 : 1;
 	if (depth < base + first + 1) return;
-	ms_emit<true, kV>(a, levels, ns, base, first, depth - 1 - base, base != 0, lev);
+	ms_emit<true, kV, kW>(a, levels, ns, base, first, depth - 1 - base, base != 0, lev);
+}
+
+// chunk_slot[c]: the index of chunk c's destination in in_big (ascending).
+__global__ void k_ms_chunk_slots(const uint32_t *chunk_v, uint32_t nchunks, const uint32_t *in_big, uint32_t nbig,
+		uint32_t *chunk_slot) {
+	for (uint32_t c = blockIdx.x * blockDim.x + threadIdx.x; c < nchunks; c += gridDim.x * blockDim.x) {
+		const uint32_t v = chunk_v[c];
+		uint32_t lo = 0, hi = nbig - 1;
+		while (lo < hi) {
+			const uint32_t mid = (lo + hi) / 2;
+			if (in_big[mid] < v) lo = mid + 1;
+			else hi = mid;
+		}
+		chunk_slot[c] = lo;
+	}
+}
+
+int ms_chunk_slots(const uint32_t *chunk_v, uint32_t nchunks, const uint32_t *in_big, uint32_t nbig, uint32_t *chunk_slot) {
+	if (!nchunks || !nbig) return BFS_OK;
+	k_ms_chunk_slots<<<std::min<uint32_t>((nchunks + 255) / 256, 1024), 256>>>(chunk_v, nchunks, in_big, nbig, chunk_slot);
+	return cudaGetLastError() == cudaSuccess && cudaStreamSynchronize(0) == cudaSuccess ? BFS_OK : BFS_ECUDA;
 }
 
 int ms_launch(const MsArgs &a, const uint32_t *d_sources, uint32_t ns, uint8_t *levels, int num_sms, cudaStream_t st,
@@ -1000,13 +1129,14 @@ int ms_launch(const MsArgs &a, const uint32_t *d_sources, uint32_t ns, uint8_t *
 	if (between2 && cudaEventRecord(between2, st) != cudaSuccess) return BFS_ECUDA;
 	if (levels) {
 		const bool wide = a.out_tile ? a.out_tile == 128 : a.n >= kEmitWideMinVertices;
-		const void *fn = wide ? (const void *) k_ms_emit<512> : (const void *) k_ms_emit<256>;
-		const int threads = wide ? 512 : 256;
+		const uint32_t words = a.out_tile || a.K > 2 ? kEmitW : a.K;  // an explicit tile width is one of four-word tiles
+		void (*fn)(MsArgs, uint32_t, uint8_t *) = words == 1 ? k_ms_emit<256, 1> : words == 2 ? k_ms_emit<256, 2> :
+				wide ? k_ms_emit<512, kEmitW> : k_ms_emit<256, kEmitW>;
+		const int threads = words == kEmitW && wide ? 512 : 256;
 		int out_per_sm = 0;
 		if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&out_per_sm, fn, threads, 0) != cudaSuccess || out_per_sm < 1)
 			return BFS_ECUDA;
-		if (wide) k_ms_emit<512><<<num_sms * out_per_sm, 512, 0, st>>>(a, ns, levels);
-		else k_ms_emit<256><<<num_sms * out_per_sm, 256, 0, st>>>(a, ns, levels);
+		fn<<<num_sms * out_per_sm, threads, 0, st>>>(a, ns, levels);
 	}
 	return cudaGetLastError() == cudaSuccess ? BFS_OK : BFS_ECUDA;
 }

@@ -42,6 +42,7 @@ struct MsControl {
 	unsigned bar[2];
 	int err;
 	unsigned push_chunks;  // push level: 1024-edge chunks of its high-degree frontier vertices
+	unsigned work[kMsMaxLevel + 1];  // per pull level: the next work item (chunks, then blocks of destinations)
 	MsCounters ctr[3];
 	MsStats stats;
 	// active[l % 3][k]: OR of word k over level l's frontier rows -- the
@@ -61,6 +62,9 @@ struct MsArgs {
 	const uint32_t *row_off, *col, *in_off, *in_src;
 	const uint32_t *in_big;              // [nbig_in] those destinations
 	const uint32_t *chunk_v, *chunk_beg; // [nchunks] destination and first in-edge of each chunk
+	uint32_t *chunk_slot;                // [nchunks] the destination's index in in_big
+	uint64_t *big_acc;                   // [nbig_in][K] words their chunks gathered (0 between levels)
+	unsigned *big_cnt;                   // [nbig_in] their chunks done (0 between levels)
 	uint32_t *push_u, *push_beg;         // [push_cap] push: vertex and first edge of each 1024-edge chunk
 	uint32_t push_cap;
 	uint64_t *vis;        // [n][K] sources that reached v
@@ -83,6 +87,9 @@ struct MsArgs {
 // *grid receives the launch's CTA count.  levels == null: no output pass, the
 // planes stay for a later pass, and a traversal deeper than the planes stops
 // with BFS_EUNSUPPORTED.
+// Fills chunk_slot (once per allocation); waits for it.
+int ms_chunk_slots(const uint32_t *chunk_v, uint32_t nchunks, const uint32_t *in_big, uint32_t nbig, uint32_t *chunk_slot);
+
 int ms_launch(const MsArgs &a, const uint32_t *d_sources, uint32_t ns, uint8_t *levels, int num_sms, cudaStream_t st,
 		int *grid, cudaEvent_t between, cudaEvent_t between2);
 

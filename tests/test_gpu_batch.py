@@ -298,3 +298,29 @@ def test_output_tile_widths_give_the_same_levels(native, oracle, num_sources):
         import bfs_simd_benchmarks_gb300._native as N
         with pytest.raises(N.BfsError):
             g.set_options(batch_output_tile=96)
+
+
+@pytest.mark.parametrize("words", [1, 2, 3, 4, 5, 8, 9, 33, 64])
+@pytest.mark.parametrize("push_div", [1, 1 << 30])
+def test_words_per_vertex_and_degrees(native, oracle, words, push_div):
+    """Every shape of the pull (and of the push) by words per vertex, on a graph whose
+    in-degrees lie at its edges: 31-33 (a lane), 255-257 (a chunk), 511-513."""
+    import bfs_simd_benchmarks_gb300 as B
+    rng = np.random.default_rng(words)
+    n = 3001
+    degs = [31, 32, 33, 255, 256, 257, 511, 512, 513, 1, 2]
+    src = [rng.integers(0, n, size=d) for d in degs] + [rng.integers(0, n, size=4 * n)]
+    dst = [np.full(d, 100 + 37 * i) for i, d in enumerate(degs)] + [rng.integers(200 + 37 * len(degs), n, size=4 * n)]
+    src, dst = np.concatenate(src).astype(np.uint32), np.concatenate(dst).astype(np.uint32)
+    arr = oracle.csr_arrays(n, src, dst)
+    k = 64 * words - (rng.integers(0, 64) if words < 64 else 0)
+    sources = rng.integers(0, n, size=k).astype(np.uint32)
+    with B.Graph.from_edges(n, src, dst, 256, 4) as g:
+        g.set_options(batch_single_max=0, batch_push_div=push_div)
+        expect = {}
+        for s in set(sources.tolist()):
+            lev = oracle.bfs_levels(arr, int(s))
+            expect[s] = np.where(lev < 0, 255, lev).astype(np.uint8)
+        exp = np.stack([expect[int(s)] for s in sources])
+        for _ in range(2):  # the second run finds the first one's state
+            _check(oracle, arr, g, sources, exp)
