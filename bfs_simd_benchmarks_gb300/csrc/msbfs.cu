@@ -48,13 +48,15 @@ constexpr int kMsWarps = kMsThreads / 32;
 constexpr uint32_t kMsWq = 64;          // per-warp staged queue appends (pull)
 constexpr uint32_t kMsBig = 1024;       // push: higher-degree vertices are spread over the grid
 constexpr int kMsGather = 4;            // pull: frontier rows gathered per round
+constexpr int kMsFinishRows = 2;        // push: touched rows finished per round
 constexpr uint32_t kLaneMaxDeg = 32;    // pull, few words: destinations of at most this in-degree go one per lane
 constexpr uint32_t kGroupMaxWords = 8;  // pull: up to this many words, in-neighbour rows in lane groups
 constexpr uint32_t kEmitW = 4;          // output tile: kV vertices x kW words (4: 256 sources), kV = threads / kW
 // shared bytes of an output tile of kV vertices: rows of one source quad (kV + 4
 // words, 16-byte aligned; `bufs` copies) and the nibble table
-__host__ __device__ constexpr uint32_t emit_bytes(uint32_t kV, uint32_t bufs = 1, uint32_t kW = kEmitW) {
-	return (bufs * kW * 16 * (kV + 4) + 16) * 4;
+// (shifted rows: one copy, and the rows themselves)
+__host__ __device__ constexpr uint32_t emit_bytes(uint32_t kV, uint32_t bufs = 1, uint32_t kW = kEmitW, bool shift = false) {
+	return shift ? (kW * 16 * (kV + 4) + 16) * 4 + kW * 64 * (kV + 16) : (bufs * kW * 16 * (kV + 4) + 16) * 4;
 }
 constexpr uint32_t kMsRowWords = 4;     // pull: up to this many words per vertex, rows are read whole
 constexpr uint32_t kEmitV = kMsThreads / kEmitW;  // the traversal kernel's tiles (its early output passes)
@@ -161,6 +163,40 @@ __device__ void ms_push_chunk_list(const MsArgs &a, uint32_t lvl, uint32_t nb, u
 	if (threadIdx.x == 0) a.ctl->push_chunks = min(running, a.push_cap);
 }
 
+// Push level with few edges: clears only the rows that will receive words (the
+// first edge to reach one claims it in `touched`), instead of the whole plane.
+// R-MAT scale 22 with 64 words per vertex: a plane is 2 GiB, 0.33 ms to clear;
+// levels of up to n / kMsMarkDiv edges take 0.02 to 0.06 ms this way.
+constexpr uint32_t kMsMarkDiv = 8;
+constexpr uint32_t kMsMarkBig = 64;  // high-degree frontier vertices, one after the other by the whole grid
+__device__ __forceinline__ void ms_mark_edges(const MsArgs &a, uint64_t *nxt, uint32_t e0, uint32_t end) {
+	const unsigned lane = lane_id();
+	const uint32_t e = e0 + lane;
+	const uint32_t v = e < end ? __ldg(a.col + e) : 0u;
+	bool mine = e < end && !ld_cg_u8(a.touched + v);
+	if (mine) {
+		const uint32_t bit = 1u << (8 * (v & 3u));
+		mine = !(atomicOr(reinterpret_cast<unsigned *>(a.touched + (v & ~3u)), bit) & bit);
+	}
+	for (uint32_t m = __ballot_sync(kFull, mine); m; m &= m - 1) {
+		uint64_t *row = nxt + (size_t) __shfl_sync(kFull, v, __ffs(m) - 1) * a.K;
+		for (uint32_t k = lane; k < a.K; k += 32) row[k] = 0ull;
+	}
+}
+__device__ void ms_push_mark(const MsArgs &a, uint32_t lvl, uint64_t *nxt, uint32_t nq, uint32_t nb) {
+	const uint32_t *q = a.queue[lvl & 1];
+	const uint32_t gwarp = blockIdx.x * kMsWarps + warp_id();
+	const uint32_t nwarps = gridDim.x * kMsWarps;
+	for (uint32_t i = gwarp; i < nq; i += nwarps) {
+		const uint32_t u = ld_cg(q + i), end = __ldg(a.row_off + u + 1);
+		for (uint32_t e = __ldg(a.row_off + u); e < end; e += 32) ms_mark_edges(a, nxt, e, end);
+	}
+	for (uint32_t i = 0; i < nb; ++i) {
+		const uint32_t u = ld_cg(q + a.n - 1 - i), end = __ldg(a.row_off + u + 1);
+		for (uint32_t e = __ldg(a.row_off + u) + 32 * gwarp; e < end; e += 32 * nwarps) ms_mark_edges(a, nxt, e, end);
+	}
+}
+
 __device__ void ms_push(const MsArgs &a, uint32_t lvl, const uint64_t *cur, const uint64_t *actc, uint64_t *nxt, uint32_t nq,
 		uint32_t nb) {
 	const uint32_t *q = a.queue[lvl & 1];
@@ -200,25 +236,40 @@ __device__ void ms_push_finish(const MsArgs &a, uint32_t lvl, uint64_t *nxt, uin
 		const uint32_t v = vb + lane;
 		const bool t = v < a.n && ld_cg_u8(a.touched + v);
 		uint32_t anym = 0;
-		for (uint32_t tm = __ballot_sync(kFull, t); tm; tm &= tm - 1) {
-			const int j = __ffs(tm) - 1;
-			const size_t row = (size_t) (vb + j) * K;
-			uint64_t nw[2] = {0ull, 0ull};
+		for (uint32_t tm = __ballot_sync(kFull, t); tm;) {
+			// kMsFinishRows touched rows at a time, the loads of all of them in flight
+			size_t row[kMsFinishRows];
+			uint32_t j[kMsFinishRows];
+			uint64_t w[kMsFinishRows][2], vv[kMsFinishRows][2];
 #pragma unroll
-			for (int h = 0; h < 2; ++h) {
-				const uint32_t k = lane + 32 * h;
-				if (k >= K) continue;
-				const uint64_t w = ld_cg64(nxt + row + k);
-				if (!w) continue;
-				const uint64_t vv = ld_cg64(a.vis + row + k);
-				nw[h] = w & ~vv;
-				if (nw[h] != w) nxt[row + k] = nw[h];
-				if (nw[h]) a.vis[row + k] = vv | nw[h];
-				newacc[h] |= nw[h];
+			for (int r = 0; r < kMsFinishRows; ++r) {
+				j[r] = tm ? (uint32_t) __ffs(tm) - 1 : 32u;
+				tm &= tm - 1;
+				row[r] = (size_t) (vb + (j[r] & 31u)) * K;
+#pragma unroll
+				for (int h = 0; h < 2; ++h) {
+					const uint32_t k = lane + 32 * h;
+					const bool ld = j[r] < 32 && k < K;
+					w[r][h] = ld ? ld_cg64(nxt + row[r] + k) : 0ull;
+					vv[r][h] = ld ? ld_cg64(a.vis + row[r] + k) : 0ull;
+				}
 			}
-			const uint64_t mask = row_mask(nw[0], nw[1]);
-			if (lane == 0) actn[vb + j] = mask;
-			if (mask) anym |= 1u << j;
+#pragma unroll
+			for (int r = 0; r < kMsFinishRows; ++r) {
+				if (j[r] == 32u) break;
+				uint64_t nw[2];
+#pragma unroll
+				for (int h = 0; h < 2; ++h) {
+					const uint32_t k = lane + 32 * h;
+					nw[h] = w[r][h] & ~vv[r][h];
+					if (nw[h] != w[r][h]) nxt[row[r] + k] = nw[h];
+					if (nw[h]) a.vis[row[r] + k] = vv[r][h] | nw[h];
+					newacc[h] |= nw[h];
+				}
+				const uint64_t mask = row_mask(nw[0], nw[1]);
+				if (lane == 0) actn[vb + j[r]] = mask;
+				if (mask) anym |= 1u << j[r];
+			}
 		}
 		if (t) a.touched[v] = 0;
 		else if (v < a.n) actn[v] = 0;
@@ -812,11 +863,63 @@ __device__ __forceinline__ uint64_t emit_ld(const uint64_t *p) {
 // kCached also selects two row buffers used in turn, so that a tile needs one
 // barrier (between its two phases): a buffer is written again two tiles
 // later, after the barrier that every thread reaches once done reading it.
-template <bool kCached, uint32_t kV, uint32_t kW>
+//
+// kShift: rows that do not start on 16-byte boundaries (n or `levels` not a
+// multiple of 16).  Phase 2 then leaves its bytes in shared memory, row by row,
+// and a third phase writes every row in 16-byte pieces of its own alignment,
+// each put together from five words by funnel shifts; only the up to 15 bytes
+// at either end of a tile's row go out in smaller stores.  (Straight from phase
+// 2, a row on an odd address went out a byte at a time: Pokec shape, 64
+// sources, 0.23 ms.)
+__host__ __device__ constexpr uint32_t emit_row_bytes(uint32_t kV) { return kV + 16; }
+
+// 4 bytes at any byte offset of shared memory
+__device__ __forceinline__ uint32_t smem_u32(const uint8_t *p, uint32_t o) {
+	const uint32_t *w = reinterpret_cast<const uint32_t *>(p + (o & ~3u));
+	return __funnelshift_r(w[0], w[1], 8 * (o & 3u));
+}
+// The row's bytes [0, nv) at src -> dst: piece 0 up to dst's first 16-byte
+// boundary, piece i the 16 bytes from the i-th one on.
+__device__ __forceinline__ void emit_shifted(const uint8_t *src, uint8_t *dst, uint32_t nv, uint32_t piece, bool merge) {
+	const uint32_t head = min(nv, (uint32_t) (-(uintptr_t) dst & 15u));
+	uint32_t o = piece ? head + 16 * (piece - 1) : 0u;
+	if (o >= nv) return;
+	const uint32_t len = piece ? min(16u, nv - o) : head;
+	if (merge) {
+		for (uint32_t i = o; i < o + len; ++i) dst[i] = min(src[i], ld_cg_u8(dst + i));
+		return;
+	}
+	if (len == 16) {
+		const uint32_t *w = reinterpret_cast<const uint32_t *>(src + (o & ~3u));
+		const uint32_t sh = 8 * (o & 3u);
+		uint32_t x[5];
+#pragma unroll
+		for (int q = 0; q < 5; ++q) x[q] = w[q];
+		*reinterpret_cast<uint4 *>(dst + o) =
+				make_uint4(__funnelshift_r(x[0], x[1], sh), __funnelshift_r(x[1], x[2], sh),
+						__funnelshift_r(x[2], x[3], sh), __funnelshift_r(x[3], x[4], sh));
+		return;
+	}
+	// a head grows to the 16-byte boundary, a tail shrinks from it
+	if (piece == 0 && head == nv && ((uintptr_t) (dst + nv) & 15u)) {  // both ends inside one piece
+		for (; o < nv; ++o) dst[o] = src[o];
+		return;
+	}
+	for (uint32_t b = piece ? 8u : 1u; b && b <= 8u; b = piece ? b / 2 : b * 2) {
+		if (!(len & b)) continue;
+		if (b == 1) dst[o] = src[o];
+		else if (b == 2) *reinterpret_cast<uint16_t *>(dst + o) = (uint16_t) smem_u32(src, o);
+		else if (b == 4) *reinterpret_cast<uint32_t *>(dst + o) = smem_u32(src, o);
+		else *reinterpret_cast<uint2 *>(dst + o) = make_uint2(smem_u32(src, o), smem_u32(src, o + 4));
+		o += b;
+	}
+}
+
+template <bool kCached, uint32_t kV, uint32_t kW, bool kShift>
 __device__ __noinline__ void ms_emit(const MsArgs &a, uint8_t *levels, uint32_t ns, uint32_t base, uint32_t first, uint32_t last,
 		bool merge, uint8_t *lev) {
 	constexpr uint32_t kEmitV = kV, kEmitW = kW, kEmitRow = kV + 4;
-	constexpr uint32_t kBufs = kCached ? 2 : 1, kBufWords = kEmitW * 16 * kEmitRow;
+	constexpr uint32_t kBufs = kCached && !kShift ? 2 : 1, kBufWords = kEmitW * 16 * kEmitRow;
 	constexpr uint32_t kRows = kEmitW * 64;
 	const uint32_t K = a.K, n = a.n;
 	const uint32_t vtiles = (n + kEmitV - 1) / kEmitV, wtiles = (K + kEmitW - 1) / kEmitW;
@@ -824,6 +927,7 @@ __device__ __noinline__ void ms_emit(const MsArgs &a, uint8_t *levels, uint32_t 
 	const size_t pstride = (size_t) n * K;
 	uint32_t *const sw0 = reinterpret_cast<uint32_t *>(lev);  // [buffer][wi * 16 + quad][kEmitRow]
 	uint32_t *lut = sw0 + kBufs * kBufWords;                 // nibble -> byte mask
+	uint8_t *const rows = reinterpret_cast<uint8_t *>(lut + 16);  // kShift: [source][emit_row_bytes]
 	if (threadIdx.x < 16) lut[threadIdx.x] = nibble_bytes(threadIdx.x);
 	// phase 2's item: rows of source quad rq (word rq / 16), vertices 16 cc ...
 	const uint32_t rq = threadIdx.x / (kEmitV / 16), cc = threadIdx.x % (kEmitV / 16);
@@ -845,10 +949,10 @@ __device__ __noinline__ void ms_emit(const MsArgs &a, uint8_t *levels, uint32_t 
 			// 8 planes per round: their word masks (one round trip), then the
 			// non-zero words (one more)
 			for (uint32_t l = first; l <= last; l += 8) {
-				uint32_t nz = 0;
+				uint32_t nz = K <= kMsRowWords ? 0xFFu >> (l + 7 <= last ? 0u : l + 7 - last) : 0u;  // rows are zero where nothing is
 #pragma unroll
 				for (int t = 0; t < 8; ++t)
-					if (l + t <= last)
+					if (K > kMsRowWords && l + t <= last)
 						nz |= (uint32_t) ((emit_ld<kCached>(pm + (size_t) (l - first + t) * n) >> k) & 1ull) << t;
 				uint64_t w[8];
 #pragma unroll
@@ -899,11 +1003,25 @@ __device__ __noinline__ void ms_emit(const MsArgs &a, uint8_t *levels, uint32_t 
 			const uint32_t cnt = min(16u, nv - c);
 #pragma unroll
 			for (int b = 0; b < 4; ++b) {
+				if constexpr (kShift) {
+					*reinterpret_cast<uint4 *>(rows + (r0 + b) * emit_row_bytes(kV) + c) =
+							make_uint4(y[b][0], y[b][1], y[b][2], y[b][3]);
+					continue;
+				}
 				if (r0 + b >= nrows) break;
 				emit_piece(levels + (size_t) (k0 * 64 + r0 + b) * n + v0 + c, y[b], cnt, merge);
 			}
 		}
-		if (kBufs == 1) __syncthreads();
+		if (kShift) {
+			__syncthreads();
+			constexpr uint32_t kPieces = kV / 16 + 1;
+			for (uint32_t i = threadIdx.x; i < nrows * kPieces; i += blockDim.x) {
+				const uint32_t r = i / kPieces;
+				emit_shifted(rows + r * emit_row_bytes(kV), levels + (size_t) (k0 * 64 + r) * n + v0, nv, i % kPieces, merge);
+			}
+		} else if (kBufs == 1) {
+			__syncthreads();
+		}
 	}
 }
 
@@ -972,7 +1090,7 @@ __global__ void __launch_bounds__(kMsThreads, 2) k_ms_bfs(const __grid_constant_
 				break;
 			}
 			// planes full: write them out, keep the frontier's plane as plane 0
-			ms_emit<false, kEmitV, kEmitW>(a, levels, ns, base, base == 0 ? 0 : 1, lvl - base, base != 0, lev);
+			ms_emit<false, kEmitV, kEmitW, false>(a, levels, ns, base, base == 0 ? 0 : 1, lvl - base, base != 0, lev);
 			if (!(ok = grid_sync(ctl->bar, epoch, &ctl->err, a.wait_limit_ns, a.hold_barrier))) break;
 			const uint64_t *src = a.hist + (size_t) (lvl - base) * nK;
 			for (size_t i = t0; i < nK; i += stride) a.hist[i] = ld_cg64(src + i);
@@ -1005,10 +1123,12 @@ __global__ void __launch_bounds__(kMsThreads, 2) k_ms_bfs(const __grid_constant_
 		uint64_t *actn = a.pmask + (size_t) (lvl + 1 - base) * a.n;
 		unsigned long long *tph = lvl < kMsTraceLevels ? ctl->stats.t_phase[lvl] : nullptr;
 		unsigned long long actdeg = 0;
+		const bool masked = levels != nullptr && a.K > kMsRowWords;  // rows with an empty mask need no clearing
 		const bool push = qdeg * (unsigned long long) a.push_div < (unsigned long long) a.m;
 		if (push) {
 			if (blockIdx.x == 0 && nb) ms_push_chunk_list(a, lvl, nb, wq);
-			for (size_t i = t0; i < nK; i += stride) nxt[i] = 0;
+			if (masked && nb <= kMsMarkBig && qdeg < a.n / kMsMarkDiv) ms_push_mark(a, lvl, nxt, nq, nb);
+			else for (size_t i = t0; i < nK; i += stride) nxt[i] = 0;
 			if (!(ok = grid_sync(ctl->bar, epoch, &ctl->err, a.wait_limit_ns, a.hold_barrier))) break;
 			if (leader && tph) tph[0] = global_timer_ns();
 			ms_push(a, lvl, cur, actc, nxt, nq, nb);
@@ -1017,7 +1137,7 @@ __global__ void __launch_bounds__(kMsThreads, 2) k_ms_bfs(const __grid_constant_
 			ms_push_finish(a, lvl, nxt, actn, actdeg, s_act);
 		} else {
 			const MsPull p{cur, actc, nxt, actn, act, &ctl->ctr[(lvl + 1) % 3], a.queue[(lvl + 1) & 1],
-					levels != nullptr && a.K > kMsRowWords};
+					masked};
 			ms_pull(a, p, &ctl->work[lvl], actdeg, gathered, wq, s_act);
 		}
 		// the next frontier's out-degree: per-CTA sum, one atomic per CTA
@@ -1075,16 +1195,30 @@ __global__ void __launch_bounds__(kMsThreads, 2) k_ms_bfs(const __grid_constant_
 // tiles on small CTAs keep more chains going per SM.  A tile is kW words wide,
 // a thread per (vertex, word): with one or two words per vertex, tiles of four
 // would leave most threads idle.
-template <int kThreads, uint32_t kW>
+template <int kThreads, uint32_t kW, bool kShift>
 __global__ void __launch_bounds__(kThreads, kThreads == 256 ? 4 : 2) k_ms_emit(MsArgs a, uint32_t ns, uint8_t *levels) {
 	constexpr uint32_t kV = kThreads / kW;
-	__shared__ __align__(16) uint8_t lev[emit_bytes(kV, 2, kW)];
+	extern __shared__ __align__(16) uint8_t lev[];
 	const MsStats &st = a.ctl->stats;
 	if (!st.complete) return;
 	const uint32_t base = st.base, depth = st.depth;
 	const uint32_t first = base == 0 ? 0 : 1;
 	if (depth < base + first + 1) return;
-	ms_emit<true, kV, kW>(a, levels, ns, base, first, depth - 1 - base, base != 0, lev);
+	ms_emit<true, kV, kW, kShift>(a, levels, ns, base, first, depth - 1 - base, base != 0, lev);
+}
+
+// The output pass's launch for a tile of kThreads / kW vertices x kW words.
+template <int kThreads, uint32_t kW, bool kShift>
+int emit_launch(const MsArgs &a, uint32_t ns, uint8_t *levels, int num_sms, cudaStream_t st) {
+	constexpr int kBytes = (int) emit_bytes(kThreads / kW, 2, kW, kShift);
+	auto fn = k_ms_emit<kThreads, kW, kShift>;
+	if (kBytes > 48 * 1024 && cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, kBytes) != cudaSuccess)
+		return BFS_ECUDA;
+	int per_sm = 0;
+	if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, fn, kThreads, kBytes) != cudaSuccess || per_sm < 1)
+		return BFS_ECUDA;
+	fn<<<num_sms * per_sm, kThreads, kBytes, st>>>(a, ns, levels);
+	return cudaGetLastError() == cudaSuccess ? BFS_OK : BFS_ECUDA;
 }
 
 // chunk_slot[c]: the index of chunk c's destination in in_big (ascending).
@@ -1130,13 +1264,13 @@ int ms_launch(const MsArgs &a, const uint32_t *d_sources, uint32_t ns, uint8_t *
 	if (levels) {
 		const bool wide = a.out_tile ? a.out_tile == 128 : a.n >= kEmitWideMinVertices;
 		const uint32_t words = a.out_tile || a.K > 2 ? kEmitW : a.K;  // an explicit tile width is one of four-word tiles
-		void (*fn)(MsArgs, uint32_t, uint8_t *) = words == 1 ? k_ms_emit<256, 1> : words == 2 ? k_ms_emit<256, 2> :
-				wide ? k_ms_emit<512, kEmitW> : k_ms_emit<256, kEmitW>;
-		const int threads = words == kEmitW && wide ? 512 : 256;
-		int out_per_sm = 0;
-		if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&out_per_sm, fn, threads, 0) != cudaSuccess || out_per_sm < 1)
-			return BFS_ECUDA;
-		fn<<<num_sms * out_per_sm, threads, 0, st>>>(a, ns, levels);
+		const bool shift = a.n % 16 != 0 || (uintptr_t) levels % 16 != 0;
+		const auto launch = words == 1 ? (shift ? emit_launch<256, 1, true> : emit_launch<256, 1, false>)
+				: words == 2 ? (shift ? emit_launch<256, 2, true> : emit_launch<256, 2, false>)
+				: wide ? (shift ? emit_launch<512, kEmitW, true> : emit_launch<512, kEmitW, false>)
+				: (shift ? emit_launch<256, kEmitW, true> : emit_launch<256, kEmitW, false>);
+		const int rc = launch(a, ns, levels, num_sms, st);
+		if (rc) return rc;
 	}
 	return cudaGetLastError() == cudaSuccess ? BFS_OK : BFS_ECUDA;
 }

@@ -324,3 +324,29 @@ def test_words_per_vertex_and_degrees(native, oracle, words, push_div):
         exp = np.stack([expect[int(s)] for s in sources])
         for _ in range(2):  # the second run finds the first one's state
             _check(oracle, arr, g, sources, exp)
+
+
+@pytest.mark.parametrize("planes", [0, 3])
+@pytest.mark.parametrize("n", [1, 15, 16, 17, 63, 64, 65, 127, 129, 255, 256, 257, 1000, 4099])
+def test_rows_at_every_alignment(native, oracle, n, planes):
+    """Level rows that start on any byte (odd vertex counts, level buffers at odd
+    addresses), for tiles of one, two and four words, also when the output is
+    written early and merged (three level planes); nothing is written outside."""
+    import torch
+    import bfs_simd_benchmarks_gb300 as B
+    rng = np.random.default_rng(n)
+    src = np.concatenate([rng.integers(0, n, size=2 * n), np.arange(n - 1)]).astype(np.uint32)
+    dst = np.concatenate([rng.integers(0, n, size=2 * n), np.arange(1, n)]).astype(np.uint32)
+    arr = oracle.csr_arrays(n, src, dst)
+    with B.Graph.from_edges(n, src, dst, 64, 4) as g:
+        g.set_options(batch_single_max=0, batch_planes=planes)
+        for k in (5, 70, 150, 260):
+            sources = rng.integers(0, n, size=k).astype(np.uint32)
+            exp = _expect(oracle, arr, sources)
+            for offset in (0, 1, 6, 8):
+                buf = torch.full((k * n + 64,), 77, dtype=torch.uint8, device="cuda")
+                st = g.run_batch_device(sources, buf.data_ptr() + offset, stats=True)
+                assert st["status"] == 0
+                got = buf.cpu().numpy()
+                np.testing.assert_array_equal(got[offset:offset + k * n].reshape(k, n), exp)
+                assert (got[:offset] == 77).all() and (got[offset + k * n:] == 77).all()
