@@ -232,6 +232,35 @@ template <class T> int dev_alloc(bfs_graph *g, T **out, size_t count) {
 	return BFS_OK;
 }
 
+// Several device arrays in one allocation: add() them all, then allocate.
+struct DevArena {
+	struct Part {
+		void **out;
+		size_t bytes;
+	};
+	std::vector<Part> parts;
+	template <class T> void add(T **out, size_t count) {
+		parts.push_back({(void **) out, (std::max<size_t>(sizeof(T) * count, 16) + 255) & ~size_t(255)});
+	}
+	size_t bytes() const {
+		size_t b = 0;
+		for (const Part &p : parts) b += p.bytes;
+		return b;
+	}
+	void place(uint8_t *base) const {
+		for (const Part &p : parts) {
+			*p.out = base;
+			base += p.bytes;
+		}
+	}
+};
+int dev_alloc_all(bfs_graph *g, const DevArena &a) {
+	uint8_t *p = nullptr;
+	const int st = dev_alloc(g, &p, a.bytes());
+	if (!st) a.place(p);
+	return st;
+}
+
 template <class T> int dev_upload(bfs_graph *g, const T **out, const std::vector<T> &v) {
 	T *p = nullptr;
 	int st = dev_alloc(g, &p, v.size());
@@ -387,24 +416,25 @@ int alloc_run(bfs_graph *g) {
 	DevGraph &d = g->dg;
 	RunCtx &r = g->rc;
 	int st;
-	if ((st = dev_alloc(g, &r.vis, d.nwords))) return st;
+	DevArena ar;
+	ar.add(&r.vis, d.nwords);
 	for (int i = 0; i < 3; ++i) {
-		if ((st = dev_alloc(g, &r.bm[i], d.bm_words))) return st;
-		if ((st = dev_alloc(g, &r.sf[i], d.num_stripes))) return st;
+		ar.add(&r.bm[i], d.bm_words);
+		ar.add(&r.sf[i], d.num_stripes);
 	}
 	for (int set = 0; set < 2; ++set)
-		for (int b = 0; b < 3; ++b)
-			if ((st = dev_alloc(g, &r.q[set][b], g->n))) return st;
-	if ((st = dev_alloc(g, &r.ctr, 3))) return st;
-	if ((st = dev_alloc(g, &r.part, 6 * (size_t) kMaxGrid))) return st;
-	if ((st = dev_alloc(g, &r.stats, 1))) return st;
-	if ((st = dev_alloc(g, &r.bar, 2))) return st;
-	if ((st = dev_alloc(g, &r.err, 1))) return st;
+		for (int b = 0; b < 3; ++b) ar.add(&r.q[set][b], g->n);
+	ar.add(&r.ctr, 3);
+	ar.add(&r.part, 6 * (size_t) kMaxGrid);
+	ar.add(&r.stats, 1);
+	ar.add(&r.bar, 2);
+	ar.add(&r.err, 1);
+	ar.add(&g->level_buf, g->n);
+	ar.add(&g->parent_buf, g->n);
+	if ((st = dev_alloc_all(g, ar))) return st;
 	// the persistent kernel expects its barrier and status words zero at launch
 	if (cudaMemset(r.bar, 0, 2 * sizeof(unsigned)) != cudaSuccess || cudaMemset(r.err, 0, sizeof(int)) != cudaSuccess)
 		return BFS_ECUDA;
-	if ((st = dev_alloc(g, &g->level_buf, g->n))) return st;
-	if ((st = dev_alloc(g, &g->parent_buf, g->n))) return st;
 	if (cudaMallocHost(&g->h_stats, sizeof(DevStats)) != cudaSuccess) return BFS_ENOMEM;
 	if (cudaMallocHost(&g->h_part, sizeof(unsigned long long) * 2 * kMaxGrid) != cudaSuccess) return BFS_ENOMEM;
 	if (cudaEventCreate(&g->ev0) != cudaSuccess || cudaEventCreate(&g->ev1) != cudaSuccess ||
@@ -474,16 +504,34 @@ struct TmpDev {
 		*p = (T *) q;
 		return BFS_OK;
 	}
+	int alloc_all(const DevArena &a) {
+		uint8_t *p = nullptr;
+		const int st = alloc(&p, a.bytes());
+		if (!st) a.place(p);
+		return st;
+	}
 	~TmpDev() {
 		for (void *p : ptrs) cudaFree(p);
 	}
 };
 
+bool on_device(const void *p, int device) {
+	cudaPointerAttributes at{};
+	if (cudaPointerGetAttributes(&at, p) != cudaSuccess) {
+		cudaGetLastError();
+		return false;
+	}
+	return at.type == cudaMemoryTypeDevice && at.device == device;
+}
+
 // The device layout of an edge list built on the GPU (build_device.cu): CSR
-// and in-edge lists by degree histograms, scans and scatters; the packed
-// column-major segments by a segment histogram, the host's group plan and
-// segment offsets, and a scatter; the out-degrees and in-edge offsets come
-// back for the host-side fields.
+// and in-edge lists by degree histograms, scans and scatters; the batched
+// pull's lists from the degrees; the packed column-major segments by a segment
+// histogram over the in-edge lists, the host's group plan and segment offsets,
+// and a fill; the out-degrees come back for the host-side fields.  (Pokec
+// shape from device arrays, with a first traversal: 10.6 ms when the largest
+// degree and the lists were found on the host and every edge went to a global
+// counter for its segment.)
 int upload_device_build(bfs_graph *g, uint32_t n, uint64_t m, const uint32_t *src, const uint32_t *dst, uint32_t w,
 		uint32_t s, std::vector<uint32_t> *degree_order_out) {
 	g->n = n;
@@ -498,18 +546,31 @@ int upload_device_build(bfs_graph *g, uint32_t n, uint64_t m, const uint32_t *sr
 	cudaStream_t cs = nullptr;
 	TmpDev tmp;
 	DevGraph &d = g->dg;
-	uint32_t *d_src = nullptr, *d_dst = nullptr, *out_deg = nullptr, *in_deg = nullptr, *cursor = nullptr, *scan_tmp = nullptr;
+	// edge arrays already on this device are read where they are; host arrays
+	// (and edges to be relabelled) are copied
+	const bool in_place = m && !degree_order_out && on_device(src, g->device) && on_device(dst, g->device);
+	uint32_t *c_src = nullptr, *c_dst = nullptr, *out_deg = nullptr, *in_deg = nullptr, *cursor = nullptr, *scan_tmp = nullptr;
+	uint32_t *chunks = nullptr, *is_big = nullptr, *chunk_off = nullptr, *big_off = nullptr, *d_max = nullptr;
+	uint32_t *col_edges = nullptr;
 	int *d_err = nullptr;
-	if ((st = tmp.alloc(&d_src, m)) || (st = tmp.alloc(&d_dst, m)) || (st = tmp.alloc(&out_deg, n)) ||
-			(st = tmp.alloc(&in_deg, n)) || (st = tmp.alloc(&cursor, (size_t) n + 1)) ||
-			(st = tmp.alloc(&scan_tmp, dbuild_scan_tmp_words(n))) || (st = tmp.alloc(&d_err, 1)))
-		return st;
-	// host or device edge arrays (unified addressing tells them apart)
-	if (m && (cudaMemcpy(d_src, src, m * 4, cudaMemcpyDefault) != cudaSuccess ||
-			cudaMemcpy(d_dst, dst, m * 4, cudaMemcpyDefault) != cudaSuccess))
+	DevArena ta;
+	if (!in_place) {
+		ta.add(&c_src, m);
+		ta.add(&c_dst, m);
+	}
+	for (uint32_t **p : {&out_deg, &in_deg, &chunks, &is_big}) ta.add(p, n);
+	for (uint32_t **p : {&cursor, &chunk_off, &big_off}) ta.add(p, (size_t) n + 1);
+	ta.add(&scan_tmp, dbuild_scan_tmp_words(n));
+	ta.add(&col_edges, g->side);
+	ta.add(&d_err, 1);
+	ta.add(&d_max, 1);
+	if ((st = tmp.alloc_all(ta))) return st;
+	if (m && !in_place && (cudaMemcpy(c_src, src, m * 4, cudaMemcpyDefault) != cudaSuccess ||
+			cudaMemcpy(c_dst, dst, m * 4, cudaMemcpyDefault) != cudaSuccess))
 		return BFS_ECUDA;
+	const uint32_t *d_src = in_place ? src : c_src, *d_dst = in_place ? dst : c_dst;
 	if (cudaMemset(out_deg, 0, (size_t) n * 4) != cudaSuccess || cudaMemset(in_deg, 0, (size_t) n * 4) != cudaSuccess ||
-			cudaMemset(d_err, 0, 4) != cudaSuccess)
+			cudaMemset(d_err, 0, 4) != cudaSuccess || cudaMemset(d_max, 0, 4) != cudaSuccess)
 		return BFS_ECUDA;
 	if ((st = dbuild_degrees(d_src, d_dst, m, n, out_deg, in_deg, d_err, g->num_sms, cs))) return st;
 	int herr = 0;
@@ -524,16 +585,20 @@ int upload_device_build(bfs_graph *g, uint32_t n, uint64_t m, const uint32_t *sr
 		if ((st = tmp.alloc(&d_map, n))) return st;
 		if (cudaMemcpy(d_map, degree_order_out->data(), (size_t) n * 4, cudaMemcpyHostToDevice) != cudaSuccess)
 			return BFS_ECUDA;
-		k_relabel_edges<<<g->num_sms * 8, 512, 0, cs>>>(m, d_map, d_src, d_dst);
+		k_relabel_edges<<<g->num_sms * 8, 512, 0, cs>>>(m, d_map, c_src, c_dst);
 		if (cudaMemset(out_deg, 0, (size_t) n * 4) != cudaSuccess || cudaMemset(in_deg, 0, (size_t) n * 4) != cudaSuccess)
 			return BFS_ECUDA;
 		if ((st = dbuild_degrees(d_src, d_dst, m, n, out_deg, in_deg, d_err, g->num_sms, cs))) return st;
 	}
 	// CSR and in-edge lists
-	uint32_t *row_off = nullptr, *col = nullptr, *in_off = nullptr, *in_src = nullptr;
-	if ((st = dev_alloc(g, &row_off, (size_t) n + 1)) || (st = dev_alloc(g, &col, m)) ||
-			(st = dev_alloc(g, &in_off, (size_t) n + 1)) || (st = dev_alloc(g, &in_src, m)))
-		return st;
+	uint32_t *row_off = nullptr, *col = nullptr, *in_off = nullptr, *in_src = nullptr, *hasin = nullptr;
+	DevArena la;
+	la.add(&row_off, (size_t) n + 1);
+	la.add(&in_off, (size_t) n + 1);
+	la.add(&hasin, ((size_t) n + 31) / 32);
+	la.add(&col, m);
+	la.add(&in_src, m);
+	if ((st = dev_alloc_all(g, la))) return st;
 	if ((st = dbuild_exclusive_scan(out_deg, n, scan_tmp, row_off, cs))) return st;
 	if (cudaMemcpy(cursor, row_off, (size_t) n * 4, cudaMemcpyDeviceToDevice) != cudaSuccess) return BFS_ECUDA;
 	if ((st = dbuild_scatter(d_src, d_dst, m, cursor, col, g->num_sms, cs))) return st;
@@ -544,25 +609,34 @@ int upload_device_build(bfs_graph *g, uint32_t n, uint64_t m, const uint32_t *sr
 	d.col = col;
 	d.in_off = in_off;
 	d.in_src = in_src;
-	// host-side fields
+	// what follows from the degrees: the has-in bitmap, the largest out-degree,
+	// the batched pull's lists, the in-edges per tile column
+	if ((st = dbuild_vertex_facts(out_deg, in_deg, n, kMsPullBig, kMsChunk, hasin, chunks, is_big, d_max, g->num_sms, cs)) ||
+			(st = dbuild_exclusive_scan(chunks, n, scan_tmp, chunk_off, cs)) ||
+			(st = dbuild_exclusive_scan(is_big, n, scan_tmp, big_off, cs)) ||
+			(st = dbuild_col_edges(in_off, n, w, g->side, col_edges, cs)))
+		return st;
 	g->degrees.resize(n);
-	std::vector<uint32_t> h_in_off((size_t) n + 1);
-	if (cudaMemcpy(g->degrees.data(), out_deg, (size_t) n * 4, cudaMemcpyDeviceToHost) != cudaSuccess ||
-			cudaMemcpy(h_in_off.data(), in_off, ((size_t) n + 1) * 4, cudaMemcpyDeviceToHost) != cudaSuccess)
-		return BFS_ECUDA;
-	g->max_degree = 0;
-	for (uint32_t v = 0; v < n; ++v) g->max_degree = std::max(g->max_degree, g->degrees[v]);
-	if ((st = upload_big_in(g, h_in_off))) return st;
-	// packed column-major segments
-	uint32_t *col_edges = nullptr, *hasin = nullptr;
-	if ((st = tmp.alloc(&col_edges, g->side)) || (st = dev_alloc(g, &hasin, ((size_t) n + 31) / 32))) return st;
-	if (cudaMemset(col_edges, 0, (size_t) g->side * 4) != cudaSuccess ||
-			cudaMemset(hasin, 0, ((size_t) n + 31) / 32 * 4) != cudaSuccess)
-		return BFS_ECUDA;
-	if ((st = dbuild_col_hist(d_dst, m, w, g->side, col_edges, hasin, g->num_sms, cs))) return st;
 	std::vector<uint32_t> h_col32(g->side);
-	if (cudaMemcpy(h_col32.data(), col_edges, (size_t) g->side * 4, cudaMemcpyDeviceToHost) != cudaSuccess)
+	if (cudaMemcpy(g->degrees.data(), out_deg, (size_t) n * 4, cudaMemcpyDeviceToHost) != cudaSuccess ||
+			cudaMemcpy(&g->max_degree, d_max, 4, cudaMemcpyDeviceToHost) != cudaSuccess ||
+			cudaMemcpy(&g->ms_nchunks, chunk_off + n, 4, cudaMemcpyDeviceToHost) != cudaSuccess ||
+			cudaMemcpy(&g->ms_nbig_in, big_off + n, 4, cudaMemcpyDeviceToHost) != cudaSuccess ||
+			cudaMemcpy(h_col32.data(), col_edges, (size_t) g->side * 4, cudaMemcpyDeviceToHost) != cudaSuccess)
 		return BFS_ECUDA;
+	uint32_t *in_big = nullptr, *chunk_v = nullptr, *chunk_beg = nullptr;
+	DevArena ca;
+	ca.add(&in_big, g->ms_nbig_in);
+	ca.add(&chunk_v, g->ms_nchunks);
+	ca.add(&chunk_beg, g->ms_nchunks);
+	if ((st = dev_alloc_all(g, ca)) ||
+			(st = dbuild_big_lists(n, big_off, chunk_off, in_off, g->ms_nchunks, kMsChunk, in_big, chunk_v, chunk_beg,
+					 g->num_sms, cs)))
+		return st;
+	g->ms_in_big = in_big;
+	g->ms_chunk_v = chunk_v;
+	g->ms_chunk_beg = chunk_beg;
+	// packed column-major segments
 	std::vector<uint64_t> h_col(h_col32.begin(), h_col32.end());
 	PackedTiles pk;
 	if ((st = plan_groups(n, w, s, g->side, h_col, m, (uint32_t) g->num_sms * 2 * kGroupsPerCta, kMaxGroupVertices, pk)))
@@ -571,17 +645,28 @@ int upload_device_build(bfs_graph *g, uint32_t n, uint64_t m, const uint32_t *sr
 	for (uint32_t gi = 0; gi < pk.num_groups; ++gi)
 		for (uint32_t c = pk.group_col[gi]; c < pk.group_col[gi + 1]; ++c) group_of[c] = gi;
 	const uint64_t nseg = (uint64_t) g->num_stripes * pk.num_groups;
+	const bool by_lists = dbuild_seg_items_fit(g->num_stripes);
+	std::vector<SegItem> items;
+	if (by_lists) items = dbuild_seg_items(pk.group_col, h_col);
 	uint32_t *d_group_of = nullptr, *seg_count = nullptr, *seg_cursor = nullptr, *pad = nullptr;
-	if ((st = tmp.alloc(&d_group_of, g->side)) || (st = tmp.alloc(&seg_count, nseg)) || (st = tmp.alloc(&seg_cursor, nseg)) ||
-			(st = tmp.alloc(&pad, pk.num_groups)))
-		return st;
+	SegItem *d_items = nullptr;
+	DevArena sa;
+	if (by_lists) sa.add(&d_items, items.size());
+	else sa.add(&d_group_of, g->side);
+	sa.add(&seg_count, nseg);
+	sa.add(&seg_cursor, nseg);
+	sa.add(&pad, pk.num_groups);
+	if ((st = tmp.alloc_all(sa))) return st;
 	const uint32_t *group_col = nullptr;
 	if ((st = dev_upload(g, &group_col, pk.group_col))) return st;
-	if (cudaMemcpy(d_group_of, group_of.data(), (size_t) g->side * 4, cudaMemcpyHostToDevice) != cudaSuccess ||
+	if ((by_lists ? cudaMemcpy(d_items, items.data(), items.size() * sizeof(SegItem), cudaMemcpyHostToDevice)
+	              : cudaMemcpy(d_group_of, group_of.data(), (size_t) g->side * 4, cudaMemcpyHostToDevice)) != cudaSuccess ||
 			cudaMemset(seg_count, 0, nseg * 4) != cudaSuccess)
 		return BFS_ECUDA;
 	DeviceBuildShape sh{w, s, g->num_stripes, pk.vbits, pk.cbits};
-	if ((st = dbuild_seg_hist(d_src, d_dst, m, sh, d_group_of, seg_count, g->num_sms, cs))) return st;
+	st = by_lists ? dbuild_seg_count(in_src, d_items, (uint32_t) items.size(), s * w, g->num_stripes, seg_count, cs)
+	              : dbuild_seg_hist(d_src, d_dst, m, sh, d_group_of, seg_count, g->num_sms, cs);
+	if (st) return st;
 	std::vector<uint32_t> h_seg32(nseg);
 	if (cudaMemcpy(h_seg32.data(), seg_count, nseg * 4, cudaMemcpyDeviceToHost) != cudaSuccess) return BFS_ECUDA;
 	std::vector<uint64_t> h_seg(h_seg32.begin(), h_seg32.end());
@@ -595,7 +680,9 @@ int upload_device_build(bfs_graph *g, uint32_t n, uint64_t m, const uint32_t *sr
 	if (cudaMemcpy(seg_cursor, seg_off, nseg * 4, cudaMemcpyDeviceToDevice) != cudaSuccess ||
 			cudaMemcpy(pad, pad_word.data(), pk.num_groups * 4, cudaMemcpyHostToDevice) != cudaSuccess)
 		return BFS_ECUDA;
-	if ((st = dbuild_seg_fill(d_src, d_dst, m, sh, d_group_of, group_col, seg_cursor, packed, g->num_sms, cs))) return st;
+	st = by_lists ? dbuild_seg_pack(in_off, in_src, d_items, (uint32_t) items.size(), sh, group_col, n, seg_cursor, packed, cs)
+	              : dbuild_seg_fill(d_src, d_dst, m, sh, d_group_of, group_col, seg_cursor, packed, g->num_sms, cs);
+	if (st) return st;
 	if ((st = dbuild_seg_pad(seg_off, seg_count, nseg, g->num_stripes, pad, packed, g->num_sms, cs))) return st;
 	if (cudaDeviceSynchronize() != cudaSuccess) return BFS_ECUDA;
 	d.packed = packed;

@@ -3,6 +3,8 @@
 #pragma once
 
 #include <cstdint>
+#include <vector>
+
 #include <cuda_runtime.h>
 
 namespace bfsg {
@@ -23,9 +25,31 @@ int dbuild_exclusive_scan(const uint32_t *in, uint32_t n, uint32_t *tmp, uint32_
 // out[cursor[key[i]]++] = val[i]
 int dbuild_scatter(const uint32_t *key, const uint32_t *val, uint64_t m, uint32_t *cursor, uint32_t *out, int num_sms,
 		cudaStream_t st);
-// in-edges per tile column and the has-in-edge bitmap (both zeroed by the caller)
-int dbuild_col_hist(const uint32_t *dst, uint64_t m, uint32_t w, uint32_t side, uint32_t *col_edges, uint32_t *hasin,
-		int num_sms, cudaStream_t st);
+// From the degrees: the has-in-edge bitmap, per vertex the batched pull's
+// chunks of `chunk` in-edges (0 up to `big` of them) and whether there are
+// any, and the largest out-degree (*max_degree zeroed by the caller).
+int dbuild_vertex_facts(const uint32_t *out_deg, const uint32_t *in_deg, uint32_t n, uint32_t big, uint32_t chunk,
+		uint32_t *hasin, uint32_t *chunks, uint32_t *is_big, uint32_t *max_degree, int num_sms, cudaStream_t st);
+// The batched pull's lists from the exclusive scans of is_big and chunks.
+int dbuild_big_lists(uint32_t n, const uint32_t *big_off, const uint32_t *chunk_off, const uint32_t *in_off,
+		uint32_t nchunks, uint32_t chunk, uint32_t *in_big, uint32_t *chunk_v, uint32_t *chunk_beg, int num_sms,
+		cudaStream_t st);
+// in-edges per tile column
+int dbuild_col_edges(const uint32_t *in_off, uint32_t n, uint32_t w, uint32_t side, uint32_t *col_edges, cudaStream_t st);
+
+// A run of one column group's in-edges, the work of one CTA.
+struct SegItem {
+	uint32_t group, beg, end;
+};
+// Whether a CTA can count this many stripes in shared memory; graphs with more
+// take the per-edge dbuild_seg_hist and dbuild_seg_fill.
+bool dbuild_seg_items_fit(uint32_t stripes);
+std::vector<SegItem> dbuild_seg_items(const std::vector<uint32_t> &group_col, const std::vector<uint64_t> &col_edges);
+// dbuild_seg_hist and dbuild_seg_fill from the in-edge lists
+int dbuild_seg_count(const uint32_t *in_src, const SegItem *items, uint32_t num_items, uint32_t sw, uint32_t stripes,
+		uint32_t *seg_count, cudaStream_t st);
+int dbuild_seg_pack(const uint32_t *in_off, const uint32_t *in_src, const SegItem *items, uint32_t num_items,
+		const DeviceBuildShape &sh, const uint32_t *group_col, uint32_t n, uint32_t *cursor, uint32_t *words, cudaStream_t st);
 // edges per packed segment (group(v) * stripes + stripe(u)), zeroed by the caller
 int dbuild_seg_hist(const uint32_t *src, const uint32_t *dst, uint64_t m, const DeviceBuildShape &sh,
 		const uint32_t *group_of, uint32_t *seg_count, int num_sms, cudaStream_t st);

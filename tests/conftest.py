@@ -1,6 +1,7 @@
 """Shared test setup: the `gpu` marker, library builds and golden fixtures."""
 from __future__ import annotations
 
+import gc
 import json
 import os
 import sys
@@ -16,6 +17,13 @@ if ROOT not in sys.path:
 
 def pytest_configure(config):
     config.addinivalue_line("markers", "gpu: needs a CUDA GPU (GB300); runs the CUDA path through the C ABI")
+
+
+@pytest.fixture(scope="module", autouse=True)
+def _no_garbage_from_other_files():
+    """Tensors that a caught exception's traceback keeps are freed before a file starts,
+    not at some allocation inside a test that compares device memory."""
+    gc.collect()
 
 
 @pytest.fixture(scope="session")

@@ -370,3 +370,59 @@ def test_bfs_run_into_pinned_host_memory(native, oracle):
         # pageable buffers through the same call
         lev2, par2, _ = g.run(int(sources[0]))
         np.testing.assert_array_equal(lev2, oracle.bfs_levels(arr, int(sources[0])))
+
+
+def _lists_case(name):
+    rng = np.random.default_rng(len(name))
+    if name == "many_stripes":      # more stripes than a CTA counts in shared memory
+        n, w, s = 16 * 12289, 16, 1
+    elif name == "stripes_at_limit":
+        n, w, s = 16 * 12288, 16, 1
+    else:
+        n, w, s = 50_001, 256, 4
+    if name == "gaps":               # few destinations, far apart; long lists and lists of 255-257
+        heads = np.concatenate([np.full(40_000, 17), np.full(255, 900), np.full(256, 901), np.full(257, 49_000),
+                                np.full(32_768, 50_000)])
+        src, dst = rng.integers(0, n, size=heads.size), heads
+    elif name == "one_edge":
+        src, dst = np.array([3]), np.array([50_000])
+    elif name == "empty":
+        src, dst = np.zeros(0, np.int64), np.zeros(0, np.int64)
+    else:
+        src, dst = rng.integers(0, n, size=6 * n), rng.integers(0, n, size=6 * n)
+    return n, w, s, src.astype(np.uint32), dst.astype(np.uint32)
+
+
+@pytest.mark.parametrize("where", ["host", "device"])
+@pytest.mark.parametrize("name", ["many_stripes", "stripes_at_limit", "random", "gaps", "one_edge", "empty"])
+def test_device_build_lists_and_segments(native, oracle, name, where):
+    """The device build's lists and packed segments, through every traversal that reads
+    them (pull, streamed tiles, batched), from host and from device edge arrays."""
+    import torch
+    import bfs_simd_benchmarks_gb300 as B
+    n, w, s, src, dst = _lists_case(name)
+    arr = oracle.arrays_from_edges(n, src, dst, w, s)
+    if where == "host":
+        g = B.Graph.from_edges(n, src, dst, w, s, device_build=True)
+    else:
+        ds, dd = torch.from_numpy(src.astype(np.int32)).cuda(), torch.from_numpy(dst.astype(np.int32)).cuda()
+        g = B.Graph.from_device_edges(n, ds.data_ptr(), dd.data_ptr(), src.size, w, s)
+        assert (ds.cpu().numpy() == src.astype(np.int32)).all() and (dd.cpu().numpy() == dst.astype(np.int32)).all()
+        del ds, dd
+    with g, B.Graph.from_edges(n, src, dst, w, s) as host:
+        np.testing.assert_array_equal(g.degrees(), arr["degrees"])
+        a, b = g.info(), host.info()
+        for k in ("num_groups", "packed_words", "max_out_degree", "num_stripes"):
+            assert a[k] == b[k], k
+        sources = [int(x) for x in (src[:3] if src.size else np.array([0, n - 1]))]
+        for bottom_up in ("pull", "stream"):
+            g.set_options(bottom_up=bottom_up, to_dense_ratio=1 << 30, to_sparse_ratio=1 << 30)
+            for x in sources:
+                lev, par, st = g.run(x)
+                np.testing.assert_array_equal(lev, oracle.bfs_levels(arr, x))
+                assert oracle.check_parents(arr, x, lev, par) == 0
+        g.set_options(batch_single_max=0, batch_push_div=1 << 30)
+        rows, _ = g.run_batch(np.asarray(sources, np.uint32))
+        for i, x in enumerate(sources):
+            ref = oracle.bfs_levels(arr, x)
+            np.testing.assert_array_equal(rows[i].cpu().numpy(), np.where(ref < 0, 255, ref).astype(np.uint8))
