@@ -198,8 +198,7 @@ class Stats(C.Structure):
     ]
 
     def as_dict(self) -> dict:
-        arrays = ("trace", "step_ms", "step_work_min_ms", "step_work_max_ms", "bu_cycles")
-        d = {k: getattr(self, k) for k, _ in self._fields_ if k not in arrays}
+        d = {k: getattr(self, k) for k in _STATS_SCALARS}
         d["bu_cycles"] = list(self.bu_cycles[:6])
         k = min(self.num_steps, BFS_TRACE_MAX)
         d["trace"] = list(self.trace[:k])
@@ -207,6 +206,8 @@ class Stats(C.Structure):
             d[name] = [round(x, 5) for x in getattr(self, name)[:k]]
         return d
 
+
+_STATS_SCALARS = tuple(k for k, t in Stats._fields_ if not issubclass(t, C.Array))
 
 BFS_TUNE_SINGLE, BFS_TUNE_BATCH, BFS_TUNE_MAX_TRIALS = 1, 2, 256
 BFS_TUNE_DEVICE_BUILD, BFS_TUNE_LAYOUTS = 4, 8

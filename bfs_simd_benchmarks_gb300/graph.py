@@ -21,6 +21,9 @@ def _u32(a) -> np.ndarray:
     return np.ascontiguousarray(a, dtype=np.uint32)
 
 
+_i32p, _u32p = C.POINTER(C.c_int32), C.POINTER(C.c_uint32)
+
+
 def _ptr(a: np.ndarray, ctype):
     return a.ctypes.data_as(C.POINTER(ctype))
 
@@ -30,6 +33,7 @@ class Graph:
 
     def __init__(self, handle: C.c_void_p):
         self._h = handle
+        self._n = None  # vertices, fixed for a handle
 
     # ---- construction -------------------------------------------------
     @classmethod
@@ -128,7 +132,9 @@ class Graph:
 
     @property
     def num_vertices(self) -> int:
-        return self.info()["num_vertices"]
+        if self._n is None:
+            self._n = self.info()["num_vertices"]
+        return self._n
 
     def degrees(self) -> np.ndarray:
         n = self.num_vertices
@@ -168,9 +174,10 @@ class Graph:
         lev = np.empty(n, dtype=np.int32)
         par = np.empty(n, dtype=np.uint32) if parents else None
         st = N.Stats()
-        N.check(N.load().bfs_run(self._h, int(source), _ptr(lev, C.c_int32),
-                                 None if par is None else _ptr(par, C.c_uint32), C.byref(st)),
-                f"bfs_run(source={source})")
+        rc = N.load().bfs_run(self._h, int(source), C.cast(lev.ctypes.data, _i32p),
+                              None if par is None else C.cast(par.ctypes.data, _u32p), C.byref(st))
+        if rc:
+            N.check(rc, f"bfs_run(source={source})")
         return lev, par, st.as_dict()
 
     def bfs_order(self, source: int = 0) -> np.ndarray:
