@@ -53,6 +53,7 @@ struct bfs_graph {
 	size_t smem = 0;
 	// by bottom-up variant: CTAs of the cooperative grid at full occupancy and
 	// their shared memory (grid, smem: as the options ask)
+	int cluster = 0;   // CTAs of the one-cluster traversal, 0: not for this graph
 	int grid_max[2] = {0, 0};
 	size_t smem_of[2] = {0, 0};
 	std::vector<DevBuf> bufs;
@@ -75,6 +76,7 @@ struct bfs_graph {
 	bool stats_fresh = false;
 	bool have_run = false;
 	bool stepwise_last = false;
+	bool cluster_last = false;       // the last run was in one cluster
 	bfs_stats host_stats{};          // stepwise-mode bookkeeping
 	bfs_options opt{};
 	uint32_t num_groups = 0;
@@ -477,8 +479,21 @@ int alloc_run(bfs_graph *g) {
 	g->batch = std::max<uint32_t>(1, std::min<uint32_t>(kMaxSliceBatch, kSliceBudgetWords / std::max<uint32_t>(1, d.slice_words)));
 	for (uint32_t bu : {BFS_BU_PULL, BFS_BU_STREAM})
 		if ((st = persistent_grid(d, g->batch, bu, g->device, g->num_sms, &g->grid_max[bu], &g->smem_of[bu]))) return st;
+	g->cluster = cluster_ctas(d);
 	apply_grid(g);
 	return BFS_OK;
+}
+
+// Whether a traversal runs in one cluster: small graphs with the default
+// variant and launch shape (and no test hook on the grid barriers).
+bool in_cluster(const bfs_graph *g) {
+	const bfs_options &o = g->opt;
+	return g->cluster && o.mode == BFS_MODE_PERSISTENT && o.bottom_up == BFS_BU_PULL && o.ctas_per_sm == 0 &&
+			o.test_hold_barrier == 0;
+}
+int launch_traversal(bfs_graph *g, const RunCtx &r, const StepParams &p, cudaStream_t st) {
+	return in_cluster(g) ? launch_cluster(g->dg, r, p, g->cluster, st)
+	                     : launch_persistent(g->dg, r, p, g->batch, g->grid, g->smem, st);
 }
 
 // Builds the device copy of a validated host graph.
@@ -868,6 +883,7 @@ int run_impl(bfs_graph *g, uint32_t source, int32_t *levels, uint32_t *parents, 
 	p.beta = g->opt.td_beta;
 	int rc;
 	g->stepwise_last = g->opt.mode == BFS_MODE_STEPWISE;
+	g->cluster_last = in_cluster(g);
 	if (cudaEventRecord(g->ev0, st) != cudaSuccess) return BFS_ECUDA;
 	// the persistent kernel clears the run state and seeds the source itself;
 	// the stepwise host loop clears and seeds with launches of their own
@@ -876,7 +892,7 @@ int run_impl(bfs_graph *g, uint32_t source, int32_t *levels, uint32_t *parents, 
 	if (g->stepwise_last) {
 		if ((rc = run_stepwise(g, r, p, st))) return rc;
 	} else {
-		if ((rc = launch_persistent(g->dg, r, p, g->batch, g->grid, g->smem, st))) return rc;
+		if ((rc = launch_traversal(g, r, p, st))) return rc;
 	}
 	if (g->relabeled) {
 		k_unrelabel<<<g->num_sms * 4, 512, 0, st>>>(g->n, g->d_new_of_old, g->d_old_of_new, r.level, r.parent, levels,
@@ -933,7 +949,7 @@ int collect_stats(bfs_graph *g, bfs_stats *out) {
 	s.bu_vertices = d.bu_vertices;
 	s.status = g->stepwise_last ? BFS_OK : d.status;
 	s.max_level = s.num_steps ? s.num_steps - 1 : 0;
-	s.grid_ctas = (uint32_t) g->grid;
+	s.grid_ctas = (uint32_t) (g->cluster_last ? g->cluster : g->grid);
 	float ms = 0, kms = 0;
 	cudaEventElapsedTime(&ms, g->ev0, g->ev1);
 	cudaEventElapsedTime(&kms, g->evm, g->ev1);
@@ -1121,7 +1137,7 @@ int run_batch_impl(bfs_graph *g, const uint32_t *sources, uint32_t ns, uint8_t *
 		p.beta = g->opt.td_beta;
 		for (uint32_t i = 0; i < ns; ++i) {
 			p.source = sources[i];
-			if ((rc = launch_persistent(g->dg, r, p, g->batch, g->grid, g->smem, st))) return rc;
+			if ((rc = launch_traversal(g, r, p, st))) return rc;
 			k_levels_u8<<<g->num_sms * 4, 512, 0, st>>>(g->level_buf, levels + (size_t) i * g->n, g->n, r.stats, a.ctl);
 		}
 		if (cudaGetLastError() != cudaSuccess) return BFS_ECUDA;
@@ -1265,7 +1281,7 @@ int bc_enqueue(bfs_graph *g, uint32_t source, uint32_t *sigma, float *delta, flo
 	p.beta = g->opt.td_beta;
 	int rc;
 	if (cudaEventRecord(b.e0, st) != cudaSuccess) return BFS_ECUDA;
-	if ((rc = launch_persistent(g->dg, r, p, g->batch, g->grid, g->smem, st))) return rc;
+	if ((rc = launch_traversal(g, r, p, st))) return rc;
 	if (cudaEventRecord(b.e1, st) != cudaSuccess) return BFS_ECUDA;
 	BcArgs a{};
 	a.n = g->n;

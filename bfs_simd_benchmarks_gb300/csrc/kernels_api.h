@@ -30,6 +30,13 @@ int persistent_grid(const DevGraph &g, uint32_t batch, uint32_t bottom_up, int d
 int launch_init(const DevGraph &g, const RunCtx &r, cudaStream_t st, int num_sms);
 int launch_persistent(const DevGraph &g, const RunCtx &r, const StepParams &p, uint32_t batch, int grid,
 		size_t smem, cudaStream_t st);
+// The one-cluster traversal (bfs_cluster.cu): CTAs of its cluster for a graph,
+// 0 where the graph is too large for it (or the device takes no such cluster).
+constexpr uint32_t kClusterMaxVertices = 3u << 15;
+constexpr uint32_t kClusterMaxEdges = 1u << 24;
+constexpr uint32_t kClusterVerticesPerCta = 1024;
+int cluster_ctas(const DevGraph &g);
+int launch_cluster(const DevGraph &g, const RunCtx &r, const StepParams &p, int ctas, cudaStream_t st);
 int launch_step(int kind, const DevGraph &g, const RunCtx &r, const StepParams &p, uint32_t step,
 		uint32_t batch, int grid, size_t smem, cudaStream_t st);
 int kernel_threads();

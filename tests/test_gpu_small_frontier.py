@@ -109,3 +109,48 @@ def test_a_smaller_graph_leaves_a_larger_one_callable(native, oracle):
                     assert st["status"] == 0
                     np.testing.assert_array_equal(lev, ref)
             np.testing.assert_array_equal(small.run(0)[0], [0, 1, 2])
+
+
+def _mixed(n, seed):
+    """Random edges, a hub whose long in-edge list starts at unreachable vertices, a hub with many out-edges."""
+    rng = np.random.default_rng(seed)
+    src = [rng.integers(0, n, size=3 * n)]
+    dst = [rng.integers(0, n, size=3 * n)]
+    if n > 1000:
+        island = np.arange(n - n // 8, n)          # only out-edges: never reached
+        keep = dst[0] < n - n // 8
+        src[0], dst[0] = src[0][keep], dst[0][keep]
+        src.append(np.repeat(island, 2)[:9000])
+        dst.append(np.full(src[-1].size, 5))
+        src.append(np.full(3000, 7))
+        dst.append(rng.integers(0, n // 2, size=3000))
+    return np.concatenate(src).astype(np.uint32), np.concatenate(dst).astype(np.uint32)
+
+
+@pytest.mark.parametrize("n", [1, 31, 33, 1024, 1025, 4097, 20_000, 98_304, 98_305])
+def test_one_cluster_traversal(native, oracle, n):
+    """Small graphs are traversed in one cluster: its sizes, both directions at every
+    step and mixed ones, against the oracle and the whole grid's step sequence."""
+    import bfs_simd_benchmarks_gb300 as B
+    src, dst = _mixed(n, n)
+    arr = oracle.arrays_from_edges(n, src, dst, 256, 4)
+    deg = arr["degrees"].astype(np.uint64)
+    with B.Graph.from_edges(n, src, dst, 256, 4) as g:
+        for s in sorted({0, n // 3, min(7, n - 1)}):
+            ref = oracle.bfs_levels(arr, s)
+            for opts in ({}, {"switch_rule": 1}, {"to_dense_ratio": 1, "to_sparse_ratio": 1},
+                         {"to_dense_ratio": 1 << 30, "to_sparse_ratio": 1 << 30}):
+                g.set_options(**{"switch_rule": 0, "to_dense_ratio": 20, "to_sparse_ratio": 20, "ctas_per_sm": 0, **opts})
+                lev, par, st = g.run(s)
+                np.testing.assert_array_equal(lev, ref)
+                assert oracle.check_parents(arr, s, lev, par) == 0
+                assert st["reached"] == int((ref >= 0).sum()) and st["num_steps"] == ref.max() + 1
+                assert st["edges_traversed"] == int(deg[ref >= 0].sum())
+                assert (st["grid_ctas"] <= 16) == (n <= 98_304)
+                np.testing.assert_array_equal(g.run(s, parents=False)[0], ref)
+                g.set_options(ctas_per_sm=2)
+                lev2, _, st2 = g.run(s)
+                assert st2["grid_ctas"] > 16
+                np.testing.assert_array_equal(lev2, ref)
+                for k in ("trace", "dense_steps", "td_edges", "td_vertices", "num_steps"):
+                    assert st[k] == st2[k], (k, opts)
