@@ -1224,8 +1224,19 @@ __global__ void k_seed(DevGraph g, RunCtx r, StepParams p) {
 // ---------------------------------------------------------------------------
 // A step of the whole grid costs about 6 us however little it does: the grid
 // barrier, the totals and a chain of round trips.  While the frontier has at
-// most kSoloCap vertices and out-edges, CTA 0 therefore takes the steps by
+// most solo_cap vertices and out-edges, CTA 0 therefore takes the steps by
 // itself, and the other CTAs wait at the round's grid barrier.
+//
+// The cap is kSoloCap while the visited bits fit in shared memory.  On larger
+// graphs one SM's claims and row offsets are slow, and so are the queues on
+// either side of a round (one step of 128 edges 9.9 us, the grid's 7.7; one of
+// 1700 edges at 2^20 vertices 16 us, the grid's 10): it pays only when many
+// such steps follow, so there the frontier's out-edges must have neither
+// doubled nor halved since the frontier before (`prev` out-edges).
+__device__ __forceinline__ uint32_t solo_cap(const DevGraph &g, unsigned long long prev, unsigned long long ne) {
+	return g.nwords <= kSoloVisWords || (ne <= 2 * prev && prev <= 2 * ne) ? kSoloCap : 0u;
+}
+
 // Called by every thread of CTA 0: expands the frontier of `step` (queue
 // sizes tails[]) and the ones after it until one is too large, goes
 // bottom-up, is empty, or kSoloLevels steps are done; that one becomes the
@@ -1270,9 +1281,10 @@ __device__ __forceinline__ void phase_solo(const DevGraph &g, const RunCtx &r, c
 		else solo_expand<kTdPerLane, kThreads>(g, r, cur, nxt, cn, ne, nl, vis_s);
 		__syncthreads();
 		++done;
+		const uint32_t prev = ne;
 		nv = cn[0];
 		ne = cn[1];
-		if (nv == 0 || ne > kSoloCap || done == kSoloLevels ||
+		if (nv == 0 || ne > solo_cap(g, prev, ne) || done == kSoloLevels ||
 				goes_dense(g, p, nv, ne, seen + skipped + ne, false))
 			break;
 		skipped += ne;
@@ -1320,6 +1332,7 @@ __global__ void __launch_bounds__(kThreads, 2) k_bfs_persistent(DevGraph g, RunC
 	uint32_t st_dense = 0;
 	unsigned epoch = 0;  // grid barriers this CTA has passed
 	unsigned long long seen = 0;  // out-edges of the vertices reached so far (frontiers included)
+	unsigned long long prev_dsum = 0;  // out-edges of the round before's frontier
 	bool last_dense = false;
 	uint32_t step = 0;
 	CTA_STAMP(15, 0);  // profiling builds: the prologue in the slot of step 15
@@ -1369,10 +1382,12 @@ __global__ void __launch_bounds__(kThreads, 2) k_bfs_persistent(DevGraph g, RunC
 				tails[2] = s_conv_tails[2];
 			}
 			CTA_STAMP(step, 3);
-			solo = fsize <= kSoloCap && dsum <= kSoloCap;
+			const uint32_t cap = solo_cap(g, prev_dsum, dsum);
+			solo = fsize <= cap && dsum <= cap;
 			if (!solo) phase_expand(g, r, p, rnd, (int32_t) step + 1, tails[0], tails[1], tails[2], smem, acc);
 			else if (blockIdx.x == 0) phase_solo(g, r, p, rnd, step, tails, seen, smem, acc, st_reached, st_edges);
 		}
+		prev_dsum = dsum;
 		CTA_STAMP(step, 4);
 		flush_step(acc, r, rnd % 3);
 		CTA_STAMP(step, 5);

@@ -51,8 +51,7 @@ __device__ __forceinline__ SoloList solo_list(uint32_t *smem, uint32_t which) {
 
 // Appends the lanes' vertices v[q] (ok[q]; out-edges beg[q], deg[q]) to `l`;
 // cnt[0], cnt[1]: its vertices and out-edges.  All 32 lanes call it.  Slots
-// past kSoloCap are not filled: a list with that many edges is never expanded
-// here.
+// past kSoloCap are not filled: a list with more edges is never expanded here.
 template <int Q>
 __device__ __forceinline__ void solo_append(const SoloList &l, uint32_t *cnt, const bool (&ok)[Q], const uint32_t (&v)[Q],
 		const uint32_t (&beg)[Q], const uint32_t (&deg)[Q]) {
