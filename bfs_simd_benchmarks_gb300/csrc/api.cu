@@ -414,7 +414,7 @@ void set_shape(bfs_graph *g, const PackedTiles &pk, uint64_t packed_words) {
 	d.bm_words = d.num_stripes * d.slice_words;  // bulk copies read whole slices
 	d.tma = (d.sw % 128 == 0) ? 1u : 0u;
 	d.tma_batch = std::max<uint32_t>(1, std::min<uint32_t>(kMaxSliceBatch, kTmaSliceWords / d.slice_words));
-	d.pull_long_cap = 4096;
+	d.pull_long_cap = 2816;  // 3 words each; with the bitmaps no more than the top-down step uses
 }
 
 // Batched pull: destinations with many in-edges and their chunks.

@@ -50,8 +50,13 @@ __device__ unsigned long long g_cta_prof[16][kProfPoints][kMaxGrid];
 #define CTA_STAMP(step, k) do { } while (0)
 #endif
 
+// One thread's share.  A vertex is reached and expanded once, so its sums over
+// a traversal are below 2^32 like the graph's edges; bu_words counts an edge
+// again in every bottom-up step.
 struct ThreadAcc {
-	unsigned long long count, degsum, td_edges, td_vertices, bu_words, bu_slices, bu_groups, bu_vertices;
+	uint32_t count, degsum;  // of the current step
+	uint32_t td_edges, td_vertices, bu_slices, bu_groups, bu_vertices;
+	unsigned long long bu_words;
 };
 
 __device__ __forceinline__ uint32_t bucket_of(uint32_t deg, const StepParams &p) {
@@ -899,9 +904,13 @@ __device__ __forceinline__ void phase_dense_tma(const DevGraph &g, const RunCtx 
 // reference's dense step tests every edge of the active rows instead,
 // apps/bfs_simd/bfs.cpp:194-217, with the same levels).  Pass 1 gives each
 // destination one lane and its first kPullShort in-edges; destinations not
-// settled by then go to a shared-memory queue that whole warps scan 32 edges
-// at a time with a ballot to stop at the first hit.
-constexpr uint32_t kPullShort = 4;
+// settled by then go to a shared-memory queue (with what is left of their
+// lists) that 4 lanes each scan, 8 edges at a time, up to the first hit.
+// What bounds it is chains of round trips: the edges of a destination one
+// after the other and a warp per queued destination took 155 us for the first
+// pull of a uniform graph of 2^20 vertices and 2^24 edges (now 100), 1.86 ms for
+// the Twitter shape's (now 0.9).
+constexpr uint32_t kPullShort = 3;
 // Work items of a pull step: each column group in this many parts, handed
 // out dynamically (whole groups left a few CTAs with most of the work: the
 // early exit makes a group's cost depend on where its frontier sources are).
@@ -909,6 +918,25 @@ constexpr uint32_t kPullSplit = 4;
 
 __device__ __forceinline__ bool frontier_bit(const uint32_t *cur, uint32_t u) {
 	return (ld_cg(cur + (u >> 5)) >> (u & 31)) & 1u;
+}
+
+// A frontier source among the in-edges e, e + stride, ... (kPullDeep of them,
+// below end), or kUnvisitedWord.
+constexpr int kPullDeep = 2;
+constexpr uint32_t kPullRounds = 16;
+__device__ __forceinline__ uint32_t pull_hit(const DevGraph &g, const uint32_t *cur, uint32_t e, uint32_t end,
+		uint32_t stride, uint32_t &edges) {
+	uint32_t u[kPullDeep], fw[kPullDeep], hit = kUnvisitedWord;
+#pragma unroll
+	for (int q = 0; q < kPullDeep; ++q) u[q] = e + stride * q < end ? __ldg(g.in_src + e + stride * q) : kUnvisitedWord;
+#pragma unroll
+	for (int q = 0; q < kPullDeep; ++q) fw[q] = u[q] != kUnvisitedWord ? ld_cg(cur + (u[q] >> 5)) : 0u;
+#pragma unroll
+	for (int q = 0; q < kPullDeep; ++q) {
+		edges += u[q] != kUnvisitedWord;
+		if ((fw[q] >> (u[q] & 31)) & 1u) hit = u[q];
+	}
+	return hit;
 }
 
 __device__ __forceinline__ void phase_pull(const DevGraph &g, const RunCtx &r, uint32_t step, int32_t nl, uint32_t *smem,
@@ -955,39 +983,49 @@ __device__ __forceinline__ void phase_pull(const DevGraph &g, const RunCtx &r, u
 					end[q] = __ldg(g.in_off + v + 1);
 				}
 			}
+			// the first in-edge of all four destinations, then for those it
+			// does not settle the next kPullShort - 1 together
 #pragma unroll
-			for (int q = 0; q < 4; ++q) u[q] = (beg[q] < end[q]) ? __ldg(g.in_src + beg[q]) : 0u;
+			for (int q = 0; q < 4; ++q) u[q] = beg[q] < end[q] ? __ldg(g.in_src + beg[q]) : kUnvisitedWord;
 #pragma unroll
 			for (int q = 0; q < 4; ++q) {
-				if (beg[q] < end[q]) {
-					++tested;
-					++edges;
-					found[q] = frontier_bit(cur, u[q]);
-				}
+				if (u[q] == kUnvisitedWord) continue;
+				++tested;
+				++edges;
+				found[q] = frontier_bit(cur, u[q]);
 			}
+			uint32_t x[4][kPullShort - 1];
+#pragma unroll
+			for (int q = 0; q < 4; ++q)
+#pragma unroll
+				for (uint32_t t = 0; t < kPullShort - 1; ++t)
+					x[q][t] = !found[q] && beg[q] + 1 + t < end[q] ? __ldg(g.in_src + beg[q] + 1 + t) : kUnvisitedWord;
+#pragma unroll
+			for (int q = 0; q < 4; ++q)
+#pragma unroll
+				for (uint32_t t = 0; t < kPullShort - 1; ++t) {
+					if (x[q][t] == kUnvisitedWord) continue;
+					++edges;
+					if (frontier_bit(cur, x[q][t])) {
+						found[q] = true;
+						u[q] = x[q][t];
+					}
+				}
 #pragma unroll
 			for (int q = 0; q < 4; ++q) {
-				if (beg[q] < end[q] && !found[q]) {
-					// the next few in-edges, then the long queue
-					const uint32_t v = v0 + 32u * (j0 + q) + lane;
-					const uint32_t stop = min(end[q], beg[q] + kPullShort);
-					uint32_t e = beg[q] + 1;
-					for (; e < stop; ++e) {
-						++edges;
-						u[q] = __ldg(g.in_src + e);
-						if (frontier_bit(cur, u[q])) { found[q] = true; break; }
-					}
-					if (!found[q] && e < end[q]) {
-						const uint32_t pos = atomicAdd(&dsh.nlist, 1u);
-						if (pos < long_cap) {
-							longq[pos] = v;
-						} else {
-							// queue full: finish the scan here
-							for (; e < end[q]; ++e) {
-								++edges;
-								u[q] = __ldg(g.in_src + e);
-								if (frontier_bit(cur, u[q])) { found[q] = true; break; }
-							}
+				if (!found[q] && end[q] - beg[q] > kPullShort) {
+					// the rest of a longer list: the queue
+					const uint32_t pos = atomicAdd(&dsh.nlist, 1u);
+					if (pos < long_cap) {
+						longq[pos] = v0 + 32u * (j0 + q) + lane;
+						longq[long_cap + pos] = beg[q] + kPullShort;
+						longq[2 * long_cap + pos] = end[q];
+					} else {
+						// queue full: finish the scan here
+						for (uint32_t e = beg[q] + kPullShort; e < end[q]; ++e) {
+							++edges;
+							u[q] = __ldg(g.in_src + e);
+							if (frontier_bit(cur, u[q])) { found[q] = true; break; }
 						}
 					}
 				}
@@ -998,27 +1036,40 @@ __device__ __forceinline__ void phase_pull(const DevGraph &g, const RunCtx &r, u
 		}
 		__syncthreads();
 		{ long long t1 = clock64(); cyc[1] += t1 - t0; t0 = t1; }
-		// Pass 2: a warp per remaining destination, 32 in-edges at a time.
-		const uint32_t nlong = min(dsh.nlist, long_cap);
-		for (uint32_t x = wid; x < nlong; x += kWarps) {
-			const uint32_t v = longq[x];
-			const uint32_t end = __ldg(g.in_off + v + 1);
-			for (uint32_t e0 = __ldg(g.in_off + v) + kPullShort; e0 < end; e0 += 32) {
-				const uint32_t e = e0 + lane;
-				uint32_t u = 0;
-				const bool hit = e < end && frontier_bit(cur, u = __ldg(g.in_src + e));
-				const uint32_t hm = __ballot_sync(kFull, hit);
-				if (hm) {
-					const int first = __ffs(hm) - 1;
-					if (lane == (unsigned) first) {
-						if (parent) parent[v] = u;
-						const uint32_t d = v - v0;
+		// Pass 2: eight queued destinations of a warp side by side, 4 lanes and
+		// kPullDeep in-edges per lane each; what is left of a list after
+		// kPullRounds of these is the whole warp's.
+		const uint32_t nlong = min(dsh.nlist, long_cap), sub = lane & 3u;
+		for (uint32_t x0 = wid * 8; x0 < nlong; x0 += kWarps * 8) {
+			const uint32_t x = x0 + lane / 4;
+			bool open = x < nlong;
+			const uint32_t v = open ? longq[x] : 0u, end = open ? longq[2 * long_cap + x] : 0u;
+			uint32_t e = open ? longq[long_cap + x] : 0u;
+			for (uint32_t round = 0; round < kPullRounds && __any_sync(kFull, open); ++round) {
+				const uint32_t hit = pull_hit(g, cur, e + sub, open ? end : 0u, 4, edges);
+				const uint32_t m = (__ballot_sync(kFull, hit != kUnvisitedWord) >> (lane & 28u)) & 0xFu;
+				if (m && sub == (unsigned) __ffs(m) - 1) {
+					if (parent) parent[v] = hit;
+					const uint32_t d = v - v0;
+					atomicOr(&vis_s[d >> 5], 1u << (d & 31));
+				}
+				e += 4 * kPullDeep;
+				open = open && !m && e < end;
+			}
+			for (uint32_t om = __ballot_sync(kFull, open && sub == 0); om; om &= om - 1) {
+				const int src = __ffs(om) - 1;
+				const uint32_t ov = __shfl_sync(kFull, v, src), oend = __shfl_sync(kFull, end, src);
+				for (uint32_t oe = __shfl_sync(kFull, e, src); oe < oend; oe += 32 * kPullDeep) {
+					const uint32_t hit = pull_hit(g, cur, oe + lane, oend, 32, edges);
+					const uint32_t m = __ballot_sync(kFull, hit != kUnvisitedWord);
+					if (!m) continue;
+					if (lane == (unsigned) __ffs(m) - 1) {
+						if (parent) parent[ov] = hit;
+						const uint32_t d = ov - v0;
 						atomicOr(&vis_s[d >> 5], 1u << (d & 31));
 					}
-					if (lane == 0) edges += (uint32_t) first + 1;
 					break;
 				}
-				if (lane == 0) edges += min(32u, end - e0);
 			}
 		}
 		acc.bu_words += edges;
@@ -1067,7 +1118,7 @@ __device__ __forceinline__ unsigned long long *part_at(const RunCtx &r, uint32_t
 __device__ __forceinline__ void flush_step(ThreadAcc &acc, const RunCtx &r, uint32_t slot) {
 	__shared__ unsigned long long red[2][kWarps];
 	const unsigned lane = lane_id(), wid = warp_id();
-	const unsigned long long c = warp_sum(acc.count), d = warp_sum(acc.degsum);
+	const unsigned long long c = warp_sum((unsigned long long) acc.count), d = warp_sum((unsigned long long) acc.degsum);
 	if (lane == 0) { red[0][wid] = c; red[1][wid] = d; }
 	__syncthreads();
 	if (threadIdx.x < 2) {
@@ -1321,12 +1372,17 @@ __device__ __forceinline__ void phase_solo(const DevGraph &g, const RunCtx &r, c
 // waits for) takes no extra round trips.  The grid barrier's arrival count,
 // the exit count and the status word are zero when the launch starts: the
 // last CTA to exit resets them.
+//
+// One kernel per bottom-up variant (kStream: p.bottom_up == BFS_BU_STREAM), so
+// that the pull's carries neither the streamed variant's code nor its
+// registers.
+template <bool kStream>
 __global__ void __launch_bounds__(kThreads, 2) k_bfs_persistent(DevGraph g, RunCtx r, StepParams p, uint32_t batch) {
 	extern __shared__ __align__(128) uint32_t smem[];
 	__shared__ uint32_t s_conv_tails[3];
-	ThreadAcc acc{0, 0, 0, 0, 0, 0, 0, 0};
+	ThreadAcc acc{};
 	bool ok = true;
-	dense_tma_init();
+	if (kStream) dense_tma_init();
 	const bool leader = blockIdx.x == 0 && threadIdx.x == 0;
 	unsigned long long st_reached = 0, st_edges = 0;
 	uint32_t st_dense = 0;
@@ -1363,13 +1419,15 @@ __global__ void __launch_bounds__(kThreads, 2) k_bfs_persistent(DevGraph g, RunC
 		if (dense) {
 			// the top-down step that produced this frontier also set its
 			// bitmap; only the streaming variant needs the stripe flags built
-			if (!last_dense && p.bottom_up != 0) {
+			if (kStream && !last_dense) {
 				phase_to_dense(g, r, rnd, true);
 				if (!(ok = grid_sync(r.bar, epoch, r.err, p.wait_limit_ns, p.hold_barrier))) break;
 				if (leader && step < 256) r.stats->t_conv[step] = global_timer_ns();
 			}
 			CTA_STAMP(step, 3);
-			phase_dense(g, r, p, rnd, (int32_t) step + 1, batch, smem, acc);
+			if (!kStream) phase_pull(g, r, rnd, (int32_t) step + 1, smem, acc);
+			else if (g.tma) phase_dense_tma(g, r, rnd, (int32_t) step + 1, smem, acc);
+			else phase_dense_generic(g, r, rnd, (int32_t) step + 1, batch, smem, acc);
 		} else {
 			if (last_dense) {
 				phase_to_sparse(g, r, p, rnd);
@@ -1384,8 +1442,9 @@ __global__ void __launch_bounds__(kThreads, 2) k_bfs_persistent(DevGraph g, RunC
 			CTA_STAMP(step, 3);
 			const uint32_t cap = solo_cap(g, prev_dsum, dsum);
 			solo = fsize <= cap && dsum <= cap;
-			if (!solo) phase_expand(g, r, p, rnd, (int32_t) step + 1, tails[0], tails[1], tails[2], smem, acc);
-			else if (blockIdx.x == 0) phase_solo(g, r, p, rnd, step, tails, seen, smem, acc, st_reached, st_edges);
+			if (__builtin_expect(!solo, 1)) phase_expand(g, r, p, rnd, (int32_t) step + 1, tails[0], tails[1], tails[2], smem, acc);
+			else if (blockIdx.x == 0)
+				phase_solo(g, r, p, rnd, step, tails, seen, smem, acc, st_reached, st_edges);
 		}
 		prev_dsum = dsum;
 		CTA_STAMP(step, 4);
@@ -1436,7 +1495,7 @@ __global__ void __launch_bounds__(kThreads) k_step_to_sparse(DevGraph g, RunCtx 
 }
 __global__ void __launch_bounds__(kThreads) k_step_expand(DevGraph g, RunCtx r, StepParams p, uint32_t step) {
 	extern __shared__ __align__(128) uint32_t smem[];
-	ThreadAcc acc{0, 0, 0, 0, 0, 0, 0, 0};
+	ThreadAcc acc{};
 	const StepCounters *in = r.ctr + (step + 2) % 3;
 	phase_expand(g, r, p, step, (int32_t) step + 1, ld_volatile(&in->tail[0]), ld_volatile(&in->tail[1]), ld_volatile(&in->tail[2]),
 			smem, acc);
@@ -1446,7 +1505,7 @@ __global__ void __launch_bounds__(kThreads) k_step_expand(DevGraph g, RunCtx r, 
 __global__ void __launch_bounds__(kThreads, 2) k_step_dense(DevGraph g, RunCtx r, StepParams p, uint32_t step,
 		uint32_t batch) {
 	extern __shared__ __align__(128) uint32_t smem[];
-	ThreadAcc acc{0, 0, 0, 0, 0, 0, 0, 0};
+	ThreadAcc acc{};
 	dense_tma_init();
 	phase_dense(g, r, p, step, (int32_t) step + 1, batch, smem, acc);
 	flush_step(acc, r, step % 3);
@@ -1465,7 +1524,7 @@ size_t traversal_smem_bytes(const DevGraph &g, uint32_t batch, uint32_t bottom_u
 	size_t words = (size_t) 2 * (g.max_group_words + 1) + 3 * kThreads;
 	if (g.tma) words += (size_t) kTmaStages * (kTmaEdgeWords + (size_t) g.tma_batch * g.slice_words);
 	else words += (size_t) batch * g.slice_words;
-	const size_t pull = (size_t) 3 * (g.max_group_words + 1) + g.pull_long_cap;
+	const size_t pull = (size_t) 3 * (g.max_group_words + 1 + g.pull_long_cap);
 	const size_t expand = (size_t) kWarps * 3 * kWqCap + 3 * (size_t) kFlatChunk;
 	size_t need = bottom_up == BFS_BU_PULL || pull > words ? pull : words;
 	need = need > expand ? need : expand;
@@ -1481,7 +1540,8 @@ int persistent_grid(const DevGraph &g, uint32_t batch, uint32_t bottom_up, int d
 	*smem = traversal_smem_bytes(g, batch, bottom_up);
 	int optin = 0;
 	if (cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, device) != cudaSuccess) return BFS_ECUDA;
-	for (const void *fn : {(const void *) k_bfs_persistent, (const void *) k_step_dense, (const void *) k_step_expand}) {
+	const void *run = bottom_up == BFS_BU_STREAM ? (const void *) k_bfs_persistent<true> : (const void *) k_bfs_persistent<false>;
+	for (const void *fn : {run, (const void *) k_step_dense, (const void *) k_step_expand}) {
 		cudaFuncAttributes at{};
 		if (cudaFuncGetAttributes(&at, fn) != cudaSuccess) return BFS_ECUDA;
 		const int most = optin - (int) at.sharedSizeBytes;
@@ -1489,7 +1549,7 @@ int persistent_grid(const DevGraph &g, uint32_t batch, uint32_t bottom_up, int d
 		if (cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, most) != cudaSuccess) return BFS_ECUDA;
 	}
 	int per_sm = 0;
-	if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_bfs_persistent, kThreads, *smem) != cudaSuccess)
+	if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, run, kThreads, *smem) != cudaSuccess)
 		return BFS_ECUDA;
 	if (per_sm < 1) return BFS_EUNSUPPORTED;
 	if (per_sm > 2) per_sm = 2;
@@ -1510,7 +1570,8 @@ int launch_persistent(const DevGraph &g, const RunCtx &r, const StepParams &p, u
 	StepParams pp = p;
 	uint32_t bb = batch;
 	void *args[] = {&gg, &rr, &pp, &bb};
-	cudaError_t e = cudaLaunchCooperativeKernel((const void *) k_bfs_persistent, dim3(grid), dim3(kThreads), args, smem, st);
+	const void *fn = p.bottom_up == BFS_BU_STREAM ? (const void *) k_bfs_persistent<true> : (const void *) k_bfs_persistent<false>;
+	cudaError_t e = cudaLaunchCooperativeKernel(fn, dim3(grid), dim3(kThreads), args, smem, st);
 	return e == cudaSuccess ? BFS_OK : BFS_ECUDA;
 }
 
