@@ -63,6 +63,10 @@ __device__ __forceinline__ uint32_t bucket_of(uint32_t deg, const StepParams &p)
 	return deg <= p.warp_max_degree ? 0u : (deg <= p.cta_max_degree ? 1u : 2u);
 }
 
+// Frontiers with this many out-edges, once the reached vertices hold more than
+// half of the edges, look a destination up in the visited bitmap before they
+// claim its level (see visit_and_append).
+constexpr uint32_t kScreenEdges = 1u << 17;
 constexpr int kTdPerLane = 4;  // candidate edges a lane handles per top-down iteration
 // Medium-degree buckets up to this size join the grid-flat expansion of the
 // large ones (a few chunks); larger ones are spread over CTAs in chunks.
@@ -105,24 +109,36 @@ __device__ __forceinline__ void wq_flush_all(WarpQ &wq) {
 // u[q] -> v[q] each (has[q] false for an empty slot).  Each stage -- the
 // claiming compare-and-swap, the degree load of the claimed -- is issued for
 // all candidates before any result is used, so a lane waits for two round
-// trips per batch of edges, not per edge.  (A visited-bitmap pre-load before
-// the claim kept visited destinations off the atomic unit but cost a round
-// trip per batch: measured slower on R-MAT frontiers.)
+// trips per batch of edges, not per edge.  `screen`: visited destinations are
+// dropped by the visited bitmap first, one more round trip per batch.  That
+// pays after the bottom-up steps, when most are visited and the levels' random
+// sectors come from DRAM (Twitter shape, 30 M edges: 715 -> 414 us; R-MAT scale
+// 22: 35 -> 28 us); a growing frontier loses (uniform graph of 2^20 vertices, 31 ->
+// 37 us), a small one has the round trip only.
 // Claimed vertices get their level and parent, their bit in the next
 // frontier's bitmap `nbm` (so that a bottom-up step after this one needs no
 // queue -> bitmap conversion) and are staged for the next queue bucket of
 // their out-degree.
 __device__ __forceinline__ void visit_and_append(const bool (&has)[kTdPerLane], const uint32_t (&u)[kTdPerLane],
 		const uint32_t (&v)[kTdPerLane], int32_t next_level, const DevGraph &g, const RunCtx &r, uint32_t *nbm,
-		WarpQ &wq, const StepParams &p, ThreadAcc &acc) {
+		WarpQ &wq, const StepParams &p, ThreadAcc &acc, bool screen) {
 	// The claim is a compare-and-swap on the destination's own level (-1 ->
 	// next level): only edges to the same destination contend, not the 32
 	// destinations of a bitmap word.  The visited bit follows with a
 	// reduction whose result nobody waits for.
 	bool claimed[kTdPerLane];
 #pragma unroll
+	for (int q = 0; q < kTdPerLane; ++q) claimed[q] = has[q];
+	if (screen) {
+		uint32_t vw[kTdPerLane];
+#pragma unroll
+		for (int q = 0; q < kTdPerLane; ++q) vw[q] = has[q] ? ld_cg(r.vis + (v[q] >> 5)) : 0u;
+#pragma unroll
+		for (int q = 0; q < kTdPerLane; ++q) claimed[q] = has[q] && !((vw[q] >> (v[q] & 31)) & 1u);
+	}
+#pragma unroll
 	for (int q = 0; q < kTdPerLane; ++q)
-		claimed[q] = has[q] && atomicCAS((int *) r.level + v[q], -1, next_level) == -1;
+		claimed[q] = claimed[q] && atomicCAS((int *) r.level + v[q], -1, next_level) == -1;
 	uint32_t deg[kTdPerLane];
 #pragma unroll
 	for (int q = 0; q < kTdPerLane; ++q) {
@@ -188,7 +204,7 @@ __device__ __forceinline__ uint32_t block_incl_scan(uint32_t x) {
 // The frontier's queue sizes nS, nM, nL (small, medium, large out-degree)
 // come from the caller, which loads them together with the step totals.
 __device__ __forceinline__ void phase_expand(const DevGraph &g, const RunCtx &r, const StepParams &p, uint32_t step,
-		int32_t nl, uint32_t nS, uint32_t nM, uint32_t nL, uint32_t *smem, ThreadAcc &acc) {
+		int32_t nl, uint32_t nS, uint32_t nM, uint32_t nL, uint32_t *smem, ThreadAcc &acc, bool screen) {
 	const uint32_t cur = step & 1, nxt = (step + 1) & 1;
 	StepCounters *out = r.ctr + step % 3;
 	uint32_t *nbm = r.bm[step % 3];
@@ -260,7 +276,7 @@ __device__ __forceinline__ void phase_expand(const DevGraph &g, const RunCtx &r,
 				uu[q] = fu[jj];
 				vv[q] = has[q] ? __ldg(g.col + fbeg[jj] + (uint32_t) (f - prev)) : 0u;
 			}
-			visit_and_append(has, uu, vv, nl, g, r, nbm, wq, p, acc);
+			visit_and_append(has, uu, vv, nl, g, r, nbm, wq, p, acc, screen);
 		}
 		if (blockIdx.x == 0 && threadIdx.x == 0) { acc.td_edges += total; acc.td_vertices += cn; }
 		__syncthreads();
@@ -311,7 +327,7 @@ __device__ __forceinline__ void phase_expand(const DevGraph &g, const RunCtx &r,
 					uu[q] = xsh.u[jj];
 					vv[q] = has[q] ? __ldg(g.col + xsh.beg[jj] + (uint32_t) (f - prev)) : 0u;
 				}
-				visit_and_append(has, uu, vv, nl, g, r, nbm, wq, p, acc);
+				visit_and_append(has, uu, vv, nl, g, r, nbm, wq, p, acc, screen);
 			}
 			if (threadIdx.x == 0) {
 				acc.td_edges += total;
@@ -354,7 +370,7 @@ __device__ __forceinline__ void phase_expand(const DevGraph &g, const RunCtx &r,
 				const uint32_t oe = __shfl_sync(kFull, excl, lo);
 				vv[q] = has[q] ? __ldg(g.col + ob + (f - oe)) : 0u;
 			}
-			visit_and_append(has, uu, vv, nl, g, r, nbm, wq, p, acc);
+			visit_and_append(has, uu, vv, nl, g, r, nbm, wq, p, acc, screen);
 		}
 		const unsigned nvalid = (unsigned) __popc(__ballot_sync(kFull, valid));
 		if (lane == 0) {
@@ -1442,7 +1458,8 @@ __global__ void __launch_bounds__(kThreads, 2) k_bfs_persistent(DevGraph g, RunC
 			CTA_STAMP(step, 3);
 			const uint32_t cap = solo_cap(g, prev_dsum, dsum);
 			solo = fsize <= cap && dsum <= cap;
-			if (__builtin_expect(!solo, 1)) phase_expand(g, r, p, rnd, (int32_t) step + 1, tails[0], tails[1], tails[2], smem, acc);
+			if (__builtin_expect(!solo, 1)) phase_expand(g, r, p, rnd, (int32_t) step + 1, tails[0], tails[1], tails[2], smem, acc,
+						dsum >= kScreenEdges && seen > g.m / 2);
 			else if (blockIdx.x == 0)
 				phase_solo(g, r, p, rnd, step, tails, seen, smem, acc, st_reached, st_edges);
 		}
@@ -1498,7 +1515,7 @@ __global__ void __launch_bounds__(kThreads) k_step_expand(DevGraph g, RunCtx r, 
 	ThreadAcc acc{};
 	const StepCounters *in = r.ctr + (step + 2) % 3;
 	phase_expand(g, r, p, step, (int32_t) step + 1, ld_volatile(&in->tail[0]), ld_volatile(&in->tail[1]), ld_volatile(&in->tail[2]),
-			smem, acc);
+			smem, acc, false);
 	flush_step(acc, r, step % 3);
 	flush_stats(acc, r.stats);
 }

@@ -154,3 +154,66 @@ def test_one_cluster_traversal(native, oracle, n):
                 np.testing.assert_array_equal(lev2, ref)
                 for k in ("trace", "dense_steps", "td_edges", "td_vertices", "num_steps"):
                     assert st[k] == st2[k], (k, opts)
+
+
+@pytest.mark.parametrize("ctas_per_sm", [0, 1])
+@pytest.mark.parametrize("layers", ["few", "many"])
+def test_grid_pull_lists(native, oracle, layers, ctas_per_sm):
+    """The whole grid's bottom-up step on in-edge lists whose frontier source comes
+    first, in the lane's share, in the queue's rounds, in the warp's rounds and
+    never; top-down steps with and without the visited screen."""
+    import bfs_simd_benchmarks_gb300 as B
+    n = 200_003
+    rng = np.random.default_rng(3)
+    island = np.arange(n - 20_000, n)  # no in-edges: never reached
+    src, dst = [rng.integers(0, 1000, size=4000)], [rng.integers(0, 1000, size=4000)]
+    at = 1000
+    for length in (1, 2, 3, 4, 5, 11, 12, 67, 68, 69, 131, 132, 133, 700):
+        for _ in range(40):
+            u = rng.choice(island, size=length)
+            if rng.random() < 0.8:
+                u[rng.integers(0, length)] = rng.integers(0, 1000)
+            src.append(u)
+            dst.append(np.full(length, at))
+            at += 1
+    last = np.arange(at, n - 20_000)
+    per = 5 if layers == "many" else 1
+    src.append(rng.integers(0, at, size=per * last.size))
+    dst.append(np.repeat(last, per))
+    if layers == "many":  # edges back to visited vertices, for the screened top-down steps
+        src.append(np.repeat(last, 2))
+        dst.append(rng.integers(0, n - 20_000, size=2 * last.size))
+    src, dst = np.concatenate(src).astype(np.uint32), np.concatenate(dst).astype(np.uint32)
+    arr = oracle.arrays_from_edges(n, src, dst, 256, 4)
+    with B.Graph.from_edges(n, src, dst, 256, 4, device_build=False) as g:
+        for opts in ({}, {"switch_rule": 1}, {"to_dense_ratio": 1 << 30, "to_sparse_ratio": 1 << 30},
+                     {"to_dense_ratio": 1 << 30, "to_sparse_ratio": 2}, {"to_dense_ratio": 1, "to_sparse_ratio": 1}):
+            g.set_options(**{"switch_rule": 0, "to_dense_ratio": 20, "to_sparse_ratio": 20, "ctas_per_sm": ctas_per_sm, **opts})
+            for s in (0, 17):
+                lev, par, st = g.run(s)
+                np.testing.assert_array_equal(lev, oracle.bfs_levels(arr, s))
+                assert oracle.check_parents(arr, s, lev, par) == 0
+                assert st["grid_ctas"] > 16
+
+
+def test_grid_pull_queue_overflow(native, oracle):
+    """More long in-edge lists in a work item than its queue holds."""
+    import torch
+    import bfs_simd_benchmarks_gb300 as B
+    n = 4_200_000
+    gen = torch.Generator(device="cuda")
+    gen.manual_seed(9)
+    island = 1000  # vertices n - 1000 ..: no in-edges
+    heads = torch.arange(2, n - island, device="cuda", dtype=torch.int32).repeat_interleave(5)
+    tails = torch.randint(n - island, n, (heads.numel(),), device="cuda", dtype=torch.int32, generator=gen)
+    chain = torch.tensor([0, 1, 2, 3], device="cuda", dtype=torch.int32)
+    src = torch.cat([tails, chain[:3]]).contiguous()
+    dst = torch.cat([heads, chain[1:]]).contiguous()
+    arr = oracle.csr_arrays(n, src.cpu().numpy().astype(np.uint32), dst.cpu().numpy().astype(np.uint32))
+    with B.Graph.from_device_edges(n, src.data_ptr(), dst.data_ptr(), src.numel(), 1024, 16) as g:
+        g.set_options(to_dense_ratio=1 << 30, to_sparse_ratio=1 << 30)
+        for s in (0, n - 5):
+            lev, par, st = g.run(s)
+            np.testing.assert_array_equal(lev, oracle.bfs_levels(arr, s))
+            assert oracle.check_parents(arr, s, lev, par) == 0
+            assert st["dense_steps"] > 0
