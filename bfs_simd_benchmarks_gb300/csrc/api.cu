@@ -105,6 +105,7 @@ struct bfs_graph {
 	struct Bc {
 		uint32_t *sigma = nullptr, *order = nullptr, *cnt = nullptr, *kstart = nullptr, *partial = nullptr;
 		uint32_t *cpre = nullptr;
+		unsigned *big_done = nullptr;
 		float *delta = nullptr, *acc = nullptr;
 		uint2 *lvx = nullptr;
 		uint8_t *lv8 = nullptr;
@@ -1244,7 +1245,7 @@ int bc_prepare(bfs_graph *g) {
 			(rc = bc_alloc(g, &b.acc, g->n)) || (rc = bc_alloc(g, &b.cnt, kBcCntCap)) ||
 			(rc = bc_alloc(g, &b.kstart, kBcClasses * (size_t) kBcMaxLevels + 1)) ||
 			(rc = bc_alloc(g, &b.partial, bc_partial_capacity(g->n, g->m))) ||
-			(rc = bc_alloc(g, &b.cpre, (size_t) g->n + 1)) || (rc = bc_alloc(g, &b.ctl, 1))) {
+			(rc = bc_alloc(g, &b.cpre, (size_t) g->n + 1)) || (rc = bc_alloc(g, &b.big_done, g->n)) || (rc = bc_alloc(g, &b.ctl, 1))) {
 		release_bc(g);
 		return rc;
 	}
@@ -1285,6 +1286,7 @@ int bc_enqueue(bfs_graph *g, uint32_t source, uint32_t *sigma, float *delta, flo
 	if (cudaEventRecord(b.e1, st) != cudaSuccess) return BFS_ECUDA;
 	BcArgs a{};
 	a.n = g->n;
+	a.m = (uint32_t) g->m;
 	a.source = source;
 	a.row_off = g->dg.row_off;
 	a.col = g->dg.col;
@@ -1303,6 +1305,7 @@ int bc_enqueue(bfs_graph *g, uint32_t source, uint32_t *sigma, float *delta, flo
 	a.cnt = b.cnt;
 	a.kstart = b.kstart;
 	a.partial = b.partial;
+	a.big_done = b.big_done;
 	a.cpre = b.cpre;
 	a.ctl = b.ctl;
 	if ((rc = bc_launch(a, g->num_sms, st, &b.grid))) return rc;

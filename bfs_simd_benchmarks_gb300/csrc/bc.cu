@@ -9,8 +9,9 @@
 // dependencies (:2032-2061).
 //
 // Here the levels come from the single-source traversal (k_bfs_persistent),
-// and one cooperative launch does the rest with pulls instead of pushes, so
-// that no atomics touch the values and every sum has a fixed order:
+// and one cooperative launch does the rest with pulls instead of pushes (but
+// for some of the integer path counts), so that every float sum has a fixed
+// order:
 //   1. level sort: reached vertices are ordered by (level, class), with the
 //      vertices whose in- or out-degree exceeds kBcBig first in each level.
 //      Each warp owns a range of 32*q vertices and counts / places them with
@@ -23,11 +24,10 @@
 //      (D - 1/sigma) / (1/sigma), 0 where sigma is 0 -- the reference's float
 //      formulas, with its signed int -> float conversion of the counts.
 // Per level, the edge lists of big vertices are cut into kBcChunk-edge chunks
-// that CTAs all over the grid sum (partials added in chunk order after a grid
-// barrier), medium vertices are summed by half-warps, and small ones by warps
-// that take 32 vertices and walk their concatenated edge lists 32 edges at a
-// time (owner by a binary search over the warp's degree prefix, segmented
-// shuffle scan per 32 edges).
+// that CTAs all over the grid sum (partials added in chunk order by the CTA that
+// completes the last one), medium vertices are summed by half-warps, and small
+// ones by a lane each, with lanes of a warp in the same degree band.  Path
+// counts of levels that few edges lead to are pushed instead (integer adds).
 #include "bc.h"
 
 #include <algorithm>
@@ -42,6 +42,7 @@ namespace {
 constexpr int kBcThreads = 512;
 constexpr int kBcWarps = kBcThreads / 32;
 constexpr int kBcUnroll = 4;
+constexpr uint32_t kBcSmemKeys = 256;  // level sort: keys a warp counts in shared memory
 
 struct BcShared {
 	float f[kBcWarps];
@@ -49,8 +50,12 @@ struct BcShared {
 	unsigned long long e[kBcWarps];
 	uint32_t scan[kBcWarps];
 	uint32_t total;
-	uint32_t chunk_beg, chunk_end;
-	uint32_t cpre[kBcSmemBig + 1];   // chunk prefix of the level's big vertices
+	uint32_t chunk_beg, chunk_end, owner;
+	uint32_t lv_deg[2][kBcTraceLevels];  // this CTA's out- and in-degree sums by level
+	union {
+		uint32_t cpre[kBcSmemBig + 1];        // chunk prefix of the level's big vertices
+		uint32_t keys[kBcWarps * kBcSmemKeys];  // level sort: a warp's counters
+	};
 };
 __device__ __shared__ BcShared bsh;
 
@@ -95,7 +100,8 @@ __device__ __forceinline__ uint32_t block_excl_scan(uint32_t x, uint32_t *total)
 
 // Sort key of a vertex: kBcClasses*level + class by the larger of its in- and
 // out-degree d (0: d > 1024; 1..5: d in (512, 1024], (256, 512], (128, 256],
-// (64, 128], (32, 64]; 6: d <= 32); -1 for unreached and out-of-range ids.
+// (64, 128], (32, 64]; 6: d in (8, 32]; 7: d <= 8); -1 for unreached and
+// out-of-range ids.
 __device__ __forceinline__ int vertex_key(const BcArgs &a, uint64_t v, uint32_t depth, int *bad) {
 	if (v >= a.n) return -1;
 	const int lv = a.level[v];
@@ -105,6 +111,7 @@ __device__ __forceinline__ int vertex_key(const BcArgs &a, uint64_t v, uint32_t 
 	const uint32_t id = a.in_off[v + 1] - a.in_off[v];
 	const uint32_t dmax = od > id ? od : id;
 	int cls = (int) kBcClasses - 1;
+	if (dmax > kBcTiny && dmax <= kBcMedium) cls = (int) kBcClasses - 2;
 	if (dmax > kBcBig) cls = 0;
 	else if (dmax > kBcMedium) cls = 1 + (31 - __clz(kBcBig - 1)) - (31 - __clz(dmax - 1));
 	return (int) kBcClasses * lv + cls;
@@ -122,8 +129,10 @@ template <> __device__ __forceinline__ float Dir<false>::value(uint32_t bits) { 
 template <> __device__ __forceinline__ uint32_t Dir<true>::bits(uint32_t x) { return x; }
 template <> __device__ __forceinline__ uint32_t Dir<false>::bits(float x) { return __float_as_uint(x); }
 
-// {level, value} of a neighbour in one 8-byte load (written earlier in this launch: via L2)
-__device__ __forceinline__ uint2 ld_lvx(const uint2 *p) { return __ldcg(p); }
+// {level, value} of a neighbour in one 8-byte load.  Where the level is the one
+// asked for, the pair was written in an earlier phase; others' values may be
+// being written and are not used.
+__device__ __forceinline__ uint2 ld_lvx(const uint2 *p) { return ld_phase(p); }
 
 // Level tags and value bits of the neighbours nb[] (0xFFFFFFFF: none): with
 // use8 the byte level first and the value only where it matches `target`,
@@ -168,47 +177,87 @@ __device__ __forceinline__ typename Dir<kFwd>::T cta_range_sum(const BcArgs &a, 
 }
 
 
-// Big vertices order[bb .. bb+nbig) (nbig <= kBcSmemBig) cut into chunks of
-// kBcChunk edges: every CTA builds the same chunk prefix in shared memory,
-// then CTA c sums chunks c, c + grid, ... into partial[] (value bits).
+// Chunk prefix of the vertices order[bb .. bb+cnt) (cnt <= kBcSmemBig, `per`
+// edges per chunk) in bsh.cpre, the same in every CTA; returns the total.
 template <bool kFwd>
-__device__ __forceinline__ void big_chunks(const BcArgs &a, uint32_t bb, uint32_t nbig, int target, bool use8) {
+__device__ __forceinline__ uint32_t chunk_prefix(const BcArgs &a, uint32_t bb, uint32_t cnt, uint32_t per) {
 	const uint32_t *off = Dir<kFwd>::off(a);
 	uint32_t carry = 0;
-	for (uint32_t t0 = 0; t0 < nbig; t0 += kBcThreads) {
+	for (uint32_t t0 = 0; t0 < cnt; t0 += kBcThreads) {
 		const uint32_t i = t0 + threadIdx.x;
 		uint32_t c = 0;
-		if (i < nbig) {
+		if (i < cnt) {
 			const uint32_t v = ld_cg(a.order + bb + i);
-			c = (off[v + 1] - off[v] + kBcChunk - 1) / kBcChunk;
+			c = (off[v + 1] - off[v] + per - 1) / per;
 		}
 		uint32_t tot;
 		const uint32_t ex = block_excl_scan(c, &tot);
-		if (i < nbig) bsh.cpre[i] = carry + ex;
+		if (i < cnt) bsh.cpre[i] = carry + ex;
 		carry += tot;
 	}
-	if (threadIdx.x == 0) bsh.cpre[nbig] = carry;
+	if (threadIdx.x == 0) bsh.cpre[cnt] = carry;
 	__syncthreads();
-	for (uint32_t j = blockIdx.x; j < carry; j += gridDim.x) {
+	return carry;
+}
+// The largest i with cpre[i] <= j (cpre[cnt] > j).
+__device__ __forceinline__ uint32_t chunk_owner(uint32_t cnt, uint32_t j) {
+	uint32_t lo = 0, hi = cnt;
+	while (lo < hi) {
+		const uint32_t mid = (lo + hi + 1) / 2;
+		if (bsh.cpre[mid] <= j) lo = mid;
+		else hi = mid - 1;
+	}
+	return lo;
+}
+
+template <bool kFwd>
+__device__ __forceinline__ typename Dir<kFwd>::T big_finish_sum(const BcArgs &a, uint32_t i, bool global);
+
+// Writes a vertex's finished sum (one thread).
+template <bool kFwd> __device__ __forceinline__ void finish_vertex(const BcArgs &a, uint32_t v, typename Dir<kFwd>::T sum);
+
+// Big vertices order[bb .. bb+nbig) (nbig <= kBcSmemBig) cut into chunks of
+// kBcChunk edges: CTA c sums chunks c, c + grid, ... into partial[] (value
+// bits); the one that completes a vertex's last chunk adds them in chunk
+// order and writes the vertex, and leaves its count at 0.
+template <bool kFwd>
+__device__ __forceinline__ void big_chunks(const BcArgs &a, uint32_t bb, uint32_t nbig, int target, bool use8,
+		unsigned long long *edges) {
+	using T = typename Dir<kFwd>::T;
+	const uint32_t *off = Dir<kFwd>::off(a);
+	const uint32_t total = chunk_prefix<kFwd>(a, bb, nbig, kBcChunk);
+	for (uint32_t j = blockIdx.x; j < total; j += gridDim.x) {
 		if (threadIdx.x == 0) {
-			// the largest i with cpre[i] <= j (cpre[nbig] = carry > j)
-			uint32_t lo = 0, hi = nbig;
-			while (lo < hi) {
-				const uint32_t mid = (lo + hi + 1) / 2;
-				if (bsh.cpre[mid] <= j) lo = mid;
-				else hi = mid - 1;
-			}
+			const uint32_t lo = chunk_owner(nbig, j);
 			const uint32_t v = ld_cg(a.order + bb + lo);
 			const uint32_t beg = off[v] + (j - bsh.cpre[lo]) * kBcChunk;
 			const uint32_t end = off[v + 1];
+			bsh.owner = lo;
 			bsh.chunk_beg = beg;
 			bsh.chunk_end = end - beg > kBcChunk ? beg + kBcChunk : end;
 		}
 		__syncthreads();
-		const uint32_t beg = bsh.chunk_beg, end = bsh.chunk_end;
-		const typename Dir<kFwd>::T s = cta_range_sum<kFwd>(a, beg, end, target, use8);
-		if (threadIdx.x == 0) a.partial[j] = Dir<kFwd>::bits(s);
+		const uint32_t beg = bsh.chunk_beg, end = bsh.chunk_end, lo = bsh.owner;
+		const T s = cta_range_sum<kFwd>(a, beg, end, target, use8);
+		if (warp_id() != 0) continue;
+		const uint32_t c0 = bsh.cpre[lo], c1 = bsh.cpre[lo + 1];
+		uint32_t before = 0;
+		if (lane_id() == 0) {
+			a.partial[j] = Dir<kFwd>::bits(s);
+			// releases this partial to, and acquires the others' from, the chunks that count here
+			asm volatile("atom.acq_rel.gpu.global.add.u32 %0, [%1], 1;" : "=r"(before) : "l"(a.big_done + lo) : "memory");
+		}
+		if (__shfl_sync(kFull, before, 0) != c1 - c0 - 1) continue;
+		__syncwarp();
+		const T t = big_finish_sum<kFwd>(a, lo, false);
+		if (lane_id() == 0) {
+			const uint32_t v = ld_cg(a.order + bb + lo);
+			a.big_done[lo] = 0u;
+			finish_vertex<kFwd>(a, v, t);
+			*edges += off[v + 1] - off[v];
+		}
 	}
+	__syncthreads();
 }
 
 // The same for a level with more than kBcSmemBig big vertices: the chunk
@@ -216,7 +265,8 @@ __device__ __forceinline__ void big_chunks(const BcArgs &a, uint32_t bb, uint32_
 // the contiguous chunk range [c*per, (c+1)*per).  Returns false when a barrier
 // gave up.
 template <bool kFwd>
-__device__ __forceinline__ bool big_chunks_global(const BcArgs &a, uint32_t bb, uint32_t nbig, int target, bool use8) {
+__device__ __forceinline__ bool big_chunks_global(const BcArgs &a, uint32_t bb, uint32_t nbig, int target, bool use8,
+		unsigned &epoch) {
 	const uint32_t *off = Dir<kFwd>::off(a);
 	BcControl *ctl = a.ctl;
 	const uint32_t L = (nbig + gridDim.x - 1) / gridDim.x;
@@ -231,7 +281,7 @@ __device__ __forceinline__ bool big_chunks_global(const BcArgs &a, uint32_t bb, 
 		s = block_sum(s);
 		if (threadIdx.x == 0) ctl->blk[blockIdx.x] = s;
 	}
-	if (!grid_barrier(ctl->bar, &ctl->err)) return false;
+	if (!grid_sync(ctl->bar, epoch, &ctl->err)) return false;
 	uint32_t base = 0, total = 0;
 	for (uint32_t c = threadIdx.x; c < gridDim.x; c += kBcThreads) {
 		const uint32_t x = ld_cg(ctl->blk + c);
@@ -261,7 +311,7 @@ __device__ __forceinline__ bool big_chunks_global(const BcArgs &a, uint32_t bb, 
 		base += tot;
 	}
 	if (blockIdx.x == 0 && threadIdx.x == 0) a.cpre[nbig] = total;
-	if (!grid_barrier(ctl->bar, &ctl->err)) return false;
+	if (!grid_sync(ctl->bar, epoch, &ctl->err)) return false;
 	const uint32_t per = (total + gridDim.x - 1) / gridDim.x;
 	const uint32_t j0 = blockIdx.x * per < total ? blockIdx.x * per : total;
 	const uint32_t j1 = j0 + per < total ? j0 + per : total;
@@ -337,67 +387,80 @@ __device__ __forceinline__ typename Dir<kFwd>::T half_vertex_sum(const BcArgs &a
 	return s;
 }
 
-// Sums of the edge lists of 32 vertices order[first .. min(first+32, end))
-// by one warp; lane i gets vertex i's sum (0 for lanes past `end`).
+// Sum over the edge list of one vertex by one lane, in edge order: the list in
+// aligned 16-byte pieces, kBcQuads of them and their neighbours' values in
+// flight.  (32 vertices' concatenated lists walked by the warp, with an owner
+// search and a segmented scan per 32 edges, spent about 60 shuffles per 32
+// edges: 0.11 ms for the 8 M edges of a Pokec-shape level.)
+constexpr int kBcQuads = 2;
 template <bool kFwd>
-__device__ __forceinline__ typename Dir<kFwd>::T warp_group_sum(const BcArgs &a, uint32_t v, bool valid, int target,
-		bool skip, bool use8, unsigned long long *edges) {
+__device__ __forceinline__ typename Dir<kFwd>::T lane_vertex_sum(const BcArgs &a, uint32_t v, bool valid, int target,
+		bool use8, unsigned long long *edges) {
 	using T = typename Dir<kFwd>::T;
-	const unsigned lane = lane_id();
-	uint32_t beg = 0, deg = 0;
+	const uint32_t *adj = Dir<kFwd>::adj(a);
+	uint32_t beg = 0, end = 0;
 	if (valid) {
 		beg = Dir<kFwd>::off(a)[v];
-		deg = Dir<kFwd>::off(a)[v + 1] - beg;
+		end = Dir<kFwd>::off(a)[v + 1];
 	}
-	if (skip) deg = 0;
-	*edges += deg;
-	const uint32_t incl = warp_incl_scan(deg);
-	const uint32_t excl = incl - deg;
-	const uint32_t total = __shfl_sync(kFull, incl, 31);
-	const uint32_t *adj = Dir<kFwd>::adj(a);
-	T acc = T(0);
-	for (uint32_t f0 = 0; f0 < total; f0 += 32u * kBcUnroll) {
-		uint32_t nb[kBcUnroll], own[kBcUnroll];
-		uint2 lx[kBcUnroll];
-		T val[kBcUnroll];
+	*edges += end - beg;
+	T s = T(0);
+	for (uint32_t q = beg & ~3u; q < end; q += 4 * kBcQuads) {
+		uint32_t nb[4 * kBcQuads];
+		uint2 lx[4 * kBcQuads];
 #pragma unroll
-		for (int k = 0; k < kBcUnroll; ++k) {
-			const uint32_t f = f0 + (uint32_t) k * 32u + lane;
-			// owner = number of lanes whose inclusive prefix is <= f
-			uint32_t o = 0;
+		for (int k = 0; k < kBcQuads; ++k) {
+			const uint32_t e = q + 4 * k;
+			if (e >= end) {
+				nb[4 * k] = nb[4 * k + 1] = nb[4 * k + 2] = nb[4 * k + 3] = 0xFFFFFFFFu;
+			} else if (a.m - e >= 4) {
+				const uint4 x = ldg_v4(adj + e);
+				nb[4 * k] = e >= beg ? x.x : 0xFFFFFFFFu;
+				nb[4 * k + 1] = e + 1 >= beg && e + 1 < end ? x.y : 0xFFFFFFFFu;
+				nb[4 * k + 2] = e + 2 >= beg && e + 2 < end ? x.z : 0xFFFFFFFFu;
+				nb[4 * k + 3] = e + 3 >= beg && e + 3 < end ? x.w : 0xFFFFFFFFu;
+			} else {  // the last edges of the array
 #pragma unroll
-			for (uint32_t step = 16; step > 0; step >>= 1) {
-				const uint32_t x = __shfl_sync(kFull, incl, o + step - 1);
-				if (x <= f) o += step;
+				for (uint32_t t = 0; t < 4; ++t) nb[4 * k + t] = e + t >= beg && e + t < end ? __ldg(adj + e + t) : 0xFFFFFFFFu;
 			}
-			const uint32_t ob = __shfl_sync(kFull, beg, o);
-			const uint32_t oe = __shfl_sync(kFull, excl, o);
-			const bool on = f < total;
-			own[k] = on ? o : 32u;
-			nb[k] = on ? __ldg(adj + ob + (f - oe)) : 0xFFFFFFFFu;
 		}
 		gather_tags(a, nb, lx, use8, target);
 #pragma unroll
-		for (int k = 0; k < kBcUnroll; ++k) val[k] = (int) lx[k].x == target ? Dir<kFwd>::value(lx[k].y) : T(0);
+		for (int k = 0; k < 4 * kBcQuads; ++k)
+			if ((int) lx[k].x == target) s += Dir<kFwd>::value(lx[k].y);
+	}
+	return s;
+}
+
+// Path counts of level d pushed along the out-edges of the vertices of level
+// d - 1 (order[bb .. bb+cnt), cnt <= kBcSmemBig): integer adds, whose order does
+// not matter.  Warps take chunks of kBcPushChunk edges.
+constexpr uint32_t kBcPushChunk = 512;
+__device__ __forceinline__ void push_paths(const BcArgs &a, uint32_t bb, uint32_t cnt, int target, bool use8,
+		unsigned long long *edges) {
+	const uint32_t total = chunk_prefix<false>(a, bb, cnt, kBcPushChunk);
+	const unsigned lane = lane_id();
+	const uint32_t gw = blockIdx.x + warp_id() * gridDim.x, tw = gridDim.x * kBcWarps;
+	for (uint32_t j = gw; j < total; j += tw) {
+		const uint32_t lo = chunk_owner(cnt, j);
+		const uint32_t u = ld_cg(a.order + bb + lo);
+		const uint32_t beg = a.row_off[u] + (j - bsh.cpre[lo]) * kBcPushChunk;
+		const uint32_t end = min(beg + kBcPushChunk, a.row_off[u + 1]);
+		const uint32_t su = ld_cg(reinterpret_cast<const uint32_t *>(a.lvx + u) + 1);
+		if (lane == 0) *edges += end - beg;
+		for (uint32_t e = beg + lane; e < end; e += 32 * kBcUnroll) {
+			uint32_t v[kBcUnroll], lv[kBcUnroll];
 #pragma unroll
-		for (int k = 0; k < kBcUnroll; ++k) {
-			T x = val[k];
-			const uint32_t o = own[k];
+			for (int k = 0; k < kBcUnroll; ++k) v[k] = e + 32 * k < end ? __ldg(a.col + e + 32 * k) : 0xFFFFFFFFu;
 #pragma unroll
-			for (uint32_t dd = 1; dd < 32; dd <<= 1) {
-				const T y = __shfl_up_sync(kFull, x, dd);
-				const uint32_t oo = __shfl_up_sync(kFull, o, dd);
-				if (lane >= dd && oo == o) x += y;
-			}
-			// the last lane of this vertex's run in these 32 edges holds its sum
-			const uint32_t base = f0 + (uint32_t) k * 32u;
-			const bool mine = deg > 0 && incl > base && excl < base + 32u;
-			const uint32_t src = mine ? min(incl, base + 32u) - 1u - base : 0u;
-			const T got = __shfl_sync(kFull, x, src);
-			if (mine) acc += got;
+			for (int k = 0; k < kBcUnroll; ++k)
+				lv[k] = v[k] == 0xFFFFFFFFu ? 0xFFFFFFFEu
+						: use8 ? (uint32_t) ld_cg_u8(a.lv8 + v[k]) : ld_cg(reinterpret_cast<const uint32_t *>(a.lvx + v[k]));
+#pragma unroll
+			for (int k = 0; k < kBcUnroll; ++k)
+				if ((int) lv[k] == target) atomicAdd(reinterpret_cast<uint32_t *>(a.lvx + v[k]) + 1, su);
 		}
 	}
-	return acc;
 }
 
 __device__ __forceinline__ void finish_dependency(const BcArgs &a, uint32_t v, float sum) {
@@ -408,6 +471,14 @@ __device__ __forceinline__ void finish_dependency(const BcArgs &a, uint32_t v, f
 	const float del = inv != 0.0f ? (dv - inv) / inv : 0.0f;
 	a.delta[v] = del;
 	if (a.acc && v != a.source) a.acc[v] += del;
+}
+
+template <> __device__ __forceinline__ void finish_vertex<true>(const BcArgs &a, uint32_t v, uint32_t sum) {
+	a.sigma[v] = sum;
+	a.lvx[v].y = sum;
+}
+template <> __device__ __forceinline__ void finish_vertex<false>(const BcArgs &a, uint32_t v, float sum) {
+	finish_dependency(a, v, sum);
 }
 
 __global__ void __launch_bounds__(kBcThreads, 2) k_bc(BcArgs a) {
@@ -435,14 +506,26 @@ __global__ void __launch_bounds__(kBcThreads, 2) k_bc(BcArgs a) {
 		++q;
 		R = (W32 + q - 1) / q;
 	}
+	// few keys: ranges as long as a warp's share, counted in shared memory (one
+	// range per 32 vertices has KR = 2.5 M scattered counters on the Pokec shape)
+	const bool skeys = K <= kBcSmemKeys;
+	if (skeys) {
+		q = max(q, (W32 + tw - 1) / tw);
+		R = (W32 + q - 1) / q;
+	}
+	uint32_t *my_cnt = bsh.keys + (skeys ? warp_id() * K : 0u);
 	const uint64_t KR = (uint64_t) K * R;
+	unsigned epoch = 0;
+	for (uint32_t i = threadIdx.x; i < 2 * kBcTraceLevels; i += kBcThreads) bsh.lv_deg[i / kBcTraceLevels][i % kBcTraceLevels] = 0;
+	__syncthreads();
 
 	// ---- 1a. count (level key, range) and initialise the outputs ----------
 	unsigned long long my_edges = 0;
 	uint32_t my_reached = 0;
 	int bad = 0;
 	for (uint64_t r = gw; r < R; r += tw) {
-		for (uint32_t k = lane; k < K; k += 32) a.cnt[(uint64_t) k * R + r] = 0;
+		if (skeys) for (uint32_t k = lane; k < K; k += 32) my_cnt[k] = 0;
+		else for (uint32_t k = lane; k < K; k += 32) a.cnt[(uint64_t) k * R + r] = 0;
 		__syncwarp();
 		const uint64_t v0 = r * 32 * q;
 		for (uint64_t j = 0; j < q; ++j) {
@@ -450,6 +533,7 @@ __global__ void __launch_bounds__(kBcThreads, 2) k_bc(BcArgs a) {
 			const int key = vertex_key(a, v, depth, &bad);
 			if (v < a.n) {
 				a.sigma[v] = v == a.source ? 1u : 0u;
+				a.big_done[v] = 0u;
 				a.delta[v] = 0.0f;
 				const int lv = a.level[v];
 				a.lvx[v] = make_uint2((uint32_t) lv, v == a.source ? 1u : 0u);
@@ -457,12 +541,28 @@ __global__ void __launch_bounds__(kBcThreads, 2) k_bc(BcArgs a) {
 			}
 			if (key >= 0) {
 				++my_reached;
-				my_edges += a.row_off[v + 1] - a.row_off[v];
+				const uint32_t od = a.row_off[v + 1] - a.row_off[v];
+				my_edges += od;
+				const uint32_t lv = (uint32_t) key / kBcClasses;
+				if (lv < kBcTraceLevels) {
+					atomicAdd(&bsh.lv_deg[0][lv], od);
+					atomicAdd(&bsh.lv_deg[1][lv], a.in_off[v + 1] - a.in_off[v]);
+				}
 			}
 			const unsigned mm = __match_any_sync(kFull, key);
-			if (key >= 0 && lane == (unsigned) (__ffs(mm) - 1)) a.cnt[(uint64_t) key * R + r] += __popc(mm);
+			if (key >= 0 && lane == (unsigned) (__ffs(mm) - 1)) {
+				if (skeys) my_cnt[key] += __popc(mm);
+				else a.cnt[(uint64_t) key * R + r] += __popc(mm);
+			}
 			__syncwarp();
 		}
+		if (skeys) for (uint32_t k = lane; k < K; k += 32) a.cnt[(uint64_t) k * R + r] = my_cnt[k];
+		__syncwarp();
+	}
+	__syncthreads();
+	if (threadIdx.x < 2 * kBcTraceLevels) {
+		const uint32_t x = (&bsh.lv_deg[0][0])[threadIdx.x];
+		if (x) atomicAdd(&ctl->lv_deg[0][0] + threadIdx.x, x);
 	}
 	{
 		const unsigned long long e = block_sum(my_edges);
@@ -474,7 +574,7 @@ __global__ void __launch_bounds__(kBcThreads, 2) k_bc(BcArgs a) {
 			if (b) atomicExch(&ctl->err, BFS_ECUDA);
 		}
 	}
-	if (!grid_barrier(ctl->bar, &ctl->err)) return;
+	if (!grid_sync(ctl->bar, epoch, &ctl->err)) return;
 
 	// ---- 1b. exclusive scan of the counters (key-major) --------------------
 	const uint64_t L = (KR + gridDim.x - 1) / gridDim.x;
@@ -486,7 +586,7 @@ __global__ void __launch_bounds__(kBcThreads, 2) k_bc(BcArgs a) {
 		s = block_sum(s);
 		if (threadIdx.x == 0) ctl->blk[blockIdx.x] = s;
 	}
-	if (!grid_barrier(ctl->bar, &ctl->err)) return;
+	if (!grid_sync(ctl->bar, epoch, &ctl->err)) return;
 	{
 		uint32_t base = 0;
 		for (uint32_t c = threadIdx.x; c < blockIdx.x; c += kBcThreads) base += ld_cg(ctl->blk + c);
@@ -508,11 +608,13 @@ __global__ void __launch_bounds__(kBcThreads, 2) k_bc(BcArgs a) {
 		}
 		if (blockIdx.x == 0 && threadIdx.x == 0) a.kstart[K] = ld_cg(&ctl->reached);
 	}
-	if (!grid_barrier(ctl->bar, &ctl->err)) return;
+	if (!grid_sync(ctl->bar, epoch, &ctl->err)) return;
 
 	// ---- 1c. place the vertices ------------------------------------------
 	for (uint64_t r = gw; r < R; r += tw) {
 		const uint64_t v0 = r * 32 * q;
+		if (skeys) for (uint32_t k = lane; k < K; k += 32) my_cnt[k] = ld_cg(a.cnt + (uint64_t) k * R + r);
+		__syncwarp();
 		for (uint64_t j = 0; j < q; ++j) {
 			const uint64_t v = v0 + j * 32 + lane;
 			int dummy = 0;
@@ -520,42 +622,64 @@ __global__ void __launch_bounds__(kBcThreads, 2) k_bc(BcArgs a) {
 			const unsigned mm = __match_any_sync(kFull, key);
 			const unsigned leader = (unsigned) (__ffs(mm) - 1);
 			uint32_t base = 0;
-			if (key >= 0 && lane == leader) base = ld_cg(a.cnt + (uint64_t) key * R + r);
+			if (key >= 0 && lane == leader) base = skeys ? my_cnt[key] : ld_cg(a.cnt + (uint64_t) key * R + r);
 			base = __shfl_sync(kFull, base, leader);
 			if (key >= 0) {
 				a.order[base + __popc(mm & lanemask_lt())] = (uint32_t) v;
-				if (lane == leader) a.cnt[(uint64_t) key * R + r] = base + __popc(mm);
+				if (lane == leader) {
+					if (skeys) my_cnt[key] = base + __popc(mm);
+					else a.cnt[(uint64_t) key * R + r] = base + __popc(mm);
+				}
 			}
 			__syncwarp();
 		}
 	}
 	if (blockIdx.x == 0 && threadIdx.x == 0) ctl->t[1] = global_timer_ns();
-	if (!grid_barrier(ctl->bar, &ctl->err)) return;
+	if (!grid_sync(ctl->bar, epoch, &ctl->err)) return;
 
 	// ---- 2. path counts, level by level ----------------------------------
 	unsigned long long e_fwd = 0, e_rev = 0;
+	bool pushed = false;      // the level before was pushed
+	uint32_t pb = ld_cg(a.kstart);  // where the level before starts in `order`
 	for (uint32_t d = 1; d <= depth; ++d) {
 		const uint32_t bb = ld_cg(a.kstart + kBcClasses * d), be = ld_cg(a.kstart + kBcClasses * d + 1);
-		const uint32_t me = ld_cg(a.kstart + kBcClasses * d + kBcClasses - 1);
+		const uint32_t me = ld_cg(a.kstart + kBcClasses * d + kBcClasses - 2);
 		const uint32_t se = ld_cg(a.kstart + kBcClasses * d + kBcClasses);
-		const uint32_t nbig = be - bb;
-		if (nbig > 0) {
-			const bool global = nbig > kBcSmemBig;
-			if (global) {
-				if (!big_chunks_global<true>(a, bb, nbig, (int) d - 1, use8)) return;
-			} else {
-				big_chunks<true>(a, bb, nbig, (int) d - 1, use8);
+		// the counts of a pushed level are in lvx alone so far
+		if (pushed)
+			for (uint32_t i = pb + blockIdx.x * kBcThreads + threadIdx.x; i < bb; i += gridDim.x * kBcThreads) {
+				const uint32_t v = ld_cg(a.order + i);
+				a.sigma[v] = ld_cg(reinterpret_cast<const uint32_t *>(a.lvx + v) + 1);
 			}
-			if (!grid_barrier(ctl->bar, &ctl->err)) return;
+		// push where the level before has few vertices and less than half the
+		// out-edges of this one's in-edges (the first levels, whose vertices
+		// have the hubs' long in-edge lists: 94 us for the second level of a
+		// Pokec-shape source whose first has two vertices)
+		const uint32_t before = bb - pb;
+		pushed = d < kBcTraceLevels && before <= kBcSmemBig &&
+				2ull * ld_cg(&ctl->lv_deg[0][d - 1]) < ld_cg(&ctl->lv_deg[1][d]);
+		if (pushed) {
+			push_paths(a, pb, before, (int) d, use8, &e_fwd);
+			pb = bb;
+			if (!grid_sync(ctl->bar, epoch, &ctl->err)) return;
+			if (blockIdx.x == 0 && threadIdx.x == 0 && d < kBcTraceLevels) ctl->t_fwd[d] = global_timer_ns();
+			continue;
+		}
+		pb = bb;
+		const uint32_t nbig = be - bb;
+		if (nbig > kBcSmemBig) {
+			if (!big_chunks_global<true>(a, bb, nbig, (int) d - 1, use8, epoch)) return;
+			if (!grid_sync(ctl->bar, epoch, &ctl->err)) return;
 			for (uint32_t i = gw; i < nbig; i += tw) {
 				const uint32_t v = ld_cg(a.order + bb + i);
-				const uint32_t s = big_finish_sum<true>(a, i, global);
+				const uint32_t s = big_finish_sum<true>(a, i, true);
 				if (lane == 0) {
-					a.sigma[v] = s;
-					a.lvx[v].y = s;
+					finish_vertex<true>(a, v, s);
 					e_fwd += a.in_off[v + 1] - a.in_off[v];
 				}
 			}
+		} else if (nbig > 0) {
+			big_chunks<true>(a, bb, nbig, (int) d - 1, use8, &e_fwd);
 		}
 		for (uint32_t i0 = be + 2 * (tw - 1 - gw); i0 < me; i0 += 2 * tw) {
 			const uint32_t i = i0 + (lane >> 4);
@@ -563,8 +687,7 @@ __global__ void __launch_bounds__(kBcThreads, 2) k_bc(BcArgs a) {
 			const uint32_t v = ok ? ld_cg(a.order + i) : 0u;
 			const uint32_t s = half_vertex_sum<true>(a, v, ok, (int) d - 1, use8);
 			if (ok && (lane & 15u) == 0) {
-				a.sigma[v] = s;
-				a.lvx[v].y = s;
+				finish_vertex<true>(a, v, s);
 				e_fwd += a.in_off[v + 1] - a.in_off[v];
 			}
 		}
@@ -573,14 +696,19 @@ __global__ void __launch_bounds__(kBcThreads, 2) k_bc(BcArgs a) {
 			const uint32_t idx = me + grp * 32 + lane;
 			const bool valid = idx < se;
 			const uint32_t v = valid ? ld_cg(a.order + idx) : 0u;
-			const uint32_t s = warp_group_sum<true>(a, v, valid, (int) d - 1, false, use8, &e_fwd);
-			if (valid) {
-				a.sigma[v] = s;
-				a.lvx[v].y = s;
-			}
+			const uint32_t s = lane_vertex_sum<true>(a, v, valid, (int) d - 1, use8, &e_fwd);
+			if (valid) finish_vertex<true>(a, v, s);
 		}
-		if (!grid_barrier(ctl->bar, &ctl->err)) return;
+		if (!grid_sync(ctl->bar, epoch, &ctl->err)) return;
 		if (blockIdx.x == 0 && threadIdx.x == 0 && d < kBcTraceLevels) ctl->t_fwd[d] = global_timer_ns();
+	}
+	if (pushed) {
+		const uint32_t end = ld_cg(a.kstart + kBcClasses * (depth + 1));
+		for (uint32_t i = pb + blockIdx.x * kBcThreads + threadIdx.x; i < end; i += gridDim.x * kBcThreads) {
+			const uint32_t v = ld_cg(a.order + i);
+			a.sigma[v] = ld_cg(reinterpret_cast<const uint32_t *>(a.lvx + v) + 1);
+		}
+		if (!grid_sync(ctl->bar, epoch, &ctl->err)) return;
 	}
 	if (blockIdx.x == 0 && threadIdx.x == 0) ctl->t[2] = global_timer_ns();
 
@@ -588,28 +716,25 @@ __global__ void __launch_bounds__(kBcThreads, 2) k_bc(BcArgs a) {
 	for (int d = (int) depth; d >= 0; --d) {
 		const bool deepest = (uint32_t) d == depth;
 		const uint32_t bb = ld_cg(a.kstart + kBcClasses * d), be = ld_cg(a.kstart + kBcClasses * d + 1);
-		const uint32_t me = ld_cg(a.kstart + kBcClasses * d + kBcClasses - 1);
+		const uint32_t me = ld_cg(a.kstart + kBcClasses * d + kBcClasses - 2);
 		const uint32_t se = ld_cg(a.kstart + kBcClasses * d + kBcClasses);
 		const uint32_t nbig = be - bb;
 		if (deepest) {
 			for (uint32_t i = gw; i < nbig; i += tw)
 				if (lane == 0) finish_dependency(a, ld_cg(a.order + bb + i), 0.0f);
-		} else if (nbig > 0) {
-			const bool global = nbig > kBcSmemBig;
-			if (global) {
-				if (!big_chunks_global<false>(a, bb, nbig, d + 1, use8)) return;
-			} else {
-				big_chunks<false>(a, bb, nbig, d + 1, use8);
-			}
-			if (!grid_barrier(ctl->bar, &ctl->err)) return;
+		} else if (nbig > kBcSmemBig) {
+			if (!big_chunks_global<false>(a, bb, nbig, d + 1, use8, epoch)) return;
+			if (!grid_sync(ctl->bar, epoch, &ctl->err)) return;
 			for (uint32_t i = gw; i < nbig; i += tw) {
 				const uint32_t v = ld_cg(a.order + bb + i);
-				const float s = big_finish_sum<false>(a, i, global);
+				const float s = big_finish_sum<false>(a, i, true);
 				if (lane == 0) {
 					finish_dependency(a, v, s);
 					e_rev += a.row_off[v + 1] - a.row_off[v];
 				}
 			}
+		} else if (nbig > 0) {
+			big_chunks<false>(a, bb, nbig, d + 1, use8, &e_rev);
 		}
 		for (uint32_t i0 = be + 2 * (tw - 1 - gw); i0 < me; i0 += 2 * tw) {
 			const uint32_t i = i0 + (lane >> 4);
@@ -626,10 +751,10 @@ __global__ void __launch_bounds__(kBcThreads, 2) k_bc(BcArgs a) {
 			const uint32_t idx = me + grp * 32 + lane;
 			const bool valid = idx < se;
 			const uint32_t v = valid ? ld_cg(a.order + idx) : 0u;
-			const float s = warp_group_sum<false>(a, v, valid, d + 1, deepest, use8, &e_rev);
+			const float s = deepest ? 0.0f : lane_vertex_sum<false>(a, v, valid, d + 1, use8, &e_rev);
 			if (valid) finish_dependency(a, v, s);
 		}
-		if (d > 0 && !grid_barrier(ctl->bar, &ctl->err)) return;
+		if (d > 0 && !grid_sync(ctl->bar, epoch, &ctl->err)) return;
 		if (blockIdx.x == 0 && threadIdx.x == 0 && (uint32_t) d < kBcTraceLevels) {
 			ctl->t_rev[d] = global_timer_ns();
 			ctl->lv_vertices[d] = se - bb;

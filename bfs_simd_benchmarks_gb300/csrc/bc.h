@@ -11,11 +11,13 @@ namespace bfsg {
 constexpr uint32_t kBcMaxLevels = 1u << 19;   // deeper traversals are refused (BFS_EUNSUPPORTED)
 constexpr uint32_t kBcCntCap = 1u << 22;      // (level key, vertex range) counters of the level sort
 constexpr uint32_t kBcBig = 1024;             // in- or out-degree above which a whole CTA reduces a vertex
-constexpr uint32_t kBcMedium = 32;            // above this (and up to kBcBig) one warp reduces a vertex;
-                                              // at most this, a warp takes 32 vertices at once
-constexpr uint32_t kBcClasses = 7;            // sort keys per level: big, five medium degree bands
+constexpr uint32_t kBcMedium = 32;            // above this (and up to kBcBig) a half-warp reduces a vertex;
+                                              // at most this, a lane does
+constexpr uint32_t kBcTiny = 8;               // small vertices come in two bands, so that a warp's lanes
+                                              // have similar lists
+constexpr uint32_t kBcClasses = 8;            // sort keys per level: big, five medium degree bands
                                               // (highest first, so that warps dealt medium vertices in
-                                              // turn get similar work), small
+                                              // turn get similar work), two small bands
 constexpr uint32_t kBcMaxGrid = 1024;
 constexpr uint32_t kBcTraceLevels = 64;       // per-level timers and sizes kept for the first levels
 static_assert(kBcClasses * kBcMaxLevels <= kBcCntCap, "every sort key needs a counter");
@@ -34,12 +36,13 @@ struct BcControl {
 	uint32_t depth;             // deepest level
 	uint32_t reached;
 	uint32_t pad;
-	unsigned long long edges_fwd;      // in-edges read by the path-count sweep
+	unsigned long long edges_fwd;      // edges read by the path-count sweep
 	unsigned long long edges_rev;      // out-edges read by the dependency sweep
 	unsigned long long edges_reached;  // sum of out-degrees of reached vertices
 	unsigned long long t[4];           // global timer: start, sorted, path counts done, end
 	unsigned long long t_fwd[kBcTraceLevels];  // end of the path counts of level d
 	unsigned long long t_rev[kBcTraceLevels];  // end of the dependency sums of level d
+	uint32_t lv_deg[2][kBcTraceLevels];        // out-degree and in-degree sums of level d's vertices
 	uint32_t lv_vertices[kBcTraceLevels];      // vertices of level d
 	uint32_t lv_big[kBcTraceLevels];           // of which reduced by a whole CTA
 	uint32_t lv_medium[kBcTraceLevels];        // of which reduced by one warp
@@ -47,7 +50,7 @@ struct BcControl {
 };
 
 struct BcArgs {
-	uint32_t n, source;
+	uint32_t n, m, source;
 	uint32_t byte_levels;              // 1: test lv8 first (used when the traversal is at most 254 deep)
 	const uint32_t *row_off, *col;     // CSR
 	const uint32_t *in_off, *in_src;   // in-edge lists (the reverse graph)
@@ -65,6 +68,7 @@ struct BcArgs {
 	uint32_t *cnt;                     // [kBcCntCap] counters of the level sort
 	uint32_t *kstart;                  // [kBcClasses * kBcMaxLevels + 1] start of every key in `order`
 	uint32_t *partial;                 // [bc_partial_capacity(n, m)] chunk sums of big vertices (value bits)
+	unsigned *big_done;                // [n] a level's big vertices: chunks summed so far (0 between levels)
 	uint32_t *cpre;                    // [n + 1] chunk prefix of a level with more than kBcSmemBig big vertices
 	BcControl *ctl;
 };

@@ -933,7 +933,7 @@ constexpr uint32_t kPullShort = 3;
 constexpr uint32_t kPullSplit = 4;
 
 __device__ __forceinline__ bool frontier_bit(const uint32_t *cur, uint32_t u) {
-	return (ld_cg(cur + (u >> 5)) >> (u & 31)) & 1u;
+	return (ld_phase(cur + (u >> 5)) >> (u & 31)) & 1u;
 }
 
 // A frontier source among the in-edges e, e + stride, ... (kPullDeep of them,
@@ -946,7 +946,7 @@ __device__ __forceinline__ uint32_t pull_hit(const DevGraph &g, const uint32_t *
 #pragma unroll
 	for (int q = 0; q < kPullDeep; ++q) u[q] = e + stride * q < end ? __ldg(g.in_src + e + stride * q) : kUnvisitedWord;
 #pragma unroll
-	for (int q = 0; q < kPullDeep; ++q) fw[q] = u[q] != kUnvisitedWord ? ld_cg(cur + (u[q] >> 5)) : 0u;
+	for (int q = 0; q < kPullDeep; ++q) fw[q] = u[q] != kUnvisitedWord ? ld_phase(cur + (u[q] >> 5)) : 0u;
 #pragma unroll
 	for (int q = 0; q < kPullDeep; ++q) {
 		edges += u[q] != kUnvisitedWord;

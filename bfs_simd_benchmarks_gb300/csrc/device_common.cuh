@@ -28,6 +28,18 @@ __device__ __forceinline__ uint32_t ld_cg(const uint32_t *p) { return __ldcg(p);
 __device__ __forceinline__ uint8_t ld_cg_u8(const uint8_t *p) {
 	return (uint8_t) __ldcg((const unsigned char *) p);
 }
+// The same data through L1, where nobody writes it until the next grid barrier
+// and the reads repeat (hubs' rows and bits): an ordinary load.  A grid barrier
+// orders it after the writes of the phase before -- every CTA's writes, its
+// barrier, thread 0's fence and arrival; here thread 0's poll, its fence
+// (which drops this SM's L1 lines), the barrier -- so no older line is read.
+template <class T> __device__ __forceinline__ T ld_phase(const T *p) {
+	T x;
+	static_assert(sizeof(T) == 4 || sizeof(T) == 8, "32 or 64 bits");
+	if constexpr (sizeof(T) == 4) asm volatile("ld.global.ca.u32 %0, [%1];" : "=r"(reinterpret_cast<uint32_t &>(x)) : "l"(p));
+	else asm volatile("ld.global.ca.u64 %0, [%1];" : "=l"(reinterpret_cast<unsigned long long &>(x)) : "l"(p));
+	return x;
+}
 __device__ __forceinline__ uint32_t ld_volatile(const uint32_t *p) { return *(const volatile uint32_t *) p; }
 __device__ __forceinline__ unsigned long long ld_volatile_u64(const unsigned long long *p) {
 	return *(const volatile unsigned long long *) p;

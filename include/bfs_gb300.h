@@ -502,7 +502,7 @@ typedef struct bfs_bc_stats {
 	uint32_t reached;         /* vertices reached from the (last) source */
 	uint32_t status;          /* BFS_* status of the device run */
 	uint64_t edges_reached;   /* sum of the out-degrees of reached vertices, over the runs */
-	uint64_t edges_forward;   /* in-edges read by the path-count sweeps */
+	uint64_t edges_forward;   /* edges read by the path-count sweeps (in-edges, or out-edges where a level is pushed) */
 	uint64_t edges_reverse;   /* out-edges read by the dependency sweeps */
 	float device_ms;          /* traversals + dependency launches, device events */
 	float traversal_ms;       /* of which the single-source traversals */
