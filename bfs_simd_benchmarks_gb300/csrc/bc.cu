@@ -50,7 +50,10 @@ struct BcShared {
 	unsigned long long e[kBcWarps];
 	uint32_t scan[kBcWarps];
 	uint32_t total;
-	uint32_t chunk_beg, chunk_end, owner;
+	uint32_t chunk_beg, chunk_end;
+	uint32_t beg[kBcClasses + 1];        // the level's classes in `order`
+	uint32_t items[kBcClasses + 1];      // work items before each class
+	uint32_t per[kBcClasses];            // vertices per item
 	uint32_t lv_deg[2][kBcTraceLevels];  // this CTA's out- and in-degree sums by level
 	union {
 		uint32_t cpre[kBcSmemBig + 1];        // chunk prefix of the level's big vertices
@@ -182,22 +185,29 @@ __device__ __forceinline__ typename Dir<kFwd>::T cta_range_sum(const BcArgs &a, 
 template <bool kFwd>
 __device__ __forceinline__ uint32_t chunk_prefix(const BcArgs &a, uint32_t bb, uint32_t cnt, uint32_t per) {
 	const uint32_t *off = Dir<kFwd>::off(a);
-	uint32_t carry = 0;
-	for (uint32_t t0 = 0; t0 < cnt; t0 += kBcThreads) {
-		const uint32_t i = t0 + threadIdx.x;
-		uint32_t c = 0;
-		if (i < cnt) {
-			const uint32_t v = ld_cg(a.order + bb + i);
-			c = (off[v + 1] - off[v] + per - 1) / per;
-		}
-		uint32_t tot;
-		const uint32_t ex = block_excl_scan(c, &tot);
-		if (i < cnt) bsh.cpre[i] = carry + ex;
-		carry += tot;
+	constexpr uint32_t kPer = kBcSmemBig / kBcThreads;  // consecutive entries per thread, their loads together
+	uint32_t v[kPer], c[kPer], sum = 0;
+#pragma unroll
+	for (uint32_t k = 0; k < kPer; ++k) {
+		const uint32_t i = threadIdx.x * kPer + k;
+		v[k] = i < cnt ? ld_cg(a.order + bb + i) : 0xFFFFFFFFu;
 	}
-	if (threadIdx.x == 0) bsh.cpre[cnt] = carry;
+#pragma unroll
+	for (uint32_t k = 0; k < kPer; ++k) {
+		c[k] = v[k] != 0xFFFFFFFFu ? (off[v[k] + 1] - off[v[k]] + per - 1) / per : 0u;
+		sum += c[k];
+	}
+	uint32_t total;
+	uint32_t run = block_excl_scan(sum, &total);
+#pragma unroll
+	for (uint32_t k = 0; k < kPer; ++k) {
+		const uint32_t i = threadIdx.x * kPer + k;
+		if (i < cnt) bsh.cpre[i] = run;
+		run += c[k];
+	}
+	if (threadIdx.x == 0) bsh.cpre[cnt] = total;
 	__syncthreads();
-	return carry;
+	return total;
 }
 // The largest i with cpre[i] <= j (cpre[cnt] > j).
 __device__ __forceinline__ uint32_t chunk_owner(uint32_t cnt, uint32_t j) {
@@ -216,48 +226,46 @@ __device__ __forceinline__ typename Dir<kFwd>::T big_finish_sum(const BcArgs &a,
 // Writes a vertex's finished sum (one thread).
 template <bool kFwd> __device__ __forceinline__ void finish_vertex(const BcArgs &a, uint32_t v, typename Dir<kFwd>::T sum);
 
-// Big vertices order[bb .. bb+nbig) (nbig <= kBcSmemBig) cut into chunks of
-// kBcChunk edges: CTA c sums chunks c, c + grid, ... into partial[] (value
-// bits); the one that completes a vertex's last chunk adds them in chunk
-// order and writes the vertex, and leaves its count at 0.
+// Chunk j (kBcWarpChunk edges) of the level's big vertices order[bb .. bb+nbig)
+// (prefix in bsh.cpre) by one warp, into partial[j] (value bits); the warp
+// that completes a vertex's last chunk adds them in a fixed order and writes
+// the vertex, and leaves its count at 0.
 template <bool kFwd>
-__device__ __forceinline__ void big_chunks(const BcArgs &a, uint32_t bb, uint32_t nbig, int target, bool use8,
+__device__ __forceinline__ void big_chunk(const BcArgs &a, uint32_t bb, uint32_t nbig, uint32_t j, int target, bool use8,
 		unsigned long long *edges) {
 	using T = typename Dir<kFwd>::T;
-	const uint32_t *off = Dir<kFwd>::off(a);
-	const uint32_t total = chunk_prefix<kFwd>(a, bb, nbig, kBcChunk);
-	for (uint32_t j = blockIdx.x; j < total; j += gridDim.x) {
-		if (threadIdx.x == 0) {
-			const uint32_t lo = chunk_owner(nbig, j);
-			const uint32_t v = ld_cg(a.order + bb + lo);
-			const uint32_t beg = off[v] + (j - bsh.cpre[lo]) * kBcChunk;
-			const uint32_t end = off[v + 1];
-			bsh.owner = lo;
-			bsh.chunk_beg = beg;
-			bsh.chunk_end = end - beg > kBcChunk ? beg + kBcChunk : end;
-		}
-		__syncthreads();
-		const uint32_t beg = bsh.chunk_beg, end = bsh.chunk_end, lo = bsh.owner;
-		const T s = cta_range_sum<kFwd>(a, beg, end, target, use8);
-		if (warp_id() != 0) continue;
-		const uint32_t c0 = bsh.cpre[lo], c1 = bsh.cpre[lo + 1];
-		uint32_t before = 0;
-		if (lane_id() == 0) {
-			a.partial[j] = Dir<kFwd>::bits(s);
-			// releases this partial to, and acquires the others' from, the chunks that count here
-			asm volatile("atom.acq_rel.gpu.global.add.u32 %0, [%1], 1;" : "=r"(before) : "l"(a.big_done + lo) : "memory");
-		}
-		if (__shfl_sync(kFull, before, 0) != c1 - c0 - 1) continue;
-		__syncwarp();
-		const T t = big_finish_sum<kFwd>(a, lo, false);
-		if (lane_id() == 0) {
-			const uint32_t v = ld_cg(a.order + bb + lo);
-			a.big_done[lo] = 0u;
-			finish_vertex<kFwd>(a, v, t);
-			*edges += off[v + 1] - off[v];
-		}
+	const uint32_t *off = Dir<kFwd>::off(a), *adj = Dir<kFwd>::adj(a);
+	const uint32_t lo = chunk_owner(nbig, j), c0 = bsh.cpre[lo], c1 = bsh.cpre[lo + 1];
+	const uint32_t v = ld_cg(a.order + bb + lo);
+	const uint32_t vbeg = off[v], vend = off[v + 1];
+	const uint32_t beg = vbeg + (j - c0) * kBcWarpChunk, end = min(beg + kBcWarpChunk, vend);
+	T s = T(0);
+	for (uint32_t e = beg + lane_id(); e < end; e += 32 * kBcUnroll) {
+		uint32_t nb[kBcUnroll];
+		uint2 lx[kBcUnroll];
+#pragma unroll
+		for (int k = 0; k < kBcUnroll; ++k) nb[k] = e + 32 * k < end ? __ldg(adj + e + 32 * k) : 0xFFFFFFFFu;
+		gather_tags(a, nb, lx, use8, target);
+#pragma unroll
+		for (int k = 0; k < kBcUnroll; ++k)
+			if ((int) lx[k].x == target) s += Dir<kFwd>::value(lx[k].y);
 	}
-	__syncthreads();
+	__syncwarp();
+	s = warp_sum(s);
+	uint32_t before = 0;
+	if (lane_id() == 0) {
+		a.partial[j] = Dir<kFwd>::bits(s);
+		// releases this partial to, and acquires the others' from, the chunks that count here
+		asm volatile("atom.acq_rel.gpu.global.add.u32 %0, [%1], 1;" : "=r"(before) : "l"(a.big_done + lo) : "memory");
+	}
+	if (__shfl_sync(kFull, before, 0) != c1 - c0 - 1) return;
+	__syncwarp();
+	const T t = big_finish_sum<kFwd>(a, lo, false);
+	if (lane_id() == 0) {
+		a.big_done[lo] = 0u;
+		finish_vertex<kFwd>(a, v, t);
+		*edges += vend - vbeg;
+	}
 }
 
 // The same for a level with more than kBcSmemBig big vertices: the chunk
@@ -355,19 +363,14 @@ __device__ __forceinline__ typename Dir<kFwd>::T big_finish_sum(const BcArgs &a,
 	return warp_sum(s);
 }
 
-// Sum over the edge list of one vertex by a half-warp (16 lanes); v_ok false
-// gives 0.  Both halves call it together (the reduction shuffles the warp).
+// Sum over the edges [beg, end) of one vertex by a half-warp (16 lanes).  Both
+// halves call it together (the reduction shuffles the warp).
 template <bool kFwd>
-__device__ __forceinline__ typename Dir<kFwd>::T half_vertex_sum(const BcArgs &a, uint32_t v, bool v_ok, int target,
+__device__ __forceinline__ typename Dir<kFwd>::T half_vertex_sum(const BcArgs &a, uint32_t beg, uint32_t end, int target,
 		bool use8) {
 	using T = typename Dir<kFwd>::T;
 	const uint32_t *adj = Dir<kFwd>::adj(a);
 	const uint32_t hl = lane_id() & 15u;
-	uint32_t beg = 0, end = 0;
-	if (v_ok) {
-		beg = Dir<kFwd>::off(a)[v];
-		end = Dir<kFwd>::off(a)[v + 1];
-	}
 	T s = T(0);
 	for (uint32_t e = beg + hl; e < end; e += 16u * kBcUnroll) {
 		uint32_t nb[kBcUnroll];
@@ -387,23 +390,17 @@ __device__ __forceinline__ typename Dir<kFwd>::T half_vertex_sum(const BcArgs &a
 	return s;
 }
 
-// Sum over the edge list of one vertex by one lane, in edge order: the list in
+// Sum over the edges [beg, end) of one vertex by one lane, in edge order: the list in
 // aligned 16-byte pieces, kBcQuads of them and their neighbours' values in
 // flight.  (32 vertices' concatenated lists walked by the warp, with an owner
 // search and a segmented scan per 32 edges, spent about 60 shuffles per 32
 // edges: 0.11 ms for the 8 M edges of a Pokec-shape level.)
 constexpr int kBcQuads = 2;
 template <bool kFwd>
-__device__ __forceinline__ typename Dir<kFwd>::T lane_vertex_sum(const BcArgs &a, uint32_t v, bool valid, int target,
-		bool use8, unsigned long long *edges) {
+__device__ __forceinline__ typename Dir<kFwd>::T lane_vertex_sum(const BcArgs &a, uint32_t beg, uint32_t end, int target,
+		bool use8) {
 	using T = typename Dir<kFwd>::T;
 	const uint32_t *adj = Dir<kFwd>::adj(a);
-	uint32_t beg = 0, end = 0;
-	if (valid) {
-		beg = Dir<kFwd>::off(a)[v];
-		end = Dir<kFwd>::off(a)[v + 1];
-	}
-	*edges += end - beg;
 	T s = T(0);
 	for (uint32_t q = beg & ~3u; q < end; q += 4 * kBcQuads) {
 		uint32_t nb[4 * kBcQuads];
@@ -463,8 +460,8 @@ __device__ __forceinline__ void push_paths(const BcArgs &a, uint32_t bb, uint32_
 	}
 }
 
-__device__ __forceinline__ void finish_dependency(const BcArgs &a, uint32_t v, float sum) {
-	const uint32_t sg = ld_cg(a.sigma + v);
+// sg: the vertex's path count
+__device__ __forceinline__ void finish_dependency(const BcArgs &a, uint32_t v, float sum, uint32_t sg) {
 	const float inv = sg ? 1.0f / (float) (int) sg : 0.0f;
 	const float dv = sum + inv;
 	a.lvx[v].y = __float_as_uint(dv);
@@ -478,7 +475,111 @@ template <> __device__ __forceinline__ void finish_vertex<true>(const BcArgs &a,
 	a.lvx[v].y = sum;
 }
 template <> __device__ __forceinline__ void finish_vertex<false>(const BcArgs &a, uint32_t v, float sum) {
-	finish_dependency(a, v, sum);
+	finish_dependency(a, v, sum, ld_cg(a.sigma + v));
+}
+
+// The vertices order[i], order[i + step], ... below `last`, one per half-warp
+// (kHalf) or lane: their sums for a level (none of their edges with `skip`).
+// The next vertex's edge range and path count and the one after's id are
+// loaded while a vertex is summed: without that, the chain order -> offsets ->
+// edges -> values -> count of each vertex is what a level waits for.
+template <bool kFwd, bool kHalf>
+__device__ __forceinline__ void sum_vertices(const BcArgs &a, uint32_t i, uint32_t step, uint32_t last, int target,
+		bool skip, bool use8, unsigned long long *edges) {
+	using T = typename Dir<kFwd>::T;
+	const uint32_t *off = Dir<kFwd>::off(a);
+	const bool writer = !kHalf || (lane_id() & 15u) == 0;
+	auto id_at = [&](uint32_t k) { return k < last ? ld_cg(a.order + k) : 0xFFFFFFFFu; };
+	uint32_t v = id_at(i), next = id_at(i + step);
+	uint32_t beg = 0, end = 0, sg = 0;
+	if (v != 0xFFFFFFFFu) {
+		beg = off[v];
+		end = off[v + 1];
+		if (!kFwd && writer) sg = ld_cg(a.sigma + v);
+	}
+	while (__any_sync(kFull, v != 0xFFFFFFFFu)) {
+		const uint32_t next2 = next != 0xFFFFFFFFu ? id_at(i + 2 * step) : 0xFFFFFFFFu;
+		uint32_t nbeg = 0, nend = 0, nsg = 0;
+		if (next != 0xFFFFFFFFu) {
+			nbeg = off[next];
+			nend = off[next + 1];
+			if (!kFwd && writer) nsg = ld_cg(a.sigma + next);
+		}
+		T s = T(0);
+		if (!skip) {
+			if constexpr (kHalf) s = half_vertex_sum<kFwd>(a, beg, end, target, use8);
+			else s = lane_vertex_sum<kFwd>(a, beg, end, target, use8);
+		}
+		if (writer && v != 0xFFFFFFFFu) {
+			if constexpr (kFwd) finish_vertex<true>(a, v, s);
+			else finish_dependency(a, v, s, sg);
+			if (!skip) *edges += end - beg;
+		}
+		__syncwarp();
+		v = next;
+		next = next2;
+		beg = nbeg;
+		end = nend;
+		sg = nsg;
+		i += step;
+	}
+}
+
+// Of cnt vertices of class c (1 .. kBcClasses - 1), how many a warp takes at a
+// time: at most about 2048 edges' worth, fewer where that would leave less than
+// two items per warp of the grid, at least one step's (a vertex per half-warp
+// or lane).
+__device__ __forceinline__ uint32_t class_item(uint32_t c, uint32_t cnt) {
+	const uint32_t least = c + 2 < kBcClasses ? 2u : 32u;
+	const uint32_t most = c + 2 < kBcClasses ? 1u << c : c + 2 == kBcClasses ? 128u : 256u;
+	return least * max(1u, min(most / least, cnt / (least * 2 * gridDim.x * kBcWarps)));
+}
+
+// All vertices of level d: big ones in chunks (`big`: not done by
+// big_chunks_global), then the medium bands, then the small ones, dealt to the
+// grid's warps in turn.  (With a CTA per chunk of 4096 edges, warps spent 39%
+// of their cycles at block barriers; handed out through a counter, small
+// levels paid more for the claims than large ones gained.)  What bounds a large
+// level is the L1 pipeline: a neighbour's pair is a 32-byte sector of its own
+// (18 M in-edges of a Pokec-shape level in 0.10 ms, 0.6 a cycle and SM).
+// `skip`: the level's sums are all empty.
+template <bool kFwd>
+__device__ __forceinline__ void level_sums(const BcArgs &a, uint32_t d, int target, bool big, bool skip, bool use8,
+		unsigned long long *edges) {
+	__syncthreads();
+	if (threadIdx.x <= kBcClasses) bsh.beg[threadIdx.x] = ld_cg(a.kstart + kBcClasses * d + threadIdx.x);
+	__syncthreads();
+	const uint32_t bb = bsh.beg[0], nbig = bsh.beg[1] - bb;
+	uint32_t chunks = 0;
+	if (big && nbig && !skip) chunks = chunk_prefix<kFwd>(a, bb, nbig, kBcWarpChunk);
+	if (threadIdx.x == 0) {
+		uint32_t n = chunks;
+		for (uint32_t c = 1; c < kBcClasses; ++c) {
+			bsh.items[c] = n;
+			const uint32_t cnt = bsh.beg[c + 1] - bsh.beg[c], per = class_item(c, cnt);
+			bsh.per[c] = per;
+			n += (cnt + per - 1) / per;
+		}
+		bsh.items[kBcClasses] = n;
+	}
+	__syncthreads();
+	const unsigned lane = lane_id();
+	if (skip)
+		for (uint32_t i = blockIdx.x * kBcThreads + threadIdx.x; i < nbig; i += gridDim.x * kBcThreads)
+			finish_vertex<kFwd>(a, ld_cg(a.order + bb + i), typename Dir<kFwd>::T(0));
+	const uint32_t total = bsh.items[kBcClasses];
+	// warps numbered across CTAs first, so that a few items are spread over all SMs
+	const uint32_t step = gridDim.x * kBcWarps;
+	uint32_t item = warp_id() * gridDim.x + blockIdx.x;
+	for (; item < chunks; item += step) big_chunk<kFwd>(a, bb, nbig, item, target, use8, edges);
+	for (; item < total; item += step) {
+		uint32_t c = 1;
+		while (item >= bsh.items[c + 1]) ++c;
+		const uint32_t first = bsh.beg[c] + (item - bsh.items[c]) * bsh.per[c];
+		const uint32_t last = min(first + bsh.per[c], bsh.beg[c + 1]);
+		if (c + 2 < kBcClasses) sum_vertices<kFwd, true>(a, first + (lane >> 4), 2, last, target, skip, use8, edges);
+		else sum_vertices<kFwd, false>(a, first + lane, 32, last, target, skip, use8, edges);
+	}
 }
 
 __global__ void __launch_bounds__(kBcThreads, 2) k_bc(BcArgs a) {
@@ -643,8 +744,6 @@ __global__ void __launch_bounds__(kBcThreads, 2) k_bc(BcArgs a) {
 	uint32_t pb = ld_cg(a.kstart);  // where the level before starts in `order`
 	for (uint32_t d = 1; d <= depth; ++d) {
 		const uint32_t bb = ld_cg(a.kstart + kBcClasses * d), be = ld_cg(a.kstart + kBcClasses * d + 1);
-		const uint32_t me = ld_cg(a.kstart + kBcClasses * d + kBcClasses - 2);
-		const uint32_t se = ld_cg(a.kstart + kBcClasses * d + kBcClasses);
 		// the counts of a pushed level are in lvx alone so far
 		if (pushed)
 			for (uint32_t i = pb + blockIdx.x * kBcThreads + threadIdx.x; i < bb; i += gridDim.x * kBcThreads) {
@@ -678,27 +777,8 @@ __global__ void __launch_bounds__(kBcThreads, 2) k_bc(BcArgs a) {
 					e_fwd += a.in_off[v + 1] - a.in_off[v];
 				}
 			}
-		} else if (nbig > 0) {
-			big_chunks<true>(a, bb, nbig, (int) d - 1, use8, &e_fwd);
 		}
-		for (uint32_t i0 = be + 2 * (tw - 1 - gw); i0 < me; i0 += 2 * tw) {
-			const uint32_t i = i0 + (lane >> 4);
-			const bool ok = i < me;
-			const uint32_t v = ok ? ld_cg(a.order + i) : 0u;
-			const uint32_t s = half_vertex_sum<true>(a, v, ok, (int) d - 1, use8);
-			if (ok && (lane & 15u) == 0) {
-				finish_vertex<true>(a, v, s);
-				e_fwd += a.in_off[v + 1] - a.in_off[v];
-			}
-		}
-		const uint32_t groups = (se - me + 31) / 32;
-		for (uint32_t grp = gw; grp < groups; grp += tw) {
-			const uint32_t idx = me + grp * 32 + lane;
-			const bool valid = idx < se;
-			const uint32_t v = valid ? ld_cg(a.order + idx) : 0u;
-			const uint32_t s = lane_vertex_sum<true>(a, v, valid, (int) d - 1, use8, &e_fwd);
-			if (valid) finish_vertex<true>(a, v, s);
-		}
+		level_sums<true>(a, d, (int) d - 1, nbig <= kBcSmemBig, false, use8, &e_fwd);
 		if (!grid_sync(ctl->bar, epoch, &ctl->err)) return;
 		if (blockIdx.x == 0 && threadIdx.x == 0 && d < kBcTraceLevels) ctl->t_fwd[d] = global_timer_ns();
 	}
@@ -719,41 +799,19 @@ __global__ void __launch_bounds__(kBcThreads, 2) k_bc(BcArgs a) {
 		const uint32_t me = ld_cg(a.kstart + kBcClasses * d + kBcClasses - 2);
 		const uint32_t se = ld_cg(a.kstart + kBcClasses * d + kBcClasses);
 		const uint32_t nbig = be - bb;
-		if (deepest) {
-			for (uint32_t i = gw; i < nbig; i += tw)
-				if (lane == 0) finish_dependency(a, ld_cg(a.order + bb + i), 0.0f);
-		} else if (nbig > kBcSmemBig) {
+		if (!deepest && nbig > kBcSmemBig) {
 			if (!big_chunks_global<false>(a, bb, nbig, d + 1, use8, epoch)) return;
 			if (!grid_sync(ctl->bar, epoch, &ctl->err)) return;
 			for (uint32_t i = gw; i < nbig; i += tw) {
 				const uint32_t v = ld_cg(a.order + bb + i);
 				const float s = big_finish_sum<false>(a, i, true);
 				if (lane == 0) {
-					finish_dependency(a, v, s);
+					finish_vertex<false>(a, v, s);
 					e_rev += a.row_off[v + 1] - a.row_off[v];
 				}
 			}
-		} else if (nbig > 0) {
-			big_chunks<false>(a, bb, nbig, d + 1, use8, &e_rev);
 		}
-		for (uint32_t i0 = be + 2 * (tw - 1 - gw); i0 < me; i0 += 2 * tw) {
-			const uint32_t i = i0 + (lane >> 4);
-			const bool ok = i < me;
-			const uint32_t v = ok ? ld_cg(a.order + i) : 0u;
-			const float s = half_vertex_sum<false>(a, v, ok && !deepest, d + 1, use8);
-			if (ok && (lane & 15u) == 0) {
-				finish_dependency(a, v, s);
-				if (!deepest) e_rev += a.row_off[v + 1] - a.row_off[v];
-			}
-		}
-		const uint32_t groups = (se - me + 31) / 32;
-		for (uint32_t grp = gw; grp < groups; grp += tw) {
-			const uint32_t idx = me + grp * 32 + lane;
-			const bool valid = idx < se;
-			const uint32_t v = valid ? ld_cg(a.order + idx) : 0u;
-			const float s = deepest ? 0.0f : lane_vertex_sum<false>(a, v, valid, d + 1, use8, &e_rev);
-			if (valid) finish_dependency(a, v, s);
-		}
+		level_sums<false>(a, (uint32_t) d, d + 1, nbig <= kBcSmemBig, deepest, use8, &e_rev);
 		if (d > 0 && !grid_sync(ctl->bar, epoch, &ctl->err)) return;
 		if (blockIdx.x == 0 && threadIdx.x == 0 && (uint32_t) d < kBcTraceLevels) {
 			ctl->t_rev[d] = global_timer_ns();

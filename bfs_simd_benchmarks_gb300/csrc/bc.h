@@ -24,11 +24,12 @@ static_assert(kBcClasses * kBcMaxLevels <= kBcCntCap, "every sort key needs a co
 constexpr uint32_t kBcByteLevelsMinVertices = 1u << 22;  // default: byte levels from here (the 8-byte
                                                          // {level, value} array outgrows L2)
 constexpr uint32_t kBcChunk = 4096;           // edges of a big vertex one CTA sums as one task
+constexpr uint32_t kBcWarpChunk = 512;        // ... and a warp, where the chunk list is in shared memory
 constexpr uint32_t kBcSmemBig = 4096;         // big vertices of a level whose chunk list every CTA keeps in shared
                                               // memory; a level with more builds it in global memory
 
 // Chunk partial sums a graph of n vertices and m edges can need in one level.
-inline size_t bc_partial_capacity(uint64_t n, uint64_t m) { return n + kBcSmemBig + m / kBcChunk + 2; }
+inline size_t bc_partial_capacity(uint64_t n, uint64_t m) { return n + kBcSmemBig + m / kBcWarpChunk + 2; }
 
 struct BcControl {
 	unsigned bar[2];            // grid barrier

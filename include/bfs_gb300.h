@@ -512,8 +512,8 @@ typedef struct bfs_bc_stats {
 	uint32_t grid_ctas;
 	/* the (last) run, per level d < BFS_BC_TRACE_LEVELS: path-count and
 	 * dependency times, vertices, and of those the ones whose in- or
-	 * out-degree is above 1024 (reduced by whole CTAs) or above 32 (one warp
-	 * each; the rest are taken 32 to a warp) */
+	 * out-degree is above 1024 (summed in chunks) or above 32 (a half-warp
+	 * each; the rest a lane each) */
 	float level_paths_ms[BFS_BC_TRACE_LEVELS];
 	float level_dependencies_ms[BFS_BC_TRACE_LEVELS];
 	uint32_t level_vertices[BFS_BC_TRACE_LEVELS];
