@@ -390,7 +390,7 @@ __device__ __forceinline__ typename Dir<kFwd>::T half_vertex_sum(const BcArgs &a
 	return s;
 }
 
-// Sum over the edges [beg, end) of one vertex by one lane, in edge order: the list in
+// Sum over the edges [beg, end) of one vertex by one lane: the list in
 // aligned 16-byte pieces, kBcQuads of them and their neighbours' values in
 // flight.  (32 vertices' concatenated lists walked by the warp, with an owner
 // search and a segmented scan per 32 edges, spent about 60 shuffles per 32
@@ -422,9 +422,15 @@ __device__ __forceinline__ typename Dir<kFwd>::T lane_vertex_sum(const BcArgs &a
 			}
 		}
 		gather_tags(a, nb, lx, use8, target);
+		// pairwise: a list of 32 takes 3 + 4 roundings in a row, not 32
+		T x[4 * kBcQuads];
 #pragma unroll
-		for (int k = 0; k < 4 * kBcQuads; ++k)
-			if ((int) lx[k].x == target) s += Dir<kFwd>::value(lx[k].y);
+		for (int k = 0; k < 4 * kBcQuads; ++k) x[k] = (int) lx[k].x == target ? Dir<kFwd>::value(lx[k].y) : T(0);
+#pragma unroll
+		for (int d = 1; d < 4 * kBcQuads; d *= 2)
+#pragma unroll
+			for (int k = 0; k + d < 4 * kBcQuads; k += 2 * d) x[k] += x[k + d];
+		s += x[0];
 	}
 	return s;
 }
