@@ -52,20 +52,26 @@ constexpr int kMsFinishRows = 2;        // push: touched rows finished per round
 constexpr uint32_t kLaneMaxDeg = 32;    // pull, few words: destinations of at most this in-degree go one per lane
 constexpr uint32_t kGroupMaxWords = 8;  // pull: up to this many words, in-neighbour rows in lane groups
 constexpr uint32_t kEmitW = 4;          // output tile: kV vertices x kW words (4: 256 sources), kV = threads / kW
-// shared bytes of an output tile of kV vertices: rows of one source quad (kV + 4
-// words, 16-byte aligned; `bufs` copies) and the nibble table
-// (shifted rows: one copy, and the rows themselves)
-__host__ __device__ constexpr uint32_t emit_bytes(uint32_t kV, uint32_t bufs = 1, uint32_t kW = kEmitW, bool shift = false) {
-	return shift ? (kW * 16 * (kV + 4) + 16) * 4 + kW * 64 * (kV + 16) : (bufs * kW * 16 * (kV + 4) + 16) * 4;
+constexpr uint32_t kEmitPlanes = 7;  // planes that a 3-bit index tells apart, with one value left for "none of them"
+constexpr uint32_t kEmitUnits = 8;   // output tiles' words are split among CTAs below this many per CTA
+// Words of a tile's shared memory per word of its vertices: 16 source quads, each
+// a row of kV words with 4 more after every 16 (the second phase's 16-byte reads
+// of 16 vertices per lane then fall on different banks), and the shift that puts
+// the kW words of 32 / kW vertices on 32 different banks.
+__host__ __device__ constexpr uint32_t emit_row(uint32_t kV) { return kV / 16 * 20; }
+__host__ __device__ constexpr uint32_t emit_word_stride(uint32_t kV, uint32_t kW) { return 16 * emit_row(kV) + 32 / kW; }
+// planes whose words are fetched a step ahead: two groups of seven; one where a
+// vertex has more words, whose masks leave the second group nearly empty
+__host__ __device__ constexpr uint32_t emit_slots(uint32_t kW) { return kW == 4 ? kEmitPlanes : 2 * kEmitPlanes; }
+// shared bytes of an output tile: its quads' rows (or, in their place, its
+// source rows); ahead: per thread a slot per plane of a step, and with kW = 4 its
+// word masks
+__host__ __device__ constexpr uint32_t emit_bytes(uint32_t kV, uint32_t kW, bool ahead) {
+	return kW * emit_word_stride(kV, kW) * 4 + (ahead ? (emit_slots(kW) + (kW == 4 ? 4 : 0)) * kV * kW * 8 : 0);
 }
 constexpr uint32_t kMsRowWords = 4;     // pull: up to this many words per vertex, rows are read whole
 constexpr uint32_t kEmitV = kMsThreads / kEmitW;  // the traversal kernel's tiles (its early output passes)
-constexpr uint32_t kEmitBytes = emit_bytes(kEmitV);
-// The output pass launch: tiles of 64 vertices (256 threads, 4 CTAs per SM)
-// or 128 vertices (512 threads, 2 per SM); by default the wide tiles from
-// kEmitWideMinVertices vertices (measured: 64 wins on 2^22 vertices, 128 on
-// 4.2e7, where the half-line row pieces of narrow tiles cost more)
-constexpr uint32_t kEmitWideMinVertices = 1u << 24;
+constexpr uint32_t kEmitBytes = emit_bytes(kEmitV, kEmitW, false);
 
 __device__ __forceinline__ uint64_t ld_cg64(const uint64_t *p) { return __ldcg((const unsigned long long *) p); }
 __device__ __forceinline__ uint64_t shfl64(uint64_t x, int src) {
@@ -793,22 +799,47 @@ __device__ __forceinline__ void ms_pull(const MsArgs &a, const MsPull &p, unsign
 
 // Planes [first, last] (levels base + p) -> uint8 levels [source][vertex].
 // A CTA of 512 threads takes tiles of 128 vertices x 4 words (256 sources).
-// 1. thread (vertex, word) -- a warp holds 32 consecutive vertices of one
-//    word -- builds the 64 level bytes of its word's sources in 16 registers:
-//    for every plane whose word mask says the word is non-zero it loads the
-//    word and, four sources at a time, looks the nibble up in a 16-entry
-//    shared table of byte masks and writes the plane's level under it.  A
-//    byte starts at 255 and is written at most once (a source reaches a vertex
-//    at one level), so "write" is an XOR with 255 ^ level.  The 16 words go to
-//    shared memory as [word][source quad][vertex].
+// 1. thread (vertex, word) -- the words of a vertex on neighbouring lanes, so
+//    that a warp's load touches one sector per vertex -- builds the 64 level
+//    bytes of its word's sources in 16 registers.  For every plane whose word
+//    mask says the word is non-zero it loads the word.  Of 7 planes, a source's
+//    bit is set in one at most: three words hold that plane's number in binary
+//    (7: none), their bits are brought together as one nibble per source, and a
+//    byte permute looks four nibbles up in the 8 bytes {lvl .. lvl + 6, 255} at
+//    once.  That is about 100 instructions per 7 planes whatever they hold; an
+//    XOR of looked-up byte masks per plane took 80 for each of them, the output
+//    was bound by it (rmat, 2^20 vertices, 1,024 sources: 0.74 ms, 57% of the
+//    issue slots, 58% of L1; now 0.40) and each lane of a warp read another
+//    sector.  The 16 registers go to shared memory as [word][source quad][vertex].
 // 2. thread (word, source quad, 16 vertices) reads its 16 words with 16-byte
 //    loads, transposes them 4 x 4 bytes at a time (byte permutes) into the
 //    16-byte pieces of its 4 source rows and stores those.
 // `merge` combines with the bytes already in `levels` (a later segment of a
 // traversal deeper than the planes) by a byte-wise minimum: every byte is
 // below 255 in at most one segment.
-__device__ __forceinline__ uint32_t nibble_bytes(uint32_t nib) {
-	return ((nib * 0x00204081u) & 0x01010101u) * 0xFFu;  // bit i -> byte i all ones
+// Source j of quad q (j < 4, q < 16) among its word's 64.
+__device__ __forceinline__ constexpr uint32_t emit_source(uint32_t q, uint32_t j) { return q / 4 * 16 + q % 4 + 4 * j; }
+
+// The 64 level bytes of a word's sources, lvl + t where plane w[t] has the
+// source's bit and 255 where none has, combined into o (a source's bit is set
+// in one plane at most, and 255 is all ones: an AND).
+__device__ __forceinline__ void emit_bytes_of(const uint64_t (&w)[kEmitPlanes], uint32_t lvl, uint32_t (&o)[16]) {
+	const uint32_t lo = lvl * 0x01010101u + 0x03020100u, hi = (lvl * 0x00010101u + 0x00060504u) | 0xFF000000u;
+#pragma unroll
+	for (int h = 0; h < 2; ++h) {
+		uint32_t x[kEmitPlanes];
+#pragma unroll
+		for (uint32_t t = 0; t < kEmitPlanes; ++t) x[t] = (uint32_t) (w[t] >> (32 * h));
+		const uint32_t none = ~(x[0] | x[1] | x[2] | x[3] | x[4] | x[5] | x[6]);
+		const uint32_t b0 = x[1] | x[3] | x[5] | none, b1 = x[2] | x[3] | x[6] | none, b2 = x[4] | x[5] | x[6] | none;
+#pragma unroll
+		for (uint32_t r = 0; r < 4; ++r) {  // nibble i of sel: the index of source 32 h + 4 i + r
+			const uint32_t c1 = r ? b1 >> (r - 1) : b1 << 1, c2 = r < 2 ? b2 << (2 - r) : b2 >> (r - 2);
+			const uint32_t sel = ((b0 >> r) & 0x11111111u) | (c1 & 0x22222222u) | (c2 & 0x44444444u);
+			o[8 * h + r] &= __byte_perm(lo, hi, sel);
+			o[8 * h + 4 + r] &= __byte_perm(lo, hi, sel >> 16);
+		}
+	}
 }
 
 // 16 level bytes (x, vertices in order) -> levels at dst, cnt <= 16 of them,
@@ -852,17 +883,17 @@ __device__ __forceinline__ void emit_piece(uint8_t *dst, const uint32_t (&x)[4],
 	}
 }
 
-// kCached: the planes may be read through L1 (a launch of its own after the
-// traversal; the four warps of a tile read neighbouring words of the same
-// sectors); inside the traversal kernel they are read around L1.
-template <bool kCached>
-__device__ __forceinline__ uint64_t emit_ld(const uint64_t *p) {
-	return kCached ? (uint64_t) __ldg((const unsigned long long *) p) : ld_cg64(p);
+__device__ __forceinline__ void cp_async8(void *dst, const void *src) {
+	asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" :: "r"((uint32_t) __cvta_generic_to_shared(dst)), "l"(src) : "memory");
 }
+__device__ __forceinline__ void cp_async_wait() { asm volatile("cp.async.wait_all;" ::: "memory"); }
 
-// kCached also selects two row buffers used in turn, so that a tile needs one
-// barrier (between its two phases): a buffer is written again two tiles
-// later, after the barrier that every thread reaches once done reading it.
+// kAhead (the launch of its own after the traversal): a step's words are copied
+// to shared memory while the step before is looked up, transposed and stored;
+// every thread copies what it reads itself, so that no barrier is between.  A
+// CTA goes through a tile's words before it takes another tile, so that a
+// tile's masks come from L1 and the neighbouring sectors of its rows from L2.
+// Without kAhead (inside the traversal kernel) everything is read around L1.
 //
 // kShift: rows that do not start on 16-byte boundaries (n or `levels` not a
 // multiple of 16).  Phase 2 then leaves its bytes in shared memory, row by row,
@@ -915,69 +946,130 @@ __device__ __forceinline__ void emit_shifted(const uint8_t *src, uint8_t *dst, u
 	}
 }
 
-template <bool kCached, uint32_t kV, uint32_t kW, bool kShift>
+template <bool kAhead, uint32_t kV, uint32_t kW, bool kShift>
 __device__ __noinline__ void ms_emit(const MsArgs &a, uint8_t *levels, uint32_t ns, uint32_t base, uint32_t first, uint32_t last,
 		bool merge, uint8_t *lev) {
-	constexpr uint32_t kEmitV = kV, kEmitW = kW, kEmitRow = kV + 4;
-	constexpr uint32_t kBufs = kCached && !kShift ? 2 : 1, kBufWords = kEmitW * 16 * kEmitRow;
-	constexpr uint32_t kRows = kEmitW * 64;
+	static_assert(!kShift || kW * 64 * emit_row_bytes(kV) <= kW * emit_word_stride(kV, kW) * 4, "source rows fit in the quads' place");
+	constexpr uint32_t kThreads = kV * kW, kRow = emit_row(kV), kSlots = emit_slots(kW), kWordStride = emit_word_stride(kV, kW), kRows = kW * 64;
 	const uint32_t K = a.K, n = a.n;
-	const uint32_t vtiles = (n + kEmitV - 1) / kEmitV, wtiles = (K + kEmitW - 1) / kEmitW;
-	const uint32_t vi = threadIdx.x % kEmitV, wi = threadIdx.x / kEmitV;
+	const uint32_t vtiles = (n + kV - 1) / kV, wtiles = (K + kW - 1) / kW;
+	const uint32_t vi = threadIdx.x / kW, wi = threadIdx.x % kW;
 	const size_t pstride = (size_t) n * K;
-	uint32_t *const sw0 = reinterpret_cast<uint32_t *>(lev);  // [buffer][wi * 16 + quad][kEmitRow]
-	uint32_t *lut = sw0 + kBufs * kBufWords;                 // nibble -> byte mask
-	uint8_t *const rows = reinterpret_cast<uint8_t *>(lut + 16);  // kShift: [source][emit_row_bytes]
-	if (threadIdx.x < 16) lut[threadIdx.x] = nibble_bytes(threadIdx.x);
+	uint32_t *const sw = reinterpret_cast<uint32_t *>(lev);  // [wi][quad][kRow]
+	uint8_t *const rows = lev;  // kShift: then [source][emit_row_bytes]
+	// this thread's words of one step, a slot per plane (kAhead)
+	uint64_t *const slot = reinterpret_cast<uint64_t *>(lev + kW * kWordStride * 4) + threadIdx.x;
+	uint2 *const group = reinterpret_cast<uint2 *>(slot + kSlots * kThreads);
 	// phase 2's item: rows of source quad rq (word rq / 16), vertices 16 cc ...
-	const uint32_t rq = threadIdx.x / (kEmitV / 16), cc = threadIdx.x % (kEmitV / 16);
-	__syncthreads();
-	uint32_t turn = 0;
-	for (uint32_t tile = blockIdx.x; tile < vtiles * wtiles; tile += gridDim.x, ++turn) {
-		uint32_t *sw = sw0 + (turn % kBufs) * kBufWords;
-		const uint32_t v0 = (tile % vtiles) * kEmitV, k0 = (tile / vtiles) * kEmitW;
-		const uint32_t nv = min(kEmitV, n - v0);
-		const uint32_t nrows = min(kRows, ns - k0 * 64);
-		// 1. this thread's 64 level bytes
-		if (vi < nv && k0 + wi < K) {
-			const uint32_t v = v0 + vi, k = k0 + wi;
-			const uint64_t *pw = a.hist + ((size_t) first * n + v) * K + k;
-			const uint64_t *pm = a.pmask + (size_t) first * n + v;
-			uint32_t o[16];
+	const uint32_t rq = threadIdx.x / (kV / 16), cc = threadIdx.x % (kV / 16);
+	const uint32_t rw = rq / 16, q2 = rq % 16;
+	// a CTA takes a tile's words one after another, as many as leave every CTA work
+	uint32_t len = wtiles;
+	while (len > 1 && (uint64_t) vtiles * ((wtiles + len - 1) / len) < (uint64_t) kEmitUnits * gridDim.x) len = (len + 1) / 2;
+	const uint32_t units = vtiles * ((wtiles + len - 1) / len);
+	uint32_t unit = blockIdx.x, v0 = 0, kt = 0, kend = 0, l = first;
+	const auto place = [&] {  // the unit's first tile
+		v0 = unit % vtiles * kV;
+		kt = unit / vtiles * len;
+		kend = min(kt + len, wtiles);
+	};
+	// which of the step's planes have a non-zero word for this thread
+	const auto step_planes = [&] { return min(last + 1 - l, 2 * kEmitPlanes); };
+	const auto inside = [&] { return v0 + vi < n && kt * kW + wi < K; };
+	const auto nonzero = [&] {
+		if (!inside()) return 0u;
+		const uint32_t cnt = step_planes(), k = kt * kW + wi;
+		if (K <= kMsRowWords) return (1u << cnt) - 1u;  // rows of so few words are zero where nothing is
+		if constexpr (kAhead) {
+			const uint2 g[4] = {group[0], group[kThreads], group[2 * kThreads], group[3 * kThreads]};
+			uint32_t nz = 0;
 #pragma unroll
-			for (int q = 0; q < 16; ++q) o[q] = 0xFFFFFFFFu;
-			// 8 planes per round: their word masks (one round trip), then the
-			// non-zero words (one more)
-			for (uint32_t l = first; l <= last; l += 8) {
-				uint32_t nz = K <= kMsRowWords ? 0xFFu >> (l + 7 <= last ? 0u : l + 7 - last) : 0u;  // rows are zero where nothing is
+			for (int i = 0; i < 4; ++i) nz |= ((kt < 8 ? g[i].x : g[i].y) >> (4 * (kt % 8)) & 15u) << (4 * i);
+			return nz;
+		}
+		uint32_t nz = 0;
+		for (uint32_t t = 0; t < cnt; ++t) nz |= (uint32_t) (ld_cg64(a.pmask + (size_t) (l + t) * n + v0 + vi) >> k & 1u) << t;
+		return nz;
+	};
+	// kAhead: the bits of this thread's words (every kW-th) in the step's masks, nibble kt of group i planes 4 i ..
+	const auto masks = [&] {
+		if (K <= kMsRowWords || !inside()) return;
+		const uint32_t cnt = step_planes();
+		const unsigned long long *pm = reinterpret_cast<const unsigned long long *>(a.pmask) + (size_t) l * n + v0 + vi;
 #pragma unroll
-				for (int t = 0; t < 8; ++t)
-					if (K > kMsRowWords && l + t <= last)
-						nz |= (uint32_t) ((emit_ld<kCached>(pm + (size_t) (l - first + t) * n) >> k) & 1ull) << t;
-				uint64_t w[8];
+		for (uint32_t i = 0; i < 4; ++i) {
+			unsigned long long g = 0;
 #pragma unroll
-				for (int t = 0; t < 8; ++t)
-					w[t] = ((nz >> t) & 1u) ? emit_ld<kCached>(pw + (size_t) (l - first + t) * pstride) : 0ull;
+			for (uint32_t t = 4 * i; t < min(4 * i + 4, 2 * kEmitPlanes); ++t)
+				if (t < cnt) g |= (__ldg(pm + (size_t) t * n) >> wi & 0x1111111111111111ull) << (t % 4);
+			group[i * kThreads] = make_uint2((uint32_t) g, (uint32_t) (g >> 32));
+		}
+	};
+	const auto plane_words = [&] { return a.hist + (size_t) l * pstride + (size_t) (v0 + vi) * K + kt * kW + wi; };
+	const auto fetch = [&] {  // kAhead: the step's words -> the slots, asynchronously
+		const uint32_t nz = nonzero();
+		const uint64_t *pw = plane_words();
 #pragma unroll
-				for (int t = 0; t < 8; ++t) {
-					if (!w[t]) continue;
-					const uint32_t inv = ~((uint32_t) (base + l + t) * 0x01010101u);
-					const uint32_t lo = (uint32_t) w[t], hi = (uint32_t) (w[t] >> 32);
+		for (uint32_t h = 0; h < kSlots / kEmitPlanes; ++h) {
+			if (!(nz >> (h * kEmitPlanes))) break;
 #pragma unroll
-					for (int q = 0; q < 8; ++q) o[q] ^= lut[(lo >> (4 * q)) & 0xFu] & inv;
+			for (uint32_t t = h * kEmitPlanes; t < (h + 1) * kEmitPlanes; ++t)
+				if ((nz >> t) & 1u) cp_async8(slot + t * kThreads, pw + (size_t) t * pstride);
+		}
+		return nz;
+	};
+	if (unit >= units) return;
+	place();
+	if (kAhead) masks();
+	uint32_t nz = kAhead ? fetch() : 0u;
+	uint32_t o[16];
 #pragma unroll
-					for (int q = 0; q < 8; ++q) o[8 + q] ^= lut[(hi >> (4 * q)) & 0xFu] & inv;
-				}
+	for (int q = 0; q < 16; ++q) o[q] = 0xFFFFFFFFu;
+	for (;;) {
+		// 1. this thread's 64 level bytes, 14 planes a step
+		if (!kAhead) nz = nonzero();
+		else cp_async_wait();
+#pragma unroll
+		for (uint32_t h = 0; h < 2; ++h) {
+			if (!(nz >> (h * kEmitPlanes))) break;
+			const uint64_t *pw = plane_words();
+			uint64_t w[kEmitPlanes];
+#pragma unroll
+			for (uint32_t t = 0; t < kEmitPlanes; ++t) {
+				const uint32_t p = h * kEmitPlanes + t;
+				w[t] = !((nz >> p) & 1u) ? 0ull : kAhead && p < kSlots ? slot[p * kThreads] : ld_cg64(pw + (size_t) p * pstride);
 			}
-			uint32_t *col = sw + wi * 16 * kEmitRow + vi;
+			emit_bytes_of(w, base + l + h * kEmitPlanes, o);
+		}
+		const uint32_t tv0 = v0, k0 = kt * kW;
+		const bool out = l + 2 * kEmitPlanes > last;
+		bool more = true;
+		l += 2 * kEmitPlanes;
+		if (out) {
+			l = first;
+			if (++kt == kend) {
+				unit += gridDim.x;
+				more = unit < units;
+				if (more) place();
+			}
+		}
+		if (kAhead && more && (!out || kt == unit / vtiles * len || last - first >= 2 * kEmitPlanes)) masks();
+		if (kAhead) nz = more ? fetch() : 0u;
+		if (!out) continue;
+		const uint32_t nv = min(kV, n - tv0), nrows = min(kRows, ns - k0 * 64);
+		uint32_t *col = sw + wi * kWordStride + vi + vi / 16 * 4;
 #pragma unroll
-			for (int q = 0; q < 16; ++q) col[q * kEmitRow] = o[q];
+		for (int q = 0; q < 16; ++q) {
+			col[q * kRow] = o[q];
+			o[q] = 0xFFFFFFFFu;
 		}
 		__syncthreads();
 		// 2. rows out: 16 vertices x 4 source rows per thread
-		const uint32_t c = cc * 16, r0 = rq * 4;
-		if (k0 + rq / 16 < K && r0 < nrows && c < nv) {
-			const uint4 *sp = reinterpret_cast<const uint4 *>(sw + rq * kEmitRow + c);
+		const uint32_t c = cc * 16, r0 = rw * 64 + emit_source(q2, 0);
+		const bool piece = k0 + rw < K && r0 < nrows && c < nv;
+		uint32_t y[4][4];  // y[b][g]: source r0 + 4 b, vertices c + 4g .. c + 4g + 3
+		if (piece) {
+			const uint4 *sp = reinterpret_cast<const uint4 *>(sw + rw * kWordStride + q2 * kRow + cc * 20);
 			uint32_t x[16];
 #pragma unroll
 			for (int j = 0; j < 4; ++j) {
@@ -987,8 +1079,6 @@ __device__ __noinline__ void ms_emit(const MsArgs &a, uint8_t *levels, uint32_t 
 				x[4 * j + 2] = u.z;
 				x[4 * j + 3] = u.w;
 			}
-			// y[b][g]: source 4 rq + b, vertices c + 4g .. c + 4g + 3
-			uint32_t y[4][4];
 #pragma unroll
 			for (int g = 0; g < 4; ++g) {
 				const uint32_t t0 = __byte_perm(x[4 * g], x[4 * g + 1], 0x5140);
@@ -1000,16 +1090,29 @@ __device__ __noinline__ void ms_emit(const MsArgs &a, uint8_t *levels, uint32_t 
 				y[2][g] = __byte_perm(t2, t3, 0x5410);
 				y[3][g] = __byte_perm(t2, t3, 0x7632);
 			}
+		}
+		if (kShift) __syncthreads();  // the source rows take the quads' place
+		if (piece) {
 			const uint32_t cnt = min(16u, nv - c);
 #pragma unroll
 			for (int b = 0; b < 4; ++b) {
 				if constexpr (kShift) {
-					*reinterpret_cast<uint4 *>(rows + (r0 + b) * emit_row_bytes(kV) + c) =
+					*reinterpret_cast<uint4 *>(rows + (r0 + 4 * b) * emit_row_bytes(kV) + c) =
 							make_uint4(y[b][0], y[b][1], y[b][2], y[b][3]);
 					continue;
 				}
-				if (r0 + b >= nrows) break;
-				emit_piece(levels + (size_t) (k0 * 64 + r0 + b) * n + v0 + c, y[b], cnt, merge);
+				if (r0 + 4 * b >= nrows) break;
+				if constexpr (kAhead) {  // whole pieces of aligned rows: see the launch
+					uint4 *const d = reinterpret_cast<uint4 *>(levels + (size_t) (k0 * 64 + r0 + 4 * b) * n + tv0 + c);
+					uint4 z = make_uint4(y[b][0], y[b][1], y[b][2], y[b][3]);
+					if (merge) {
+						const uint4 old = __ldcg(d);
+						z = make_uint4(__vminu4(z.x, old.x), __vminu4(z.y, old.y), __vminu4(z.z, old.z), __vminu4(z.w, old.w));
+					}
+					*d = z;
+					continue;
+				}
+				emit_piece(levels + (size_t) (k0 * 64 + r0 + 4 * b) * n + tv0 + c, y[b], cnt, merge);
 			}
 		}
 		if (kShift) {
@@ -1017,11 +1120,11 @@ __device__ __noinline__ void ms_emit(const MsArgs &a, uint8_t *levels, uint32_t 
 			constexpr uint32_t kPieces = kV / 16 + 1;
 			for (uint32_t i = threadIdx.x; i < nrows * kPieces; i += blockDim.x) {
 				const uint32_t r = i / kPieces;
-				emit_shifted(rows + r * emit_row_bytes(kV), levels + (size_t) (k0 * 64 + r) * n + v0, nv, i % kPieces, merge);
+				emit_shifted(rows + r * emit_row_bytes(kV), levels + (size_t) (k0 * 64 + r) * n + tv0, nv, i % kPieces, merge);
 			}
-		} else if (kBufs == 1) {
-			__syncthreads();
 		}
+		if (!more) return;
+		__syncthreads();
 	}
 }
 
@@ -1188,13 +1291,14 @@ __global__ void __launch_bounds__(kMsThreads, 2) k_ms_bfs(const __grid_constant_
 	if (leader) ctl->stats.depth = lvl;
 }
 
-// The final output pass, its own launch after k_ms_bfs (more CTAs per SM than
-// the cooperative kernel, so more plane loads in flight).  Plane depth - base
-// is the empty frontier; after an early output pass, plane 0 was written too.
-// A tile's plane loads and its barriers form a chain of round trips; narrow
-// tiles on small CTAs keep more chains going per SM.  A tile is kW words wide,
-// a thread per (vertex, word): with one or two words per vertex, tiles of four
-// would leave most threads idle.
+// The final output pass, its own launch after k_ms_bfs.  Plane depth - base is
+// the empty frontier; after an early output pass, plane 0 was written too.  A
+// tile is kW words wide, a thread per (vertex, word): with one or two words per
+// vertex, tiles of four would leave most threads idle.  512 threads: level rows
+// go out in pieces of 128 bytes or more, 5.5 ms for 2^22 vertices and 4,096
+// sources (17 GB of levels, 4 TB/s with the planes read; 11.7 ms before the words
+// came ahead and by permute), where pieces of 64 bytes (256 threads, option
+// batch_output_tile) take 7.3 and of 256 bytes (1,024) 5.9.
 template <int kThreads, uint32_t kW, bool kShift>
 __global__ void __launch_bounds__(kThreads, kThreads == 256 ? 4 : 2) k_ms_emit(MsArgs a, uint32_t ns, uint8_t *levels) {
 	constexpr uint32_t kV = kThreads / kW;
@@ -1210,7 +1314,7 @@ __global__ void __launch_bounds__(kThreads, kThreads == 256 ? 4 : 2) k_ms_emit(M
 // The output pass's launch for a tile of kThreads / kW vertices x kW words.
 template <int kThreads, uint32_t kW, bool kShift>
 int emit_launch(const MsArgs &a, uint32_t ns, uint8_t *levels, int num_sms, cudaStream_t st) {
-	constexpr int kBytes = (int) emit_bytes(kThreads / kW, 2, kW, kShift);
+	constexpr int kBytes = (int) emit_bytes(kThreads / kW, kW, true);
 	auto fn = k_ms_emit<kThreads, kW, kShift>;
 	if (kBytes > 48 * 1024 && cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, kBytes) != cudaSuccess)
 		return BFS_ECUDA;
@@ -1262,13 +1366,12 @@ int ms_launch(const MsArgs &a, const uint32_t *d_sources, uint32_t ns, uint8_t *
 	if (between && cudaEventRecord(between, st) != cudaSuccess) return BFS_ECUDA;
 	if (between2 && cudaEventRecord(between2, st) != cudaSuccess) return BFS_ECUDA;
 	if (levels) {
-		const bool wide = a.out_tile ? a.out_tile == 128 : a.n >= kEmitWideMinVertices;
 		const uint32_t words = a.out_tile || a.K > 2 ? kEmitW : a.K;  // an explicit tile width is one of four-word tiles
 		const bool shift = a.n % 16 != 0 || (uintptr_t) levels % 16 != 0;
-		const auto launch = words == 1 ? (shift ? emit_launch<256, 1, true> : emit_launch<256, 1, false>)
-				: words == 2 ? (shift ? emit_launch<256, 2, true> : emit_launch<256, 2, false>)
-				: wide ? (shift ? emit_launch<512, kEmitW, true> : emit_launch<512, kEmitW, false>)
-				: (shift ? emit_launch<256, kEmitW, true> : emit_launch<256, kEmitW, false>);
+		const auto launch = words == 1 ? (shift ? emit_launch<512, 1, true> : emit_launch<512, 1, false>)
+				: words == 2 ? (shift ? emit_launch<512, 2, true> : emit_launch<512, 2, false>)
+				: a.out_tile == 64 ? (shift ? emit_launch<256, kEmitW, true> : emit_launch<256, kEmitW, false>)
+				: (shift ? emit_launch<512, kEmitW, true> : emit_launch<512, kEmitW, false>);
 		const int rc = launch(a, ns, levels, num_sms, st);
 		if (rc) return rc;
 	}

@@ -350,3 +350,29 @@ def test_rows_at_every_alignment(native, oracle, n, planes):
                 got = buf.cpu().numpy()
                 np.testing.assert_array_equal(got[offset:offset + k * n].reshape(k, n), exp)
                 assert (got[:offset] == 77).all() and (got[offset + k * n:] == 77).all()
+
+
+@pytest.mark.parametrize("levels", [7, 8, 14, 15, 29])
+@pytest.mark.parametrize("n", [1024, 4099])
+def test_planes_per_output_step(native, oracle, n, levels):
+    """The output pass takes 14 level planes a step, in two groups of seven: depths at
+    those edges, for words per vertex with and without masks, in both tile widths."""
+    import bfs_simd_benchmarks_gb300 as B
+    rng = np.random.default_rng(levels)
+    layer = np.arange(n) % levels
+    src = rng.integers(0, n, size=6 * n)
+    src = src[layer[src] < levels - 1]
+    dst = np.minimum(src // levels * levels + layer[src] + 1 + levels * rng.integers(-2, 3, size=len(src)), n - 1)
+    dst = np.where(dst < 0, layer[src] + 1, dst)
+    arr = oracle.csr_arrays(n, src.astype(np.uint32), dst.astype(np.uint32))
+    with B.Graph.from_edges(n, src.astype(np.uint32), dst.astype(np.uint32), 64, 4) as g:
+        for k in (60, 100, 250, 300, 1090, 4096):
+            sources = (rng.integers(0, n, size=k) // levels * levels).clip(0, n - 1).astype(np.uint32)
+            expect = {int(s): None for s in sources}
+            for s in expect:
+                lev = oracle.bfs_levels(arr, s)
+                expect[s] = np.where(lev < 0, 255, lev).astype(np.uint8)
+            exp = np.stack([expect[int(s)] for s in sources])
+            for tile in (0, 64) if k > 128 else (0,):
+                g.set_options(batch_single_max=0, batch_planes=36, batch_output_tile=tile)
+                _check(oracle, arr, g, sources, exp)
