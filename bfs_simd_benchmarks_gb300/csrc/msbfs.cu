@@ -22,11 +22,11 @@
 //     frontier has reached them (per-destination early exit).  Up to
 //     kMsRowWords words per vertex a lane (or 8 lanes) takes a destination and
 //     reads whole rows; with more, a warp takes one and reads the non-zero
-//     words it still lacks.  Destinations with many in-edges are cut into
+//     words it still lacks, in groups of 8, 16 or 32 lanes per row.  Destinations with many in-edges are cut into
 //     chunks that warps all over the grid gather and OR together; the last one
 //     finishes the destination, so that a pull level has one grid barrier.
 //     (R-MAT scale 22, 4096 sources: the level with the most gathers 7.8 ->
-//     6.1 ms; Pokec shape, 64 sources: 0.54 -> 0.26 ms.)
+//     4.8 ms; Pokec shape, 64 sources: 0.54 -> 0.26 ms.)
 // Clearing, seeding, all levels and the edge count run in one cooperative
 // launch, levels separated by a bounded-spin grid barrier; the output pass,
 // its own launch, turns planes into uint8 levels [source][vertex] (255 =
@@ -50,10 +50,11 @@ constexpr uint32_t kMsBig = 1024;       // push: higher-degree vertices are spre
 constexpr int kMsGather = 4;            // pull: frontier rows gathered per round
 constexpr int kMsFinishRows = 2;        // push: touched rows finished per round
 constexpr uint32_t kLaneMaxDeg = 32;    // pull, few words: destinations of at most this in-degree go one per lane
-constexpr uint32_t kGroupMaxWords = 8;  // pull: up to this many words, in-neighbour rows in lane groups
+constexpr uint32_t kMsMaxWords = 64;    // 4,096 sources
+constexpr uint32_t kGroupMaxWords = 16; // pull: up to this many words, in-neighbour rows in lane groups
 constexpr uint32_t kEmitW = 4;          // output tile: kV vertices x kW words (4: 256 sources), kV = threads / kW
-constexpr uint32_t kEmitPlanes = 7;  // planes that a 3-bit index tells apart, with one value left for "none of them"
-constexpr uint32_t kEmitUnits = 8;   // output tiles' words are split among CTAs below this many per CTA
+constexpr uint32_t kEmitPlanes = 7;     // planes that a 3-bit index tells apart, with one value left for "none of them"
+constexpr uint32_t kEmitUnits = 8;      // output tiles' words are split among CTAs below this many per CTA
 // Words of a tile's shared memory per word of its vertices: 16 source quads, each
 // a row of kV words with 4 more after every 16 (the second phase's 16-byte reads
 // of 16 vertices per lane then fall on different banks), and the shift that puts
@@ -325,16 +326,15 @@ struct FullMask {
 // the neighbour's row and still incomplete in the destination's are read.
 // Returns true when it stopped early.  Warp-uniform.
 __device__ __forceinline__ bool ms_gather(const MsArgs &a, const uint64_t *cur, const uint64_t *actc, uint32_t beg,
-		uint32_t end, const FullMask &fm, uint64_t vis0, uint64_t vis1, uint64_t &acc0, uint64_t &acc1,
+		uint32_t end, uint32_t u, uint64_t um, const FullMask &fm, uint64_t vis0, uint64_t vis1, uint64_t &acc0, uint64_t &acc1,
 		unsigned long long &gathered) {
 	const uint32_t K = a.K;
 	const unsigned lane = lane_id();
 	bool done = false;
 	uint32_t loads = 0;
 	for (uint32_t e0 = beg; e0 < end && !done; e0 += 32) {
-		const uint32_t e = e0 + lane;
-		const uint32_t u = e < end ? __ldg(a.in_src + e) : 0u;
-		const uint64_t um = e < end ? ld_cg64(actc + u) : 0ull;
+		if (e0 != beg) um = e0 + lane < end ? ld_cg64(actc + u) : 0ull;
+		const uint32_t en = e0 + 32 + lane, un = en < end ? __ldg(a.in_src + en) : 0u;
 		uint32_t lm = __ballot_sync(kFull, um != 0ull);
 		while (lm && !done) {
 			const bool need0 = ((acc0 | vis0) & fm.f0) != fm.f0;
@@ -360,6 +360,7 @@ __device__ __forceinline__ bool ms_gather(const MsArgs &a, const uint64_t *cur, 
 			for (int t = 0; t < kMsGather; ++t) { acc0 |= g0[t]; acc1 |= g1[t]; }
 			done = fm.complete(acc0 | vis0, acc1 | vis1);
 		}
+		u = un;
 	}
 	gathered += loads;
 	return done;
@@ -371,47 +372,48 @@ __device__ __forceinline__ uint64_t warp_or64(uint64_t x) {
 	return x;
 }
 
-// ms_gather for 2 < K <= 16 words per vertex: the warp is split into
-// 32 / kp groups of kp lanes (kp = K rounded up to a power of two); a group
-// reads one in-neighbour row (lane k its word k), so a round reads
-// kMsGather * 32 / kp rows; the groups' words are OR-ed together after every
-// round for the early exit.  `vis` and `f` are the lane's word k (the same in
-// every group); acc comes back in every group.
+// ms_gather for kMsRowWords < K <= kGroupMaxWords words per vertex: the warp is
+// split into groups of kLanes (8 or 16) lanes; of g groups, each takes every g-th
+// in-neighbour and reads its row (lane k its word k), so a round reads
+// g kMsGather rows; the groups' words are
+// OR-ed together after every round for the early exit.  `vis` and `f` are the
+// lane's word k (the same in every group); acc comes back in every group.
+// (Sharing the frontier's neighbours out evenly, by __fns, cost more than idle
+// groups: uniform, 2^18 vertices, 2^22 edges, 300 sources: 1.13 against 0.80 ms.
+// With a warp per row as above 16 words, rmat, 2^20 vertices, 2^24 edges, 1,024
+// sources: 3.81 against 2.63 ms.)
+template <uint32_t kLanes>
 __device__ __forceinline__ void ms_gather_grouped(const MsArgs &a, const uint64_t *cur, const uint64_t *actc,
-		uint32_t beg, uint32_t end, uint32_t kp, uint64_t f, uint64_t vis, uint64_t &acc, unsigned long long &gathered) {
+		uint32_t beg, uint32_t end, uint32_t u, uint64_t um, uint64_t f, uint64_t vis, uint64_t &acc,
+		unsigned long long &gathered) {
 	const uint32_t K = a.K;
 	const unsigned lane = lane_id();
-	const uint32_t k = lane & (kp - 1), grp = lane / kp, ngrp = 32 / kp;
-	const bool wk = k < K;
+	const uint32_t k = lane % kLanes;
 	uint32_t loads = 0;
 	bool done = __all_sync(kFull, ((vis | acc) & f) == f);
 	for (uint32_t e0 = beg; e0 < end && !done; e0 += 32) {
-		const uint32_t e = e0 + lane;
-		const uint32_t u = e < end ? __ldg(a.in_src + e) : 0u;
-		const uint64_t um = e < end ? ld_cg64(actc + u) : 0ull;
-		uint32_t lm = __ballot_sync(kFull, um != 0ull);
-		while (lm && !done) {
-			const bool need = ((vis | acc) & f) != f;
-			const uint32_t nlive = __popc(lm);
+		if (e0 != beg) um = e0 + lane < end ? ld_cg64(actc + u) : 0ull;
+		const uint32_t en = e0 + 32 + lane, un = en < end ? __ldg(a.in_src + en) : 0u;
+		uint32_t lm = __ballot_sync(kFull, um != 0ull) & ((kLanes == 8 ? 0x11111111u : 0x55555555u) << (lane / kLanes));
+		while (!done && __any_sync(kFull, lm)) {
+			const bool need = ((vis | acc) & f) != f;  // f is zero beyond the last word
 			uint64_t gv[kMsGather];
 #pragma unroll
 			for (int t = 0; t < kMsGather; ++t) {
-				const uint32_t idx = t * ngrp + grp;
-				const int src = idx < nlive ? (int) __fns(lm, 0, idx + 1) : 0;
-				const uint32_t ut = __shfl_sync(kFull, u, src);
-				const uint64_t mt = shfl64(um, src);
-				const bool ld = idx < nlive && need && wk && ((mt >> k) & 1ull);
+				const int src = __ffs(lm) - 1;
+				const uint32_t ut = __shfl_sync(kFull, u, src & 31);
+				const uint64_t mt = shfl64(um, src & 31);
+				const bool ld = lm && need && ((mt >> k) & 1ull);
 				gv[t] = ld ? ld_cg64(cur + (size_t) ut * K + k) : 0ull;
 				loads += ld;
+				lm &= lm - 1;
 			}
 #pragma unroll
 			for (int t = 0; t < kMsGather; ++t) acc |= gv[t];
-			for (uint32_t d = kp; d < 32; d <<= 1) acc |= shfl_xor64(acc, d);
-			const uint32_t took = min(nlive, (uint32_t) kMsGather * ngrp);
-			if (took == nlive) lm = 0;
-			else lm &= ~((1u << __fns(lm, 0, took + 1)) - 1u);
+			for (uint32_t d = kLanes; d < 32; d <<= 1) acc |= shfl_xor64(acc, d);
 			done = __all_sync(kFull, ((vis | acc) & f) == f);
 		}
+		u = un;
 	}
 	gathered += loads;
 }
@@ -588,6 +590,7 @@ __device__ __forceinline__ uint64_t ms_chunk_rows(const MsArgs &a, const uint64_
 // A warp screens 32 consecutive destinations at once (their in-edge ranges and
 // "every source has arrived" flags, lane-parallel), then works through those
 // with something to do one at a time: lane l owns words l and l + 32.
+template <int KK>
 __device__ __forceinline__ void ms_pull_words(const MsArgs &a, const MsPull &p, uint32_t vb, const FullMask &fm,
 		uint64_t &new0, uint64_t &new1, unsigned long long &actdeg, unsigned long long &gathered, uint32_t *wbuf,
 		uint32_t &wn) {
@@ -609,21 +612,34 @@ __device__ __forceinline__ void ms_pull_words(const MsArgs &a, const MsPull &p, 
 		for (uint32_t x = lane; x < nb * K; x += 32)
 			if (!(((needm | bigm) >> (x / K)) & 1u)) blk[x] = 0ull;
 	}
+	// a destination's first 32 in-neighbours are read, and its visited row is sent
+	// for, while the one before it gathers (2^22 vertices, 4,096 sources: 24.6 -> 24.0 ms)
+	const auto first_neighbours = [&](uint32_t m) {
+		const int jj = __ffs(m) - 1;
+		const uint32_t e = __shfl_sync(kFull, lbeg, jj) + lane;
+		const uint64_t *r = a.vis + (size_t) (vb + jj) * K + 16 * lane;  // a line per lane
+		if (16 * lane < K) asm volatile("prefetch.global.L2 [%0];" :: "l"(r));
+		return e < __shfl_sync(kFull, lend, jj) ? __ldg(a.in_src + e) : 0u;
+	};
+	uint32_t un = needm ? first_neighbours(needm) : 0u;
 	for (uint32_t m = needm; m; m &= m - 1) {
 		const int jj = __ffs(m) - 1;
 		const uint32_t v = vb + jj;
 		const uint32_t beg = __shfl_sync(kFull, lbeg, jj), end = __shfl_sync(kFull, lend, jj);
 		const size_t row = (size_t) v * K;
+		const uint32_t u = un;
+		const uint64_t um = beg + lane < end ? ld_cg64(p.actc + u) : 0ull;
 		const uint64_t vis0 = w0 ? ld_cg64(a.vis + row + lane) : 0ull;
 		const uint64_t vis1 = w1 ? ld_cg64(a.vis + row + lane + 32) : 0ull;
+		if (m & (m - 1)) un = first_neighbours(m & (m - 1));
 		uint64_t acc0 = 0, acc1 = 0;
-		if (K <= kGroupMaxWords) {
-			const uint32_t kw = lane & 7u;
+		if constexpr (KK <= (int) kGroupMaxWords) {
+			const uint32_t kw = lane % KK;
 			uint64_t ag = 0;
-			ms_gather_grouped(a, p.cur, p.actc, beg, end, 8, shfl64(fm.f0, kw), shfl64(vis0, kw), ag, gathered);
-			acc0 = lane < 8 ? ag : 0ull;
+			ms_gather_grouped<KK>(a, p.cur, p.actc, beg, end, u, um, shfl64(fm.f0, kw), shfl64(vis0, kw), ag, gathered);
+			acc0 = lane < KK ? ag : 0ull;
 		} else if (!fm.complete(vis0, vis1)) {
-			ms_gather(a, p.cur, p.actc, beg, end, fm, vis0, vis1, acc0, acc1, gathered);
+			ms_gather(a, p.cur, p.actc, beg, end, u, um, fm, vis0, vis1, acc0, acc1, gathered);
 		}
 		const uint64_t n0 = acc0 & ~vis0 & fm.f0, n1 = acc1 & ~vis1 & fm.f1;
 		new0 |= n0;
@@ -657,6 +673,7 @@ __device__ __forceinline__ void ms_pull_words(const MsArgs &a, const MsPull &p, 
 // words it gathers are OR-ed into the destination's row of big_acc; the warp
 // that completes the destination's last chunk writes its row, mask and queue
 // entry and leaves its row of big_acc and its count at 0.
+template <int KK>
 __device__ __forceinline__ void ms_pull_chunk(const MsArgs &a, const MsPull &p, uint32_t c, const FullMask &fm,
 		uint64_t &new0, uint64_t &new1, unsigned long long &actdeg, unsigned long long &gathered) {
 	const uint32_t K = a.K;
@@ -666,25 +683,26 @@ __device__ __forceinline__ void ms_pull_chunk(const MsArgs &a, const MsPull &p, 
 	const uint32_t vbeg = __ldg(a.in_off + v), vend = __ldg(a.in_off + v + 1);
 	const uint32_t end = min(beg + kMsChunk, vend);
 	const size_t row = (size_t) v * K;
+	uint32_t u = 0;
+	uint64_t um = 0;
+	if (KK > (int) kMsRowWords && beg + lane < end) {
+		u = __ldg(a.in_src + beg + lane);
+		um = ld_cg64(p.actc + u);
+	}
 	const uint64_t vis0 = w0 ? ld_cg64(a.vis + row + lane) : 0ull;
 	const uint64_t vis1 = w1 ? ld_cg64(a.vis + row + lane + 32) : 0ull;
 	uint64_t *bacc = a.big_acc + (size_t) slot * K;
 	if (!fm.complete(vis0, vis1)) {
 		uint64_t acc0 = 0, acc1 = 0;
-		switch (K) {
-		case 1: acc0 = ms_chunk_rows<1>(a, p.cur, beg, end, gathered); break;
-		case 2: acc0 = ms_chunk_rows<2>(a, p.cur, beg, end, gathered); break;
-		case 3: acc0 = ms_chunk_rows<3>(a, p.cur, beg, end, gathered); break;
-		case 4: acc0 = ms_chunk_rows<4>(a, p.cur, beg, end, gathered); break;
-		default:
-			if (K <= kGroupMaxWords) {
-				const uint32_t kw = lane & 7u;
-				uint64_t ag = 0;
-				ms_gather_grouped(a, p.cur, p.actc, beg, end, 8, shfl64(fm.f0, kw), shfl64(vis0, kw), ag, gathered);
-				acc0 = lane < 8 ? ag : 0ull;
-			} else {
-				ms_gather(a, p.cur, p.actc, beg, end, fm, vis0, vis1, acc0, acc1, gathered);
-			}
+		if constexpr (KK <= (int) kMsRowWords) {
+			acc0 = ms_chunk_rows<KK>(a, p.cur, beg, end, gathered);
+		} else if constexpr (KK <= (int) kGroupMaxWords) {
+			const uint32_t kw = lane % KK;
+			uint64_t ag = 0;
+			ms_gather_grouped<KK>(a, p.cur, p.actc, beg, end, u, um, shfl64(fm.f0, kw), shfl64(vis0, kw), ag, gathered);
+			acc0 = lane < KK ? ag : 0ull;
+		} else {
+			ms_gather(a, p.cur, p.actc, beg, end, u, um, fm, vis0, vis1, acc0, acc1, gathered);
 		}
 		const uint64_t n0 = acc0 & ~vis0 & fm.f0, n1 = acc1 & ~vis1 & fm.f1;
 		if (n0) atomicOr((unsigned long long *) (bacc + lane), (unsigned long long) n0);
@@ -723,13 +741,14 @@ __device__ __forceinline__ void ms_pull_chunk(const MsArgs &a, const MsPull &p, 
 }
 
 // The chunks from `item` on; returns the first item after them that this warp got.
-__device__ __noinline__ uint32_t ms_pull_chunks(const MsArgs &a, const MsPull &p, uint32_t item, unsigned *counter,
+template <int KK>
+__device__ __forceinline__ uint32_t ms_pull_chunks(const MsArgs &a, const MsPull &p, uint32_t item, unsigned *counter,
 		const FullMask &fm, unsigned long long &actdeg, unsigned long long &gathered, unsigned long long *s_act) {
 	const unsigned lane = lane_id();
 	uint64_t new0 = 0, new1 = 0;
 	while (item < a.nchunks) {
 		const uint32_t next = lane == 0 ? atomicAdd(counter, 1u) : 0u;
-		ms_pull_chunk(a, p, item, fm, new0, new1, actdeg, gathered);
+		ms_pull_chunk<KK>(a, p, item, fm, new0, new1, actdeg, gathered);
 		item = __shfl_sync(kFull, next, 0);
 	}
 	if (new0) atomicOr(s_act + lane, (unsigned long long) new0);
@@ -737,30 +756,30 @@ __device__ __noinline__ uint32_t ms_pull_chunks(const MsArgs &a, const MsPull &p
 	return item;
 }
 
-// The blocks of 32 destinations from `item` on, for KK words per vertex (0:
-// more than kMsRowWords).
+// The blocks of 32 destinations from `item` on.
 template <int KK>
-__device__ __noinline__ void ms_pull_blocks(const MsArgs &a, const MsPull &p, uint32_t item, unsigned *counter,
+__device__ __forceinline__ void ms_pull_blocks(const MsArgs &a, const MsPull &p, uint32_t item, unsigned *counter,
 		const FullMask &fm, unsigned long long &actdeg, unsigned long long &gathered, uint32_t *wbuf,
 		unsigned long long *s_act) {
 	const unsigned lane = lane_id();
 	const uint32_t nblk = (a.n + 31) / 32;
-	constexpr int kN = KK ? KK : 2;
+	constexpr bool kRowWords = KK <= (int) kMsRowWords;
+	constexpr int kN = kRowWords ? KK : 2;
 	uint64_t f[kN], acc[kN];
 #pragma unroll
 	for (int k = 0; k < kN; ++k) {
-		f[k] = KK ? shfl64(fm.f0, k) : 0ull;
+		f[k] = kRowWords ? shfl64(fm.f0, k) : 0ull;
 		acc[k] = 0ull;
 	}
 	uint32_t wn = 0;
 	while (item < a.nchunks + nblk) {
 		const uint32_t next = lane == 0 ? atomicAdd(counter, 1u) : 0u;
 		const uint32_t vb = (item - a.nchunks) * 32;
-		if constexpr (KK != 0) ms_pull_rows<KK>(a, p, vb, f, acc, actdeg, gathered);
-		else ms_pull_words(a, p, vb, fm, acc[0], acc[1], actdeg, gathered, wbuf, wn);
+		if constexpr (kRowWords) ms_pull_rows<KK>(a, p, vb, f, acc, actdeg, gathered);
+		else ms_pull_words<KK>(a, p, vb, fm, acc[0], acc[1], actdeg, gathered, wbuf, wn);
 		item = __shfl_sync(kFull, next, 0);
 	}
-	if constexpr (KK != 0) {
+	if constexpr (kRowWords) {
 #pragma unroll
 		for (int k = 0; k < KK; ++k) {
 			const uint64_t x = warp_or64(acc[k]);
@@ -776,6 +795,7 @@ __device__ __noinline__ void ms_pull_blocks(const MsArgs &a, const MsPull &p, ui
 // A pull level: the chunks of the many-in-edge destinations, then the blocks of
 // 32 destinations, handed to the warps one at a time through a counter (the
 // next one claimed while one runs), so that no barrier is needed between them.
+template <int KK>
 __device__ __forceinline__ void ms_pull(const MsArgs &a, const MsPull &p, unsigned *counter, unsigned long long &actdeg_out,
 		unsigned long long &gathered_out, uint32_t *wq_base, unsigned long long *s_act) {
 	const unsigned lane = lane_id();
@@ -783,16 +803,9 @@ __device__ __forceinline__ void ms_pull(const MsArgs &a, const MsPull &p, unsign
 	unsigned long long actdeg = 0, gathered = 0;
 	uint32_t item = lane == 0 ? atomicAdd(counter, 1u) : 0u;
 	item = __shfl_sync(kFull, item, 0);
-	if (item < a.nchunks) item = ms_pull_chunks(a, p, item, counter, fm, actdeg, gathered, s_act);
+	if (item < a.nchunks) item = ms_pull_chunks<KK>(a, p, item, counter, fm, actdeg, gathered, s_act);
 	uint32_t *wbuf = wq_base + warp_id() * kMsWq;
-	switch (a.K) {
-	case 1: ms_pull_blocks<1>(a, p, item, counter, fm, actdeg, gathered, wbuf, s_act); break;
-	case 2: ms_pull_blocks<2>(a, p, item, counter, fm, actdeg, gathered, wbuf, s_act); break;
-	case 3: ms_pull_blocks<3>(a, p, item, counter, fm, actdeg, gathered, wbuf, s_act); break;
-	case 4: ms_pull_blocks<4>(a, p, item, counter, fm, actdeg, gathered, wbuf, s_act); break;
-	default: ms_pull_blocks<0>(a, p, item, counter, fm, actdeg, gathered, wbuf, s_act); break;
-	}
-	static_assert(kMsRowWords == 4, "a case for each");
+	ms_pull_blocks<KK>(a, p, item, counter, fm, actdeg, gathered, wbuf, s_act);
 	actdeg_out += actdeg;
 	gathered_out += gathered;
 }
@@ -1128,6 +1141,12 @@ __device__ __noinline__ void ms_emit(const MsArgs &a, uint8_t *levels, uint32_t 
 	}
 }
 
+// KK: words per vertex up to kMsRowWords; for more, 8, 16 (kGroupMaxWords) or 64
+// (kMsMaxWords) for up to as many: one kernel each, so that only one form of the pull shares
+// the registers and its arguments are read where they lie (as calls of one
+// kernel, with arguments by reference, the pulls' accesses to local memory were
+// a third of their L1 traffic: 2^22 vertices, 4,096 sources, 28.6 against 24.6 ms).
+template <int KK>
 __global__ void __launch_bounds__(kMsThreads, 2) k_ms_bfs(const __grid_constant__ MsArgs a, const uint32_t *sources, uint32_t ns,
 		uint8_t *levels) {
 	__shared__ unsigned long long red[kMsWarps];
@@ -1241,7 +1260,7 @@ __global__ void __launch_bounds__(kMsThreads, 2) k_ms_bfs(const __grid_constant_
 		} else {
 			const MsPull p{cur, actc, nxt, actn, act, &ctl->ctr[(lvl + 1) % 3], a.queue[(lvl + 1) & 1],
 					masked};
-			ms_pull(a, p, &ctl->work[lvl], actdeg, gathered, wq, s_act);
+			ms_pull<KK>(a, p, &ctl->work[lvl], actdeg, gathered, wq, s_act);
 		}
 		// the next frontier's out-degree: per-CTA sum, one atomic per CTA
 		const unsigned long long d = warp_sum(actdeg);
@@ -1348,8 +1367,11 @@ int ms_chunk_slots(const uint32_t *chunk_v, uint32_t nchunks, const uint32_t *in
 
 int ms_launch(const MsArgs &a, const uint32_t *d_sources, uint32_t ns, uint8_t *levels, int num_sms, cudaStream_t st,
 		int *grid, cudaEvent_t between, cudaEvent_t between2) {
+	static_assert(kMsRowWords == 4, "a kernel for each");
+	const auto fn = a.K == 1 ? k_ms_bfs<1> : a.K == 2 ? k_ms_bfs<2> : a.K == 3 ? k_ms_bfs<3> : a.K == 4 ? k_ms_bfs<4>
+			: a.K <= 8 ? k_ms_bfs<8> : a.K <= kGroupMaxWords ? k_ms_bfs<kGroupMaxWords> : k_ms_bfs<kMsMaxWords>;
 	int per_sm = 0;
-	if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_ms_bfs, kMsThreads, 0) != cudaSuccess || per_sm < 1)
+	if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, fn, kMsThreads, 0) != cudaSuccess || per_sm < 1)
 		return BFS_ECUDA;
 	per_sm = std::min(per_sm, 2);
 	if (a.ctas_per_sm) per_sm = std::min(per_sm, (int) a.ctas_per_sm);
@@ -1360,7 +1382,7 @@ int ms_launch(const MsArgs &a, const uint32_t *d_sources, uint32_t ns, uint8_t *
 	uint32_t nsrc = ns;
 	uint8_t *out = levels;
 	void *args[] = {&aa, (void *) &src, &nsrc, &out};
-	if (cudaLaunchCooperativeKernel((const void *) k_ms_bfs, dim3(num_sms * per_sm), dim3(kMsThreads), args, 0, st) !=
+	if (cudaLaunchCooperativeKernel((const void *) fn, dim3(num_sms * per_sm), dim3(kMsThreads), args, 0, st) !=
 			cudaSuccess)
 		return BFS_ECUDA;
 	if (between && cudaEventRecord(between, st) != cudaSuccess) return BFS_ECUDA;

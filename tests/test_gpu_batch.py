@@ -300,7 +300,7 @@ def test_output_tile_widths_give_the_same_levels(native, oracle, num_sources):
             g.set_options(batch_output_tile=96)
 
 
-@pytest.mark.parametrize("words", [1, 2, 3, 4, 5, 8, 9, 33, 64])
+@pytest.mark.parametrize("words", [1, 2, 3, 4, 5, 8, 9, 12, 16, 17, 33, 64])
 @pytest.mark.parametrize("push_div", [1, 1 << 30])
 def test_words_per_vertex_and_degrees(native, oracle, words, push_div):
     """Every shape of the pull (and of the push) by words per vertex, on a graph whose
