@@ -53,7 +53,11 @@ namespace {
 constexpr int kBbThreads = 512;
 constexpr int kBbWarps = kBbThreads / 32;
 constexpr int kBbUnroll = 4;   // chunk partial rows added per round (finish)
-constexpr int kBbPairs = 2;    // pairs of served edges per round (their rows loaded together)
+// Pairs of served edges per round (their rows loaded together).  3 with the next
+// step's neighbours read ahead: Pokec shape, 64 sources, 6.62 -> 6.25 ms, uniform
+// 2^20 vertices 6.12 -> 5.86 (2 pairs: 6.40 and 6.08; 4, which spill: 6.71 and
+// 7.03; the neighbours' words read ahead as well: 6.40 and 6.65).
+constexpr int kBbPairs = 3;
 constexpr uint32_t kBbOutV = 64;   // output pass: vertices per tile
 constexpr int kBbOutThreads = 256;
 
@@ -279,23 +283,32 @@ __device__ void bb_block(const BbArgs &a, uint32_t L, uint32_t w, bool has_nb, u
 	uint64_t hcur = 0;
 	BbOpen<kFwd> op;
 	uint32_t flushed = 0;
-	for (uint32_t e0 = 0; e0 < total; e0 += 32) {
-		const uint32_t e = e0 + lane;
-		// the edge's vertex slot: the first lane whose inclusive prefix exceeds e
+	// an edge's vertex slot: the first lane whose inclusive prefix exceeds e
+	const auto slot_of = [&](uint32_t e) {
 		uint32_t o = 0;
 #pragma unroll
 		for (uint32_t s = 16; s; s >>= 1) {
 			const uint32_t x = __shfl_sync(kFull, incl, o + s - 1);
 			if (x <= e) o += s;
 		}
+		return o;
+	};
+	const auto neighbour = [&](uint32_t e, uint32_t o) {
 		const uint32_t obeg = __shfl_sync(kFull, beg, o), oex = __shfl_sync(kFull, excl, o);
-		const uint64_t ohv = bb_shfl64(hv, o);
-		uint32_t u = 0;
-		uint64_t m = 0;
-		if (e < total) {
-			u = __ldg(adj + obeg + (e - oex));
-			m = ohv & bb_word(nb, a, u);
-			u += rw;
+		return e < total ? __ldg(adj + obeg + (e - oex)) : 0u;
+	};
+	uint32_t o2 = 0, u2 = 0;
+	if (total) {
+		o2 = slot_of(lane);
+		u2 = neighbour(lane, o2);
+	}
+	for (uint32_t e0 = 0; e0 < total; e0 += 32) {
+		const uint32_t e = e0 + lane, o = o2, u = u2 + rw;
+		uint64_t m = bb_shfl64(hv, o);
+		m = e < total ? m & bb_word(nb, a, u2) : 0ull;
+		if (e0 + 32 < total) {
+			o2 = slot_of(e + 32);
+			u2 = neighbour(e + 32, o2);
 		}
 		uint32_t bal = __ballot_sync(kFull, m != 0ull);
 		if (lane == 0) {
@@ -406,15 +419,11 @@ __device__ void bb_chunk(const BbArgs &a, uint32_t L, uint32_t w, bool has_nb, u
 	const uint32_t beg = __ldg(cb + c), vbeg = __ldg(off + v), vend = __ldg(off + v + 1);
 	const uint32_t end = min(beg + a.chunk, vend);
 	T acc[4] = {T(0), T(0), T(0), T(0)};
+	uint32_t u2 = has_nb && beg + lane < end ? __ldg(adj + beg + lane) : 0u;
 	for (uint32_t e0 = beg; has_nb && e0 < end; e0 += 32) {
-		const uint32_t e = e0 + lane;
-		uint32_t u = 0;
-		uint64_t m = 0;
-		if (e < end) {
-			u = __ldg(adj + e);
-			m = hv & bb_word(nb, a, u);
-			u += rw;
-		}
+		const uint32_t e = e0 + lane, u = u2 + rw;
+		const uint64_t m = e < end ? hv & bb_word(nb, a, u2) : 0ull;
+		u2 = e + 32 < end ? __ldg(adj + e + 32) : 0u;
 		uint32_t bal = __ballot_sync(kFull, m != 0ull);
 		if (lane == 0) {
 			cnt.edges += min(32u, end - e0);
