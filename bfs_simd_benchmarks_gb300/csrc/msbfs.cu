@@ -45,11 +45,28 @@ namespace bfsg {
 
 constexpr int kMsThreads = 512;
 constexpr int kMsWarps = kMsThreads / 32;
-constexpr uint32_t kMsWq = 64;          // per-warp staged queue appends (pull)
+constexpr uint32_t kMsWq = 512;         // per-warp staged queue appends (pull)
+// push: edges per lane and round trip (2^14 vertices, whose first frontier has a
+// vertex of almost kMsBig edges: that level 38 -> 24 us)
+constexpr int kMsPushEdges = 4;
 constexpr uint32_t kMsBig = 1024;       // push: higher-degree vertices are spread over the grid
 constexpr int kMsGather = 4;            // pull: frontier rows gathered per round
 constexpr int kMsFinishRows = 2;        // push: touched rows finished per round
 constexpr uint32_t kLaneMaxDeg = 32;    // pull, few words: destinations of at most this in-degree go one per lane
+// Pull with more than kMsRowWords words: a block of 32 destinations is halved
+// down to 4 while there are fewer than kMsBlocks per warp, and further while
+// there are not blocks for half of the warps: a warp takes a block's destinations
+// one after another (rmat, 16 edges a vertex: 2^12 vertices, 1,000 sources 549 ->
+// 214 us; 2^14 546 -> 275; 2^16 543 -> 377; 2^18 1,142 -> 903).
+constexpr uint32_t kMsBlocks = 4;
+// Up to kMsRowWords words and this many words of state, one CTA per SM: a level
+// is then a few chains of round trips and a grid barrier, which costs less among
+// fewer CTAs (rmat, 16 edges a vertex, 60 sources: 2^14 vertices 177 -> 157 us,
+// 2^16 162 -> 147, 2^17 206 -> 194; 2^18 264 -> 268).
+// Up to kMsTinyState, a CTA on every other SM (2^14 vertices 155 -> 147 us, uniform
+// 126 -> 115; 2^16 150 -> 163).
+constexpr uint32_t kMsSmallState = 1u << 18, kMsTinyState = 1u << 15;
+constexpr uint32_t kMsRun = 8;          // pull, few words: chunks taken at once
 constexpr uint32_t kMsMaxWords = 64;    // 4,096 sources
 constexpr uint32_t kGroupMaxWords = 16; // pull: up to this many words, in-neighbour rows in lane groups
 constexpr uint32_t kEmitW = 4;          // output tile: kV vertices x kW words (4: 256 sources), kV = threads / kW
@@ -108,29 +125,41 @@ __device__ __forceinline__ void ms_append(const MsArgs &a, MsCounters *cn, uint3
 // Push: ORs u's non-zero frontier words into the next words of its out-edges
 // [beg + first, end), taking 32 edges per warp step of `step`.  Warp-uniform.
 __device__ __forceinline__ void ms_push_edges(const MsArgs &a, const uint64_t *cur, const uint64_t *actc,
-		uint64_t *nxt, uint32_t u, uint32_t beg, uint32_t end, uint32_t first, uint32_t step) {
+		uint64_t *nxt, uint32_t u, uint32_t beg, uint32_t end) {
 	const uint32_t K = a.K;
 	const unsigned lane = lane_id();
 	const uint64_t um = ld_cg64(actc + u);  // which of u's words are non-zero
 	const uint32_t nz0 = (uint32_t) um, nz1 = (uint32_t) (um >> 32);
 	const uint64_t w0 = (nz0 >> lane) & 1u ? ld_cg64(cur + (size_t) u * K + lane) : 0ull;
 	const uint64_t w1 = (nz1 >> lane) & 1u ? ld_cg64(cur + (size_t) u * K + lane + 32) : 0ull;
-	for (uint32_t e0 = beg + first; e0 < end; e0 += step) {
-		const uint32_t e = e0 + lane;
-		const bool ok = e < end;
-		const uint32_t v = ok ? __ldg(a.col + e) : 0u;
-		unsigned long long *dst = (unsigned long long *) (nxt + (size_t) v * K);
+	for (uint32_t e0 = beg; e0 < end; e0 += 32 * kMsPushEdges) {
+		uint32_t v[kMsPushEdges];
+		bool ok[kMsPushEdges], fresh[kMsPushEdges];
+#pragma unroll
+		for (int j = 0; j < kMsPushEdges; ++j) {
+			const uint32_t e = e0 + 32 * j + lane;
+			ok[j] = e < end;
+			v[j] = ok[j] ? __ldg(a.col + e) : 0u;
+		}
+#pragma unroll
+		for (int j = 0; j < kMsPushEdges; ++j) fresh[j] = ok[j] && !ld_cg_u8(a.touched + v[j]);
 		for (uint32_t m = nz0; m; m &= m - 1) {
 			const int k = __ffs(m) - 1;
 			const uint64_t w = shfl64(w0, k);
-			if (ok) atomicOr(dst + k, (unsigned long long) w);
+#pragma unroll
+			for (int j = 0; j < kMsPushEdges; ++j)
+				if (ok[j]) atomicOr((unsigned long long *) (nxt + (size_t) v[j] * K + k), (unsigned long long) w);
 		}
 		for (uint32_t m = nz1; m; m &= m - 1) {
 			const int k = __ffs(m) - 1;
 			const uint64_t w = shfl64(w1, k);
-			if (ok) atomicOr(dst + 32 + k, (unsigned long long) w);
+#pragma unroll
+			for (int j = 0; j < kMsPushEdges; ++j)
+				if (ok[j]) atomicOr((unsigned long long *) (nxt + (size_t) v[j] * K + k + 32), (unsigned long long) w);
 		}
-		if (ok && !ld_cg_u8(a.touched + v)) a.touched[v] = 1;
+#pragma unroll
+		for (int j = 0; j < kMsPushEdges; ++j)
+			if (fresh[j]) a.touched[v[j]] = 1;
 	}
 }
 
@@ -211,14 +240,14 @@ __device__ void ms_push(const MsArgs &a, uint32_t lvl, const uint64_t *cur, cons
 	const uint32_t nwarps = gridDim.x * kMsWarps;
 	for (uint32_t i = gwarp; i < nq; i += nwarps) {
 		const uint32_t u = ld_cg(q + i);
-		ms_push_edges(a, cur, actc, nxt, u, __ldg(a.row_off + u), __ldg(a.row_off + u + 1), 0, 32);
+		ms_push_edges(a, cur, actc, nxt, u, __ldg(a.row_off + u), __ldg(a.row_off + u + 1));
 	}
 	if (!nb) return;
 	const uint32_t nc = ld_volatile(&a.ctl->push_chunks);
 	for (uint32_t c = gwarp; c < nc; c += nwarps) {
 		const uint32_t u = ld_cg(a.push_u + c), beg = ld_cg(a.push_beg + c);
 		const uint32_t end = min(beg + kMsPushChunk, __ldg(a.row_off + u + 1));
-		ms_push_edges(a, cur, actc, nxt, u, beg, end, 0, 32);
+		ms_push_edges(a, cur, actc, nxt, u, beg, end);
 	}
 }
 
@@ -486,12 +515,12 @@ __device__ __forceinline__ bool row_complete(const uint64_t (&x)[KK], const uint
 // at a time, 32 edges of each per round; a list's walk stops when every source
 // that has a frontier has arrived.  All lanes then write their own destination.
 template <int KK>
-__device__ __forceinline__ void ms_pull_rows(const MsArgs &a, const MsPull &p, uint32_t vb, const uint64_t (&f)[KK],
-		uint64_t (&newacc)[KK], unsigned long long &actdeg, unsigned long long &gathered) {
+__device__ __forceinline__ void ms_pull_rows(const MsArgs &a, const MsPull &p, uint32_t vb, uint32_t nv, const uint64_t (&f)[KK],
+		uint64_t (&newacc)[KK], unsigned long long &actdeg, unsigned long long &gathered, uint32_t *wbuf, uint32_t &wn) {
 	constexpr int kRows = KK == 1 ? 8 : 4;
 	const unsigned lane = lane_id();
 	const uint32_t v = vb + lane;
-	const bool valid = v < a.n;
+	const bool valid = lane < nv;
 	const uint32_t beg = valid ? __ldg(a.in_off + v) : 0u, end = valid ? __ldg(a.in_off + v + 1) : 0u;
 	const bool small = valid && end - beg <= kMsPullBig;
 	const bool needy = small && end > beg && !ld_cg_u8(a.done + v);
@@ -560,30 +589,91 @@ __device__ __forceinline__ void ms_pull_rows(const MsArgs &a, const MsPull &p, u
 	}
 	const uint32_t d = mask ? deg_of(a, v) : 0u;
 	actdeg += d;
-	ms_append(a, p.cn, p.qn, v, mask && d <= kMsBig, mask && d > kMsBig);
+	const uint32_t ms = __ballot_sync(kFull, mask && d <= kMsBig);
+	if (wn + __popc(ms) > kMsWq) ms_wq_flush(p.cn, p.qn, wbuf, wn);
+	if ((ms >> lane) & 1u) wbuf[wn + __popc(ms & lanemask_lt())] = v;
+	wn += __popc(ms);
+	if (mask && d > kMsBig) p.qn[a.n - 1 - atomicAdd(&p.cn->nbig, 1u)] = v;
 }
 
-// A chunk's frontier words for KK words per vertex: OR over its in-edges, in
-// every lane's acc.
+// Chunks c0 .. c0 + cnt - 1 (at most 32 of them) of the destinations with more
+// than kMsPullBig in-edges: lane t holds chunk c0 + t's facts; neighbouring
+// chunks of one destination are read as one list and counted together, so that
+// a destination costs one release of its words and not one per chunk (Pokec
+// shape, 64 sources: 1.07 -> 0.88 ms; 11% of the warps' time was waiting for them).
 template <int KK>
-__device__ __forceinline__ uint64_t ms_chunk_rows(const MsArgs &a, const uint64_t *cur, uint32_t beg, uint32_t end,
-		unsigned long long &gathered) {
+__device__ __forceinline__ void ms_pull_runs(const MsArgs &a, const MsPull &p, uint32_t c0, uint32_t cnt, const uint64_t (&f)[KK],
+		uint64_t (&newacc)[KK], unsigned long long &actdeg, unsigned long long &gathered) {
 	constexpr int kRows = KK == 1 ? 8 : 4;
 	const unsigned lane = lane_id();
-	uint64_t acc[KK];
-#pragma unroll
-	for (int k = 0; k < KK; ++k) acc[k] = 0ull;
+	const uint32_t c = c0 + min(lane, cnt - 1);
+	const uint32_t v = __ldg(a.chunk_v + c), beg = __ldg(a.chunk_beg + c), slot = __ldg(a.chunk_slot + c);
+	const uint32_t vbeg = __ldg(a.in_off + v), vend = __ldg(a.in_off + v + 1);
+	uint64_t vis[KK];
+	row_ld<KK>(a.vis + (size_t) v * KK, vis);
+	const uint32_t openm = __ballot_sync(kFull, !row_complete(vis, vis, f));
 	uint32_t read = 0;
-	for (uint32_t e = beg + lane; e < end; e += 32 * kRows) read += rows_or<KK, kRows>(a, cur, e, 32, end, acc);
-	__syncwarp();
-	gathered += read;
-	uint64_t mine = 0;
+	for (uint32_t t = 0; t < cnt;) {
+		const uint32_t rv = __shfl_sync(kFull, v, t), rend = __shfl_sync(kFull, vend, t), rslot = __shfl_sync(kFull, slot, t);
+		const uint32_t len = __popc(__ballot_sync(kFull, lane < cnt && v == rv));
+		uint64_t acc[KK], have[KK];
 #pragma unroll
-	for (int k = 0; k < KK; ++k) {
-		const uint64_t x = warp_or64(acc[k]);
-		if (lane == (unsigned) k) mine = x;
+		for (int k = 0; k < KK; ++k) {
+			acc[k] = 0ull;
+			have[k] = shfl64(vis[k], t);
+		}
+		uint64_t *bacc = a.big_acc + (size_t) rslot * KK;
+		if ((openm >> t) & 1u) {
+			uint32_t e = __shfl_sync(kFull, beg, t);
+			const uint32_t end = min(e + len * kMsChunk, rend);
+			for (bool go = true; go && e < end; e += 32 * kRows) {
+				read += rows_or<KK, kRows>(a, p.cur, e + lane, 32, end, acc);
+				__syncwarp();
+#pragma unroll
+				for (int k = 0; k < KK; ++k) acc[k] = warp_or64(acc[k]);
+				go = !row_complete(have, acc, f);
+			}
+#pragma unroll
+			for (int k = 0; k < KK; ++k) {
+				const uint64_t n = acc[k] & ~have[k] & f[k];
+				if (lane == (unsigned) k && n) atomicOr((unsigned long long *) (bacc + k), (unsigned long long) n);
+			}
+		}
+		__syncwarp();
+		uint32_t before = 0;
+		// releases this warp's words to, and acquires the other warps' from, those that count here
+		if (lane == 0)
+			asm volatile("atom.acq_rel.gpu.global.add.u32 %0, [%1], %2;" : "=r"(before) : "l"(a.big_cnt + rslot), "r"(len) : "memory");
+		before = __shfl_sync(kFull, before, 0);
+		if (before + len == (rend - __shfl_sync(kFull, vbeg, t) + kMsChunk - 1) / kMsChunk) {
+			// every chunk is in: lane 0 finishes the destination
+			if (lane == 0) {
+				uint64_t mask = 0;
+#pragma unroll
+				for (int k = 0; k < KK; ++k) {
+					const uint64_t n = ld_cg64(bacc + k);
+					if (n) {
+						bacc[k] = 0ull;
+						a.vis[(size_t) rv * KK + k] = have[k] | n;
+						newacc[k] |= n;
+						mask |= 1ull << k;
+					}
+					p.nxt[(size_t) rv * KK + k] = n;
+				}
+				a.big_cnt[rslot] = 0u;
+				p.actn[rv] = mask;
+				if (mask) {
+					const uint32_t d = deg_of(a, rv);
+					actdeg += d;
+					if (d > kMsBig) p.qn[a.n - 1 - atomicAdd(&p.cn->nbig, 1u)] = rv;
+					else p.qn[atomicAdd(&p.cn->nact, 1u)] = rv;
+				}
+			}
+			__syncwarp();
+		}
+		t += len;
 	}
-	return mine;
+	gathered += read;
 }
 
 // ---- pull with more words per vertex --------------------------------------
@@ -591,14 +681,14 @@ __device__ __forceinline__ uint64_t ms_chunk_rows(const MsArgs &a, const uint64_
 // "every source has arrived" flags, lane-parallel), then works through those
 // with something to do one at a time: lane l owns words l and l + 32.
 template <int KK>
-__device__ __forceinline__ void ms_pull_words(const MsArgs &a, const MsPull &p, uint32_t vb, const FullMask &fm,
+__device__ __forceinline__ void ms_pull_words(const MsArgs &a, const MsPull &p, uint32_t vb, uint32_t nv, const FullMask &fm,
 		uint64_t &new0, uint64_t &new1, unsigned long long &actdeg, unsigned long long &gathered, uint32_t *wbuf,
 		uint32_t &wn) {
 	const uint32_t K = a.K;
 	const unsigned lane = lane_id();
 	const bool w0 = lane < K, w1 = lane + 32 < K;
 	const uint32_t vl = vb + lane;
-	const bool valid = vl < a.n;
+	const bool valid = lane < nv;
 	const uint32_t lbeg = valid ? __ldg(a.in_off + vl) : 0u, lend = valid ? __ldg(a.in_off + vl + 1) : 0u;
 	const bool big = lend - lbeg > kMsPullBig;
 	const bool needy = valid && !big && lend > lbeg && !ld_cg_u8(a.done + vl);
@@ -607,9 +697,8 @@ __device__ __forceinline__ void ms_pull_words(const MsArgs &a, const MsPull &p, 
 	if (!p.masked) {
 		// rows of the block with nothing to do are zero
 		const uint32_t bigm = __ballot_sync(kFull, big);
-		const uint32_t nb = min(32u, a.n - vb);
 		uint64_t *blk = p.nxt + (size_t) vb * K;
-		for (uint32_t x = lane; x < nb * K; x += 32)
+		for (uint32_t x = lane; x < nv * K; x += 32)
 			if (!(((needm | bigm) >> (x / K)) & 1u)) blk[x] = 0ull;
 	}
 	// a destination's first 32 in-neighbours are read, and its visited row is sent
@@ -685,7 +774,7 @@ __device__ __forceinline__ void ms_pull_chunk(const MsArgs &a, const MsPull &p, 
 	const size_t row = (size_t) v * K;
 	uint32_t u = 0;
 	uint64_t um = 0;
-	if (KK > (int) kMsRowWords && beg + lane < end) {
+	if (beg + lane < end) {
 		u = __ldg(a.in_src + beg + lane);
 		um = ld_cg64(p.actc + u);
 	}
@@ -694,9 +783,7 @@ __device__ __forceinline__ void ms_pull_chunk(const MsArgs &a, const MsPull &p, 
 	uint64_t *bacc = a.big_acc + (size_t) slot * K;
 	if (!fm.complete(vis0, vis1)) {
 		uint64_t acc0 = 0, acc1 = 0;
-		if constexpr (KK <= (int) kMsRowWords) {
-			acc0 = ms_chunk_rows<KK>(a, p.cur, beg, end, gathered);
-		} else if constexpr (KK <= (int) kGroupMaxWords) {
+		if constexpr (KK <= (int) kGroupMaxWords) {
 			const uint32_t kw = lane % KK;
 			uint64_t ag = 0;
 			ms_gather_grouped<KK>(a, p.cur, p.actc, beg, end, u, um, shfl64(fm.f0, kw), shfl64(vis0, kw), ag, gathered);
@@ -762,7 +849,6 @@ __device__ __forceinline__ void ms_pull_blocks(const MsArgs &a, const MsPull &p,
 		const FullMask &fm, unsigned long long &actdeg, unsigned long long &gathered, uint32_t *wbuf,
 		unsigned long long *s_act) {
 	const unsigned lane = lane_id();
-	const uint32_t nblk = (a.n + 31) / 32;
 	constexpr bool kRowWords = KK <= (int) kMsRowWords;
 	constexpr int kN = kRowWords ? KK : 2;
 	uint64_t f[kN], acc[kN];
@@ -772,13 +858,24 @@ __device__ __forceinline__ void ms_pull_blocks(const MsArgs &a, const MsPull &p,
 		acc[k] = 0ull;
 	}
 	uint32_t wn = 0;
-	while (item < a.nchunks + nblk) {
-		const uint32_t next = lane == 0 ? atomicAdd(counter, 1u) : 0u;
-		const uint32_t vb = (item - a.nchunks) * 32;
-		if constexpr (kRowWords) ms_pull_rows<KK>(a, p, vb, f, acc, actdeg, gathered);
-		else ms_pull_words<KK>(a, p, vb, fm, acc[0], acc[1], actdeg, gathered, wbuf, wn);
-		item = __shfl_sync(kFull, next, 0);
+	const uint32_t nruns = kRowWords ? a.nruns : a.nchunks;
+	if constexpr (kRowWords) {
+		while (item < nruns) {
+			const uint32_t next = lane == 0 ? atomicAdd(counter, 1u) : 0u;
+			const uint32_t c0 = item * a.run;
+			ms_pull_runs<KK>(a, p, c0, min(a.run, a.nchunks - c0), f, acc, actdeg, gathered);
+			item = gridDim.x * kMsWarps + __shfl_sync(kFull, next, 0);
+		}
 	}
+	while (item < nruns + a.nblk) {
+		const uint32_t next = lane == 0 ? atomicAdd(counter, 1u) : 0u;
+		const uint32_t vb = (item - nruns) << a.blk_shift;
+		const uint32_t nv = min(1u << a.blk_shift, a.n - vb);
+		if constexpr (kRowWords) ms_pull_rows<KK>(a, p, vb, nv, f, acc, actdeg, gathered, wbuf, wn);
+		else ms_pull_words<KK>(a, p, vb, nv, fm, acc[0], acc[1], actdeg, gathered, wbuf, wn);
+		item = (kRowWords ? gridDim.x * kMsWarps : 0u) + __shfl_sync(kFull, next, 0);
+	}
+	ms_wq_flush(p.cn, p.qn, wbuf, wn);
 	if constexpr (kRowWords) {
 #pragma unroll
 		for (int k = 0; k < KK; ++k) {
@@ -786,24 +883,28 @@ __device__ __forceinline__ void ms_pull_blocks(const MsArgs &a, const MsPull &p,
 			if (lane == 0 && x) atomicOr(s_act + k, (unsigned long long) x);
 		}
 	} else {
-		ms_wq_flush(p.cn, p.qn, wbuf, wn);
 		if (acc[0]) atomicOr(s_act + lane, (unsigned long long) acc[0]);
 		if (acc[1]) atomicOr(s_act + lane + 32, (unsigned long long) acc[1]);
 	}
 }
 
 // A pull level: the chunks of the many-in-edge destinations, then the blocks of
-// 32 destinations, handed to the warps one at a time through a counter (the
-// next one claimed while one runs), so that no barrier is needed between them.
+// destinations, handed to the warps one at a time, so that no barrier is needed
+// between them: through a counter, the next one claimed while one runs; with few
+// words a warp's first by its number (with more, that was 10% slower on 4,096
+// sources).  The frontier's vertices are staged per warp:
+// one atomic on the queue's length per kMsWq of them and not per block (together
+// 2^18 vertices, 64 sources: 282 -> 270 us; 2^20 604 -> 586).  Two or more blocks
+// at a time cost more in balance than they save (2^20: 618).
 template <int KK>
 __device__ __forceinline__ void ms_pull(const MsArgs &a, const MsPull &p, unsigned *counter, unsigned long long &actdeg_out,
 		unsigned long long &gathered_out, uint32_t *wq_base, unsigned long long *s_act) {
 	const unsigned lane = lane_id();
 	const FullMask fm(a, lane, p.act);
 	unsigned long long actdeg = 0, gathered = 0;
-	uint32_t item = lane == 0 ? atomicAdd(counter, 1u) : 0u;
-	item = __shfl_sync(kFull, item, 0);
-	if (item < a.nchunks) item = ms_pull_chunks<KK>(a, p, item, counter, fm, actdeg, gathered, s_act);
+	uint32_t item = warp_id() * gridDim.x + blockIdx.x;
+	if (KK > (int) kMsRowWords) item = __shfl_sync(kFull, lane == 0 ? atomicAdd(counter, 1u) : 0u, 0);
+	if (KK > (int) kMsRowWords && item < a.nchunks) item = ms_pull_chunks<KK>(a, p, item, counter, fm, actdeg, gathered, s_act);
 	uint32_t *wbuf = wq_base + warp_id() * kMsWq;
 	ms_pull_blocks<KK>(a, p, item, counter, fm, actdeg, gathered, wbuf, s_act);
 	actdeg_out += actdeg;
@@ -1150,8 +1251,10 @@ template <int KK>
 __global__ void __launch_bounds__(kMsThreads, 2) k_ms_bfs(const __grid_constant__ MsArgs a, const uint32_t *sources, uint32_t ns,
 		uint8_t *levels) {
 	__shared__ unsigned long long red[kMsWarps];
-	__shared__ uint32_t wq[kMsWarps * kMsWq];
+	// an early output pass's tile; while levels run, the warps' staged appends
 	__shared__ __align__(16) uint8_t lev[kEmitBytes];
+	static_assert(kMsWarps * kMsWq * 4 <= kEmitBytes, "the appends fit in the tile");
+	uint32_t *const wq = reinterpret_cast<uint32_t *>(lev);
 	MsControl *ctl = a.ctl;
 	const uint32_t stride = gridDim.x * blockDim.x;
 	const uint32_t t0 = blockIdx.x * blockDim.x + threadIdx.x;
@@ -1373,16 +1476,29 @@ int ms_launch(const MsArgs &a, const uint32_t *d_sources, uint32_t ns, uint8_t *
 	int per_sm = 0;
 	if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, fn, kMsThreads, 0) != cudaSuccess || per_sm < 1)
 		return BFS_ECUDA;
-	per_sm = std::min(per_sm, 2);
-	if (a.ctas_per_sm) per_sm = std::min(per_sm, (int) a.ctas_per_sm);
-	if (grid) *grid = num_sms * per_sm;
+	const uint64_t state = a.K <= kMsRowWords ? (uint64_t) a.n * a.K : ~0ull;
+	per_sm = std::min(per_sm, a.ctas_per_sm ? (int) a.ctas_per_sm : state <= kMsSmallState ? 1 : 2);
+	const int ctas = !a.ctas_per_sm && state <= kMsTinyState ? std::max(num_sms / 2, 1) : num_sms * per_sm;
+	if (grid) *grid = ctas;
 	if (cudaMemsetAsync(a.ctl, 0, sizeof(MsControl), st) != cudaSuccess) return BFS_ECUDA;
 	MsArgs aa = a;
+	// the pull's items: see ms_pull
+	const uint32_t nwarps = (uint32_t) ctas * kMsWarps;
+	aa.run = 1;
+	aa.blk_shift = 5;
+	if (a.K <= kMsRowWords) {
+		aa.run = std::min(std::max(a.nchunks / (nwarps * 2), 1u), kMsRun);
+	} else {
+		while (aa.blk_shift > 2 && a.n >> aa.blk_shift < kMsBlocks * nwarps) --aa.blk_shift;
+		while (aa.blk_shift > 0 && a.n >> aa.blk_shift < nwarps / 2) --aa.blk_shift;
+	}
+	aa.nruns = (a.nchunks + aa.run - 1) / aa.run;
+	aa.nblk = (uint32_t) (((uint64_t) a.n + (1u << aa.blk_shift) - 1) >> aa.blk_shift);
 	const uint32_t *src = d_sources;
 	uint32_t nsrc = ns;
 	uint8_t *out = levels;
 	void *args[] = {&aa, (void *) &src, &nsrc, &out};
-	if (cudaLaunchCooperativeKernel((const void *) fn, dim3(num_sms * per_sm), dim3(kMsThreads), args, 0, st) !=
+	if (cudaLaunchCooperativeKernel((const void *) fn, dim3(ctas), dim3(kMsThreads), args, 0, st) !=
 			cudaSuccess)
 		return BFS_ECUDA;
 	if (between && cudaEventRecord(between, st) != cudaSuccess) return BFS_ECUDA;

@@ -376,3 +376,35 @@ def test_planes_per_output_step(native, oracle, n, levels):
             for tile in (0, 64) if k > 128 else (0,):
                 g.set_options(batch_single_max=0, batch_planes=36, batch_output_tile=tile)
                 _check(oracle, arr, g, sources, exp)
+
+
+@pytest.mark.parametrize("words", [1, 3, 4, 6, 20])
+@pytest.mark.parametrize("n", [40, 4097, 9000, 70000])
+def test_grid_and_blocks_by_state(native, oracle, n, words):
+    """Graph sizes on each side of the rules that choose the grid and the pull's blocks
+    of destinations, with destinations of several chunks of in-edges each."""
+    import bfs_simd_benchmarks_gb300 as B
+    rng = np.random.default_rng(n + words)
+    hubs = rng.integers(0, n, size=3)
+    src = np.concatenate([rng.integers(0, n, size=4 * n)] + [rng.integers(0, n, size=d) for d in (2100, 1025, 300)])
+    dst = np.concatenate([rng.integers(0, n, size=4 * n)] + [np.full(d, h) for d, h in zip((2100, 1025, 300), hubs)])
+    src, dst = src.astype(np.uint32), dst.astype(np.uint32)
+    arr = oracle.csr_arrays(n, src, dst)
+    k = 64 * words - 5
+    sources = rng.integers(0, n, size=k).astype(np.uint32)
+    sources[k // 2:] = sources[rng.integers(0, 20, size=k - k // 2)]
+    with B.Graph.from_edges(n, src, dst, 256, 4) as g:
+        levels = {}
+        for s in set(sources[:20].tolist()) | set(sources[20:40].tolist()):
+            lev = oracle.bfs_levels(arr, s)
+            levels[s] = np.where(lev < 0, 255, lev).astype(np.uint8)
+        for push_div in (1, 1 << 30):
+            g.set_options(batch_single_max=0, batch_push_div=push_div)
+            for ctas in (0, 1, 2):
+                g.set_options(ctas_per_sm=ctas)
+                out, st = g.run_batch(sources)
+                assert st["status"] == 0
+                got = out.cpu().numpy()
+                for i, s in enumerate(sources.tolist()):
+                    if s in levels:
+                        np.testing.assert_array_equal(got[i], levels[s], err_msg=f"row {i} (source {s})")
