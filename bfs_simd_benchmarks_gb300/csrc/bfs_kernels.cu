@@ -474,32 +474,23 @@ __device__ __shared__ TmaMeta tma_meta[kTmaStages];
 __device__ __shared__ alignas(8) uint64_t tma_bar[kTmaStages];    // stage filled
 __device__ __shared__ alignas(8) uint64_t tma_empty[kTmaStages];  // stage released by every consumer warp
 
-// Claims the next work item -- a column group, or with `split` > 1 one of
-// `split` equal parts (in 32-vertex words) of a column group -- loads its
-// visited bits into vis_s and a copy into nxt_s, and counts the vertices
-// with an in-edge that are still unvisited.  Returns false when no item is
-// left.  Uniform across the CTA.
+// Claims the next column group, loads its visited bits into vis_s and a copy into
+// nxt_s, and counts the vertices with an in-edge that are still unvisited.
+// Returns false when none is left.  Uniform across the CTA.
 __device__ __forceinline__ bool dense_group_begin(const DevGraph &g, const RunCtx &r, StepCounters *out, uint32_t *vis_s,
-		uint32_t *nxt_s, DenseGroup &gr, uint32_t *hin_s = nullptr, uint32_t split = 1, bool first = false) {
+		uint32_t *nxt_s, DenseGroup &gr) {
 	__syncthreads();
 	if (threadIdx.x == 0) {
-		// with `first`, a CTA's first item is its own index (no atomic: the
-		// whole grid asking at once queued on one line); later items are
-		// counted from gridDim.x
-		dsh.group = first ? blockIdx.x : (split > 1 ? gridDim.x : 0u) + atomicAdd(&out->work, 1u);
+		dsh.group = atomicAdd(&out->work, 1u);
 		dsh.unsettled = 0;
 		dsh.stop = 0;
 	}
 	__syncthreads();
-	const uint32_t item = dsh.group;
-	if (item >= g.num_groups * split) return false;
-	gr.gi = item / split;
-	const uint32_t part = item % split;
+	gr.gi = dsh.group;
+	if (gr.gi >= g.num_groups) return false;
 	const uint32_t c0 = __ldg(g.group_col + gr.gi), c1 = __ldg(g.group_col + gr.gi + 1);
-	const uint64_t a = (uint64_t) c0 * g.w, b = min((uint64_t) c1 * g.w, (uint64_t) g.n);
-	const uint64_t words = (b - a + 31) / 32;
-	gr.v0 = min(b, a + 32 * (words * part / split));
-	gr.v1 = min(b, a + 32 * (words * (part + 1) / split));
+	gr.v0 = (uint64_t) c0 * g.w;
+	gr.v1 = min((uint64_t) c1 * g.w, (uint64_t) g.n);
 	gr.gw = (uint32_t) ((gr.v1 - gr.v0 + 31) / 32);
 	uint32_t uns = 0;
 	for (uint32_t j = threadIdx.x; j < gr.gw; j += kThreads) {
@@ -507,7 +498,6 @@ __device__ __forceinline__ bool dense_group_begin(const DevGraph &g, const RunCt
 		uint32_t hb = bits_at(g.hasin, gr.v0 + 32ull * j, gr.v1, 0u);
 		vis_s[j] = vb;
 		nxt_s[j] = vb;  // visited bits at the start: the new frontier is vis_s & ~nxt_s
-		if (hin_s) hin_s[j] = hb;
 		uns += __popc(hb & ~vb);
 	}
 	if (threadIdx.x == 0) vis_s[gr.gw] = kFull;  // the slot padding words point at
@@ -927,10 +917,48 @@ __device__ __forceinline__ void phase_dense_tma(const DevGraph &g, const RunCtx 
 // pull of a uniform graph of 2^20 vertices and 2^24 edges (now 100), 1.86 ms for
 // the Twitter shape's (now 0.9).
 constexpr uint32_t kPullShort = 3;
-// Work items of a pull step: each column group in this many parts, handed
-// out dynamically (whole groups left a few CTAs with most of the work: the
-// early exit makes a group's cost depend on where its frontier sources are).
-constexpr uint32_t kPullSplit = 4;
+// Work items of a pull step: ranges of the bitmap, as many for every CTA, of about
+// kPullWords words where there are more, handed out dynamically (the early exit
+// makes a range's cost depend on where its frontier sources are).  Quarters of the
+// column groups, which are planned for another kernel, gave 1,104 items of 46
+// words on the Pokec shape, less than one pass of a CTA's warps each, and a last
+// wave that was half empty: a query 147 us, now 130; uniform, 2^20 vertices, 2^24
+// edges 195 -> 163; rmat, 2^22 vertices, 2^26 edges 287 -> 254.  Ranges of 256 words:
+// 269 on the last; of 1,024: 255, but 1.32 ms on the Twitter shape (1.25).
+constexpr uint32_t kPullWords = 512, kPullMinWords = 32;
+
+// A CTA's next item of a pull step: its visited bits to vis_s and vis0_s, which
+// of its vertices have in-edges to hin_s, the unvisited of those to
+// dsh.unsettled.  A CTA's first item is its own index (no atomic: the whole grid
+// asking at once queued on one line); later items are counted from gridDim.x.
+__device__ __forceinline__ bool pull_begin(const DevGraph &g, const RunCtx &r, StepCounters *out, uint32_t per, bool first,
+		uint32_t *vis_s, uint32_t *vis0_s, uint32_t *hin_s, DenseGroup &gr) {
+	__syncthreads();
+	if (threadIdx.x == 0) {
+		dsh.group = first ? blockIdx.x : gridDim.x + atomicAdd(&out->work, 1u);
+		dsh.unsettled = 0;
+		dsh.nlist = 0;
+	}
+	__syncthreads();
+	gr.gi = 0;
+	gr.v0 = 32ull * per * dsh.group;
+	if (gr.v0 >= g.n) return false;
+	gr.v1 = min(gr.v0 + 32u * per, (uint64_t) g.n);
+	gr.gw = (uint32_t) ((gr.v1 - gr.v0 + 31) / 32);
+	uint32_t uns = 0;
+	for (uint32_t j = threadIdx.x; j < gr.gw; j += kThreads) {
+		const uint32_t vb = bits_at(r.vis, gr.v0 + 32ull * j, gr.v1, kFull);
+		const uint32_t hb = bits_at(g.hasin, gr.v0 + 32ull * j, gr.v1, 0u);
+		vis_s[j] = vb;
+		vis0_s[j] = vb;
+		hin_s[j] = hb;
+		uns += __popc(hb & ~vb);
+	}
+	uns = warp_sum(uns);
+	if (lane_id() == 0 && uns) atomicAdd(&dsh.unsettled, uns);
+	__syncthreads();
+	return true;
+}
 
 __device__ __forceinline__ bool frontier_bit(const uint32_t *cur, uint32_t u) {
 	return (ld_phase(cur + (u >> 5)) >> (u & 31)) & 1u;
@@ -972,12 +1000,14 @@ __device__ __forceinline__ void phase_pull(const DevGraph &g, const RunCtx &r, u
 	unsigned long long cyc[4] = {0, 0, 0, 0};
 	long long t0 = clock64();
 	bool first = true;
-	while (dense_group_begin(g, r, out, vis_s, vis0_s, gr, hin_s, kPullSplit, first)) {
+	const uint32_t nw = (g.n + 31) / 32, share = (nw + gridDim.x - 1) / gridDim.x;
+	const uint32_t items = max((share + kPullWords / 2) / kPullWords, 1u);
+	const uint32_t per = min(max((share + items - 1) / items, kPullMinWords), g.max_group_words);
+	while (pull_begin(g, r, out, per, first, vis_s, vis0_s, hin_s, gr)) {
 		first = false;
 		{ long long t1 = clock64(); cyc[0] += t1 - t0; t0 = t1; }
 		if (dsh.unsettled == 0) continue;
-		if (threadIdx.x == 0) { acc.bu_groups++; dsh.nlist = 0; }
-		__syncthreads();
+		if (threadIdx.x == 0) acc.bu_groups++;
 		const uint32_t v0 = (uint32_t) gr.v0;
 		uint32_t edges = 0, tested = 0;
 		// Pass 1: a warp takes four bitmap words (a lane per destination in
