@@ -923,9 +923,13 @@ constexpr uint32_t kPullShort = 3;
 // column groups, which are planned for another kernel, gave 1,104 items of 46
 // words on the Pokec shape, less than one pass of a CTA's warps each, and a last
 // wave that was half empty: a query 147 us, now 130; uniform, 2^20 vertices, 2^24
-// edges 195 -> 163; rmat, 2^22 vertices, 2^26 edges 287 -> 254.  Ranges of 256 words:
-// 269 on the last; of 1,024: 255, but 1.32 ms on the Twitter shape (1.25).
-constexpr uint32_t kPullWords = 512, kPullMinWords = 32;
+// edges 195 -> 163; rmat, 2^22 vertices, 2^26 edges 287 -> 254.  Half as long from a
+// share of kPullManyWords words per CTA on: there, long ranges' destinations
+// overflow the queue (Twitter shape, 4,282 words a CTA: 1.89 ms with 256 words and
+// with quarters, 1.94 with 384, 2.21 with 512; rmat, 2^24 vertices and 2^27 edges,
+// 1,725 words a CTA: 589, 572 and 564 us, 593 with quarters).  Emptying the queue
+// before it overflows cost more in barriers than the scans in place: 1.96.
+constexpr uint32_t kPullWords = 512, kPullManyWords = 2048, kPullMinWords = 32;
 
 // A CTA's next item of a pull step: its visited bits to vis_s and vis0_s, which
 // of its vertices have in-edges to hin_s, the unvisited of those to
@@ -1001,7 +1005,8 @@ __device__ __forceinline__ void phase_pull(const DevGraph &g, const RunCtx &r, u
 	long long t0 = clock64();
 	bool first = true;
 	const uint32_t nw = (g.n + 31) / 32, share = (nw + gridDim.x - 1) / gridDim.x;
-	const uint32_t items = max((share + kPullWords / 2) / kPullWords, 1u);
+	const uint32_t words = share < kPullManyWords ? kPullWords : kPullWords / 2;
+	const uint32_t items = max((share + words / 2) / words, 1u);
 	const uint32_t per = min(max((share + items - 1) / items, kPullMinWords), g.max_group_words);
 	while (pull_begin(g, r, out, per, first, vis_s, vis0_s, hin_s, gr)) {
 		first = false;
