@@ -68,7 +68,7 @@ constexpr uint32_t kMsBlocks = 4;
 constexpr uint32_t kMsSmallState = 1u << 18, kMsTinyState = 1u << 15;
 constexpr uint32_t kMsRun = 8;          // pull, few words: chunks taken at once
 constexpr uint32_t kMsMaxWords = 64;    // 4,096 sources
-constexpr uint32_t kGroupMaxWords = 16; // pull: up to this many words, in-neighbour rows in lane groups
+constexpr uint32_t kGroupMaxWords = 32; // pull: up to this many words, in-neighbour rows in lane groups
 constexpr uint32_t kEmitW = 4;          // output tile: kV vertices x kW words (4: 256 sources), kV = threads / kW
 constexpr uint32_t kEmitPlanes = 7;     // planes that a 3-bit index tells apart, with one value left for "none of them"
 constexpr uint32_t kEmitUnits = 8;      // output tiles' words are split among CTAs below this many per CTA
@@ -402,49 +402,66 @@ __device__ __forceinline__ uint64_t warp_or64(uint64_t x) {
 }
 
 // ms_gather for kMsRowWords < K <= kGroupMaxWords words per vertex: the warp is
-// split into groups of kLanes (8 or 16) lanes; of g groups, each takes every g-th
-// in-neighbour and reads its row (lane k its word k), so a round reads
-// g kMsGather rows; the groups' words are
-// OR-ed together after every round for the early exit.  `vis` and `f` are the
-// lane's word k (the same in every group); acc comes back in every group.
+// split into groups of kLanes lanes (8, or 16 for more than 8 words); of g groups,
+// each takes every g-th in-neighbour and reads its row (lane k its words k, and
+// k + 16 of more than 16), so a round reads g kMsGather rows; the groups' words are
+// OR-ed together after every round for the early exit.  `vis0` and `f0` are lane's
+// word; so is the result.
 // (Sharing the frontier's neighbours out evenly, by __fns, cost more than idle
 // groups: uniform, 2^18 vertices, 2^22 edges, 300 sources: 1.13 against 0.80 ms.
-// With a warp per row as above 16 words, rmat, 2^20 vertices, 2^24 edges, 1,024
-// sources: 3.81 against 2.63 ms.)
-template <uint32_t kLanes>
-__device__ __forceinline__ void ms_gather_grouped(const MsArgs &a, const uint64_t *cur, const uint64_t *actc,
-		uint32_t beg, uint32_t end, uint32_t u, uint64_t um, uint64_t f, uint64_t vis, uint64_t &acc,
-		unsigned long long &gathered) {
+// With a warp per row as above 32 words, rmat, 2^20 vertices, 2^24 edges, 1,024
+// sources: 3.81 against 2.63 ms; 2,048 sources: 4.46 against 3.71.)
+template <int KK>
+__device__ __forceinline__ uint64_t ms_gather_grouped(const MsArgs &a, const uint64_t *cur, const uint64_t *actc,
+		uint32_t beg, uint32_t end, uint32_t u, uint64_t um, uint64_t f0, uint64_t vis0, unsigned long long &gathered) {
+	constexpr uint32_t kLanes = KK > 8 ? 16 : 8;
+	constexpr int kWords = KK / (int) kLanes;
 	const uint32_t K = a.K;
 	const unsigned lane = lane_id();
 	const uint32_t k = lane % kLanes;
 	uint32_t loads = 0;
-	bool done = __all_sync(kFull, ((vis | acc) & f) == f);
+	uint64_t f[kWords], have[kWords];
+	bool full = true;
+#pragma unroll
+	for (int j = 0; j < kWords; ++j) {
+		f[j] = shfl64(f0, k + kLanes * j);  // zero beyond the last word
+		have[j] = shfl64(vis0, k + kLanes * j);
+		full &= (have[j] & f[j]) == f[j];
+	}
+	bool done = __all_sync(kFull, full);
 	for (uint32_t e0 = beg; e0 < end && !done; e0 += 32) {
 		if (e0 != beg) um = e0 + lane < end ? ld_cg64(actc + u) : 0ull;
 		const uint32_t en = e0 + 32 + lane, un = en < end ? __ldg(a.in_src + en) : 0u;
 		uint32_t lm = __ballot_sync(kFull, um != 0ull) & ((kLanes == 8 ? 0x11111111u : 0x55555555u) << (lane / kLanes));
 		while (!done && __any_sync(kFull, lm)) {
-			const bool need = ((vis | acc) & f) != f;  // f is zero beyond the last word
-			uint64_t gv[kMsGather];
+			uint64_t gv[kMsGather][kWords];
 #pragma unroll
 			for (int t = 0; t < kMsGather; ++t) {
 				const int src = __ffs(lm) - 1;
 				const uint32_t ut = __shfl_sync(kFull, u, src & 31);
 				const uint64_t mt = shfl64(um, src & 31);
-				const bool ld = lm && need && ((mt >> k) & 1ull);
-				gv[t] = ld ? ld_cg64(cur + (size_t) ut * K + k) : 0ull;
-				loads += ld;
+#pragma unroll
+				for (int j = 0; j < kWords; ++j) {
+					const bool ld = lm && (have[j] & f[j]) != f[j] && ((mt >> (k + kLanes * j)) & 1ull);
+					gv[t][j] = ld ? ld_cg64(cur + (size_t) ut * K + k + kLanes * j) : 0ull;
+					loads += ld;
+				}
 				lm &= lm - 1;
 			}
+			full = true;
 #pragma unroll
-			for (int t = 0; t < kMsGather; ++t) acc |= gv[t];
-			for (uint32_t d = kLanes; d < 32; d <<= 1) acc |= shfl_xor64(acc, d);
-			done = __all_sync(kFull, ((vis | acc) & f) == f);
+			for (int j = 0; j < kWords; ++j) {
+#pragma unroll
+				for (int t = 0; t < kMsGather; ++t) have[j] |= gv[t][j];
+				for (uint32_t d = kLanes; d < 32; d <<= 1) have[j] |= shfl_xor64(have[j], d);
+				full &= (have[j] & f[j]) == f[j];
+			}
+			done = __all_sync(kFull, full);
 		}
 		u = un;
 	}
 	gathered += loads;
+	return kWords == 2 && lane >= kLanes ? have[kWords - 1] : lane < KK ? have[0] : 0ull;
 }
 
 // What a pull level works on.
@@ -723,10 +740,7 @@ __device__ __forceinline__ void ms_pull_words(const MsArgs &a, const MsPull &p, 
 		if (m & (m - 1)) un = first_neighbours(m & (m - 1));
 		uint64_t acc0 = 0, acc1 = 0;
 		if constexpr (KK <= (int) kGroupMaxWords) {
-			const uint32_t kw = lane % KK;
-			uint64_t ag = 0;
-			ms_gather_grouped<KK>(a, p.cur, p.actc, beg, end, u, um, shfl64(fm.f0, kw), shfl64(vis0, kw), ag, gathered);
-			acc0 = lane < KK ? ag : 0ull;
+			acc0 = ms_gather_grouped<KK>(a, p.cur, p.actc, beg, end, u, um, fm.f0, vis0, gathered);
 		} else if (!fm.complete(vis0, vis1)) {
 			ms_gather(a, p.cur, p.actc, beg, end, u, um, fm, vis0, vis1, acc0, acc1, gathered);
 		}
@@ -784,10 +798,7 @@ __device__ __forceinline__ void ms_pull_chunk(const MsArgs &a, const MsPull &p, 
 	if (!fm.complete(vis0, vis1)) {
 		uint64_t acc0 = 0, acc1 = 0;
 		if constexpr (KK <= (int) kGroupMaxWords) {
-			const uint32_t kw = lane % KK;
-			uint64_t ag = 0;
-			ms_gather_grouped<KK>(a, p.cur, p.actc, beg, end, u, um, shfl64(fm.f0, kw), shfl64(vis0, kw), ag, gathered);
-			acc0 = lane < KK ? ag : 0ull;
+			acc0 = ms_gather_grouped<KK>(a, p.cur, p.actc, beg, end, u, um, fm.f0, vis0, gathered);
 		} else {
 			ms_gather(a, p.cur, p.actc, beg, end, u, um, fm, vis0, vis1, acc0, acc1, gathered);
 		}
@@ -903,8 +914,10 @@ __device__ __forceinline__ void ms_pull(const MsArgs &a, const MsPull &p, unsign
 	const FullMask fm(a, lane, p.act);
 	unsigned long long actdeg = 0, gathered = 0;
 	uint32_t item = warp_id() * gridDim.x + blockIdx.x;
-	if (KK > (int) kMsRowWords) item = __shfl_sync(kFull, lane == 0 ? atomicAdd(counter, 1u) : 0u, 0);
-	if (KK > (int) kMsRowWords && item < a.nchunks) item = ms_pull_chunks<KK>(a, p, item, counter, fm, actdeg, gathered, s_act);
+	if constexpr (KK > (int) kMsRowWords) {
+		item = __shfl_sync(kFull, lane == 0 ? atomicAdd(counter, 1u) : 0u, 0);
+		if (item < a.nchunks) item = ms_pull_chunks<KK>(a, p, item, counter, fm, actdeg, gathered, s_act);
+	}
 	uint32_t *wbuf = wq_base + warp_id() * kMsWq;
 	ms_pull_blocks<KK>(a, p, item, counter, fm, actdeg, gathered, wbuf, s_act);
 	actdeg_out += actdeg;
@@ -1242,7 +1255,7 @@ __device__ __noinline__ void ms_emit(const MsArgs &a, uint8_t *levels, uint32_t 
 	}
 }
 
-// KK: words per vertex up to kMsRowWords; for more, 8, 16 (kGroupMaxWords) or 64
+// KK: words per vertex up to kMsRowWords; for more, 8, 16, 32 (kGroupMaxWords) or 64
 // (kMsMaxWords) for up to as many: one kernel each, so that only one form of the pull shares
 // the registers and its arguments are read where they lie (as calls of one
 // kernel, with arguments by reference, the pulls' accesses to local memory were
@@ -1472,7 +1485,7 @@ int ms_launch(const MsArgs &a, const uint32_t *d_sources, uint32_t ns, uint8_t *
 		int *grid, cudaEvent_t between, cudaEvent_t between2) {
 	static_assert(kMsRowWords == 4, "a kernel for each");
 	const auto fn = a.K == 1 ? k_ms_bfs<1> : a.K == 2 ? k_ms_bfs<2> : a.K == 3 ? k_ms_bfs<3> : a.K == 4 ? k_ms_bfs<4>
-			: a.K <= 8 ? k_ms_bfs<8> : a.K <= kGroupMaxWords ? k_ms_bfs<kGroupMaxWords> : k_ms_bfs<kMsMaxWords>;
+			: a.K <= 8 ? k_ms_bfs<8> : a.K <= 16 ? k_ms_bfs<16> : a.K <= kGroupMaxWords ? k_ms_bfs<kGroupMaxWords> : k_ms_bfs<kMsMaxWords>;
 	int per_sm = 0;
 	if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, fn, kMsThreads, 0) != cudaSuccess || per_sm < 1)
 		return BFS_ECUDA;
