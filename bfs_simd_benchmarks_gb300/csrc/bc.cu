@@ -23,9 +23,10 @@
 //      over out-edges v -> w with level(w) = level(v) + 1; the output is
 //      (D - 1/sigma) / (1/sigma), 0 where sigma is 0 -- the reference's float
 //      formulas, with its signed int -> float conversion of the counts.
-// Per level, the edge lists of big vertices are cut into kBcChunk-edge chunks
-// that CTAs all over the grid sum (partials added in chunk order by the CTA that
-// completes the last one), medium vertices are summed by half-warps, and small
+// Per level, the edge lists of big vertices are cut into kBcWarpChunk-edge chunks
+// that warps all over the grid sum (kBcChunk and CTAs where a level has very many
+// big vertices; partials are added in chunk order by whoever completes the last
+// one), medium vertices are summed by half-warps, and small
 // ones by a lane each, with lanes of a warp in the same degree band.  Path
 // counts of levels that few edges lead to are pushed instead (integer adds).
 #include "bc.h"

@@ -10,7 +10,7 @@ namespace bfsg {
 
 constexpr uint32_t kBcMaxLevels = 1u << 19;   // deeper traversals are refused (BFS_EUNSUPPORTED)
 constexpr uint32_t kBcCntCap = 1u << 22;      // (level key, vertex range) counters of the level sort
-constexpr uint32_t kBcBig = 1024;             // in- or out-degree above which a whole CTA reduces a vertex
+constexpr uint32_t kBcBig = 1024;             // in- or out-degree above which a vertex is summed in chunks
 constexpr uint32_t kBcMedium = 32;            // above this (and up to kBcBig) a half-warp reduces a vertex;
                                               // at most this, a lane does
 constexpr uint32_t kBcTiny = 8;               // small vertices come in two bands, so that a warp's lanes

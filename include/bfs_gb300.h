@@ -164,8 +164,8 @@ typedef struct bfs_options {
 	                              (Beamer's rule); levels are identical, only the step directions differ */
 	uint32_t bu_alpha;         /* BFS_SWITCH_UNVISITED: alpha (default 14) */
 	uint32_t td_beta;          /* BFS_SWITCH_UNVISITED: beta (default 24) */
-	uint32_t ctas_per_sm;      /* CTAs per SM of the cooperative traversal grids: 0 = as many as fit (at most
-	                              2), or 1 or 2 */
+	uint32_t ctas_per_sm;      /* CTAs per SM of the cooperative traversal grids: 0 = chosen by graph size
+	                              (at most 2; small graphs take fewer CTAs, or one cluster), or 1 or 2 */
 	uint32_t bc_batch;         /* bfs_bc_accumulate: 1 (default) = sources in groups of up to 256 through the
 	                              batched betweenness kernel (bfs_bc_run_batch); 0 = one source at a time */
 	uint32_t batch_output_tile; /* bfs_run_batch output pass: vertices per tile, 64, 128 (both of four
