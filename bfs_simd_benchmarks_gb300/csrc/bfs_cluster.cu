@@ -428,6 +428,7 @@ int cluster_config(const DevGraph &g, int ctas, cudaStream_t st, cudaLaunchConfi
 
 int cluster_ctas(const DevGraph &g) {
 	if (g.n > kClusterMaxVertices || g.m > kClusterMaxEdges) return 0;
+	if (g.n > kClusterDenseVertices && (uint64_t) g.m > (uint64_t) kClusterSparseDegree * g.n) return 0;
 	int ctas = 1;
 	while (ctas < (int) kClMaxCtas && (uint32_t) ctas * kClusterVerticesPerCta < g.n) ctas *= 2;
 	const size_t most = sizeof(uint32_t) * ((size_t) 3 * ((kClusterMaxVertices + 31) / 32) + 3 * kClQueue + kSoloWords);

@@ -127,7 +127,7 @@ def _mixed(n, seed):
     return np.concatenate(src).astype(np.uint32), np.concatenate(dst).astype(np.uint32)
 
 
-@pytest.mark.parametrize("n", [1, 31, 33, 1024, 1025, 4097, 20_000, 98_304, 98_305])
+@pytest.mark.parametrize("n", [1, 31, 33, 1024, 1025, 4097, 20_000, 65_536, 65_537, 98_304, 98_305])
 def test_one_cluster_traversal(native, oracle, n):
     """Small graphs are traversed in one cluster: its sizes, both directions at every
     step and mixed ones, against the oracle and the whole grid's step sequence."""
@@ -146,7 +146,7 @@ def test_one_cluster_traversal(native, oracle, n):
                 assert oracle.check_parents(arr, s, lev, par) == 0
                 assert st["reached"] == int((ref >= 0).sum()) and st["num_steps"] == ref.max() + 1
                 assert st["edges_traversed"] == int(deg[ref >= 0].sum())
-                assert (st["grid_ctas"] <= 16) == (n <= 98_304)
+                assert (st["grid_ctas"] <= 16) == (n <= 65_536 or (n <= 98_304 and len(src) <= 4 * n))
                 np.testing.assert_array_equal(g.run(s, parents=False)[0], ref)
                 g.set_options(ctas_per_sm=2)
                 lev2, _, st2 = g.run(s)
