@@ -402,7 +402,7 @@ __device__ __forceinline__ typename Dir<kFwd>::T lane_vertex_sum(const BcArgs &a
 		bool use8) {
 	using T = typename Dir<kFwd>::T;
 	const uint32_t *adj = Dir<kFwd>::adj(a);
-	T s = T(0);
+	T s = T(0), lost = T(0);
 	for (uint32_t q = beg & ~3u; q < end; q += 4 * kBcQuads) {
 		uint32_t nb[4 * kBcQuads];
 		uint2 lx[4 * kBcQuads];
@@ -423,7 +423,8 @@ __device__ __forceinline__ typename Dir<kFwd>::T lane_vertex_sum(const BcArgs &a
 			}
 		}
 		gather_tags(a, nb, lx, use8, target);
-		// pairwise: a list of 32 takes 3 + 4 roundings in a row, not 32
+		// pairwise, and what is rounded off where the groups meet (Knuth's TwoSum)
+		// is added at the end: a lane's sum is then as near as a warp's tree
 		T x[4 * kBcQuads];
 #pragma unroll
 		for (int k = 0; k < 4 * kBcQuads; ++k) x[k] = (int) lx[k].x == target ? Dir<kFwd>::value(lx[k].y) : T(0);
@@ -431,9 +432,15 @@ __device__ __forceinline__ typename Dir<kFwd>::T lane_vertex_sum(const BcArgs &a
 		for (int d = 1; d < 4 * kBcQuads; d *= 2)
 #pragma unroll
 			for (int k = 0; k + d < 4 * kBcQuads; k += 2 * d) x[k] += x[k + d];
-		s += x[0];
+		if constexpr (kFwd) {
+			s += x[0];
+		} else {
+			const T t = s + x[0], b = t - s;
+			lost += (s - (t - b)) + (x[0] - b);
+			s = t;
+		}
 	}
-	return s;
+	return s + lost;
 }
 
 // Path counts of level d pushed along the out-edges of the vertices of level
