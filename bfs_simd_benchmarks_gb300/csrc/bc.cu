@@ -182,9 +182,10 @@ __device__ __forceinline__ typename Dir<kFwd>::T cta_range_sum(const BcArgs &a, 
 
 
 // Chunk prefix of the vertices order[bb .. bb+cnt) (cnt <= kBcSmemBig, `per`
-// edges per chunk) in bsh.cpre, the same in every CTA; returns the total.
+// edges per chunk, `least` chunks or more each) in bsh.cpre, the same in every
+// CTA; returns the total.
 template <bool kFwd>
-__device__ __forceinline__ uint32_t chunk_prefix(const BcArgs &a, uint32_t bb, uint32_t cnt, uint32_t per) {
+__device__ __forceinline__ uint32_t chunk_prefix(const BcArgs &a, uint32_t bb, uint32_t cnt, uint32_t per, uint32_t least) {
 	const uint32_t *off = Dir<kFwd>::off(a);
 	constexpr uint32_t kPer = kBcSmemBig / kBcThreads;  // consecutive entries per thread, their loads together
 	uint32_t v[kPer], c[kPer], sum = 0;
@@ -195,7 +196,7 @@ __device__ __forceinline__ uint32_t chunk_prefix(const BcArgs &a, uint32_t bb, u
 	}
 #pragma unroll
 	for (uint32_t k = 0; k < kPer; ++k) {
-		c[k] = v[k] != 0xFFFFFFFFu ? (off[v[k] + 1] - off[v[k]] + per - 1) / per : 0u;
+		c[k] = v[k] != 0xFFFFFFFFu ? max(least, (off[v[k] + 1] - off[v[k]] + per - 1) / per) : 0u;
 		sum += c[k];
 	}
 	uint32_t total;
@@ -449,7 +450,7 @@ __device__ __forceinline__ typename Dir<kFwd>::T lane_vertex_sum(const BcArgs &a
 constexpr uint32_t kBcPushChunk = 512;
 __device__ __forceinline__ void push_paths(const BcArgs &a, uint32_t bb, uint32_t cnt, int target, bool use8,
 		unsigned long long *edges) {
-	const uint32_t total = chunk_prefix<false>(a, bb, cnt, kBcPushChunk);
+	const uint32_t total = chunk_prefix<false>(a, bb, cnt, kBcPushChunk, 0);
 	const unsigned lane = lane_id();
 	const uint32_t gw = blockIdx.x + warp_id() * gridDim.x, tw = gridDim.x * kBcWarps;
 	for (uint32_t j = gw; j < total; j += tw) {
@@ -565,7 +566,9 @@ __device__ __forceinline__ void level_sums(const BcArgs &a, uint32_t d, int targ
 	__syncthreads();
 	const uint32_t bb = bsh.beg[0], nbig = bsh.beg[1] - bb;
 	uint32_t chunks = 0;
-	if (big && nbig && !skip) chunks = chunk_prefix<kFwd>(a, bb, nbig, kBcWarpChunk);
+	// a vertex is finished with its last chunk, so one that is big for its other
+	// side's edges and has none on this side (a sink of many in-edges) has a chunk too
+	if (big && nbig && !skip) chunks = chunk_prefix<kFwd>(a, bb, nbig, kBcWarpChunk, 1);
 	if (threadIdx.x == 0) {
 		uint32_t n = chunks;
 		for (uint32_t c = 1; c < kBcClasses; ++c) {

@@ -217,3 +217,40 @@ def test_bc_arguments(native):
         s = int(np.flatnonzero(deg == 0)[0])
         dep, sig, st = g.bc(s)
         assert st["reached"] == 1 and sig[s] == 1 and (dep == 0).all()
+
+
+def _sink_graph(k, tail, others=0):
+    """0 -> k vertices -> one sink without out-edges, 3 of them also -> a path of
+    `tail` more levels; `others` more in-edges of the sink come from the path's end
+    (with them, the sink's level has far more in-edges than the level before has
+    out-edges).  The sink's level is not the deepest."""
+    mids = np.arange(1, k + 1)
+    sink, path = k + 1, np.arange(k + 2, k + 2 + tail)
+    far = np.arange(path[-1] + 1, path[-1] + 1 + others)
+    src = [np.zeros(k, int), mids, mids[:3], path[:-1], np.full(others, path[-1]), far]
+    dst = [mids, np.full(k, sink), np.full(3, path[0]), path[1:], far, np.full(others, sink)]
+    return int(path[-1]) + 1 + others, np.concatenate(src).astype(np.uint32), np.concatenate(dst).astype(np.uint32)
+
+
+@pytest.mark.parametrize("k, tail, others", [(1024, 2, 0), (1025, 1, 0), (1025, 3, 0), (5000, 2, 0), (3, 2, 1100), (40, 3, 5000)])
+def test_bc_hub_without_out_edges(native, oracle, k, tail, others):
+    """Sinks with many in-edges on a level that others follow, reached by a pulled
+    or a pushed level: through every entry point that takes one source at a time."""
+    import torch
+    import bfs_simd_benchmarks_gb300 as B
+    n, src, dst = _sink_graph(k, tail, others)
+    arr = oracle.arrays_from_edges(n, src, dst, 256, 4)
+    with B.Graph.from_edges(n, src, dst, 256, 4) as g:
+        g.set_options(bc_batch=0)
+        for mode in (1, 2):
+            g.set_options(bc_level_bytes=mode)
+            for s in (0, 1):
+                dep, _, _ = _check_source(oracle, arr, g, s)
+                total, _ = g.betweenness(np.array([s], np.uint32))
+                want = dep.copy()
+                want[s] = 0
+                np.testing.assert_array_equal(total, want)
+                acc = torch.zeros(n, dtype=torch.float32, device="cuda")
+                g.betweenness_device(np.array([s], np.uint32), acc.data_ptr(), torch.cuda.current_stream().cuda_stream)
+                torch.cuda.synchronize()
+                np.testing.assert_array_equal(acc.cpu().numpy(), want)
