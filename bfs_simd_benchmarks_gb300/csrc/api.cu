@@ -878,6 +878,7 @@ int run_impl(bfs_graph *g, uint32_t source, int32_t *levels, uint32_t *parents, 
 	p.to_dense_threshold = g->m / std::max<uint32_t>(1, g->opt.to_dense_ratio);
 	p.to_sparse_threshold = g->m / std::max<uint32_t>(1, g->opt.to_sparse_ratio);
 	p.wait_limit_ns = wait_limit_ns(g->opt);
+	p.solo_levels = solo_levels(p.wait_limit_ns);
 	p.hold_barrier = g->opt.test_hold_barrier;
 	p.switch_rule = g->opt.switch_rule;
 	p.alpha = g->opt.bu_alpha;
@@ -1132,6 +1133,7 @@ int run_batch_impl(bfs_graph *g, const uint32_t *sources, uint32_t ns, uint8_t *
 		p.to_dense_threshold = g->m / std::max<uint32_t>(1, g->opt.to_dense_ratio);
 		p.to_sparse_threshold = g->m / std::max<uint32_t>(1, g->opt.to_sparse_ratio);
 		p.wait_limit_ns = wait_limit_ns(g->opt);
+		p.solo_levels = solo_levels(p.wait_limit_ns);
 		p.hold_barrier = g->opt.test_hold_barrier;
 		p.switch_rule = g->opt.switch_rule;
 		p.alpha = g->opt.bu_alpha;
@@ -1276,6 +1278,7 @@ int bc_enqueue(bfs_graph *g, uint32_t source, uint32_t *sigma, float *delta, flo
 	p.to_dense_threshold = g->m / std::max<uint32_t>(1, g->opt.to_dense_ratio);
 	p.to_sparse_threshold = g->m / std::max<uint32_t>(1, g->opt.to_sparse_ratio);
 	p.wait_limit_ns = wait_limit_ns(g->opt);
+	p.solo_levels = solo_levels(p.wait_limit_ns);
 	p.hold_barrier = g->opt.test_hold_barrier;
 	p.switch_rule = g->opt.switch_rule;
 	p.alpha = g->opt.bu_alpha;

@@ -1341,7 +1341,7 @@ __device__ __forceinline__ uint32_t solo_cap(const DevGraph &g, unsigned long lo
 
 // Called by every thread of CTA 0: expands the frontier of `step` (queue
 // sizes tails[]) and the ones after it until one is too large, goes
-// bottom-up, is empty, or kSoloLevels steps are done; that one becomes the
+// bottom-up, is empty, or p.solo_levels steps are done; that one becomes the
 // round's output like any step's.
 __device__ __forceinline__ void phase_solo(const DevGraph &g, const RunCtx &r, const StepParams &p, uint32_t rnd,
 		uint32_t step, const uint32_t (&tails)[3], unsigned long long seen, uint32_t *smem, ThreadAcc &acc,
@@ -1386,7 +1386,7 @@ __device__ __forceinline__ void phase_solo(const DevGraph &g, const RunCtx &r, c
 		const uint32_t prev = ne;
 		nv = cn[0];
 		ne = cn[1];
-		if (nv == 0 || ne > solo_cap(g, prev, ne) || done == kSoloLevels ||
+		if (nv == 0 || ne > solo_cap(g, prev, ne) || done == p.solo_levels ||
 				goes_dense(g, p, nv, ne, seen + skipped + ne, false))
 			break;
 		skipped += ne;
@@ -1491,7 +1491,7 @@ __global__ void __launch_bounds__(kThreads, 2) k_bfs_persistent(DevGraph g, RunC
 				tails[2] = s_conv_tails[2];
 			}
 			CTA_STAMP(step, 3);
-			const uint32_t cap = solo_cap(g, prev_dsum, dsum);
+			const uint32_t cap = p.solo_levels ? solo_cap(g, prev_dsum, dsum) : 0u;
 			solo = fsize <= cap && dsum <= cap;
 			if (__builtin_expect(!solo, 1)) phase_expand(g, r, p, rnd, (int32_t) step + 1, tails[0], tails[1], tails[2], smem, acc,
 						dsum >= kScreenEdges && seen > g.m / 2);

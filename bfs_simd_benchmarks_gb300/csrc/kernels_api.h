@@ -22,6 +22,15 @@ constexpr uint32_t kTmaSliceWords = 4096;
 
 enum StepKind { kStepSeed = 0, kStepClear, kStepToDense, kStepToSparse, kStepExpand, kStepDense };
 
+// Top-down steps that one CTA takes in a row while the rest of the grid waits at
+// one barrier: at most kSoloLevels, and no more than fit a quarter of the wait
+// limit at kSoloStepNs, the longest seen (layers of 40 vertices, 1,600 edges a step:
+// 128 steps are 0.99 ms, and a limit of 0.5 ms ran out in a sound traversal).
+constexpr uint32_t kSoloLevels = 128, kSoloStepNs = 16000;
+inline uint32_t solo_levels(uint64_t wait_limit_ns) {
+	const uint64_t fit = wait_limit_ns / (4 * kSoloStepNs);
+	return fit < kSoloLevels ? (uint32_t) fit : kSoloLevels;
+}
 // The cooperative grid at full occupancy and the dynamic shared memory of a
 // traversal whose bottom-up steps are `bottom_up` (BFS_BU_*).
 int persistent_grid(const DevGraph &g, uint32_t batch, uint32_t bottom_up, int device, int num_sms, int *grid, size_t *smem);

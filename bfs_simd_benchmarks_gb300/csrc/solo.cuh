@@ -32,8 +32,6 @@ __device__ __forceinline__ bool goes_dense(const DevGraph &g, const StepParams &
 // the grid, and the five words per edge of two lists still fit the shared
 // memory that the grid's own top-down step uses.
 constexpr uint32_t kSoloCap = 2048;
-// Steps in one round: bounds the other CTAs' wait.
-constexpr uint32_t kSoloLevels = 128;
 constexpr uint32_t kSoloWords = 5 * kSoloCap;  // dynamic shared memory of its lists ...
 constexpr uint32_t kSoloVisWords = 8192;       // ... and of the visited bits of graphs of at most 2^18 vertices
 static_assert(kSoloCap <= 0x10000, "owners are 16-bit");

@@ -154,7 +154,8 @@ typedef struct bfs_options {
 	                              vertices (default), 1 = always, 2 = never; results are identical */
 	uint32_t wait_limit_us;    /* bound of every device-side wait of bfs_run / bfs_run_batch (grid barriers):
 	                              past it the kernel gives up, returns and the run reports BFS_ETIMEOUT
-	                              (0 = the default, 2 s) */
+	                              (0 = the default, 2 s); small graphs' one-cluster traversal has hardware
+	                              barriers among resident CTAs only, and no limit */
 	uint32_t test_hold_barrier; /* TESTS ONLY: k > 0 makes CTA 0 skip its arrival at the k-th grid barrier of
 	                              the next runs, so that the other CTAs' bounded waits run out (the failure
 	                              path of the wait limit, exercised without a GPU fault); 0 = off */

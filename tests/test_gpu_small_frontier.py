@@ -217,3 +217,21 @@ def test_grid_pull_queue_overflow(native, oracle):
             np.testing.assert_array_equal(lev, oracle.bfs_levels(arr, s))
             assert oracle.check_parents(arr, s, lev, par) == 0
             assert st["dense_steps"] > 0
+
+
+@pytest.mark.parametrize("wait_limit_us", [50, 200, 400])
+def test_rounds_of_one_cta_fit_the_wait_limit(native, oracle, wait_limit_us):
+    """300 top-down steps that one CTA takes (1,600 edges, some 8 us each) on a graph
+    of more than 2^18 vertices: the wait of the other CTAs, of up to 128 of them,
+    is not what runs out."""
+    import bfs_simd_benchmarks_gb300 as B
+    n, src, dst = _chain(300, 40, 300_000)
+    src, dst = np.asarray(src, np.uint32), np.asarray(dst, np.uint32)
+    with B.Graph.from_edges(n, src, dst, 1024, 16) as g:
+        g.set_options(to_dense_ratio=1, wait_limit_us=wait_limit_us)
+        arr = oracle.csr_arrays(n, src, dst)
+        for s in (0, 41):
+            lev, par, st = g.run(s)
+            assert st["status"] == 0 and st["dense_steps"] == 0 and st["grid_ctas"] > 16
+            np.testing.assert_array_equal(lev, oracle.bfs_levels(arr, s))
+            assert oracle.check_parents(arr, s, lev, par) == 0
