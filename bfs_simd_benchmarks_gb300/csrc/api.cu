@@ -229,8 +229,10 @@ int launch_to_host(const HostCopies &h, int num_sms, cudaStream_t st) {
 }
 // The address at which the device writes host memory p: pinned and mapped
 // memory's device address; ordinary memory's own where the device shares the
-// host's page tables (`shared_pages`, Grace); null where it has none.
+// host's page tables (`shared_pages`, Grace); null where it has none, and for
+// an address that 32-bit stores cannot go to (cudaMemcpy takes any).
 uint32_t *host_address(void *p, bool shared_pages) {
+	if ((uintptr_t) p % sizeof(uint32_t)) return nullptr;
 	cudaPointerAttributes at{};
 	if (cudaPointerGetAttributes(&at, p) != cudaSuccess) {
 		cudaGetLastError();

@@ -426,3 +426,33 @@ def test_device_build_lists_and_segments(native, oracle, name, where):
         for i, x in enumerate(sources):
             ref = oracle.bfs_levels(arr, x)
             np.testing.assert_array_equal(rows[i].cpu().numpy(), np.where(ref < 0, 255, ref).astype(np.uint8))
+
+
+@pytest.mark.parametrize("pinned", [False, True])
+@pytest.mark.parametrize("offset", [0, 1, 2, 3, 4, 8])
+def test_host_outputs_at_any_address(native, oracle, offset, pinned):
+    """Level and parent buffers that start anywhere: 32-bit and 16-byte aligned ones are
+    written by the device, the others are copied."""
+    import ctypes as C
+    import torch
+    import bfs_simd_benchmarks_gb300 as B
+    n = 3001
+    src, dst = B.gen_rmat(4096, 8 * 4096, seed=12, permute=True)
+    keep = (src < n) & (dst < n)
+    src, dst = src[keep], dst[keep]
+    arr = oracle.arrays_from_edges(n, src, dst, 256, 4)
+    s = int(B.pick_sources(arr["degrees"], 1, seed=2)[0])
+    ref = oracle.bfs_levels(arr, s)
+    size = 4 * n + 32  # the buffers themselves are on 16-byte boundaries
+    raw = [torch.full((size,), 7, dtype=torch.uint8, pin_memory=pinned) for _ in range(2)]
+    with B.Graph.from_edges(n, src, dst, 256, 4) as g:
+        at = [r.data_ptr() + offset for r in raw]
+        rc = native.bfs_run(g.handle, s, C.cast(at[0], C.POINTER(C.c_int32)), C.cast(at[1], C.POINTER(C.c_uint32)), None)
+    assert rc == 0
+    out = [r.numpy() for r in raw]
+    lev = np.frombuffer(out[0][offset:offset + 4 * n].tobytes(), np.int32)
+    par = np.frombuffer(out[1][offset:offset + 4 * n].tobytes(), np.uint32)
+    np.testing.assert_array_equal(lev, ref)
+    assert oracle.check_parents(arr, s, lev, par) == 0
+    for o in out:
+        assert (o[:offset] == 7).all() and (o[offset + 4 * n:] == 7).all()
