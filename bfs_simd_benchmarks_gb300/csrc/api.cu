@@ -426,9 +426,9 @@ int upload_big_in(bfs_graph *g, const std::vector<uint32_t> &in_off) {
 	for (uint32_t v = 0; v < g->n; ++v) {
 		if (in_off[v + 1] - in_off[v] <= kMsPullBig) continue;
 		in_big.push_back(v);
-		for (uint32_t b = in_off[v]; b < in_off[v + 1]; b += kMsChunk) {
+		for (uint64_t b = in_off[v]; b < in_off[v + 1]; b += kMsChunk) {
 			chunk_v.push_back(v);
-			chunk_beg.push_back(b);
+			chunk_beg.push_back((uint32_t) b);
 		}
 	}
 	g->ms_nbig_in = (uint32_t) in_big.size();
@@ -1415,9 +1415,9 @@ int bb_upload_chunks(bfs_graph *g, const uint32_t *d_off, uint32_t chunk, const 
 	std::vector<uint32_t> cv, cb;
 	for (uint32_t v = 0; v < g->n; ++v) {
 		if (off[v + 1] - off[v] <= chunk) continue;
-		for (uint32_t e = off[v]; e < off[v + 1]; e += chunk) {
+		for (uint64_t e = off[v]; e < off[v + 1]; e += chunk) {
 			cv.push_back(v);
-			cb.push_back(e);
+			cb.push_back((uint32_t) e);
 		}
 	}
 	*count = (uint32_t) cv.size();

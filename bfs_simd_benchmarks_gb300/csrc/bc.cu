@@ -240,13 +240,13 @@ __device__ __forceinline__ void big_chunk(const BcArgs &a, uint32_t bb, uint32_t
 	const uint32_t lo = chunk_owner(nbig, j), c0 = bsh.cpre[lo], c1 = bsh.cpre[lo + 1];
 	const uint32_t v = ld_cg(a.order + bb + lo);
 	const uint32_t vbeg = off[v], vend = off[v + 1];
-	const uint32_t beg = vbeg + (j - c0) * kBcWarpChunk, end = min(beg + kBcWarpChunk, vend);
+	const uint32_t beg = vbeg + (j - c0) * kBcWarpChunk, len = min(kBcWarpChunk, vend - beg);
 	T s = T(0);
-	for (uint32_t e = beg + lane_id(); e < end; e += 32 * kBcUnroll) {
+	for (uint32_t i = lane_id(); i < len; i += 32 * kBcUnroll) {
 		uint32_t nb[kBcUnroll];
 		uint2 lx[kBcUnroll];
 #pragma unroll
-		for (int k = 0; k < kBcUnroll; ++k) nb[k] = e + 32 * k < end ? __ldg(adj + e + 32 * k) : 0xFFFFFFFFu;
+		for (int k = 0; k < kBcUnroll; ++k) nb[k] = i + 32 * k < len ? __ldg(adj + beg + i + 32 * k) : 0xFFFFFFFFu;
 		gather_tags(a, nb, lx, use8, target);
 #pragma unroll
 		for (int k = 0; k < kBcUnroll; ++k)
@@ -404,13 +404,15 @@ __device__ __forceinline__ typename Dir<kFwd>::T lane_vertex_sum(const BcArgs &a
 	using T = typename Dir<kFwd>::T;
 	const uint32_t *adj = Dir<kFwd>::adj(a);
 	T s = T(0), lost = T(0);
-	for (uint32_t q = beg & ~3u; q < end; q += 4 * kBcQuads) {
+	const uint32_t from = beg & ~3u;
+	for (uint32_t i = 0; i < end - from; i += 4 * kBcQuads) {
+		const uint32_t q = from + i;
 		uint32_t nb[4 * kBcQuads];
 		uint2 lx[4 * kBcQuads];
 #pragma unroll
 		for (int k = 0; k < kBcQuads; ++k) {
 			const uint32_t e = q + 4 * k;
-			if (e >= end) {
+			if (i + 4 * k >= end - from) {
 				nb[4 * k] = nb[4 * k + 1] = nb[4 * k + 2] = nb[4 * k + 3] = 0xFFFFFFFFu;
 			} else if (a.m - e >= 4) {
 				const uint4 x = ldg_v4(adj + e);
@@ -457,13 +459,13 @@ __device__ __forceinline__ void push_paths(const BcArgs &a, uint32_t bb, uint32_
 		const uint32_t lo = chunk_owner(cnt, j);
 		const uint32_t u = ld_cg(a.order + bb + lo);
 		const uint32_t beg = a.row_off[u] + (j - bsh.cpre[lo]) * kBcPushChunk;
-		const uint32_t end = min(beg + kBcPushChunk, a.row_off[u + 1]);
+		const uint32_t len = min(kBcPushChunk, a.row_off[u + 1] - beg);
 		const uint32_t su = ld_cg(reinterpret_cast<const uint32_t *>(a.lvx + u) + 1);
-		if (lane == 0) *edges += end - beg;
-		for (uint32_t e = beg + lane; e < end; e += 32 * kBcUnroll) {
+		if (lane == 0) *edges += len;
+		for (uint32_t i = lane; i < len; i += 32 * kBcUnroll) {
 			uint32_t v[kBcUnroll], lv[kBcUnroll];
 #pragma unroll
-			for (int k = 0; k < kBcUnroll; ++k) v[k] = e + 32 * k < end ? __ldg(a.col + e + 32 * k) : 0xFFFFFFFFu;
+			for (int k = 0; k < kBcUnroll; ++k) v[k] = i + 32 * k < len ? __ldg(a.col + beg + i + 32 * k) : 0xFFFFFFFFu;
 #pragma unroll
 			for (int k = 0; k < kBcUnroll; ++k)
 				lv[k] = v[k] == 0xFFFFFFFFu ? 0xFFFFFFFEu

@@ -417,7 +417,7 @@ __device__ void bb_chunk(const BbArgs &a, uint32_t L, uint32_t w, bool has_nb, u
 	const uint32_t v = __ldg(D::chunk_v(a) + c), rw = w * a.n;
 	const uint64_t hv = bb_word(bb_plane(a, L, w), a, v);
 	const uint32_t beg = __ldg(cb + c), vbeg = __ldg(off + v), vend = __ldg(off + v + 1);
-	const uint32_t end = min(beg + a.chunk, vend);
+	const uint32_t end = run_end(beg, a.chunk, vend);
 	T acc[4] = {T(0), T(0), T(0), T(0)};
 	uint32_t u2 = has_nb && beg + lane < end ? __ldg(adj + beg + lane) : 0u;
 	for (uint32_t e0 = beg; has_nb && e0 < end; e0 += 32) {

@@ -968,15 +968,16 @@ __device__ __forceinline__ bool frontier_bit(const uint32_t *cur, uint32_t u) {
 	return (ld_phase(cur + (u >> 5)) >> (u & 31)) & 1u;
 }
 
-// A frontier source among the in-edges e, e + stride, ... (kPullDeep of them,
-// below end), or kUnvisitedWord.
+// A frontier source among the in-edges at, at + stride, ... (kPullDeep of them) of
+// the `left` ones from e on, or kUnvisitedWord.  (Counted from e: edge numbers go up
+// to 2^32 - 1.)
 constexpr int kPullDeep = 2;
 constexpr uint32_t kPullRounds = 16;
-__device__ __forceinline__ uint32_t pull_hit(const DevGraph &g, const uint32_t *cur, uint32_t e, uint32_t end,
+__device__ __forceinline__ uint32_t pull_hit(const DevGraph &g, const uint32_t *cur, uint32_t e, uint32_t at, uint32_t left,
 		uint32_t stride, uint32_t &edges) {
 	uint32_t u[kPullDeep], fw[kPullDeep], hit = kUnvisitedWord;
 #pragma unroll
-	for (int q = 0; q < kPullDeep; ++q) u[q] = e + stride * q < end ? __ldg(g.in_src + e + stride * q) : kUnvisitedWord;
+	for (int q = 0; q < kPullDeep; ++q) u[q] = at + stride * q < left ? __ldg(g.in_src + e + at + stride * q) : kUnvisitedWord;
 #pragma unroll
 	for (int q = 0; q < kPullDeep; ++q) fw[q] = u[q] != kUnvisitedWord ? ld_phase(cur + (u[q] >> 5)) : 0u;
 #pragma unroll
@@ -1050,7 +1051,7 @@ __device__ __forceinline__ void phase_pull(const DevGraph &g, const RunCtx &r, u
 			for (int q = 0; q < 4; ++q)
 #pragma unroll
 				for (uint32_t t = 0; t < kPullShort - 1; ++t)
-					x[q][t] = !found[q] && beg[q] + 1 + t < end[q] ? __ldg(g.in_src + beg[q] + 1 + t) : kUnvisitedWord;
+					x[q][t] = !found[q] && end[q] - beg[q] > 1 + t ? __ldg(g.in_src + beg[q] + 1 + t) : kUnvisitedWord;
 #pragma unroll
 			for (int q = 0; q < 4; ++q)
 #pragma unroll
@@ -1070,7 +1071,7 @@ __device__ __forceinline__ void phase_pull(const DevGraph &g, const RunCtx &r, u
 					if (pos < long_cap) {
 						longq[pos] = v0 + 32u * (j0 + q) + lane;
 						longq[long_cap + pos] = beg[q] + kPullShort;
-						longq[2 * long_cap + pos] = end[q];
+						longq[2 * long_cap + pos] = end[q] - beg[q] - kPullShort;
 					} else {
 						// queue full: finish the scan here
 						for (uint32_t e = beg[q] + kPullShort; e < end[q]; ++e) {
@@ -1094,10 +1095,10 @@ __device__ __forceinline__ void phase_pull(const DevGraph &g, const RunCtx &r, u
 		for (uint32_t x0 = wid * 8; x0 < nlong; x0 += kWarps * 8) {
 			const uint32_t x = x0 + lane / 4;
 			bool open = x < nlong;
-			const uint32_t v = open ? longq[x] : 0u, end = open ? longq[2 * long_cap + x] : 0u;
-			uint32_t e = open ? longq[long_cap + x] : 0u;
+			const uint32_t v = open ? longq[x] : 0u;
+			uint32_t e = open ? longq[long_cap + x] : 0u, left = open ? longq[2 * long_cap + x] : 0u;
 			for (uint32_t round = 0; round < kPullRounds && __any_sync(kFull, open); ++round) {
-				const uint32_t hit = pull_hit(g, cur, e + sub, open ? end : 0u, 4, edges);
+				const uint32_t hit = pull_hit(g, cur, e, sub, open ? left : 0u, 4, edges);
 				const uint32_t m = (__ballot_sync(kFull, hit != kUnvisitedWord) >> (lane & 28u)) & 0xFu;
 				if (m && sub == (unsigned) __ffs(m) - 1) {
 					if (parent) parent[v] = hit;
@@ -1105,13 +1106,15 @@ __device__ __forceinline__ void phase_pull(const DevGraph &g, const RunCtx &r, u
 					atomicOr(&vis_s[d >> 5], 1u << (d & 31));
 				}
 				e += 4 * kPullDeep;
-				open = open && !m && e < end;
+				left -= min(left, 4u * kPullDeep);
+				open = open && !m && left;
 			}
 			for (uint32_t om = __ballot_sync(kFull, open && sub == 0); om; om &= om - 1) {
 				const int src = __ffs(om) - 1;
-				const uint32_t ov = __shfl_sync(kFull, v, src), oend = __shfl_sync(kFull, end, src);
-				for (uint32_t oe = __shfl_sync(kFull, e, src); oe < oend; oe += 32 * kPullDeep) {
-					const uint32_t hit = pull_hit(g, cur, oe + lane, oend, 32, edges);
+				const uint32_t ov = __shfl_sync(kFull, v, src);
+				uint32_t oe = __shfl_sync(kFull, e, src);
+				for (uint32_t ol = __shfl_sync(kFull, left, src); ol; oe += 32 * kPullDeep, ol -= min(ol, 32u * kPullDeep)) {
+					const uint32_t hit = pull_hit(g, cur, oe, lane, ol, 32, edges);
 					const uint32_t m = __ballot_sync(kFull, hit != kUnvisitedWord);
 					if (!m) continue;
 					if (lane == (unsigned) __ffs(m) - 1) {

@@ -185,7 +185,9 @@ __device__ __forceinline__ void seg_item_count(const uint32_t *in_src, const Seg
 		uint32_t *s_cnt) {
 	for (uint32_t k = threadIdx.x; k < stripes; k += blockDim.x) s_cnt[k] = 0;
 	__syncthreads();
-	for (uint32_t e = it.beg + threadIdx.x; e < it.end; e += blockDim.x) atomicAdd(s_cnt + __ldg(in_src + e) / sw, 1u);
+	// (counted from the item's start: edge numbers go up to 2^32 - 1)
+	for (uint32_t i = threadIdx.x; i < it.end - it.beg; i += blockDim.x)
+		atomicAdd(s_cnt + __ldg(in_src + it.beg + i) / sw, 1u);
 	__syncthreads();
 }
 
@@ -213,9 +215,9 @@ __global__ void __launch_bounds__(kSegThreads) k_seg_pack(const uint32_t *in_off
 	const uint32_t c0 = group_col[it.group], vend = (uint32_t) min((uint64_t) group_col[it.group + 1] * sh.w, (uint64_t) n);
 	const uint32_t cshift = sh.vbits, ushift = sh.vbits + sh.cbits;
 	const unsigned lane = lane_id(), nw = blockDim.x / 32;
-	const uint32_t per = ((it.end - it.beg + nw - 1) / nw + 31) / 32 * 32;
-	const uint32_t lo = it.beg + min(it.end - it.beg, warp_id() * per), hi = min(it.end, lo + per);
-	if (lo >= hi) return;
+	const uint32_t len = it.end - it.beg, per = ((len + nw - 1) / nw + 31) / 32 * 32;
+	const uint32_t i0 = min(len, warp_id() * per), i1 = min(len, i0 + per), lo = it.beg + i0;
+	if (i0 >= i1) return;
 	// the last destination whose list starts at or before lo
 	uint32_t vb = c0 * sh.w, vh = vend;
 	while (vh - vb > 1) {
@@ -223,10 +225,11 @@ __global__ void __launch_bounds__(kSegThreads) k_seg_pack(const uint32_t *in_off
 		if (__ldg(in_off + mid) <= lo) vb = mid;
 		else vh = mid;
 	}
-	for (uint32_t e0 = lo; e0 < hi; e0 += 32) {
-		const uint32_t e = e0 + lane;
+	for (uint32_t i = i0; i < i1; i += 32) {
+		const bool mine = i + lane < i1;
+		const uint32_t e = it.beg + i + lane;
 		uint32_t v = 0;
-		bool have = e >= hi;
+		bool have = !mine;
 		for (;;) {  // 32 destinations at a time until every lane has its own
 			const uint32_t off = vb + lane + 1 <= vend ? __ldg(in_off + vb + lane + 1) : 0xFFFFFFFFu;  // ends of vb + lane
 			uint32_t o = 0;  // lists of the 32 that end at or before e
@@ -244,12 +247,12 @@ __global__ void __launch_bounds__(kSegThreads) k_seg_pack(const uint32_t *in_off
 			if (__all_sync(kFull, have)) break;
 			vb += 32;
 		}
-		if (e < hi) {
+		if (mine) {
 			const uint32_t u = __ldg(in_src + e), k = u / sw, c = v / sh.w;
 			words[atomicAdd(s_cnt + k, 1u)] = (v - c * sh.w) | ((c - c0) << cshift) | ((u - k * sw) << ushift);
 		}
 		// the next 32 edges start at or after this run's last destination
-		vb = __shfl_sync(kFull, v, 31 - __clz(__ballot_sync(kFull, e < hi)));
+		vb = __shfl_sync(kFull, v, 31 - __clz(__ballot_sync(kFull, mine)));
 	}
 }
 

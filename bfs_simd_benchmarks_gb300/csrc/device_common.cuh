@@ -40,6 +40,9 @@ template <class T> __device__ __forceinline__ T ld_phase(const T *p) {
 	else asm volatile("ld.global.ca.u64 %0, [%1];" : "=l"(reinterpret_cast<unsigned long long &>(x)) : "l"(p));
 	return x;
 }
+// The end of a run of at most `most` edges from `beg` in a list that ends at
+// `end`: edge numbers go up to 2^32 - 1, so beg + most may not be one.
+__device__ __forceinline__ uint32_t run_end(uint32_t beg, uint32_t most, uint32_t end) { return beg + min(most, end - beg); }
 __device__ __forceinline__ uint32_t ld_volatile(const uint32_t *p) { return *(const volatile uint32_t *) p; }
 __device__ __forceinline__ unsigned long long ld_volatile_u64(const unsigned long long *p) {
 	return *(const volatile unsigned long long *) p;

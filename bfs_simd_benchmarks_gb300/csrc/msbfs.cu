@@ -132,14 +132,14 @@ __device__ __forceinline__ void ms_push_edges(const MsArgs &a, const uint64_t *c
 	const uint32_t nz0 = (uint32_t) um, nz1 = (uint32_t) (um >> 32);
 	const uint64_t w0 = (nz0 >> lane) & 1u ? ld_cg64(cur + (size_t) u * K + lane) : 0ull;
 	const uint64_t w1 = (nz1 >> lane) & 1u ? ld_cg64(cur + (size_t) u * K + lane + 32) : 0ull;
-	for (uint32_t e0 = beg; e0 < end; e0 += 32 * kMsPushEdges) {
+	for (uint32_t i = 0; i < end - beg; i += 32 * kMsPushEdges) {
 		uint32_t v[kMsPushEdges];
 		bool ok[kMsPushEdges], fresh[kMsPushEdges];
 #pragma unroll
 		for (int j = 0; j < kMsPushEdges; ++j) {
-			const uint32_t e = e0 + 32 * j + lane;
-			ok[j] = e < end;
-			v[j] = ok[j] ? __ldg(a.col + e) : 0u;
+			const uint32_t e = i + 32 * j + lane;
+			ok[j] = e < end - beg;
+			v[j] = ok[j] ? __ldg(a.col + beg + e) : 0u;
 		}
 #pragma unroll
 		for (int j = 0; j < kMsPushEdges; ++j) fresh[j] = ok[j] && !ld_cg_u8(a.touched + v[j]);
@@ -205,9 +205,9 @@ __device__ void ms_push_chunk_list(const MsArgs &a, uint32_t lvl, uint32_t nb, u
 // levels of up to n / kMsMarkDiv edges take 0.02 to 0.06 ms this way.
 constexpr uint32_t kMsMarkDiv = 8;
 constexpr uint32_t kMsMarkBig = 64;  // high-degree frontier vertices, one after the other by the whole grid
-__device__ __forceinline__ void ms_mark_edges(const MsArgs &a, uint64_t *nxt, uint32_t e0, uint32_t end) {
+__device__ __forceinline__ void ms_mark_edges(const MsArgs &a, uint64_t *nxt, uint64_t e0, uint32_t end) {
 	const unsigned lane = lane_id();
-	const uint32_t e = e0 + lane;
+	const uint64_t e = e0 + lane;
 	const uint32_t v = e < end ? __ldg(a.col + e) : 0u;
 	bool mine = e < end && !ld_cg_u8(a.touched + v);
 	if (mine) {
@@ -225,11 +225,11 @@ __device__ void ms_push_mark(const MsArgs &a, uint32_t lvl, uint64_t *nxt, uint3
 	const uint32_t nwarps = gridDim.x * kMsWarps;
 	for (uint32_t i = gwarp; i < nq; i += nwarps) {
 		const uint32_t u = ld_cg(q + i), end = __ldg(a.row_off + u + 1);
-		for (uint32_t e = __ldg(a.row_off + u); e < end; e += 32) ms_mark_edges(a, nxt, e, end);
+		for (uint64_t e = __ldg(a.row_off + u); e < end; e += 32) ms_mark_edges(a, nxt, e, end);
 	}
 	for (uint32_t i = 0; i < nb; ++i) {
 		const uint32_t u = ld_cg(q + a.n - 1 - i), end = __ldg(a.row_off + u + 1);
-		for (uint32_t e = __ldg(a.row_off + u) + 32 * gwarp; e < end; e += 32 * nwarps) ms_mark_edges(a, nxt, e, end);
+		for (uint64_t e = (uint64_t) __ldg(a.row_off + u) + 32 * gwarp; e < end; e += 32 * nwarps) ms_mark_edges(a, nxt, e, end);
 	}
 }
 
@@ -246,7 +246,7 @@ __device__ void ms_push(const MsArgs &a, uint32_t lvl, const uint64_t *cur, cons
 	const uint32_t nc = ld_volatile(&a.ctl->push_chunks);
 	for (uint32_t c = gwarp; c < nc; c += nwarps) {
 		const uint32_t u = ld_cg(a.push_u + c), beg = ld_cg(a.push_beg + c);
-		const uint32_t end = min(beg + kMsPushChunk, __ldg(a.row_off + u + 1));
+		const uint32_t end = run_end(beg, kMsPushChunk, __ldg(a.row_off + u + 1));
 		ms_push_edges(a, cur, actc, nxt, u, beg, end);
 	}
 }
@@ -495,13 +495,14 @@ template <int KK> __device__ __forceinline__ void row_ld(const uint64_t *p, uint
 		for (int k = 0; k < KK; ++k) x[k] = ld_cg64(p + k);
 	}
 }
-// ORs the frontier rows of U in-neighbours, in_src[e + stride * t] below end, into acc.
+// ORs the frontier rows of U in-neighbours into acc: the at, at + stride, ... -th of
+// the `left` ones from in_src[e] on.
 template <int KK, int U>
-__device__ __forceinline__ uint32_t rows_or(const MsArgs &a, const uint64_t *cur, uint32_t e, uint32_t stride, uint32_t end,
-		uint64_t (&acc)[KK]) {
+__device__ __forceinline__ uint32_t rows_or(const MsArgs &a, const uint64_t *cur, uint32_t e, uint32_t at, uint32_t stride,
+		uint32_t left, uint64_t (&acc)[KK]) {
 	uint32_t u[U], read = 0;
 #pragma unroll
-	for (int t = 0; t < U; ++t) u[t] = e + stride * t < end ? __ldg(a.in_src + e + stride * t) : 0xFFFFFFFFu;
+	for (int t = 0; t < U; ++t) u[t] = at + stride * t < left ? __ldg(a.in_src + e + at + stride * t) : 0xFFFFFFFFu;
 	uint64_t x[U][KK];
 #pragma unroll
 	for (int t = 0; t < U; ++t) {
@@ -548,8 +549,8 @@ __device__ __forceinline__ void ms_pull_rows(const MsArgs &a, const MsPull &p, u
 	const bool open = needy && !row_complete(vis, acc, f);
 	uint32_t read = 0;
 	if (open && end - beg <= kLaneMaxDeg)
-		for (uint32_t e = beg; e < end && !row_complete(vis, acc, f); e += kRows)
-			read += rows_or<KK, kRows>(a, p.cur, e, 1, end, acc);
+		for (uint32_t i = 0; i < end - beg && !row_complete(vis, acc, f); i += kRows)
+			read += rows_or<KK, kRows>(a, p.cur, beg, i, 1, end - beg, acc);
 	__syncwarp();
 	for (uint32_t wm = __ballot_sync(kFull, open && end - beg > kLaneMaxDeg); wm;) {
 		int j = -1;
@@ -569,15 +570,16 @@ __device__ __forceinline__ void ms_pull_rows(const MsArgs &a, const MsPull &p, u
 			ga[k] = 0ull;
 		}
 		uint32_t e = __shfl_sync(kFull, beg, src);
-		const uint32_t ge = __shfl_sync(kFull, end, src);
+		uint32_t left = __shfl_sync(kFull, end, src) - e;
 		for (bool go = j >= 0; __any_sync(kFull, go);) {
-			if (go) read += rows_or<KK, 4>(a, p.cur, e + (lane & 7u), 8, ge, ga);
+			if (go) read += rows_or<KK, 4>(a, p.cur, e, lane & 7u, 8, left, ga);
 			e += 32;
+			left -= min(left, 32u);
 #pragma unroll
 			for (int k = 0; k < KK; ++k)
 #pragma unroll
 				for (int d = 4; d > 0; d >>= 1) ga[k] |= shfl_xor64(ga[k], d);
-			go = go && e < ge && !row_complete(gv, ga, f);
+			go = go && left && !row_complete(gv, ga, f);
 		}
 		// each destination's words from its group to its lane
 		const int from = 8 * (__popc(taken & lanemask_lt()) & 3);
@@ -642,9 +644,9 @@ __device__ __forceinline__ void ms_pull_runs(const MsArgs &a, const MsPull &p, u
 		uint64_t *bacc = a.big_acc + (size_t) rslot * KK;
 		if ((openm >> t) & 1u) {
 			uint32_t e = __shfl_sync(kFull, beg, t);
-			const uint32_t end = min(e + len * kMsChunk, rend);
-			for (bool go = true; go && e < end; e += 32 * kRows) {
-				read += rows_or<KK, kRows>(a, p.cur, e + lane, 32, end, acc);
+			uint32_t left = min(len * kMsChunk, rend - e);
+			for (bool go = true; go && left; e += 32 * kRows, left -= min(left, 32u * kRows)) {
+				read += rows_or<KK, kRows>(a, p.cur, e, lane, 32, left, acc);
 				__syncwarp();
 #pragma unroll
 				for (int k = 0; k < KK; ++k) acc[k] = warp_or64(acc[k]);
@@ -784,7 +786,7 @@ __device__ __forceinline__ void ms_pull_chunk(const MsArgs &a, const MsPull &p, 
 	const bool w0 = lane < K, w1 = lane + 32 < K;
 	const uint32_t v = __ldg(a.chunk_v + c), beg = __ldg(a.chunk_beg + c), slot = __ldg(a.chunk_slot + c);
 	const uint32_t vbeg = __ldg(a.in_off + v), vend = __ldg(a.in_off + v + 1);
-	const uint32_t end = min(beg + kMsChunk, vend);
+	const uint32_t end = run_end(beg, kMsChunk, vend);
 	const size_t row = (size_t) v * K;
 	uint32_t u = 0;
 	uint64_t um = 0;
