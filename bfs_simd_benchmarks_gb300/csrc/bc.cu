@@ -443,7 +443,10 @@ __device__ __forceinline__ typename Dir<kFwd>::T lane_vertex_sum(const BcArgs &a
 			s = t;
 		}
 	}
-	return s + lost;
+	if constexpr (kFwd) return s;
+	// an infinite sum (path counts wrap on street grids, and their reciprocals add up
+	// past the largest float) rounds nothing off: lost is NaN then
+	else return s + (isfinite(lost) ? lost : T(0));
 }
 
 // Path counts of level d pushed along the out-edges of the vertices of level

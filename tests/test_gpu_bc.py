@@ -254,3 +254,28 @@ def test_bc_hub_without_out_edges(native, oracle, k, tail, others):
                 g.betweenness_device(np.array([s], np.uint32), acc.data_ptr(), torch.cuda.current_stream().cuda_stream)
                 torch.cuda.synchronize()
                 np.testing.assert_array_equal(acc.cpu().numpy(), want)
+
+
+@pytest.mark.parametrize("width, height, both", [(200, 200, False), (150, 170, True), (60, 300, True)])
+def test_bc_sums_past_the_largest_float(native, oracle, width, height, both):
+    """Street grids: path counts wrap, and sums of their reciprocals become infinite, of
+    either sign, or NaN where both meet: at the same vertices as in the oracle."""
+    import bfs_simd_benchmarks_gb300 as B
+    y, x = np.divmod(np.arange(width * height), width)
+    src, dst = [], []
+    for dy, dx in ((0, 1), (1, 0)) + (((0, -1), (-1, 0)) if both else ()):
+        ok = (y + dy >= 0) & (y + dy < height) & (x + dx >= 0) & (x + dx < width)
+        src.append((y * width + x)[ok])
+        dst.append(((y + dy) * width + x + dx)[ok])
+    src, dst = np.concatenate(src).astype(np.uint32), np.concatenate(dst).astype(np.uint32)
+    n = width * height
+    arr = oracle.arrays_from_edges(n, src, dst, 256, 4)
+    osig, odep, _, _ = oracle.bc_single(arr, 0)
+    assert np.isposinf(odep).any() and np.isneginf(odep).any() and np.isnan(odep).any()
+    with B.Graph.from_edges(n, src, dst, 256, 4) as g:
+        for mode in (1, 2):
+            g.set_options(bc_level_bytes=mode)
+            dep, sig, _ = g.bc(0)
+            np.testing.assert_array_equal(sig, osig)
+            for kind in (np.isposinf, np.isneginf, np.isnan):
+                np.testing.assert_array_equal(kind(dep), kind(odep))
