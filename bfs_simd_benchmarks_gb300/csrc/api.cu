@@ -467,7 +467,11 @@ int alloc_run(bfs_graph *g) {
 	ar.add(&r.err, 1);
 	ar.add(&g->level_buf, g->n);
 	ar.add(&g->parent_buf, g->n);
+	uint32_t *blocks = nullptr, *nblocks = nullptr;
+	ar.add(&blocks, (d.nwords + kPullBlock - 1) / kPullBlock);
+	ar.add(&nblocks, 1);
 	if ((st = dev_alloc_all(g, ar))) return st;
+	if ((st = dbuild_pull_blocks(d.hasin, d.nwords, blocks, nblocks, 0))) return st;
 	// the persistent kernel expects its barrier and status words zero at launch
 	if (cudaMemset(r.bar, 0, 2 * sizeof(unsigned)) != cudaSuccess || cudaMemset(r.err, 0, sizeof(int)) != cudaSuccess)
 		return BFS_ECUDA;
@@ -483,6 +487,12 @@ int alloc_run(bfs_graph *g) {
 	for (uint32_t bu : {BFS_BU_PULL, BFS_BU_STREAM})
 		if ((st = persistent_grid(d, g->batch, bu, g->device, g->num_sms, &g->grid_max[bu], &g->smem_of[bu]))) return st;
 	g->cluster = cluster_ctas(d);
+	// the pull goes through the blocks with in-edges where that saves a quarter of
+	// them; elsewhere the list would only be a load before each block's
+	const uint32_t all = (d.nwords + kPullBlock - 1) / kPullBlock;
+	if (cudaMemcpy(&d.pull_nblocks, nblocks, sizeof(uint32_t), cudaMemcpyDeviceToHost) != cudaSuccess) return BFS_ECUDA;
+	if ((uint64_t) d.pull_nblocks * 4 <= (uint64_t) all * 3) d.pull_blocks = blocks;
+	else d.pull_nblocks = all;
 	apply_grid(g);
 	return BFS_OK;
 }

@@ -8,6 +8,8 @@ namespace bfsg {
 // Upper bound of the persistent grid: per-CTA partial sums are indexed by CTA.
 constexpr uint32_t kMaxGrid = 2048;
 
+constexpr uint32_t kPullBlock = 8;  // bitmap words (a sector of them)
+
 // The graph as it sits in HBM (all read-only during a traversal).
 struct DevGraph {
 	uint32_t n;            // vertices
@@ -25,6 +27,8 @@ struct DevGraph {
 	uint32_t bm_words;          // words of a frontier bitmap, padded to whole stripe slices
 	uint32_t tma;               // 1: the bottom-up step streams segments and slices with bulk copies
 	uint32_t tma_batch;         // frontier slices per bulk-copy stage
+	uint32_t pull_nblocks;      // blocks of kPullBlock bitmap words that a pull step goes through ...
+	const uint32_t *pull_blocks;  // ... [pull_nblocks], or null: all of them
 	uint32_t pull_long_cap;     // shared-memory queue of destinations needing a long in-edge scan
 	const uint32_t *row_off;    // [n+1] CSR row starts
 	const uint32_t *col;        // [m]   CSR destinations

@@ -580,19 +580,23 @@ __device__ __forceinline__ void dense_settle(uint32_t claims) {
 // and the "stripe has a frontier vertex" flags of the next step.  Counts them
 // and sums their out-degrees (for the direction switch) with coalesced reads
 // of the row offsets: a lane per vertex, four bitmap words per warp in flight.
-__device__ __forceinline__ void dense_group_publish(const DevGraph &g, const RunCtx &r, const DenseGroup &gr,
+// gw: words of vis_s; vertex_of(j): the first vertex of word j and its three
+// neighbours (j a multiple of 4).
+template <class VertexOf>
+__device__ __forceinline__ void dense_publish(const DevGraph &g, const RunCtx &r, uint32_t gw, VertexOf vertex_of,
 		const uint32_t *vis_s, const uint32_t *vis0_s, int32_t nl, uint32_t *nxt, uint8_t *sf_nxt, ThreadAcc &acc) {
 	const unsigned lane = lane_id();
-	const uint32_t v0 = (uint32_t) gr.v0, sw = g.sw;
-	for (uint32_t j0 = warp_id() * 4; j0 < gr.gw; j0 += kWarps * 4) {
+	const uint32_t sw = g.sw;
+	for (uint32_t j0 = warp_id() * 4; j0 < gw; j0 += kWarps * 4) {
+		const uint32_t v0 = vertex_of(j0);
 		uint32_t bits[4], deg[4];
 #pragma unroll
 		for (int q = 0; q < 4; ++q) {
 			const uint32_t j = j0 + q;
-			bits[q] = (j < gr.gw) ? (vis_s[j] & ~vis0_s[j]) : 0u;
+			bits[q] = (j < gw) ? (vis_s[j] & ~vis0_s[j]) : 0u;
 			deg[q] = 0;
 			if ((bits[q] >> lane) & 1u) {
-				const uint32_t v = v0 + 32u * j + lane;
+				const uint32_t v = v0 + 32u * q + lane;
 				deg[q] = __ldg(g.row_off + v + 1) - __ldg(g.row_off + v);
 				r.level[v] = nl;
 			}
@@ -601,7 +605,7 @@ __device__ __forceinline__ void dense_group_publish(const DevGraph &g, const Run
 		for (int q = 0; q < 4; ++q) {
 			acc.degsum += deg[q];
 			if (lane == 0 && bits[q]) {
-				const uint64_t vb = gr.v0 + 32ull * (j0 + q);
+				const uint64_t vb = v0 + 32ull * q;
 				acc.count += __popc(bits[q]);
 				or_bits_at(nxt, vb, bits[q]);
 				or_bits_at(r.vis, vb, bits[q]);
@@ -616,6 +620,12 @@ __device__ __forceinline__ void dense_group_publish(const DevGraph &g, const Run
 			}
 		}
 	}
+}
+
+__device__ __forceinline__ void dense_group_publish(const DevGraph &g, const RunCtx &r, const DenseGroup &gr,
+		const uint32_t *vis_s, const uint32_t *vis0_s, int32_t nl, uint32_t *nxt, uint8_t *sf_nxt, ThreadAcc &acc) {
+	const uint32_t v0 = (uint32_t) gr.v0;
+	dense_publish(g, r, gr.gw, [v0](uint32_t j) { return v0 + 32u * j; }, vis_s, vis0_s, nl, nxt, sf_nxt, acc);
 }
 
 // Lists the group's non-empty segments in the active stripes [kb, kb+kThreads)
@@ -904,7 +914,7 @@ __device__ __forceinline__ void phase_dense_tma(const DevGraph &g, const RunCtx 
 }
 
 // Bottom-up step as a pull over in-edge lists (the column's tiles sorted by
-// destination): a CTA owns a column group with its visited bits in shared
+// destination): a CTA owns some words of the visited bitmap, in shared
 // memory; every unvisited destination that has in-edges scans them in order
 // and stops at the first source in the frontier (Beamer's bottom-up; the
 // reference's dense step tests every edge of the active rows instead,
@@ -917,26 +927,46 @@ __device__ __forceinline__ void phase_dense_tma(const DevGraph &g, const RunCtx 
 // pull of a uniform graph of 2^20 vertices and 2^24 edges (now 100), 1.86 ms for
 // the Twitter shape's (now 0.9).
 constexpr uint32_t kPullShort = 3;
-// Work items of a pull step: ranges of the bitmap, as many for every CTA, of about
-// kPullWords words where there are more, handed out dynamically (the early exit
-// makes a range's cost depend on where its frontier sources are).  Quarters of the
+// Work items of a pull step: equal numbers of bitmap words for every CTA, about
+// kPullWords in an item where there are more, handed out dynamically (the early exit
+// makes an item's cost depend on where its frontier sources are).  Quarters of the
 // column groups, which are planned for another kernel, gave 1,104 items of 46
 // words on the Pokec shape, less than one pass of a CTA's warps each, and a last
 // wave that was half empty: a query 147 us, now 130; uniform, 2^20 vertices, 2^24
 // edges 195 -> 163; rmat, 2^22 vertices, 2^26 edges 287 -> 254.  Half as long from a
-// share of kPullManyWords words per CTA on: there, long ranges' destinations
+// share of kPullManyWords words per CTA on: there, long items' destinations
 // overflow the queue (Twitter shape, 4,282 words a CTA: 1.89 ms with 256 words and
 // with quarters, 1.94 with 384, 2.21 with 512; rmat, 2^24 vertices and 2^27 edges,
 // 1,725 words a CTA: 589, 572 and 564 us, 593 with quarters).  Emptying the queue
 // before it overflows cost more in barriers than the scans in place: 1.96.
+//
+// The words of an item are blocks of kPullBlock (a sector of the bitmaps), dealt to
+// the items in turn, so that every item has its share of each part of the ids: the
+// in-edges of many graphs belong to few of them.  Where they leave a quarter of the
+// blocks empty, the graph's list of the others is dealt (pull_blocks).  A CTA per range of the ids had most of the work on such graphs:
+// uniform, 2^14 vertices of 64 edges, the first ids of 2^22: 130 us (63 with parts of
+// column groups), now 54; 2^17 of 32 edges, the first of 2^23: 210 (137), now 90;
+// rmat, 2^24 vertices of 8 edges, by degree: 1,334 us, now 683, permuted 718 and 686;
+// Twitter shape, permuted: 1,680 and 1,619.  Blocks dealt without the list are
+// a few in each of many items, with the item's chain of round trips for them (rmat,
+// 2^20 of 16 edges, the first of 2^25: 480 us, with it 131).
 constexpr uint32_t kPullWords = 512, kPullManyWords = 2048, kPullMinWords = 32;
+constexpr uint32_t kPullCap = kPullWords * 3 / 2;  // words of an item, at most
+static_assert(kPullCap % kPullBlock == 0 && kPullMinWords <= kPullCap, "whole blocks");
+
+// An item: blocks item, item + items, ... of the graph's pull_blocks.
+struct PullItem {
+	uint32_t item, items, gw;  // gw: its words
+	const uint32_t *blk;       // [kPullCap / kPullBlock] its blocks (shared memory)
+	__device__ __forceinline__ uint32_t word_of(uint32_t j) const { return blk[j / kPullBlock] * kPullBlock + j % kPullBlock; }
+};
 
 // A CTA's next item of a pull step: its visited bits to vis_s and vis0_s, which
 // of its vertices have in-edges to hin_s, the unvisited of those to
 // dsh.unsettled.  A CTA's first item is its own index (no atomic: the whole grid
 // asking at once queued on one line); later items are counted from gridDim.x.
-__device__ __forceinline__ bool pull_begin(const DevGraph &g, const RunCtx &r, StepCounters *out, uint32_t per, bool first,
-		uint32_t *vis_s, uint32_t *vis0_s, uint32_t *hin_s, DenseGroup &gr) {
+__device__ __forceinline__ bool pull_begin(const DevGraph &g, const RunCtx &r, StepCounters *out, bool first,
+		uint32_t *vis_s, uint32_t *vis0_s, uint32_t *hin_s, uint32_t *blk_s, PullItem &it) {
 	__syncthreads();
 	if (threadIdx.x == 0) {
 		dsh.group = first ? blockIdx.x : gridDim.x + atomicAdd(&out->work, 1u);
@@ -944,15 +974,16 @@ __device__ __forceinline__ bool pull_begin(const DevGraph &g, const RunCtx &r, S
 		dsh.nlist = 0;
 	}
 	__syncthreads();
-	gr.gi = 0;
-	gr.v0 = 32ull * per * dsh.group;
-	if (gr.v0 >= g.n) return false;
-	gr.v1 = min(gr.v0 + 32u * per, (uint64_t) g.n);
-	gr.gw = (uint32_t) ((gr.v1 - gr.v0 + 31) / 32);
+	it.item = dsh.group;
+	if (it.item >= it.items) return false;
+	it.gw = (g.pull_nblocks - it.item + it.items - 1) / it.items * kPullBlock;
 	uint32_t uns = 0;
-	for (uint32_t j = threadIdx.x; j < gr.gw; j += kThreads) {
-		const uint32_t vb = bits_at(r.vis, gr.v0 + 32ull * j, gr.v1, kFull);
-		const uint32_t hb = bits_at(g.hasin, gr.v0 + 32ull * j, gr.v1, 0u);
+	for (uint32_t j = threadIdx.x; j < it.gw; j += kThreads) {
+		const uint32_t x = j / kPullBlock * it.items + it.item, blk = g.pull_blocks ? __ldg(g.pull_blocks + x) : x;
+		const uint32_t w = blk * kPullBlock + j % kPullBlock;
+		if (j % kPullBlock == 0) blk_s[j / kPullBlock] = blk;
+		const uint32_t vb = w < g.nwords ? ld_cg(r.vis + w) : kFull;
+		const uint32_t hb = w < g.nwords ? __ldg(g.hasin + w) : 0u;  // (no bits past the last vertex)
 		vis_s[j] = vb;
 		vis0_s[j] = vb;
 		hin_s[j] = hb;
@@ -994,43 +1025,47 @@ __device__ __forceinline__ void phase_pull(const DevGraph &g, const RunCtx &r, u
 	uint32_t *nxt = r.bm[step % 3];
 	StepCounters *out = r.ctr + step % 3;
 	const unsigned wid = warp_id(), lane = lane_id();
-	const uint32_t mgw = g.max_group_words + 1;
 	uint32_t *vis_s = smem;
-	uint32_t *vis0_s = vis_s + mgw;
-	uint32_t *hin_s = vis0_s + mgw;
-	uint32_t *longq = hin_s + mgw;
+	uint32_t *vis0_s = vis_s + kPullCap;
+	uint32_t *hin_s = vis0_s + kPullCap;
+	uint32_t *blk_s = hin_s + kPullCap;
+	uint32_t *longq = blk_s + kPullCap / kPullBlock;
 	const uint32_t long_cap = g.pull_long_cap;
 	uint32_t *parent = r.parent;
-	DenseGroup gr;
+	PullItem it;
 	unsigned long long cyc[4] = {0, 0, 0, 0};
 	long long t0 = clock64();
 	bool first = true;
-	const uint32_t nw = (g.n + 31) / 32, share = (nw + gridDim.x - 1) / gridDim.x;
-	const uint32_t words = share < kPullManyWords ? kPullWords : kPullWords / 2;
-	const uint32_t items = max((share + words / 2) / words, 1u);
-	const uint32_t per = min(max((share + items - 1) / items, kPullMinWords), g.max_group_words);
-	while (pull_begin(g, r, out, per, first, vis_s, vis0_s, hin_s, gr)) {
+	{
+		const uint32_t share = (g.pull_nblocks * kPullBlock + gridDim.x - 1) / gridDim.x;
+		const uint32_t words = share < kPullManyWords ? kPullWords : kPullWords / 2;
+		const uint32_t n = max((share + words / 2) / words, 1u);
+		const uint32_t per = (max((share + n - 1) / n, kPullMinWords) + kPullBlock - 1) / kPullBlock;  // blocks
+		it.items = (g.pull_nblocks + per - 1) / per;
+		it.blk = blk_s;
+	}
+	while (pull_begin(g, r, out, first, vis_s, vis0_s, hin_s, blk_s, it)) {
 		first = false;
 		{ long long t1 = clock64(); cyc[0] += t1 - t0; t0 = t1; }
 		if (dsh.unsettled == 0) continue;
 		if (threadIdx.x == 0) acc.bu_groups++;
-		const uint32_t v0 = (uint32_t) gr.v0;
 		uint32_t edges = 0, tested = 0;
 		// Pass 1: a warp takes four bitmap words (a lane per destination in
 		// each); the list offsets, the first in-edge and its frontier word of
 		// all four destinations are loaded stage by stage, so a lane waits for
 		// three round trips per four destinations, not per destination.
-		for (uint32_t j0 = wid * 4; j0 < gr.gw; j0 += kWarps * 4) {
+		for (uint32_t j0 = wid * 4; j0 < it.gw; j0 += kWarps * 4) {
+			const uint32_t v0 = it.word_of(j0) * 32 + lane;  // a block holds all four words
 			uint32_t todo_w[4], beg[4], end[4], u[4];
 			bool found[4];
 #pragma unroll
 			for (int q = 0; q < 4; ++q) {
 				const uint32_t j = j0 + q;
-				todo_w[q] = (j < gr.gw) ? (hin_s[j] & ~vis0_s[j]) : 0u;
+				todo_w[q] = hin_s[j] & ~vis0_s[j];
 				found[q] = false;
 				beg[q] = end[q] = 0;
 				if ((todo_w[q] >> lane) & 1u) {
-					const uint32_t v = v0 + 32u * j + lane;
+					const uint32_t v = v0 + 32u * q;
 					beg[q] = __ldg(g.in_off + v);
 					end[q] = __ldg(g.in_off + v + 1);
 				}
@@ -1069,7 +1104,7 @@ __device__ __forceinline__ void phase_pull(const DevGraph &g, const RunCtx &r, u
 					// the rest of a longer list: the queue
 					const uint32_t pos = atomicAdd(&dsh.nlist, 1u);
 					if (pos < long_cap) {
-						longq[pos] = v0 + 32u * (j0 + q) + lane;
+						longq[pos] = 32u * (j0 + q) + lane;
 						longq[long_cap + pos] = beg[q] + kPullShort;
 						longq[2 * long_cap + pos] = end[q] - beg[q] - kPullShort;
 					} else {
@@ -1081,7 +1116,7 @@ __device__ __forceinline__ void phase_pull(const DevGraph &g, const RunCtx &r, u
 						}
 					}
 				}
-				if (found[q] && parent) parent[v0 + 32u * (j0 + q) + lane] = u[q];
+				if (found[q] && parent) parent[v0 + 32u * q] = u[q];
 				const uint32_t fmask = __ballot_sync(kFull, found[q]);
 				if (lane == 0 && fmask) atomicOr(&vis_s[j0 + q], fmask);
 			}
@@ -1095,14 +1130,13 @@ __device__ __forceinline__ void phase_pull(const DevGraph &g, const RunCtx &r, u
 		for (uint32_t x0 = wid * 8; x0 < nlong; x0 += kWarps * 8) {
 			const uint32_t x = x0 + lane / 4;
 			bool open = x < nlong;
-			const uint32_t v = open ? longq[x] : 0u;
+			const uint32_t d = open ? longq[x] : 0u;  // its slot's bit
 			uint32_t e = open ? longq[long_cap + x] : 0u, left = open ? longq[2 * long_cap + x] : 0u;
 			for (uint32_t round = 0; round < kPullRounds && __any_sync(kFull, open); ++round) {
 				const uint32_t hit = pull_hit(g, cur, e, sub, open ? left : 0u, 4, edges);
 				const uint32_t m = (__ballot_sync(kFull, hit != kUnvisitedWord) >> (lane & 28u)) & 0xFu;
 				if (m && sub == (unsigned) __ffs(m) - 1) {
-					if (parent) parent[v] = hit;
-					const uint32_t d = v - v0;
+					if (parent) parent[it.word_of(d >> 5) * 32 + (d & 31)] = hit;
 					atomicOr(&vis_s[d >> 5], 1u << (d & 31));
 				}
 				e += 4 * kPullDeep;
@@ -1111,16 +1145,15 @@ __device__ __forceinline__ void phase_pull(const DevGraph &g, const RunCtx &r, u
 			}
 			for (uint32_t om = __ballot_sync(kFull, open && sub == 0); om; om &= om - 1) {
 				const int src = __ffs(om) - 1;
-				const uint32_t ov = __shfl_sync(kFull, v, src);
+				const uint32_t od = __shfl_sync(kFull, d, src);
 				uint32_t oe = __shfl_sync(kFull, e, src);
 				for (uint32_t ol = __shfl_sync(kFull, left, src); ol; oe += 32 * kPullDeep, ol -= min(ol, 32u * kPullDeep)) {
 					const uint32_t hit = pull_hit(g, cur, oe, lane, ol, 32, edges);
 					const uint32_t m = __ballot_sync(kFull, hit != kUnvisitedWord);
 					if (!m) continue;
 					if (lane == (unsigned) __ffs(m) - 1) {
-						if (parent) parent[ov] = hit;
-						const uint32_t d = ov - v0;
-						atomicOr(&vis_s[d >> 5], 1u << (d & 31));
+						if (parent) parent[it.word_of(od >> 5) * 32 + (od & 31)] = hit;
+						atomicOr(&vis_s[od >> 5], 1u << (od & 31));
 					}
 					break;
 				}
@@ -1130,7 +1163,8 @@ __device__ __forceinline__ void phase_pull(const DevGraph &g, const RunCtx &r, u
 		acc.bu_vertices += tested;
 		__syncthreads();
 		{ long long t1 = clock64(); cyc[2] += t1 - t0; t0 = t1; }
-		dense_group_publish(g, r, gr, vis_s, vis0_s, nl, nxt, nullptr, acc);  // the pull reads no stripe flags
+		// (the pull reads no stripe flags)
+		dense_publish(g, r, it.gw, [&it](uint32_t j) { return it.word_of(j) * 32; }, vis_s, vis0_s, nl, nxt, nullptr, acc);
 		{ long long t1 = clock64(); cyc[3] += t1 - t0; t0 = t1; }
 	}
 	if (threadIdx.x == 0)
@@ -1579,7 +1613,7 @@ size_t traversal_smem_bytes(const DevGraph &g, uint32_t batch, uint32_t bottom_u
 	size_t words = (size_t) 2 * (g.max_group_words + 1) + 3 * kThreads;
 	if (g.tma) words += (size_t) kTmaStages * (kTmaEdgeWords + (size_t) g.tma_batch * g.slice_words);
 	else words += (size_t) batch * g.slice_words;
-	const size_t pull = (size_t) 3 * (g.max_group_words + 1 + g.pull_long_cap);
+	const size_t pull = (size_t) 3 * (kPullCap + g.pull_long_cap) + kPullCap / kPullBlock;
 	const size_t expand = (size_t) kWarps * 3 * kWqCap + 3 * (size_t) kFlatChunk;
 	size_t need = bottom_up == BFS_BU_PULL || pull > words ? pull : words;
 	need = need > expand ? need : expand;

@@ -13,6 +13,7 @@
 #include <cstdint>
 
 #include "../../include/bfs_gb300.h"
+#include "bfs_device.cuh"
 #include "build_device.h"
 #include "device_common.cuh"
 
@@ -163,6 +164,30 @@ __global__ void k_big_lists(uint32_t n, const uint32_t *big_off, const uint32_t 
 		chunk_v[c] = lo;
 		chunk_beg[c] = in_off[lo] + (c - chunk_off[lo]) * chunk;
 	}
+}
+
+// The non-empty blocks of the has-in-edge bitmap (one CTA, 1024 blocks at a time).
+constexpr int kPbThreads = 1024;
+__global__ void __launch_bounds__(kPbThreads) k_pull_blocks(const uint32_t *hasin, uint32_t nwords, uint32_t *blocks,
+		uint32_t *count) {
+	__shared__ uint32_t s_cnt[2][kPbThreads / 32];
+	const uint32_t nb = (nwords + kPullBlock - 1) / kPullBlock;
+	uint32_t run = 0, turn = 0;
+	for (uint64_t b0 = 0; b0 < nb; b0 += kPbThreads, turn ^= 1u) {
+		const uint64_t w0 = (b0 + threadIdx.x) * kPullBlock;
+		uint32_t bits = 0;
+#pragma unroll
+		for (uint32_t q = 0; q < kPullBlock; ++q) bits |= w0 + q < nwords ? __ldg(hasin + w0 + q) : 0u;
+		const uint32_t m = __ballot_sync(kFull, bits);
+		if (lane_id() == 0) s_cnt[turn][warp_id()] = __popc(m);
+		__syncthreads();
+		const uint32_t c = s_cnt[turn][lane_id()];
+		const uint32_t incl = warp_incl_scan(c);
+		const uint32_t at = run + __shfl_sync(kFull, incl - c, warp_id()) + __popc(m & lanemask_lt());
+		if (bits) blocks[at] = (uint32_t) b0 + threadIdx.x;
+		run += __shfl_sync(kFull, incl, 31);
+	}
+	if (threadIdx.x == 0) *count = run;
 }
 
 // In-edges per tile column: the in-edge lists of a column are one range.
@@ -332,6 +357,12 @@ int dbuild_big_lists(uint32_t n, const uint32_t *big_off, const uint32_t *chunk_
 		cudaStream_t st) {
 	k_big_lists<<<grid_for(n, num_sms), kBThreads, 0, st>>>(n, big_off, chunk_off, in_off, nchunks, chunk, in_big, chunk_v,
 			chunk_beg);
+	return cudaGetLastError() == cudaSuccess ? BFS_OK : BFS_ECUDA;
+}
+
+int dbuild_pull_blocks(const uint32_t *hasin, uint32_t nwords, uint32_t *blocks, uint32_t *count, cudaStream_t st) {
+	static_assert(kPbThreads == 32 * 32, "a count per lane");
+	k_pull_blocks<<<1, kPbThreads, 0, st>>>(hasin, nwords, blocks, count);
 	return cudaGetLastError() == cudaSuccess ? BFS_OK : BFS_ECUDA;
 }
 

@@ -34,6 +34,9 @@ int dbuild_vertex_facts(const uint32_t *out_deg, const uint32_t *in_deg, uint32_
 int dbuild_big_lists(uint32_t n, const uint32_t *big_off, const uint32_t *chunk_off, const uint32_t *in_off,
 		uint32_t nchunks, uint32_t chunk, uint32_t *in_big, uint32_t *chunk_v, uint32_t *chunk_beg, int num_sms,
 		cudaStream_t st);
+// The blocks of kPullBlock words of the has-in-edge bitmap that have a bit, in
+// order, and their number (one CTA).
+int dbuild_pull_blocks(const uint32_t *hasin, uint32_t nwords, uint32_t *blocks, uint32_t *count, cudaStream_t st);
 // in-edges per tile column
 int dbuild_col_edges(const uint32_t *in_off, uint32_t n, uint32_t w, uint32_t side, uint32_t *col_edges, cudaStream_t st);
 

@@ -235,3 +235,52 @@ def test_rounds_of_one_cta_fit_the_wait_limit(native, oracle, wait_limit_us):
             assert st["status"] == 0 and st["dense_steps"] == 0 and st["grid_ctas"] > 16
             np.testing.assert_array_equal(lev, oracle.bfs_levels(arr, s))
             assert oracle.check_parents(arr, s, lev, par) == 0
+
+
+@pytest.mark.parametrize("n, used", [
+    (1 << 22, np.arange(1 << 14)),                      # the first ids
+    ((1 << 20) + 77, np.arange((1 << 20) - 20_000, (1 << 20) + 77)),  # the last ones, the last block cut off
+    (300_000, np.arange(100_001, 120_000)),
+    (300_000, np.arange(0, 300_000, 300)),              # one in a block or none
+    (300_000, np.arange(0, 300_000, 256)),              # one in every block
+    (300_000, np.concatenate([np.arange(150_000), np.arange(200_000, 276_000)])),  # about three quarters of the blocks
+    (100_000, np.array([99_999, 5])),
+])
+def test_grid_pull_of_sparse_ids(native, oracle, tmp_path, n, used):
+    """Graphs whose edges are among some of the ids: the grid's bottom-up steps go through
+    the blocks of the bitmap that have in-edges, and share them out."""
+    import bfs_simd_benchmarks_gb300 as B
+    rng = np.random.default_rng(n + used.size)
+    src, dst = rng.choice(used, 12 * used.size).astype(np.uint32), rng.choice(used, 12 * used.size).astype(np.uint32)
+    arr = oracle.csr_arrays(n, src, dst)
+    path = str(tmp_path / "g.bin")
+    s = int(src[0])
+    ref = oracle.bfs_levels(arr, s)
+    for how in ("host", "device", "degree order", "file"):
+        if how == "file":
+            g = B.Graph.load_binary(path)
+        else:
+            g = B.Graph.from_edges(n, src, dst, 1024, 16, device_build=how != "host", degree_order=how == "degree order")
+            if how == "host":
+                g.save(path)
+        with g:
+            for opts in ({}, {"to_dense_ratio": 1 << 30, "to_sparse_ratio": 1 << 30}, {"ctas_per_sm": 1},
+                         {"mode": "stepwise"}):
+                g.set_options(**{"to_dense_ratio": 20, "to_sparse_ratio": 20, "ctas_per_sm": 2, "mode": "persistent", **opts})
+                lev, par, st = g.run(s)
+                np.testing.assert_array_equal(lev, ref)
+                assert oracle.check_parents(arr, s, lev, par) == 0
+                assert st["reached"] == int((ref >= 0).sum())
+                if "to_dense_ratio" in opts and used.size == 1 << 14:
+                    # 512 words with in-edges, by 16 CTAs or more as long as most are unvisited
+                    assert st["bu_groups"] >= 16
+
+
+def test_grid_pull_without_in_edges(native):
+    """No edges at all, and every step bottom-up: no block to go through."""
+    import bfs_simd_benchmarks_gb300 as B
+    none = np.zeros(0, np.uint32)
+    with B.Graph.from_edges(70_000, none, none, 1024, 16) as g:
+        g.set_options(ctas_per_sm=1, to_dense_ratio=1 << 30, to_sparse_ratio=1 << 30)
+        lev, _, st = g.run(69_999)
+        assert st["status"] == 0 and st["reached"] == 1 and lev[69_999] == 0 and (lev[:-1] == -1).all()
