@@ -948,8 +948,12 @@ int collect_stats(bfs_graph *g, bfs_stats *out) {
 			if (d.t_conv[i] >= t0 && d.t_conv[i] <= t1 && d.t_conv[i]) conv = (d.t_conv[i] - t0) * 1e-6;
 			s.step_ms[i] = (float) total;
 			const unsigned long long wmax = d.t_work_max[i], wmin = ~d.t_work_min_inv[i];
-			if (d.t_work_max[i] >= t0) s.step_work_max_ms[i] = (float) ((wmax - t0) * 1e-6);
-			if (d.t_work_min_inv[i] && wmin >= t0) s.step_work_min_ms[i] = (float) ((wmin - t0) * 1e-6);
+			if (!d.t_work_max[i]) {  // a step that one CTA took by itself, or one cluster
+				s.step_work_min_ms[i] = s.step_work_max_ms[i] = (float) total;
+			} else {
+				if (d.t_work_max[i] >= t0) s.step_work_max_ms[i] = (float) ((wmax - t0) * 1e-6);
+				if (d.t_work_min_inv[i] && wmin >= t0) s.step_work_min_ms[i] = (float) ((wmin - t0) * 1e-6);
+			}
 			if (s.trace[i]) { s.dense_ms += total - conv; s.to_dense_ms += conv; }
 			else { s.sparse_ms += total - conv; s.to_sparse_ms += conv; }
 		}
@@ -960,6 +964,7 @@ int collect_stats(bfs_graph *g, bfs_stats *out) {
 	s.bu_words = d.bu_words;
 	s.bu_slices = d.bu_slices;
 	s.bu_groups = d.bu_groups;
+	if (g->cluster_last) s.bu_groups = (uint64_t) d.dense_steps * std::min((uint32_t) g->cluster, g->dg.nwords);
 	s.bu_vertices = d.bu_vertices;
 	s.status = g->stepwise_last ? BFS_OK : d.status;
 	s.max_level = s.num_steps ? s.num_steps - 1 : 0;
@@ -1158,7 +1163,7 @@ int run_batch_impl(bfs_graph *g, const uint32_t *sources, uint32_t ns, uint8_t *
 		if (cudaGetLastError() != cudaSuccess) return BFS_ECUDA;
 		if (cudaEventRecord(b.em, st) != cudaSuccess) return BFS_ECUDA;
 		if (between && cudaEventRecord(between, st) != cudaSuccess) return BFS_ECUDA;
-		b.grid = g->grid;
+		b.grid = in_cluster(g) ? g->cluster : g->grid;
 		// the single-source statistics now describe the last of these runs
 		g->have_run = false;
 	} else if (dev_sources) {

@@ -202,12 +202,13 @@ typedef struct bfs_stats {
 	uint64_t td_vertices;      /* frontier vertices expanded top-down */
 	uint64_t bu_words;         /* bottom-up: packed tile words streamed (STREAM) or in-edges read (PULL) */
 	uint64_t bu_slices;        /* frontier slices staged by bottom-up steps */
-	uint64_t bu_groups;        /* column groups visited by bottom-up steps */
+	uint64_t bu_groups;        /* work items of bottom-up steps with an unvisited vertex: column groups
+	                              (STREAM), shares of the bitmap (PULL; in one cluster, a CTA's) */
 	uint64_t bu_vertices;      /* destinations tested by PULL bottom-up steps */
 	double device_ms;          /* device time of the traversal, initialisation included (CUDA events) */
 	double kernel_ms;          /* device time of the traversal kernel(s) alone */
 	int32_t status;            /* device-side status of the run (BFS_OK or BFS_ETIMEOUT) */
-	uint32_t grid_ctas;        /* CTAs of the persistent launch */
+	uint32_t grid_ctas;        /* CTAs of the traversal's launch */
 	uint8_t trace[BFS_TRACE_MAX]; /* trace[i] = 1 if step i was dense (first BFS_TRACE_MAX steps) */
 	/* Phase timers, the counterpart of the reference's dense_time, to_dense_time,
 	 * sparse_time and to_sparse_time (apps/bfs_simd/bfs.cpp:733-751), taken on the
@@ -215,11 +216,16 @@ typedef struct bfs_stats {
 	double dense_ms, to_dense_ms, sparse_ms, to_sparse_ms;
 	float step_ms[BFS_TRACE_MAX]; /* duration of each step, conversion included */
 	/* from the start of each step to the first / the last CTA done with the
-	 * step's work (the rest of step_ms is the grid barrier and the totals) */
+	 * step's work (the rest of step_ms is the barrier and the totals); step_ms for a
+	 * step that one CTA took by itself, and in the one-cluster traversal of small
+	 * graphs, whose CTAs take no times (stamps made its steps 1% longer; with
+	 * ctas_per_sm set, the whole grid runs) */
 	float step_work_min_ms[BFS_TRACE_MAX];
 	float step_work_max_ms[BFS_TRACE_MAX];
 	/* Bottom-up step profile: SM cycles summed over CTAs spent in group setup,
-	 * segment lists, consumer wait, consumer work, producer wait and publish. */
+	 * segment lists, consumer wait, consumer work, producer wait and publish
+	 * (STREAM); in setup, first in-edges, longer lists and output (PULL; 0 in the
+	 * one-cluster traversal). */
 	uint64_t bu_cycles[8];
 } bfs_stats;
 

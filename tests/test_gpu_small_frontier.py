@@ -284,3 +284,34 @@ def test_grid_pull_without_in_edges(native):
         g.set_options(ctas_per_sm=1, to_dense_ratio=1 << 30, to_sparse_ratio=1 << 30)
         lev, _, st = g.run(69_999)
         assert st["status"] == 0 and st["reached"] == 1 and lev[69_999] == 0 and (lev[:-1] == -1).all()
+
+
+@pytest.mark.parametrize("where", ["cluster", "one CTA", "grid"])
+def test_step_statistics(native, where):
+    """Every step has its time and the first and last CTA's, the bottom-up steps their
+    items, in each form of the traversal; a batch that runs as single traversals names
+    their CTAs."""
+    import torch
+    import bfs_simd_benchmarks_gb300 as B
+    n = 1 << (14 if where == "cluster" else 18)
+    src, dst = B.gen_rmat(n, 16 * n, seed=9, permute=True)
+    if where == "one CTA":
+        n, src, dst = _chain(200, 3, 1 << 17)
+        src, dst = np.asarray(src, np.uint32), np.asarray(dst, np.uint32)
+    s = int(src[0])
+    with B.Graph.from_edges(n, src, dst, 256, 4) as g:
+        if where == "one CTA":
+            g.set_options(to_dense_ratio=1)
+        _, _, st = g.run(s)
+        k = min(st["num_steps"], 256)
+        step, lo, hi = (np.array(st[x][:k]) for x in ("step_ms", "step_work_min_ms", "step_work_max_ms"))
+        assert (step > 0).all() and (lo > 0).all() and (lo <= hi).all() and (hi <= step).all()
+        if where == "one CTA":
+            assert (lo == step).sum() > k // 2
+            return
+        assert (st["grid_ctas"] <= 16) == (where == "cluster")
+        assert st["dense_steps"] > 0 and st["bu_groups"] >= st["dense_steps"]
+        g.set_options(batch_single_max=4)
+        out = torch.empty((2, n), dtype=torch.uint8, device="cuda")
+        b = g.run_batch_device(np.array([s, s], np.uint32), out.data_ptr(), torch.cuda.current_stream().cuda_stream, stats=True)
+        assert b["single_source_runs"] == 2 and b["grid_ctas"] == st["grid_ctas"]
