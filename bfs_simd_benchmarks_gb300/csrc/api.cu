@@ -999,6 +999,14 @@ uint32_t batch_planes_wanted(const bfs_graph *g, uint32_t K) {
 	return (uint32_t) std::max<size_t>(2, std::min<size_t>(kBatchDefaultPlanes, budget / std::max<size_t>(plane, 1)));
 }
 
+// Bytes of a level plane of K words per vertex (rows and word masks), and of what
+// a batch has besides.
+size_t batch_plane_bytes(const bfs_graph *g, uint32_t K) { return (size_t) g->n * K * 8 + (size_t) g->n * 8; }
+size_t batch_fixed_bytes(const bfs_graph *g, uint32_t K) {
+	return (size_t) g->n * K * 8 + (size_t) g->n * (2 + 4 + 8) + sizeof(MsControl) + 4 * BFS_BATCH_MAX_SOURCES +
+			4 * (size_t) g->ms_nchunks + (size_t) g->ms_nbig_in * (4 + 8 * (size_t) K);
+}
+
 // Makes the batch buffers hold K words per vertex and enough level planes;
 // returns the planes the call will use.  Buffers that hold at least K words
 // are reused; with the planes sized from the budget any plane count will do
@@ -1006,7 +1014,7 @@ uint32_t batch_planes_wanted(const bfs_graph *g, uint32_t K) {
 // fit.
 int batch_prepare(bfs_graph *g, uint32_t K, uint32_t *planes_out) {
 	auto &b = g->mb;
-	const size_t plane = (size_t) g->n * K * 8 + (size_t) g->n * 8;  // rows + word masks
+	const size_t plane = batch_plane_bytes(g, K);
 	uint32_t planes = batch_planes_wanted(g, K);
 	if (!b.h_ctl) {
 		if (cudaMallocHost(&b.h_ctl, sizeof(MsControl)) != cudaSuccess) return BFS_ENOMEM;
@@ -1022,8 +1030,7 @@ int batch_prepare(bfs_graph *g, uint32_t K, uint32_t *planes_out) {
 	// (re)allocate: wait for earlier batches that still use the buffers
 	if (b.have_run && cudaEventSynchronize(b.e1) != cudaSuccess) return BFS_ECUDA;
 	release_batch(g);
-	const size_t fixed = (size_t) g->n * K * 8 + (size_t) g->n * (2 + 4 + 8) + sizeof(MsControl) +
-			4 * BFS_BATCH_MAX_SOURCES + 4 * (size_t) g->ms_nchunks + (size_t) g->ms_nbig_in * (4 + 8 * (size_t) K);
+	const size_t fixed = batch_fixed_bytes(g, K);
 	size_t free_b = 0, total_b = 0;
 	if (cudaMemGetInfo(&free_b, &total_b) != cudaSuccess) return BFS_ECUDA;
 	const size_t usable = free_b > (size_t) 1 << 30 ? free_b - ((size_t) 1 << 30) : 0;  // leave 1 GiB
@@ -1440,6 +1447,33 @@ int bb_upload_chunks(bfs_graph *g, const uint32_t *d_off, uint32_t chunk, const 
 	return rc ? rc : dev_upload(g, chunk_beg, cb);
 }
 
+// Bytes of the betweenness state of `words` words of sources, and of its work
+// lists for `planes` levels.
+size_t bb_state_bytes(const bfs_graph *g, uint32_t words, uint32_t planes) {
+	const size_t rows = (size_t) words * g->n * kBbMaxSources, part = (size_t) words * std::max(g->bb_nich, g->bb_noch);
+	const size_t lists = (size_t) words * planes * ((g->n + 31) / 32 + (size_t) g->bb_nich + g->bb_noch);
+	return 8 * rows + 4 * part * (kBbMaxSources + 1) + 4 * lists;
+}
+
+// Of the `want` words of sources that one launch would take (all of the call's),
+// how many do: all where their state fits beside the level planes that the
+// traversal of these words wants, so that it gets no fewer; else one.
+uint32_t bb_words_that_fit(const bfs_graph *g, uint32_t want) {
+	const auto &b = g->bb;
+	if (want <= 1 || b.state_words >= want) return want;
+	size_t free_b = 0, total_b = 0;
+	if (cudaMemGetInfo(&free_b, &total_b) != cudaSuccess) return 1;
+	for (const auto &x : b.bufs) free_b += x.bytes;
+	for (const auto &x : b.lbufs) free_b += x.bytes;
+	const uint32_t planes = std::max(batch_planes_wanted(g, want), g->mb.planes_alloc);
+	size_t need = bb_state_bytes(g, want, planes) + ((size_t) 1 << 30);
+	if (g->mb.k_alloc < want) {
+		need += batch_fixed_bytes(g, want) + (size_t) planes * batch_plane_bytes(g, want);
+		free_b += g->mb.bytes;
+	}
+	return need <= free_b ? want : 1;
+}
+
 // Edge chunks (once per graph), the per-(vertex, source) state, and
 // (host_out) the [256][n] staging of host outputs.
 int bb_prepare(bfs_graph *g, uint32_t num_sources, bool host_deps, bool host_paths) {
@@ -1457,19 +1491,22 @@ int bb_prepare(bfs_graph *g, uint32_t num_sources, bool host_deps, bool host_pat
 		g->bb_chunks_ready = true;
 	}
 	auto &b = g->bb;
-	const uint32_t words = bb_launch_words(g, num_sources);
+	uint32_t words = bb_words_that_fit(g, bb_launch_words(g, num_sources));
 	if (b.ctl && b.state_words < words) release_bb(g);  // its cudaFree waits for earlier calls
 	if (!b.ctl) {
-		const size_t rows = (size_t) words * g->n * kBbMaxSources;
-		const size_t part = (size_t) words * std::max(g->bb_nich, g->bb_noch);
-		b.state_words = words;
-		if ((rc = bb_alloc(g, &b.sigma, rows)) || (rc = bb_alloc(g, &b.dsum, rows)) ||
-				(rc = bb_alloc(g, &b.partial, part * kBbMaxSources)) || (rc = bb_alloc(g, &b.chunks_done, part)) ||
-				(rc = bb_alloc(g, &b.ctl, kBbMaxWords)) ||
-				(rc = bb_alloc(g, &b.d_sources, kBbMaxWords * kBbMaxSources))) {
+		for (;;) {
+			const size_t rows = (size_t) words * g->n * kBbMaxSources;
+			const size_t part = (size_t) words * std::max(g->bb_nich, g->bb_noch);
+			if (!((rc = bb_alloc(g, &b.sigma, rows)) || (rc = bb_alloc(g, &b.dsum, rows)) ||
+						(rc = bb_alloc(g, &b.partial, part * kBbMaxSources)) || (rc = bb_alloc(g, &b.chunks_done, part)) ||
+						(rc = bb_alloc(g, &b.ctl, kBbMaxWords)) ||
+						(rc = bb_alloc(g, &b.d_sources, kBbMaxWords * kBbMaxSources))))
+				break;
 			release_bb(g);
-			return rc;
+			if (words == 1) return rc;
+			words = 1;
 		}
+		b.state_words = words;
 		if (cudaMallocHost(&b.h_ctl, sizeof(BbControl) * kBbMaxWords) != cudaSuccess ||
 				cudaMallocHost(&b.h_ms, sizeof(MsControl)) != cudaSuccess || cudaEventCreate(&b.e0) != cudaSuccess ||
 				cudaEventCreate(&b.e1) != cudaSuccess || cudaEventCreate(&b.e2) != cudaSuccess ||
@@ -1485,7 +1522,7 @@ int bb_prepare(bfs_graph *g, uint32_t num_sources, bool host_deps, bool host_pat
 	return BFS_OK;
 }
 
-// Enqueues the batched traversal from `sources` (host, ns <= 64) with its
+// Enqueues the batched traversal from `sources` (host, ns <= 256) with its
 // planes kept, then the path-count / dependency launch and the output pass
 // into delta / paths ([ns][n], device, either may be null) and acc.
 int bb_enqueue(bfs_graph *g, const uint32_t *sources, uint32_t ns, float *delta, uint32_t *paths, float *acc,
@@ -1496,7 +1533,7 @@ int bb_enqueue(bfs_graph *g, const uint32_t *sources, uint32_t ns, float *delta,
 	int rc = batch_prepare(g, K, &planes);
 	if (rc) return rc;
 	auto &b = g->bb;
-	if (b.list_planes < planes) {
+	while (b.list_planes < planes) {
 		// per-level work lists for this many levels (the old ones may still be in use)
 		if (cudaStreamSynchronize(st) != cudaSuccess) return BFS_ECUDA;
 		for (auto &x : b.lbufs) cudaFree(x.p);
@@ -1505,17 +1542,21 @@ int bb_enqueue(bfs_graph *g, const uint32_t *sources, uint32_t ns, float *delta,
 		const size_t nblk = (g->n + 31) / 32, levels = (size_t) planes * b.state_words;
 		const size_t sizes[3] = {levels * nblk, levels * g->bb_nich, levels * g->bb_noch};
 		uint32_t **dst[3] = {&b.blist, &b.ilist, &b.olist};
-		for (int i = 0; i < 3; ++i) {
+		int i = 0;
+		for (; i < 3; ++i) {
 			void *p = nullptr;
 			const size_t bytes = std::max<size_t>(sizeof(uint32_t) * sizes[i], 16);
-			if (cudaMalloc(&p, bytes) != cudaSuccess) {
-				cudaGetLastError();
-				return BFS_ENOMEM;
-			}
+			if (cudaMalloc(&p, bytes) != cudaSuccess) break;
 			b.lbufs.push_back({p, bytes});
 			*dst[i] = (uint32_t *) p;
 		}
-		b.list_planes = planes;
+		if (i == 3) {
+			b.list_planes = planes;
+		} else {
+			cudaGetLastError();
+			if (b.state_words == 1) return BFS_ENOMEM;
+			b.state_words = 1;  // a word at a time
+		}
 	}
 	const MsArgs a = batch_args(g, K, ns, planes);
 	if (cudaEventRecord(b.e0, st) != cudaSuccess) return BFS_ECUDA;
@@ -1554,7 +1595,7 @@ int bb_enqueue(bfs_graph *g, const uint32_t *sources, uint32_t ns, float *delta,
 	x.ctas_per_sm = g->opt.ctas_per_sm;
 	// the words of 64 sources, in launches (and output passes) of up to
 	// bb_launch_words, in source order, so that acc receives the sources in order
-	const uint32_t fused = bb_launch_words(g, ns);
+	const uint32_t fused = std::min(bb_launch_words(g, ns), b.state_words);
 	for (uint32_t w = 0; w < K; w += fused) {
 		x.word = w;
 		x.words = std::min(fused, K - w);

@@ -269,3 +269,49 @@ def test_bc_batch_chunk_length_by_edges(native, oracle, m):
         dep, sig, st = g.bc_batch(sources)
         assert st["status"] == 0 and st["batched_sources"] == 3
         _check_rows(oracle, arr, sources, dep, sig, st)
+
+
+@pytest.mark.parametrize("spare_mb, words", [(64, 1), (900, 4)])
+def test_words_one_by_one_where_all_do_not_fit(native, oracle, spare_mb, words):
+    """Four words of sources on a graph small enough for one launch: where device memory
+    holds one word's state besides the traversal's planes but not four words', the
+    words go one after the other, as deep and as exact."""
+    import torch
+    import bfs_simd_benchmarks_gb300 as B
+    n = 1 << 18
+    src, dst = B.gen_rmat(n, 4 * n, seed=33, permute=True)
+    arr = oracle.csr_arrays(n, src, dst)
+    hog = None
+    with B.Graph.from_edges(n, src, dst, 1024, 16, device_build=True) as g:
+        g.set_options(batch_planes=20)
+        sources = B.pick_sources(g.degrees(), 200, seed=4).astype(np.uint32)
+        g.bc(int(sources[0]))  # the single-source state is there before
+        torch.cuda.empty_cache()
+        # one word's state and 20 planes of four words, and the 1 GiB that a batch leaves free
+        need = n * 64 * 8 + 20 * n * 5 * 8 + 30 * (n + len(src)) + (1 << 30)
+        free, _ = torch.cuda.mem_get_info()
+        try:
+            hog = torch.empty(max(free - need - (spare_mb << 20), 0), dtype=torch.uint8, device="cuda")
+            before, _ = torch.cuda.mem_get_info()
+            total, st = g.betweenness(sources)
+            after, _ = torch.cuda.mem_get_info()
+        finally:
+            del hog
+            torch.cuda.empty_cache()
+        assert st["status"] == 0 and st["batched_sources"] == sources.size and st["fallback_sources"] == 0
+        rows = n * 64 * 8
+        assert (before - after > 4 * rows) == (words == 4)
+        want, scale = np.zeros(n), np.zeros(n)
+        for s in sources[::40]:
+            one, _ = g.betweenness(np.array([s], np.uint32))
+            _, d, _, sc = oracle.bc_single(arr, int(s))
+            d = d.astype(np.float64)
+            d[s] = 0
+            assert bc_close(one, d, sc).all()
+        for s in sources:
+            _, d, _, sc = oracle.bc_single(arr, int(s))
+            d, sc = d.astype(np.float64), sc.copy()
+            d[s] = sc[s] = 0
+            want += d
+            scale += sc
+        assert bc_close(total, want, scale).all()
