@@ -1427,24 +1427,43 @@ uint32_t bb_chunk_edges(const bfs_graph *g) { return g->m <= 1u << 21 ? 64u : g-
 // (scale 18, 64 sources: 1.86 -> 1.74 ms with quarters; scale 19: 2.70 -> 2.73).
 constexpr size_t kBbWholeBlocks = 1u << 14;
 
-// Edge chunks (once per graph) of the vertices with more than `chunk` edges in
-// the rows `d_off`, uploaded.
-int bb_upload_chunks(bfs_graph *g, const uint32_t *d_off, uint32_t chunk, const uint32_t **chunk_v,
-		const uint32_t **chunk_beg, uint32_t *count) {
-	std::vector<uint32_t> off((size_t) g->n + 1);
-	if (cudaMemcpy(off.data(), d_off, sizeof(uint32_t) * off.size(), cudaMemcpyDeviceToHost) != cudaSuccess)
-		return BFS_ECUDA;
-	std::vector<uint32_t> cv, cb;
-	for (uint32_t v = 0; v < g->n; ++v) {
-		if (off[v + 1] - off[v] <= chunk) continue;
-		for (uint64_t e = off[v]; e < off[v + 1]; e += chunk) {
-			cv.push_back(v);
-			cb.push_back((uint32_t) e);
-		}
+// Edge chunks (once per graph) of the vertices with more than bb_chunk_edges
+// out-edges and, where the batched pull's are not the same, in-edges.  (Found on the
+// host from downloaded offsets: 2^20 vertices, 2^23 edges, the first call of 64
+// sources 5.75 ms, 3.0 of them besides the run.)
+int bb_build_chunks(bfs_graph *g) {
+	const uint32_t n = g->n, chunk = bb_chunk_edges(g);
+	const bool own_in = chunk != kMsChunk;
+	const uint32_t *off[2] = {g->dg.row_off, g->dg.in_off};
+	uint32_t *counts = nullptr, *first[2] = {nullptr, nullptr}, *scan_tmp = nullptr;
+	uint32_t num[2] = {0, 0}, *cv[2] = {nullptr, nullptr}, *cb[2] = {nullptr, nullptr};
+	TmpDev tmp;
+	DevArena ta, la;
+	ta.add(&counts, n);
+	ta.add(&scan_tmp, dbuild_scan_tmp_words(n));
+	for (int d = 0; d < 1 + own_in; ++d) ta.add(&first[d], (size_t) n + 1);
+	int rc = tmp.alloc_all(ta);
+	for (int d = 0; !rc && d < 1 + own_in; ++d)
+		if (!(rc = dbuild_chunk_counts(off[d], n, chunk, counts, g->num_sms, 0)))
+			rc = dbuild_exclusive_scan(counts, n, scan_tmp, first[d], 0);
+	if (rc) return rc;
+	for (int d = 0; d < 1 + own_in; ++d) {
+		if (cudaMemcpy(&num[d], first[d] + n, sizeof(uint32_t), cudaMemcpyDeviceToHost) != cudaSuccess) return BFS_ECUDA;
+		la.add(&cv[d], num[d]);
+		la.add(&cb[d], num[d]);
 	}
-	*count = (uint32_t) cv.size();
-	const int rc = dev_upload(g, chunk_v, cv);
-	return rc ? rc : dev_upload(g, chunk_beg, cb);
+	if ((rc = dev_alloc_all(g, la))) return rc;
+	for (int d = 0; !rc && d < 1 + own_in; ++d)
+		rc = dbuild_big_lists(n, nullptr, first[d], off[d], num[d], chunk, nullptr, cv[d], cb[d], g->num_sms, 0);
+	if (rc || cudaStreamSynchronize(0) != cudaSuccess) return rc ? rc : BFS_ECUDA;  // runs on any stream read them
+	g->bb_ochunk_v = cv[0];
+	g->bb_ochunk_beg = cb[0];
+	g->bb_noch = num[0];
+	g->bb_ichunk_v = own_in ? cv[1] : g->ms_chunk_v;
+	g->bb_ichunk_beg = own_in ? cb[1] : g->ms_chunk_beg;
+	g->bb_nich = own_in ? num[1] : g->ms_nchunks;
+	g->bb_chunks_ready = true;
+	return BFS_OK;
 }
 
 // Bytes of the betweenness state of `words` words of sources, and of its work
@@ -1478,18 +1497,7 @@ uint32_t bb_words_that_fit(const bfs_graph *g, uint32_t want) {
 // (host_out) the [256][n] staging of host outputs.
 int bb_prepare(bfs_graph *g, uint32_t num_sources, bool host_deps, bool host_paths) {
 	int rc;
-	if (!g->bb_chunks_ready) {
-		const uint32_t chunk = bb_chunk_edges(g);
-		if ((rc = bb_upload_chunks(g, g->dg.row_off, chunk, &g->bb_ochunk_v, &g->bb_ochunk_beg, &g->bb_noch))) return rc;
-		if (chunk == kMsChunk) {  // the batched pull's
-			g->bb_ichunk_v = g->ms_chunk_v;
-			g->bb_ichunk_beg = g->ms_chunk_beg;
-			g->bb_nich = g->ms_nchunks;
-		} else if ((rc = bb_upload_chunks(g, g->dg.in_off, chunk, &g->bb_ichunk_v, &g->bb_ichunk_beg, &g->bb_nich))) {
-			return rc;
-		}
-		g->bb_chunks_ready = true;
-	}
+	if (!g->bb_chunks_ready && (rc = bb_build_chunks(g))) return rc;
 	auto &b = g->bb;
 	uint32_t words = bb_words_that_fit(g, bb_launch_words(g, num_sources));
 	if (b.ctl && b.state_words < words) release_bb(g);  // its cudaFree waits for earlier calls

@@ -147,11 +147,21 @@ __global__ void k_vertex_facts(const uint32_t *out_deg, const uint32_t *in_deg, 
 	if (lane_id() == 0 && mx) atomicMax(max_degree, mx);
 }
 
-// The lists of the batched pull from the scans of chunks[] and is_big[].
+// Per vertex, the chunks of `chunk` edges of its list (0 up to one chunk).
+__global__ void k_chunk_counts(const uint32_t *off, uint32_t n, uint32_t chunk, uint32_t *chunks) {
+	const uint32_t stride = gridDim.x * blockDim.x;
+	for (uint32_t v = blockIdx.x * blockDim.x + threadIdx.x; v < n; v += stride) {
+		const uint32_t d = off[v + 1] - off[v];
+		chunks[v] = d > chunk ? d / chunk + (d % chunk != 0) : 0u;
+	}
+}
+
+// The lists of the batched pull from the scans of chunks[] and is_big[]; without
+// big_off the chunks alone.
 __global__ void k_big_lists(uint32_t n, const uint32_t *big_off, const uint32_t *chunk_off, const uint32_t *in_off,
 		uint32_t nchunks, uint32_t chunk, uint32_t *in_big, uint32_t *chunk_v, uint32_t *chunk_beg) {
 	const uint32_t stride = gridDim.x * blockDim.x, t = blockIdx.x * blockDim.x + threadIdx.x;
-	for (uint32_t v = t; v < n; v += stride)
+	for (uint32_t v = t; big_off && v < n; v += stride)
 		if (big_off[v + 1] != big_off[v]) in_big[big_off[v]] = v;
 	for (uint32_t c = t; c < nchunks; c += stride) {
 		// the last vertex whose chunks start at or before c
@@ -349,6 +359,11 @@ int dbuild_vertex_facts(const uint32_t *out_deg, const uint32_t *in_deg, uint32_
 		uint32_t *hasin, uint32_t *chunks, uint32_t *is_big, uint32_t *max_degree, int num_sms, cudaStream_t st) {
 	k_vertex_facts<<<grid_for(n, num_sms), kBThreads, 0, st>>>(out_deg, in_deg, n, big, chunk, hasin, chunks, is_big,
 			max_degree);
+	return cudaGetLastError() == cudaSuccess ? BFS_OK : BFS_ECUDA;
+}
+
+int dbuild_chunk_counts(const uint32_t *off, uint32_t n, uint32_t chunk, uint32_t *chunks, int num_sms, cudaStream_t st) {
+	k_chunk_counts<<<grid_for(n, num_sms), kBThreads, 0, st>>>(off, n, chunk, chunks);
 	return cudaGetLastError() == cudaSuccess ? BFS_OK : BFS_ECUDA;
 }
 

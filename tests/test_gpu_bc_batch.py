@@ -315,3 +315,32 @@ def test_words_one_by_one_where_all_do_not_fit(native, oracle, spare_mb, words):
             want += d
             scale += sc
         assert bc_close(total, want, scale).all()
+
+
+@pytest.mark.parametrize("direction", ["out", "in"])
+@pytest.mark.parametrize("degrees", [[63, 64, 65], [127, 128, 129, 1], [0, 1, 0], [64] * 40 + [65] * 40 + [1000, 0]])
+def test_edge_chunk_lists(native, oracle, degrees, direction):
+    """Vertices whose lists in one direction end around whole chunks (64 edges on a graph
+    of so few), on two levels with others after them, built on host and device."""
+    import bfs_simd_benchmarks_gb300 as B
+    rng = np.random.default_rng(len(degrees))
+    k = len(degrees)
+    hubs, pool = np.arange(1, k + 1), np.arange(k + 1, k + 1 + 1200)
+    src, dst = [np.zeros(k, int)], [hubs]
+    for v, d in zip(hubs, degrees):
+        src.append(np.full(d, v))
+        dst.append(rng.choice(pool, d, replace=False))
+    n = k + 1 + 1200 + 3
+    src.append(pool)
+    dst.append(rng.integers(n - 3, n, pool.size))
+    src, dst = np.concatenate(src).astype(np.uint32), np.concatenate(dst).astype(np.uint32)
+    sources = np.array([0, 1, k, n - 1], np.uint32)
+    if direction == "in":
+        src, dst = dst, src
+        sources = np.array([n - 1, n - 2, k + 1, 0], np.uint32)
+    arr = oracle.csr_arrays(n, src, dst)
+    for device_build in (False, True):
+        with B.Graph.from_edges(n, src, dst, 64, 4, device_build=device_build) as g:
+            dep, sig, st = g.bc_batch(sources)
+            assert st["status"] == 0 and st["batched_sources"] == sources.size
+            _check_rows(oracle, arr, sources, dep, sig, st)
