@@ -105,6 +105,7 @@ class Graph:
         if self._h:
             N.load().bfs_graph_free(self._h)
             self._h = None
+            self._n = None
 
     def __enter__(self):
         return self

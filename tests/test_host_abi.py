@@ -332,3 +332,14 @@ def test_tile_size_range_matches_reference_tool(native):
         assert B.tile_size_range(c["vertices"], c["edges"]) == (c["min_tile_size"], c["max_tile_size"]), c
     with pytest.raises(B.BfsError):
         B.tile_size_range(10, 3)   # too few edges for any width
+
+
+def test_a_closed_graph_has_no_vertex_count(native):
+    """Every question to a closed graph is refused, one that it answered before too."""
+    import bfs_simd_benchmarks_gb300 as B
+    g = B.Graph.from_edges(5, [0, 1], [1, 2], 64, 4, host_only=True)
+    assert g.num_vertices == 5
+    g.close()
+    for ask in (lambda: g.num_vertices, g.degrees, g.info):
+        with pytest.raises(B.BfsError):
+            ask()
