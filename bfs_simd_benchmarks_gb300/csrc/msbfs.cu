@@ -66,6 +66,14 @@ constexpr uint32_t kMsBlocks = 4;
 // Up to kMsTinyState, a CTA on every other SM (2^14 vertices 155 -> 147 us, uniform
 // 126 -> 115; 2^16 150 -> 163).
 constexpr uint32_t kMsSmallState = 1u << 18, kMsTinyState = 1u << 15;
+// Pull, few words: blocks taken at once where there are more than kMsClaims per warp.
+// The counter gives out one claim in 0.8 ns, and where most destinations have no
+// in-edges that is what a level waits for (uniform, 2^18 vertices of 16 edges, the
+// first ids of 2^23, 100 sources: levels 1,411 -> 844 us; 2^20 of 8 in 2^25 6,950 ->
+// 3,185; rmat, 2^24 vertices of 8 edges, 64 sources 3,847 -> 3,517; from 8 blocks per
+// warp on rmat 2^22 loses, from 32 on 2^23 does not gain).  More words per vertex lose
+// by it at all sizes (2^23, 300 sources: 1,347 -> 2,041).
+constexpr uint32_t kMsClaims = 16, kMsMaxClaim = 8;
 constexpr uint32_t kMsRun = 8;          // pull, few words: chunks taken at once
 constexpr uint32_t kMsMaxWords = 64;    // 4,096 sources
 constexpr uint32_t kGroupMaxWords = 32; // pull: up to this many words, in-neighbour rows in lane groups
@@ -880,12 +888,16 @@ __device__ __forceinline__ void ms_pull_blocks(const MsArgs &a, const MsPull &p,
 			item = gridDim.x * kMsWarps + __shfl_sync(kFull, next, 0);
 		}
 	}
-	while (item < nruns + a.nblk) {
+	while (item < nruns + a.nclaims) {
 		const uint32_t next = lane == 0 ? atomicAdd(counter, 1u) : 0u;
-		const uint32_t vb = (item - nruns) << a.blk_shift;
-		const uint32_t nv = min(1u << a.blk_shift, a.n - vb);
-		if constexpr (kRowWords) ms_pull_rows<KK>(a, p, vb, nv, f, acc, actdeg, gathered, wbuf, wn);
-		else ms_pull_words<KK>(a, p, vb, nv, fm, acc[0], acc[1], actdeg, gathered, wbuf, wn);
+		if constexpr (kRowWords) {
+			uint32_t vb = (item - nruns) * a.claim * 32;
+			for (uint32_t c = 0; c < a.claim && vb < a.n; ++c, vb += 32)
+				ms_pull_rows<KK>(a, p, vb, min(32u, a.n - vb), f, acc, actdeg, gathered, wbuf, wn);
+		} else {
+			const uint32_t vb = (item - nruns) << a.blk_shift;
+			ms_pull_words<KK>(a, p, vb, min(1u << a.blk_shift, a.n - vb), fm, acc[0], acc[1], actdeg, gathered, wbuf, wn);
+		}
 		item = (kRowWords ? gridDim.x * kMsWarps : 0u) + __shfl_sync(kFull, next, 0);
 	}
 	ms_wq_flush(p.cn, p.qn, wbuf, wn);
@@ -908,7 +920,7 @@ __device__ __forceinline__ void ms_pull_blocks(const MsArgs &a, const MsPull &p,
 // sources).  The frontier's vertices are staged per warp:
 // one atomic on the queue's length per kMsWq of them and not per block (together
 // 2^18 vertices, 64 sources: 282 -> 270 us; 2^20 604 -> 586).  Two or more blocks
-// at a time cost more in balance than they save (2^20: 618).
+// at a time cost more in balance than they save on graphs of this size (2^20: 618).
 template <int KK>
 __device__ __forceinline__ void ms_pull(const MsArgs &a, const MsPull &p, unsigned *counter, unsigned long long &actdeg_out,
 		unsigned long long &gathered_out, uint32_t *wq_base, unsigned long long *s_act) {
@@ -1508,7 +1520,9 @@ int ms_launch(const MsArgs &a, const uint32_t *d_sources, uint32_t ns, uint8_t *
 		while (aa.blk_shift > 0 && a.n >> aa.blk_shift < nwarps / 2) --aa.blk_shift;
 	}
 	aa.nruns = (a.nchunks + aa.run - 1) / aa.run;
-	aa.nblk = (uint32_t) (((uint64_t) a.n + (1u << aa.blk_shift) - 1) >> aa.blk_shift);
+	const uint32_t nblk = (uint32_t) (((uint64_t) a.n + (1u << aa.blk_shift) - 1) >> aa.blk_shift);
+	aa.claim = a.K <= kMsRowWords ? std::min(std::max(nblk / (nwarps * kMsClaims), 1u), kMsMaxClaim) : 1u;
+	aa.nclaims = (nblk + aa.claim - 1) / aa.claim;
 	const uint32_t *src = d_sources;
 	uint32_t nsrc = ns;
 	uint8_t *out = levels;
