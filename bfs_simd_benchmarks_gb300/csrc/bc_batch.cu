@@ -52,7 +52,8 @@ namespace {
 
 constexpr int kBbThreads = 512;
 constexpr int kBbWarps = kBbThreads / 32;
-constexpr int kBbUnroll = 4;   // chunk partial rows added per round (finish)
+constexpr int kBbUnroll = 8;   // chunk partial rows added per round (finish): with 4, a star of 2^20 leaves
+                               // 2.3 ms, with 8 1.7; 16 and 32 cost 4% elsewhere (R-MAT scale 18, 20)
 // Pairs of served edges per round (their rows loaded together).  3 with the next
 // step's neighbours read ahead: Pokec shape, 64 sources, 6.62 -> 6.25 ms, uniform
 // 2^20 vertices 6.12 -> 5.86 (2 pairs: 6.40 and 6.08; 4, which spill: 6.71 and
@@ -417,7 +418,7 @@ __device__ void bb_chunk(const BbArgs &a, uint32_t L, uint32_t w, bool has_nb, u
 	const uint32_t v = __ldg(D::chunk_v(a) + c), rw = w * a.n;
 	const uint64_t hv = bb_word(bb_plane(a, L, w), a, v);
 	const uint32_t beg = __ldg(cb + c), vbeg = __ldg(off + v), vend = __ldg(off + v + 1);
-	const uint32_t end = run_end(beg, a.chunk, vend);
+	const uint32_t len = bb_chunk_len(a.chunk, vend - vbeg), end = run_end(beg, len, vend);
 	T acc[4] = {T(0), T(0), T(0), T(0)};
 	uint32_t u2 = has_nb && beg + lane < end ? __ldg(adj + beg + lane) : 0u;
 	for (uint32_t e0 = beg; has_nb && e0 < end; e0 += 32) {
@@ -458,7 +459,7 @@ __device__ void bb_chunk(const BbArgs &a, uint32_t L, uint32_t w, bool has_nb, u
 		for (int i = 0; i < 4; ++i)
 			if ((bits >> i) & 1u) a.partial[crow * 64 + bb_quad() + i] = D::to_bits(acc[i]);
 	}
-	const uint32_t k = (vend - vbeg + a.chunk - 1) / a.chunk, c0 = c - (beg - vbeg) / a.chunk;
+	const uint32_t k = (vend - vbeg + len - 1) / len, c0 = c - (beg - vbeg) / len;
 	unsigned *done = a.chunks_done + (size_t) w * D::nchunks(a) + c0;
 	__syncwarp();
 	uint32_t before = 0;

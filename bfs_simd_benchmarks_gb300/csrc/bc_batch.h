@@ -12,6 +12,13 @@ namespace bfsg {
 
 constexpr uint32_t kBbMaxSources = 64;       // sources per 64-bit word of the traversal
 constexpr uint32_t kBbMaxWords = 4;          // words per call and per launch (BFS_BC_BATCH_MAX_SOURCES = 256 sources)
+// Edges per chunk of a vertex's list: a launch's chunk, but the batched pull's longer
+// ones for lists of more than kBbHugeDegree edges, whose partial rows one warp adds
+// (a star of 2^18 leaves, 64 sources: 926 us with chunks of 64 edges, now 457)
+constexpr uint32_t kBbHugeDegree = 1u << 16;
+__host__ __device__ inline uint32_t bb_chunk_len(uint32_t chunk, uint32_t degree) {
+	return degree > kBbHugeDegree && chunk < kMsChunk ? kMsChunk : chunk;
+}
 constexpr uint32_t kBbTraceLevels = 64;      // per-level timers kept for the first levels
 
 struct BbControl {

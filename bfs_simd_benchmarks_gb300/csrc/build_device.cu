@@ -13,6 +13,7 @@
 #include <cstdint>
 
 #include "../../include/bfs_gb300.h"
+#include "bc_batch.h"
 #include "bfs_device.cuh"
 #include "build_device.h"
 #include "device_common.cuh"
@@ -147,17 +148,18 @@ __global__ void k_vertex_facts(const uint32_t *out_deg, const uint32_t *in_deg, 
 	if (lane_id() == 0 && mx) atomicMax(max_degree, mx);
 }
 
-// Per vertex, the chunks of `chunk` edges of its list (0 up to one chunk).
+// Per vertex, the chunks of its list in batched betweenness (0 up to `chunk` edges).
 __global__ void k_chunk_counts(const uint32_t *off, uint32_t n, uint32_t chunk, uint32_t *chunks) {
 	const uint32_t stride = gridDim.x * blockDim.x;
 	for (uint32_t v = blockIdx.x * blockDim.x + threadIdx.x; v < n; v += stride) {
 		const uint32_t d = off[v + 1] - off[v];
-		chunks[v] = d > chunk ? d / chunk + (d % chunk != 0) : 0u;
+		const uint32_t len = bb_chunk_len(chunk, d);
+		chunks[v] = d > chunk ? d / len + (d % len != 0) : 0u;
 	}
 }
 
 // The lists of the batched pull from the scans of chunks[] and is_big[]; without
-// big_off the chunks alone.
+// big_off the chunks of batched betweenness.
 __global__ void k_big_lists(uint32_t n, const uint32_t *big_off, const uint32_t *chunk_off, const uint32_t *in_off,
 		uint32_t nchunks, uint32_t chunk, uint32_t *in_big, uint32_t *chunk_v, uint32_t *chunk_beg) {
 	const uint32_t stride = gridDim.x * blockDim.x, t = blockIdx.x * blockDim.x + threadIdx.x;
@@ -172,7 +174,8 @@ __global__ void k_big_lists(uint32_t n, const uint32_t *big_off, const uint32_t 
 			else hi = mid;
 		}
 		chunk_v[c] = lo;
-		chunk_beg[c] = in_off[lo] + (c - chunk_off[lo]) * chunk;
+		const uint32_t len = big_off ? chunk : bb_chunk_len(chunk, in_off[lo + 1] - in_off[lo]);
+		chunk_beg[c] = in_off[lo] + (c - chunk_off[lo]) * len;
 	}
 }
 

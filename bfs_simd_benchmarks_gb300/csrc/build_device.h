@@ -30,10 +30,10 @@ int dbuild_scatter(const uint32_t *key, const uint32_t *val, uint64_t m, uint32_
 // any, and the largest out-degree (*max_degree zeroed by the caller).
 int dbuild_vertex_facts(const uint32_t *out_deg, const uint32_t *in_deg, uint32_t n, uint32_t big, uint32_t chunk,
 		uint32_t *hasin, uint32_t *chunks, uint32_t *is_big, uint32_t *max_degree, int num_sms, cudaStream_t st);
-// Per vertex of the lists `off`, its chunks of `chunk` edges (0 up to one chunk).
+// Per vertex of the lists `off`, its chunks in batched betweenness (bb_chunk_len; 0 up to `chunk` edges).
 int dbuild_chunk_counts(const uint32_t *off, uint32_t n, uint32_t chunk, uint32_t *chunks, int num_sms, cudaStream_t st);
 // The batched pull's lists from the exclusive scans of is_big and chunks; with
-// big_off null the chunks alone (of any lists, in_off).
+// big_off null the chunks of batched betweenness alone (of any lists, in_off).
 int dbuild_big_lists(uint32_t n, const uint32_t *big_off, const uint32_t *chunk_off, const uint32_t *in_off,
 		uint32_t nchunks, uint32_t chunk, uint32_t *in_big, uint32_t *chunk_v, uint32_t *chunk_beg, int num_sms,
 		cudaStream_t st);

@@ -344,3 +344,20 @@ def test_edge_chunk_lists(native, oracle, degrees, direction):
             dep, sig, st = g.bc_batch(sources)
             assert st["status"] == 0 and st["batched_sources"] == sources.size
             _check_rows(oracle, arr, sources, dep, sig, st)
+
+
+@pytest.mark.parametrize("leaves", [65_535, 65_536, 65_537, 131_200])
+def test_huge_hub(native, oracle, leaves):
+    """A hub of more than 2^16 edges, in both directions: its lists are cut into longer chunks."""
+    import bfs_simd_benchmarks_gb300 as B
+    n = leaves + 4
+    v = np.arange(1, leaves + 1)
+    src = np.concatenate([np.zeros(leaves, int), v, v[::3], np.full(3, leaves)])
+    dst = np.concatenate([v, np.zeros(leaves, int), np.minimum(v[::3] + 1, leaves), np.arange(leaves + 1, n)])
+    src, dst = src.astype(np.uint32), dst.astype(np.uint32)
+    arr = oracle.csr_arrays(n, src, dst)
+    sources = np.array([0, 1, 7, leaves, n - 1], np.uint32)
+    with B.Graph.from_edges(n, src, dst, 1024, 16) as g:
+        dep, sig, st = g.bc_batch(sources)
+        assert st["status"] == 0 and st["batched_sources"] == sources.size
+        _check_rows(oracle, arr, sources, dep, sig, st)
