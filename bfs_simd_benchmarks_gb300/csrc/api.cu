@@ -241,14 +241,16 @@ uint32_t *host_address(void *p, bool shared_pages) {
 	if (at.type == cudaMemoryTypeHost) return (uint32_t *) at.devicePointer;
 	return at.type == cudaMemoryTypeUnregistered && shared_pages ? (uint32_t *) p : nullptr;
 }
-// Writes to every page of [p, p + bytes), contents unchanged: the pages are
-// there when the device writes them, and memory that cannot be written faults
-// here, on the host.
+// Writes to every page of [p, p + bytes), which is about to be overwritten: the
+// pages are there when the device writes them, and memory that cannot be written
+// faults here, on the host.  (Stores alone: a read first maps the huge zero page into
+// a fresh buffer, which the store then splits into small ones, each with faults of
+// its own: 2^24 levels into a new array 24.4 ms, now 3.3.)
 void touch_pages(void *p, size_t bytes) {
 	static const size_t page = (size_t) sysconf(_SC_PAGESIZE);
 	volatile uint8_t *b = (volatile uint8_t *) p;
-	for (size_t o = 0; o < bytes; o += page) b[o] = b[o];
-	if (bytes) b[bytes - 1] = b[bytes - 1];
+	for (size_t o = 0; o < bytes; o += page) b[o] = 0;
+	if (bytes) b[bytes - 1] = 0;
 }
 
 template <class T> int dev_alloc(bfs_graph *g, T **out, size_t count) {

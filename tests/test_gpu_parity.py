@@ -456,3 +456,36 @@ def test_host_outputs_at_any_address(native, oracle, offset, pinned):
     assert oracle.check_parents(arr, s, lev, par) == 0
     for o in out:
         assert (o[:offset] == 7).all() and (o[offset + 4 * n:] == 7).all()
+
+
+def test_large_outputs_into_new_arrays(native, oracle):
+    """Levels and parents into memory that was never written (numpy's new arrays above
+    the allocator's limit, on huge pages where there are any): right, and in a time that
+    writing to such memory and a run into old memory explain."""
+    import ctypes as C
+    import time
+    import bfs_simd_benchmarks_gb300 as B
+    n = 1 << 24
+    src, dst = B.gen_rmat(n, n, seed=8, permute=True)
+    s = int(src[0])
+
+    def best(f):
+        out = []
+        for _ in range(5):
+            t = time.perf_counter()
+            f()
+            out.append(time.perf_counter() - t)
+        return min(out)
+
+    with B.Graph.from_edges(n, src, dst, 1024, 16, device_build=True) as g:
+        lev, par, st = g.run(s)
+        old = np.zeros(n, np.int32)
+        p_old = old.ctypes.data_as(C.POINTER(C.c_int32))
+        run_old = best(lambda: native.bfs_run(g.handle, s, p_old, None, None))
+        np.testing.assert_array_equal(lev, old)
+        arr = oracle.csr_arrays(n, src, dst)
+        np.testing.assert_array_equal(lev, oracle.bfs_levels(arr, s))
+        assert oracle.check_parents(arr, s, lev, par) == 0
+        write_new = best(lambda: np.empty(n, np.int32).fill(0))
+        run_new = best(lambda: g.run(s, parents=False))
+        assert run_new < 4 * (run_old + write_new), (run_new, run_old, write_new)
