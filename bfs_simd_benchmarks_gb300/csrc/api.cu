@@ -449,6 +449,10 @@ void apply_grid(bfs_graph *g) {
 	g->smem = g->smem_of[g->opt.bottom_up];
 }
 
+// Graphs of fewer bitmap blocks than this (2^19 vertices) have no list of those
+// with in-edges: listing them is 20 us of set-up, all of 150 for the smallest, and
+// without it each of the grid's CTAs has at most a few empty ones.
+constexpr uint32_t kPullListBlocks = 2048;
 // Run context, events and the persistent grid.
 int alloc_run(bfs_graph *g) {
 	DevGraph &d = g->dg;
@@ -470,10 +474,11 @@ int alloc_run(bfs_graph *g) {
 	ar.add(&g->level_buf, g->n);
 	ar.add(&g->parent_buf, g->n);
 	uint32_t *blocks = nullptr, *nblocks = nullptr;
-	ar.add(&blocks, (d.nwords + kPullBlock - 1) / kPullBlock);
+	ar.add(&blocks, (d.nwords + kPullBlock - 1) / kPullBlock);  // 8 words of 32 vertices each
 	ar.add(&nblocks, 1);
 	if ((st = dev_alloc_all(g, ar))) return st;
-	if ((st = dbuild_pull_blocks(d.hasin, d.nwords, blocks, nblocks, 0))) return st;
+	const uint32_t all_blocks = (d.nwords + kPullBlock - 1) / kPullBlock;
+	if (all_blocks >= kPullListBlocks && (st = dbuild_pull_blocks(d.hasin, d.nwords, blocks, nblocks, 0))) return st;
 	// the persistent kernel expects its barrier and status words zero at launch
 	if (cudaMemset(r.bar, 0, 2 * sizeof(unsigned)) != cudaSuccess || cudaMemset(r.err, 0, sizeof(int)) != cudaSuccess)
 		return BFS_ECUDA;
@@ -491,10 +496,14 @@ int alloc_run(bfs_graph *g) {
 	g->cluster = cluster_ctas(d);
 	// the pull goes through the blocks with in-edges where that saves a quarter of
 	// them; elsewhere the list would only be a load before each block's
-	const uint32_t all = (d.nwords + kPullBlock - 1) / kPullBlock;
-	if (cudaMemcpy(&d.pull_nblocks, nblocks, sizeof(uint32_t), cudaMemcpyDeviceToHost) != cudaSuccess) return BFS_ECUDA;
-	if ((uint64_t) d.pull_nblocks * 4 <= (uint64_t) all * 3) d.pull_blocks = blocks;
-	else d.pull_nblocks = all;
+	d.pull_nblocks = all_blocks;
+	uint32_t full = all_blocks;
+	if (all_blocks >= kPullListBlocks && cudaMemcpy(&full, nblocks, sizeof(uint32_t), cudaMemcpyDeviceToHost) != cudaSuccess)
+		return BFS_ECUDA;
+	if ((uint64_t) full * 4 <= (uint64_t) all_blocks * 3) {
+		d.pull_blocks = blocks;
+		d.pull_nblocks = full;
+	}
 	apply_grid(g);
 	return BFS_OK;
 }
