@@ -279,3 +279,85 @@ def test_bc_sums_past_the_largest_float(native, oracle, width, height, both):
             np.testing.assert_array_equal(sig, osig)
             for kind in (np.isposinf, np.isneginf, np.isnan):
                 np.testing.assert_array_equal(kind(dep), kind(odep))
+
+
+def _layers(sizes, seed, per=3, back=0, hubs=()):
+    """Layer i + 1's vertices get `per` edges each from random vertices of layer i (every
+    one of them is reached); `back` edges from each later layer to the one before;
+    hubs: (layer, extra in-edges from that layer's successors and from vertices that
+    nothing reaches)."""
+    rng = np.random.default_rng(seed)
+    at = np.concatenate([[0], np.cumsum(sizes)])
+    n = int(at[-1])
+    src, dst = [], []
+    for i in range(len(sizes) - 1):
+        a, b = np.arange(at[i], at[i + 1]), np.arange(at[i + 1], at[i + 2])
+        src.append(rng.choice(a, per * b.size))
+        dst.append(np.repeat(b, per))
+        if back:
+            src.append(rng.choice(b, back * b.size))
+            dst.append(rng.choice(a, back * b.size))
+    for layer, extra in hubs:
+        island = np.arange(n, n + extra)
+        src.append(island)
+        dst.append(np.full(extra, at[layer]))
+        n += extra
+    return n, np.concatenate(src).astype(np.uint32), np.concatenate(dst).astype(np.uint32)
+
+
+def _degrees(out, inn, seed):
+    """0 -> hubs -> pool -> hubs' -> end: hubs with the given out-degrees, hubs' with the given in-degrees."""
+    rng = np.random.default_rng(seed)
+    pool = max(max(out), max(inn)) + 50
+    h, p = np.arange(1, 1 + len(out)), np.arange(1 + len(out), 1 + len(out) + pool)
+    k = np.arange(p[-1] + 1, p[-1] + 1 + len(inn))
+    src, dst = [np.zeros(len(out), int)], [h]
+    for v, d in zip(h, out):
+        src.append(np.full(d, v))
+        dst.append(rng.choice(p, d, replace=False))
+    src.append(np.full(pool, h[0]))  # the whole pool is on one level
+    dst.append(p)
+    for v, d in zip(k, inn):
+        src.append(rng.choice(p, d, replace=False))
+        dst.append(np.full(d, v))
+    src.append(k)
+    dst.append(np.full(len(inn), k[-1] + 1))
+    return int(k[-1]) + 2, np.concatenate(src).astype(np.uint32), np.concatenate(dst).astype(np.uint32)
+
+
+BC_CASES = {
+    # chunks of 512 edges of vertices with more than 1024, half-warps and lanes below
+    "chunks": _degrees([1023, 1024, 1025, 1535, 1536, 1537, 2048, 2049], [1024, 1025, 1536, 1537, 2049, 4000], 1),
+    "bands": _degrees([7, 8, 9, 31, 32, 33, 63, 64, 65, 512, 513], [1, 7, 8, 9, 15, 16, 17, 32, 33, 128, 129], 2),
+    # sort counters in shared memory up to 32 levels; traced levels (and pushing) up to 64
+    **{f"levels_{k}": _layers([1] + [5 + i % 7 for i in range(k - 1)], k, back=1) for k in (31, 32, 33, 63, 64, 65, 66)},
+    # levels reached by few of their in-edges are pushed: one, two in a row, the last one, pulled ones around them
+    "push_first": _layers([1, 3, 400, 400, 50], 3, hubs=[(1, 700), (2, 5000)]),
+    "push_two": _layers([1, 40, 60, 900, 30], 4, back=1, hubs=[(2, 3000), (3, 9000)]),
+    "push_last": _layers([1, 200, 600, 20], 5, hubs=[(3, 6000)]),
+    "push_every": _layers([1, 4, 9, 30, 20], 6, hubs=[(i, 2000) for i in range(1, 5)]),
+    "push_none": _layers([1, 500, 500, 500], 7, per=8),
+    "push_deep": _layers([1] + [6] * 70, 8, hubs=[(i, 300) for i in (10, 62, 63, 64, 65, 70)]),
+}
+# lists that start at every edge number modulo 4 and end at the array's last edges
+for _k in range(4):
+    _n, _s, _d = _layers([1, 9, 40, 30, 6], 20 + _k, per=5, back=2)
+    BC_CASES[f"edges_mod_{(_s.size - _k) % 4}"] = (_n, _s[:_s.size - _k], _d[:_s.size - _k])
+
+
+@pytest.mark.parametrize("name", list(BC_CASES))
+def test_bc_shapes(native, oracle, name):
+    """The edges of k_bc's rules, in both gather modes, on graphs built on the host and on the device."""
+    import bfs_simd_benchmarks_gb300 as B
+    n, src, dst = BC_CASES[name]
+    arr = oracle.arrays_from_edges(n, src, dst, 256, 4)
+    for device_build in (False, True):
+        with B.Graph.from_edges(n, src, dst, 256, 4, device_build=device_build) as g:
+            g.set_options(bc_batch=0)
+            for mode in (1, 2):
+                g.set_options(bc_level_bytes=mode)
+                for s in (0, 2, n // 2):
+                    dep, _, _ = _check_source(oracle, arr, g, s)
+                    total, st = g.betweenness(np.array([s], np.uint32))
+                    dep[s] = 0
+                    np.testing.assert_array_equal(total, dep)
