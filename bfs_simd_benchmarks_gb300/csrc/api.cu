@@ -449,10 +449,12 @@ void apply_grid(bfs_graph *g) {
 	g->smem = g->smem_of[g->opt.bottom_up];
 }
 
-// Graphs of fewer bitmap blocks than this (2^19 vertices) have no list of those
-// with in-edges: listing them is 20 us of set-up, all of 150 for the smallest, and
-// without it each of the grid's CTAs has at most a few empty ones.
-constexpr uint32_t kPullListBlocks = 2048;
+// Graphs of fewer bitmap blocks than this (2^20 vertices) have no list of those
+// with in-edges: listing them is 20 us of a set-up of 150 to 2,000, and a CTA of the
+// grid has at most 13 of them (uniform, 2^15 vertices of 32 edges, the first ids of
+// 2^19: 64 us without the list, 66 with it; 2^17 of 32 in 2^20: 89 and 87).
+constexpr uint32_t kPullListBlocks = 4096;
+
 // Run context, events and the persistent grid.
 int alloc_run(bfs_graph *g) {
 	DevGraph &d = g->dg;

@@ -239,13 +239,13 @@ def test_rounds_of_one_cta_fit_the_wait_limit(native, oracle, wait_limit_us):
 
 @pytest.mark.parametrize("n, used", [
     (1 << 22, np.arange(1 << 14)),                      # the first ids
-    ((1 << 19) - 256, np.arange(3000)),                 # no list of blocks yet
-    (1 << 19, np.arange(3000)),                         # the smallest graph with one
+    ((1 << 20) - 256, np.arange(3000)),                 # no list of blocks yet
+    (1 << 20, np.arange(3000)),                         # the smallest graph with one
     ((1 << 20) + 77, np.arange((1 << 20) - 20_000, (1 << 20) + 77)),  # the last ones, the last block cut off
-    (600_000, np.arange(200_001, 220_000)),
-    (600_000, np.arange(0, 600_000, 300)),              # one in a block or none
-    (600_000, np.arange(0, 600_000, 256)),              # one in every block
-    (600_000, np.concatenate([np.arange(300_000), np.arange(400_000, 551_000)])),  # about three quarters of the blocks
+    (1_200_000, np.arange(200_001, 220_000)),
+    (1_200_000, np.arange(0, 1_200_000, 300)),              # one in a block or none
+    (1_200_000, np.arange(0, 1_200_000, 256)),              # one in every block
+    (1_200_000, np.concatenate([np.arange(600_000), np.arange(800_000, 1_101_000)])),  # about three quarters of the blocks
     (100_000, np.array([99_999, 5])),
 ])
 def test_grid_pull_of_sparse_ids(native, oracle, tmp_path, n, used):
