@@ -122,7 +122,7 @@ struct bfs_graph {
 		uint32_t *sigma = nullptr, *partial = nullptr, *d_sources = nullptr;
 		unsigned *chunks_done = nullptr;
 		float *dsum = nullptr;
-		float *delta = nullptr;      // [64][n] staging of host outputs (allocated when first asked for)
+		float *delta = nullptr;      // [256][n] staging of host outputs (allocated when first asked for)
 		uint32_t *paths = nullptr;
 		uint32_t *blist = nullptr, *ilist = nullptr, *olist = nullptr;  // per-level work lists
 		uint32_t list_planes = 0;    // levels they have room for
@@ -2398,7 +2398,7 @@ int bfs_bc_accumulate(bfs_graph *g, const uint32_t *sources, uint32_t num_source
 	if (!g->opt.bc_batch) {
 		rc = bc_sources_one_by_one(g, sources, num_sources, nullptr, nullptr, b.acc, total);
 	} else {
-		// groups of up to 64 sources; a group deeper than the planes one source at a time
+		// groups of up to 256 sources; a group deeper than the planes one source at a time
 		for (uint32_t i = 0; i < num_sources && rc == BFS_OK; i += BFS_BC_BATCH_MAX_SOURCES) {
 			const uint32_t k = std::min<uint32_t>(BFS_BC_BATCH_MAX_SOURCES, num_sources - i);
 			bfs_bc_stats one{};

@@ -45,8 +45,8 @@ struct BcControl {
 	unsigned long long t_rev[kBcTraceLevels];  // end of the dependency sums of level d
 	uint32_t lv_deg[2][kBcTraceLevels];        // out-degree and in-degree sums of level d's vertices
 	uint32_t lv_vertices[kBcTraceLevels];      // vertices of level d
-	uint32_t lv_big[kBcTraceLevels];           // of which reduced by a whole CTA
-	uint32_t lv_medium[kBcTraceLevels];        // of which reduced by one warp
+	uint32_t lv_big[kBcTraceLevels];           // of which summed in chunks
+	uint32_t lv_medium[kBcTraceLevels];        // of which summed by a half-warp
 	uint32_t blk[kBcMaxGrid];          // per-CTA totals of the counter scan
 };
 

@@ -947,8 +947,8 @@ constexpr uint32_t kPullShort = 3;
 // The words of an item are blocks of kPullBlock (a sector of the bitmaps), dealt to
 // the items in turn, so that every item has its share of each part of the ids: the
 // in-edges of many graphs belong to few of them.  Where they leave a quarter of the
-// blocks empty, the graph's list of the others is dealt (pull_blocks).  A CTA per range of the ids had most of the work on such graphs:
-// uniform, 2^14 vertices of 64 edges, the first ids of 2^22: 130 us (63 with parts of
+// blocks empty, the graph's list of the others is dealt (pull_blocks).  A CTA per
+// range of the ids had most of the work on such graphs: uniform, 2^14 vertices of 64 edges, the first ids of 2^22: 130 us (63 with parts of
 // column groups), now 54; 2^17 of 32 edges, the first of 2^23: 210 (137), now 90;
 // rmat, 2^24 vertices of 8 edges, by degree: 1,334 us, now 683, permuted 718 and 686;
 // Twitter shape, permuted: 1,680 and 1,619.  Blocks dealt without the list are

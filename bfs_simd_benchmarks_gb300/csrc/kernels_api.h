@@ -43,7 +43,8 @@ int launch_persistent(const DevGraph &g, const RunCtx &r, const StepParams &p, u
 // 0 where the graph is too large for it (or the device takes no such cluster).
 // Up to kClusterDenseVertices; above, up to kClusterMaxVertices, only with at most
 // kClusterSparseDegree edges a vertex (many levels of few edges): the pulls of
-// denser ones want more than 16 SMs (90,000 vertices, 2^21 edges: rmat 102 us in
+// denser ones want more than 16 SMs.  Both limits were found on dense graphs; a
+// street grid was measured at one size, and its own limit is higher (90,000 vertices, 2^21 edges: rmat 102 us in
 // the cluster, 98 on the grid; 2^20 edges: rmat 107 and 91, uniform 120 and 108; a
 // street grid of 90,000: 728 and 923; 2^16 vertices, 2^20 edges: rmat 81 and 82,
 // 2^15 vertices 59 and 77).

@@ -84,15 +84,15 @@ struct MsArgs {
 	uint32_t out_tile;                 // output pass tile width in vertices: 64, 128, or 0 = by words per vertex
 };
 
+// Fills chunk_slot (once per allocation); waits for it.
+int ms_chunk_slots(const uint32_t *chunk_v, uint32_t nchunks, const uint32_t *in_big, uint32_t nbig, uint32_t *chunk_slot);
+
 // Enqueues the whole batched traversal (one cooperative launch and the
 // output pass) on `st`; `between` and `between2` (either may be null) are
 // recorded between the two;
 // *grid receives the launch's CTA count.  levels == null: no output pass, the
 // planes stay for a later pass, and a traversal deeper than the planes stops
 // with BFS_EUNSUPPORTED.
-// Fills chunk_slot (once per allocation); waits for it.
-int ms_chunk_slots(const uint32_t *chunk_v, uint32_t nchunks, const uint32_t *in_big, uint32_t nbig, uint32_t *chunk_slot);
-
 int ms_launch(const MsArgs &a, const uint32_t *d_sources, uint32_t ns, uint8_t *levels, int num_sms, cudaStream_t st,
 		int *grid, cudaEvent_t between, cudaEvent_t between2);
 
