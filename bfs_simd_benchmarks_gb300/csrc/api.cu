@@ -1284,7 +1284,7 @@ int bc_prepare(bfs_graph *g) {
 			(rc = bc_alloc(g, &b.acc, g->n)) || (rc = bc_alloc(g, &b.cnt, kBcCntCap)) ||
 			(rc = bc_alloc(g, &b.kstart, kBcClasses * (size_t) kBcMaxLevels + 1)) ||
 			(rc = bc_alloc(g, &b.partial, bc_partial_capacity(g->n, g->m))) ||
-			(rc = bc_alloc(g, &b.cpre, (size_t) g->n + 1)) || (rc = bc_alloc(g, &b.big_done, g->n)) || (rc = bc_alloc(g, &b.ctl, 1))) {
+			(rc = bc_alloc(g, &b.cpre, (size_t) g->n + 1)) || (rc = bc_alloc(g, &b.big_done, kBcSmemBig)) || (rc = bc_alloc(g, &b.ctl, 1))) {
 		release_bc(g);
 		return rc;
 	}

@@ -656,7 +656,7 @@ __global__ void __launch_bounds__(kBcThreads, 2) k_bc(BcArgs a) {
 			const int key = vertex_key(a, v, depth, &bad);
 			if (v < a.n) {
 				a.sigma[v] = v == a.source ? 1u : 0u;
-				a.big_done[v] = 0u;
+				if (v < kBcSmemBig) a.big_done[v] = 0u;
 				a.delta[v] = 0.0f;
 				const int lv = a.level[v];
 				a.lvx[v] = make_uint2((uint32_t) lv, v == a.source ? 1u : 0u);

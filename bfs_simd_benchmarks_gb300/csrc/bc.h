@@ -69,7 +69,7 @@ struct BcArgs {
 	uint32_t *cnt;                     // [kBcCntCap] counters of the level sort
 	uint32_t *kstart;                  // [kBcClasses * kBcMaxLevels + 1] start of every key in `order`
 	uint32_t *partial;                 // [bc_partial_capacity(n, m)] chunk sums of big vertices (value bits)
-	unsigned *big_done;                // [n] a level's big vertices: chunks summed so far (0 between levels)
+	unsigned *big_done;                // [kBcSmemBig] a level's big vertices: chunks summed so far (0 between levels)
 	uint32_t *cpre;                    // [n + 1] chunk prefix of a level with more than kBcSmemBig big vertices
 	BcControl *ctl;
 };
