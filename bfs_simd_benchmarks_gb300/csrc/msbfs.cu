@@ -983,47 +983,6 @@ __device__ __forceinline__ void emit_bytes_of(const uint64_t (&w)[kEmitPlanes], 
 	}
 }
 
-// 16 level bytes (x, vertices in order) -> levels at dst, cnt <= 16 of them,
-// with the widest store the address allows.
-__device__ __forceinline__ void emit_piece(uint8_t *dst, const uint32_t (&x)[4], uint32_t cnt, bool merge) {
-	const uintptr_t al = (uintptr_t) dst;
-	if (cnt == 16 && (al & 15) == 0) {
-		uint4 y = make_uint4(x[0], x[1], x[2], x[3]);
-		if (merge) {
-			const uint4 old = __ldcg((const uint4 *) dst);
-			y.x = __vminu4(y.x, old.x);
-			y.y = __vminu4(y.y, old.y);
-			y.z = __vminu4(y.z, old.z);
-			y.w = __vminu4(y.w, old.w);
-		}
-		*(uint4 *) dst = y;
-	} else if (cnt == 16 && (al & 3) == 0) {
-#pragma unroll
-		for (int q = 0; q < 4; ++q) {
-			uint32_t y = x[q];
-			if (merge) y = __vminu4(y, __ldcg((const unsigned int *) dst + q));
-			((uint32_t *) dst)[q] = y;
-		}
-	} else if (cnt == 16 && (al & 1) == 0) {
-#pragma unroll
-		for (int q = 0; q < 8; ++q) {
-			uint32_t y = (x[q / 2] >> (16 * (q & 1))) & 0xFFFFu;
-			if (merge) {
-				const uint32_t old = __ldcg((const unsigned short *) dst + q);
-				y = __vminu4(y | 0xFFFF0000u, old | 0xFFFF0000u) & 0xFFFFu;
-			}
-			((uint16_t *) dst)[q] = (uint16_t) y;
-		}
-	} else {
-#pragma unroll
-		for (uint32_t b = 0; b < 16; ++b) {
-			if (b >= cnt) break;
-			const uint8_t y = (uint8_t) (x[b / 4] >> (8 * (b & 3)));
-			dst[b] = merge ? min(y, ld_cg_u8(dst + b)) : y;
-		}
-	}
-}
-
 __device__ __forceinline__ void cp_async8(void *dst, const void *src) {
 	asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" :: "r"((uint32_t) __cvta_generic_to_shared(dst)), "l"(src) : "memory");
 }
@@ -1057,19 +1016,23 @@ __device__ __forceinline__ void emit_shifted(const uint8_t *src, uint8_t *dst, u
 	uint32_t o = piece ? head + 16 * (piece - 1) : 0u;
 	if (o >= nv) return;
 	const uint32_t len = piece ? min(16u, nv - o) : head;
-	if (merge) {
-		for (uint32_t i = o; i < o + len; ++i) dst[i] = min(src[i], ld_cg_u8(dst + i));
-		return;
-	}
 	if (len == 16) {
 		const uint32_t *w = reinterpret_cast<const uint32_t *>(src + (o & ~3u));
 		const uint32_t sh = 8 * (o & 3u);
 		uint32_t x[5];
 #pragma unroll
 		for (int q = 0; q < 5; ++q) x[q] = w[q];
-		*reinterpret_cast<uint4 *>(dst + o) =
-				make_uint4(__funnelshift_r(x[0], x[1], sh), __funnelshift_r(x[1], x[2], sh),
-						__funnelshift_r(x[2], x[3], sh), __funnelshift_r(x[3], x[4], sh));
+		uint4 y = make_uint4(__funnelshift_r(x[0], x[1], sh), __funnelshift_r(x[1], x[2], sh),
+				__funnelshift_r(x[2], x[3], sh), __funnelshift_r(x[3], x[4], sh));
+		if (merge) {
+			const uint4 old = __ldcg(reinterpret_cast<const uint4 *>(dst + o));
+			y = make_uint4(__vminu4(y.x, old.x), __vminu4(y.y, old.y), __vminu4(y.z, old.z), __vminu4(y.w, old.w));
+		}
+		*reinterpret_cast<uint4 *>(dst + o) = y;
+		return;
+	}
+	if (merge) {
+		for (uint32_t i = o; i < o + len; ++i) dst[i] = min(src[i], ld_cg_u8(dst + i));
 		return;
 	}
 	// a head grows to the 16-byte boundary, a tail shrinks from it
@@ -1234,7 +1197,6 @@ __device__ __noinline__ void ms_emit(const MsArgs &a, uint8_t *levels, uint32_t 
 		}
 		if (kShift) __syncthreads();  // the source rows take the quads' place
 		if (piece) {
-			const uint32_t cnt = min(16u, nv - c);
 #pragma unroll
 			for (int b = 0; b < 4; ++b) {
 				if constexpr (kShift) {
@@ -1243,17 +1205,14 @@ __device__ __noinline__ void ms_emit(const MsArgs &a, uint8_t *levels, uint32_t 
 					continue;
 				}
 				if (r0 + 4 * b >= nrows) break;
-				if constexpr (kAhead) {  // whole pieces of aligned rows: see the launch
-					uint4 *const d = reinterpret_cast<uint4 *>(levels + (size_t) (k0 * 64 + r0 + 4 * b) * n + tv0 + c);
-					uint4 z = make_uint4(y[b][0], y[b][1], y[b][2], y[b][3]);
-					if (merge) {
-						const uint4 old = __ldcg(d);
-						z = make_uint4(__vminu4(z.x, old.x), __vminu4(z.y, old.y), __vminu4(z.z, old.z), __vminu4(z.w, old.w));
-					}
-					*d = z;
-					continue;
+				// whole pieces of aligned rows
+				uint4 *const d = reinterpret_cast<uint4 *>(levels + (size_t) (k0 * 64 + r0 + 4 * b) * n + tv0 + c);
+				uint4 z = make_uint4(y[b][0], y[b][1], y[b][2], y[b][3]);
+				if (merge) {
+					const uint4 old = __ldcg(d);
+					z = make_uint4(__vminu4(z.x, old.x), __vminu4(z.y, old.y), __vminu4(z.z, old.z), __vminu4(z.w, old.w));
 				}
-				emit_piece(levels + (size_t) (k0 * 64 + r0 + 4 * b) * n + tv0 + c, y[b], cnt, merge);
+				*d = z;
 			}
 		}
 		if (kShift) {
@@ -1342,7 +1301,9 @@ __global__ void __launch_bounds__(kMsThreads, 2) k_ms_bfs(const __grid_constant_
 				break;
 			}
 			// planes full: write them out, keep the frontier's plane as plane 0
-			ms_emit<false, kEmitV, kEmitW, false>(a, levels, ns, base, base == 0 ? 0 : 1, lvl - base, base != 0, lev);
+			if (a.n % 16 == 0 && (uintptr_t) levels % 16 == 0)
+				ms_emit<false, kEmitV, kEmitW, false>(a, levels, ns, base, base == 0 ? 0 : 1, lvl - base, base != 0, lev);
+			else ms_emit<false, kEmitV, kEmitW, true>(a, levels, ns, base, base == 0 ? 0 : 1, lvl - base, base != 0, lev);
 			if (!(ok = grid_sync(ctl->bar, epoch, &ctl->err, a.wait_limit_ns, a.hold_barrier))) break;
 			const uint64_t *src = a.hist + (size_t) (lvl - base) * nK;
 			for (size_t i = t0; i < nK; i += stride) a.hist[i] = ld_cg64(src + i);

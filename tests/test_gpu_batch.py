@@ -408,3 +408,33 @@ def test_grid_and_blocks_by_state(native, oracle, n, words):
                 for i, s in enumerate(sources.tolist()):
                     if s in levels:
                         np.testing.assert_array_equal(got[i], levels[s], err_msg=f"row {i} (source {s})")
+
+
+@pytest.mark.parametrize("num_sources", [3, 64, 130, 300])
+@pytest.mark.parametrize("n", [4001, 4008, 4096])
+def test_early_output_passes_at_any_alignment(native, oracle, n, num_sources):
+    """Traversals deeper than two or three planes: rows that start on any byte, first
+    written and then merged into, by the early passes and the last one."""
+    import torch
+    import bfs_simd_benchmarks_gb300 as B
+    rng = np.random.default_rng(n)
+    step = rng.integers(1, 400, 3 * n)
+    src = rng.integers(0, n, 3 * n)
+    dst = np.minimum(src + step, n - 1)  # some 20 levels
+    src, dst = src.astype(np.uint32), dst.astype(np.uint32)
+    arr = oracle.csr_arrays(n, src, dst)
+    sources = rng.integers(0, n // 8, num_sources).astype(np.uint32)
+    refs = {int(s): oracle.bfs_levels(arr, int(s)) for s in sources[:40]}
+    with B.Graph.from_edges(n, src, dst, 256, 4) as g:
+        for planes in (2, 3):
+            g.set_options(batch_planes=planes, batch_single_max=0)
+            for offset in (0, 1, 6, 8, 16):
+                buf = torch.full((num_sources * n + 64,), 77, dtype=torch.uint8, device="cuda")
+                st = g.run_batch_device(sources, buf.data_ptr() + offset, torch.cuda.current_stream().cuda_stream, stats=True)
+                assert st["status"] == 0 and st["spills"] > 3
+                out = buf.cpu().numpy()
+                assert (out[:offset] == 77).all() and (out[offset + num_sources * n:] == 77).all()
+                rows = out[offset:offset + num_sources * n].reshape(num_sources, n)
+                for i, s in enumerate(sources[:40]):
+                    ref = refs[int(s)]
+                    np.testing.assert_array_equal(rows[i], np.where(ref < 0, 255, ref).astype(np.uint8))
