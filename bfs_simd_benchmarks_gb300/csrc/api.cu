@@ -1488,9 +1488,10 @@ size_t bb_state_bytes(const bfs_graph *g, uint32_t words, uint32_t planes) {
 }
 
 // Of the `want` words of sources that one launch would take (all of the call's),
-// how many do: all where their state fits beside the level planes that the
-// traversal of these words wants, so that it gets no fewer; else one.
-uint32_t bb_words_that_fit(const bfs_graph *g, uint32_t want) {
+// how many do: all where their state fits beside the staging of host outputs and
+// the level planes that the traversal of these words wants, so that it gets no
+// fewer; else one.
+uint32_t bb_words_that_fit(const bfs_graph *g, uint32_t want, size_t stage_bytes) {
 	const auto &b = g->bb;
 	if (want <= 1 || b.state_words >= want) return want;
 	size_t free_b = 0, total_b = 0;
@@ -1498,7 +1499,7 @@ uint32_t bb_words_that_fit(const bfs_graph *g, uint32_t want) {
 	for (const auto &x : b.bufs) free_b += x.bytes;
 	for (const auto &x : b.lbufs) free_b += x.bytes;
 	const uint32_t planes = std::max(batch_planes_wanted(g, want), g->mb.planes_alloc);
-	size_t need = bb_state_bytes(g, want, planes) + ((size_t) 1 << 30);
+	size_t need = bb_state_bytes(g, want, planes) + stage_bytes + ((size_t) 1 << 30);
 	if (g->mb.k_alloc < want) {
 		need += batch_fixed_bytes(g, want) + (size_t) planes * batch_plane_bytes(g, want);
 		free_b += g->mb.bytes;
@@ -1512,35 +1513,39 @@ int bb_prepare(bfs_graph *g, uint32_t num_sources, bool host_deps, bool host_pat
 	int rc;
 	if (!g->bb_chunks_ready && (rc = bb_build_chunks(g))) return rc;
 	auto &b = g->bb;
-	uint32_t words = bb_words_that_fit(g, bb_launch_words(g, num_sources));
-	if (b.ctl && b.state_words < words) release_bb(g);  // its cudaFree waits for earlier calls
-	if (!b.ctl) {
-		for (;;) {
-			const size_t rows = (size_t) words * g->n * kBbMaxSources;
-			const size_t part = (size_t) words * std::max(g->bb_nich, g->bb_noch);
-			if (!((rc = bb_alloc(g, &b.sigma, rows)) || (rc = bb_alloc(g, &b.dsum, rows)) ||
-						(rc = bb_alloc(g, &b.partial, part * kBbMaxSources)) || (rc = bb_alloc(g, &b.chunks_done, part)) ||
-						(rc = bb_alloc(g, &b.ctl, kBbMaxWords)) ||
-						(rc = bb_alloc(g, &b.d_sources, kBbMaxWords * kBbMaxSources))))
-				break;
-			release_bb(g);
-			if (words == 1) return rc;
-			words = 1;
-		}
-		b.state_words = words;
-		if (cudaMallocHost(&b.h_ctl, sizeof(BbControl) * kBbMaxWords) != cudaSuccess ||
-				cudaMallocHost(&b.h_ms, sizeof(MsControl)) != cudaSuccess || cudaEventCreate(&b.e0) != cudaSuccess ||
-				cudaEventCreate(&b.e1) != cudaSuccess || cudaEventCreate(&b.e2) != cudaSuccess ||
-				cudaEventCreate(&b.e3) != cudaSuccess) {
-			cudaGetLastError();
-			release_bb(g);
-			return BFS_ENOMEM;
-		}
-	}
 	const size_t stage = (size_t) g->n * kBbMaxWords * kBbMaxSources;
-	if (host_deps && !b.delta && (rc = bb_alloc(g, &b.delta, stage))) return rc;
-	if (host_paths && !b.paths && (rc = bb_alloc(g, &b.paths, stage))) return rc;
-	return BFS_OK;
+	const auto alloc_all = [&](uint32_t words) {
+		const size_t rows = (size_t) words * g->n * kBbMaxSources;
+		const size_t part = (size_t) words * std::max(g->bb_nich, g->bb_noch);
+		int rc = BFS_OK;
+		if (!b.ctl) {
+			if ((rc = bb_alloc(g, &b.sigma, rows)) || (rc = bb_alloc(g, &b.dsum, rows)) ||
+					(rc = bb_alloc(g, &b.partial, part * kBbMaxSources)) || (rc = bb_alloc(g, &b.chunks_done, part)) ||
+					(rc = bb_alloc(g, &b.d_sources, kBbMaxWords * kBbMaxSources)) || (rc = bb_alloc(g, &b.ctl, kBbMaxWords)))
+				return rc;
+			b.state_words = words;
+			if (cudaMallocHost(&b.h_ctl, sizeof(BbControl) * kBbMaxWords) != cudaSuccess ||
+					cudaMallocHost(&b.h_ms, sizeof(MsControl)) != cudaSuccess || cudaEventCreate(&b.e0) != cudaSuccess ||
+					cudaEventCreate(&b.e1) != cudaSuccess || cudaEventCreate(&b.e2) != cudaSuccess ||
+					cudaEventCreate(&b.e3) != cudaSuccess) {
+				cudaGetLastError();
+				return (int) BFS_ENOMEM;
+			}
+		}
+		if (host_deps && !b.delta && (rc = bb_alloc(g, &b.delta, stage))) return rc;
+		if (host_paths && !b.paths && (rc = bb_alloc(g, &b.paths, stage))) return rc;
+		return rc;
+	};
+	const uint32_t words = bb_words_that_fit(g, bb_launch_words(g, num_sources),
+			4 * stage * ((host_deps || b.delta) + (host_paths || b.paths)));
+	if (b.ctl && b.state_words < words) release_bb(g);  // its cudaFree waits for earlier calls
+	rc = alloc_all(words);
+	if (rc && std::max(words, b.state_words) > 1) {  // what was found free is not there in one piece
+		release_bb(g);
+		rc = alloc_all(1);
+	}
+	if (rc) release_bb(g);
+	return rc;
 }
 
 // Enqueues the batched traversal from `sources` (host, ns <= 256) with its

@@ -317,6 +317,32 @@ def test_words_one_by_one_where_all_do_not_fit(native, oracle, spare_mb, words):
         assert bc_close(total, want, scale).all()
 
 
+@pytest.mark.parametrize("spare_mb", [64, 300, 1700])
+def test_host_outputs_where_all_words_do_not_fit(native, oracle, spare_mb):
+    """The same with dependencies and path counts to host memory, whose staging is 256
+    rows each: it comes before the state of more than one word."""
+    import torch
+    import bfs_simd_benchmarks_gb300 as B
+    n = 1 << 17
+    src, dst = B.gen_rmat(n, 4 * n, seed=34, permute=True)
+    arr = oracle.csr_arrays(n, src, dst)
+    hog = None
+    with B.Graph.from_edges(n, src, dst, 1024, 16, device_build=True) as g:
+        g.set_options(batch_planes=20)
+        sources = B.pick_sources(g.degrees(), 200, seed=4).astype(np.uint32)
+        torch.cuda.empty_cache()
+        need = n * 64 * 8 + 2 * n * 256 * 4 + 20 * n * 5 * 8 + 30 * (n + len(src)) + (1 << 30)
+        free, _ = torch.cuda.mem_get_info()
+        try:
+            hog = torch.empty(max(free - need - (spare_mb << 20), 0), dtype=torch.uint8, device="cuda")
+            dep, sig, st = g.bc_batch(sources)
+        finally:
+            del hog
+            torch.cuda.empty_cache()
+        assert st["status"] == 0 and st["batched_sources"] == sources.size
+        _check_rows(oracle, arr, sources[::25], dep[::25], sig[::25], {**st, "source_reached": st["source_reached"][::25]})
+
+
 @pytest.mark.parametrize("direction", ["out", "in"])
 @pytest.mark.parametrize("degrees", [[63, 64, 65], [127, 128, 129, 1], [0, 1, 0], [64] * 40 + [65] * 40 + [1000, 0]])
 def test_edge_chunk_lists(native, oracle, degrees, direction):
