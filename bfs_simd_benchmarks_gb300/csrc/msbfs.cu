@@ -66,14 +66,14 @@ constexpr uint32_t kMsBlocks = 4;
 // Up to kMsTinyState, a CTA on every other SM (2^14 vertices 155 -> 147 us, uniform
 // 126 -> 115; 2^16 150 -> 163).
 constexpr uint32_t kMsSmallState = 1u << 18, kMsTinyState = 1u << 15;
-// Pull, few words: blocks taken at once where there are more than kMsClaims per warp.
-// The counter gives out one claim in 0.8 ns, and where most destinations have no
-// in-edges that is what a level waits for (uniform, 2^18 vertices of 16 edges, the
-// first ids of 2^23, 100 sources: levels 1,411 -> 844 us; 2^20 of 8 in 2^25 6,950 ->
-// 3,185; rmat, 2^24 vertices of 8 edges, 64 sources 3,847 -> 3,517; from 8 blocks per
-// warp on rmat 2^22 loses, from 32 on 2^23 does not gain).  More words per vertex lose
-// by it at all sizes (2^23, 300 sources: 1,347 -> 2,041).
-constexpr uint32_t kMsClaims = 16, kMsMaxClaim = 8;
+// Pull, few words: blocks taken at once (a power of two), as long as there are
+// kMsClaims items per warp.  The counter gives out one claim in 0.8 ns, and where most
+// destinations have no in-edges that is what a level waits for (uniform, 2^18 vertices
+// of 16 edges, the first ids of 2^23: levels of 40 sources 1,014 -> 574 us, of 141 1,396
+// -> 984; 2^20 of 8 in 2^25, 100 sources 6,950 -> 3,185; rmat, 2^23 vertices of 8 edges,
+// 73 sources 2,340 -> 2,210).  With fewer items rmat 2^21 loses 2% and 2^22 4%.  More
+// words per vertex lose by it at all sizes (2^23, 300 sources: 1,347 -> 2,041).
+constexpr uint32_t kMsClaims = 12, kMsMaxClaim = 8;
 constexpr uint32_t kMsRun = 8;          // pull, few words: chunks taken at once
 constexpr uint32_t kMsMaxWords = 64;    // 4,096 sources
 constexpr uint32_t kGroupMaxWords = 32; // pull: up to this many words, in-neighbour rows in lane groups
@@ -891,9 +891,11 @@ __device__ __forceinline__ void ms_pull_blocks(const MsArgs &a, const MsPull &p,
 	while (item < nruns + a.nclaims) {
 		const uint32_t next = lane == 0 ? atomicAdd(counter, 1u) : 0u;
 		if constexpr (kRowWords) {
-			uint32_t vb = (item - nruns) * a.claim * 32;
-			for (uint32_t c = 0; c < a.claim && vb < a.n; ++c, vb += 32)
+			uint32_t vb = (item - nruns) * a.claim;  // (a.claim destinations, a power of two)
+			do {
 				ms_pull_rows<KK>(a, p, vb, min(32u, a.n - vb), f, acc, actdeg, gathered, wbuf, wn);
+				vb += 32;
+			} while ((vb & (a.claim - 1)) && vb < a.n);
 		} else {
 			const uint32_t vb = (item - nruns) << a.blk_shift;
 			ms_pull_words<KK>(a, p, vb, min(1u << a.blk_shift, a.n - vb), fm, acc[0], acc[1], actdeg, gathered, wbuf, wn);
@@ -1228,6 +1230,24 @@ __device__ __noinline__ void ms_emit(const MsArgs &a, uint8_t *levels, uint32_t 
 	}
 }
 
+// An early output pass: the planes base .. lvl go out, lvl's becomes plane 0.  Two
+// grid barriers after `epoch`; false where one gave up.  (A function: inside the
+// traversal kernel, its loops and calls cost the pulls registers: levels of 200 sources,
+// rmat, 2^20 vertices, 1,015 -> 930 us, of 141 885 -> 838; of 73, on a small unpermuted
+// graph, 345 -> 352.)
+__device__ __noinline__ bool ms_spill(const MsArgs &a, uint8_t *levels, uint32_t ns, uint32_t base, uint32_t lvl, uint8_t *lev,
+		unsigned epoch) {
+	const uint32_t stride = gridDim.x * blockDim.x, t0 = blockIdx.x * blockDim.x + threadIdx.x;
+	const size_t nK = (size_t) a.n * a.K;
+	ms_emit<false, kEmitV, kEmitW, true>(a, levels, ns, base, base == 0 ? 0 : 1, lvl - base, base != 0, lev);
+	if (!grid_sync(a.ctl->bar, epoch, &a.ctl->err, a.wait_limit_ns, a.hold_barrier)) return false;
+	const uint64_t *src = a.hist + (size_t) (lvl - base) * nK;
+	for (size_t i = t0; i < nK; i += stride) a.hist[i] = ld_cg64(src + i);
+	const uint64_t *msrc = a.pmask + (size_t) (lvl - base) * a.n;
+	for (uint32_t i = t0; i < a.n; i += stride) a.pmask[i] = ld_cg64(msrc + i);
+	return grid_sync(a.ctl->bar, epoch, &a.ctl->err, a.wait_limit_ns, a.hold_barrier);
+}
+
 // KK: words per vertex up to kMsRowWords; for more, 8, 16, 32 (kGroupMaxWords) or 64
 // (kMsMaxWords) for up to as many: one kernel each, so that only one form of the pull shares
 // the registers and its arguments are read where they lie (as calls of one
@@ -1301,17 +1321,10 @@ __global__ void __launch_bounds__(kMsThreads, 2) k_ms_bfs(const __grid_constant_
 				break;
 			}
 			// planes full: write them out, keep the frontier's plane as plane 0
-			if (a.n % 16 == 0 && (uintptr_t) levels % 16 == 0)
-				ms_emit<false, kEmitV, kEmitW, false>(a, levels, ns, base, base == 0 ? 0 : 1, lvl - base, base != 0, lev);
-			else ms_emit<false, kEmitV, kEmitW, true>(a, levels, ns, base, base == 0 ? 0 : 1, lvl - base, base != 0, lev);
-			if (!(ok = grid_sync(ctl->bar, epoch, &ctl->err, a.wait_limit_ns, a.hold_barrier))) break;
-			const uint64_t *src = a.hist + (size_t) (lvl - base) * nK;
-			for (size_t i = t0; i < nK; i += stride) a.hist[i] = ld_cg64(src + i);
-			const uint64_t *msrc = a.pmask + (size_t) (lvl - base) * a.n;
-			for (uint32_t i = t0; i < a.n; i += stride) a.pmask[i] = ld_cg64(msrc + i);
+			if (!(ok = ms_spill(a, levels, ns, base, lvl, lev, epoch))) break;
+			epoch += 2;
 			base = lvl;
 			if (leader) ctl->stats.spills++;
-			if (!(ok = grid_sync(ctl->bar, epoch, &ctl->err, a.wait_limit_ns, a.hold_barrier))) break;
 		}
 		// the counters of the level after next are free again
 		if (leader) {
@@ -1482,8 +1495,10 @@ int ms_launch(const MsArgs &a, const uint32_t *d_sources, uint32_t ns, uint8_t *
 	}
 	aa.nruns = (a.nchunks + aa.run - 1) / aa.run;
 	const uint32_t nblk = (uint32_t) (((uint64_t) a.n + (1u << aa.blk_shift) - 1) >> aa.blk_shift);
-	aa.claim = a.K <= kMsRowWords ? std::min(std::max(nblk / (nwarps * kMsClaims), 1u), kMsMaxClaim) : 1u;
-	aa.nclaims = (nblk + aa.claim - 1) / aa.claim;
+	uint32_t blocks = 1;
+	while (a.K <= kMsRowWords && blocks < kMsMaxClaim && nblk / (2 * blocks) >= nwarps * kMsClaims) blocks *= 2;
+	aa.claim = blocks << aa.blk_shift;
+	aa.nclaims = (nblk + blocks - 1) / blocks;
 	const uint32_t *src = d_sources;
 	uint32_t nsrc = ns;
 	uint8_t *out = levels;

@@ -68,7 +68,7 @@ struct MsArgs {
 	uint32_t *push_u, *push_beg;         // [push_cap] push: vertex and first edge of each 1024-edge chunk
 	uint32_t push_cap;
 	// set by ms_launch: chunks per item of a pull and the items they make; blocks of
-	// 2^blk_shift destinations, how many an item has, and the items they make
+	// 2^blk_shift destinations, destinations of an item, and the items they make
 	uint32_t run, nruns, blk_shift, claim, nclaims;
 	uint64_t *vis;        // [n][K] sources that reached v
 	uint64_t *hist;       // [planes][n][K] sources that reached v first at level base + plane
