@@ -1239,7 +1239,12 @@ __device__ __noinline__ bool ms_spill(const MsArgs &a, uint8_t *levels, uint32_t
 		unsigned epoch) {
 	const uint32_t stride = gridDim.x * blockDim.x, t0 = blockIdx.x * blockDim.x + threadIdx.x;
 	const size_t nK = (size_t) a.n * a.K;
-	ms_emit<false, kEmitV, kEmitW, true>(a, levels, ns, base, base == 0 ? 0 : 1, lvl - base, base != 0, lev);
+	const uint32_t first = base == 0 ? 0 : 1;
+	// rows that all start on 16 bytes need no shifting: the level with the pass, 60 sources,
+	// uniform, 2^21 vertices, 650 -> 591 us
+	if (a.n % 16 == 0 && (uintptr_t) levels % 16 == 0)
+		ms_emit<false, kEmitV, kEmitW, false>(a, levels, ns, base, first, lvl - base, base != 0, lev);
+	else ms_emit<false, kEmitV, kEmitW, true>(a, levels, ns, base, first, lvl - base, base != 0, lev);
 	if (!grid_sync(a.ctl->bar, epoch, &a.ctl->err, a.wait_limit_ns, a.hold_barrier)) return false;
 	const uint64_t *src = a.hist + (size_t) (lvl - base) * nK;
 	for (size_t i = t0; i < nK; i += stride) a.hist[i] = ld_cg64(src + i);
