@@ -343,3 +343,18 @@ def test_a_closed_graph_has_no_vertex_count(native):
     for ask in (lambda: g.num_vertices, g.degrees, g.info):
         with pytest.raises(B.BfsError):
             ask()
+
+
+@pytest.mark.parametrize("steps", [0, 1, 7, 256])
+def test_step_times_of_a_run(native, steps):
+    """Each list is its own field's, rounded, whether or not a step's three times are the same."""
+    from bfs_simd_benchmarks_gb300 import _native as N
+
+    st = N.Stats(num_steps=steps)
+    rng = np.random.default_rng(steps)
+    for i, ms in enumerate(rng.random(steps) / 100):
+        low, high = [(ms, ms), (0.0, 0.0), (ms / 3, ms / 2)][i % 3]
+        st.step_ms[i], st.step_work_min_ms[i], st.step_work_max_ms[i] = ms, low, high
+    d = st.as_dict()
+    for name in ("step_ms", "step_work_min_ms", "step_work_max_ms"):
+        assert d[name] == [round(x, 5) for x in getattr(st, name)[:steps]]
